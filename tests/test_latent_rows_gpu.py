@@ -1,0 +1,145 @@
+"""Attention of long portions over a cached latent through keys and values formed for the step: the work list (CPU), the
+kernels against plain float64 attention, and the choice between the two ways inside a layer."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from xinfer_b200 import kernels
+
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("counts,starts,window,heads,ctas", [
+    ([1], [0], None, 4, 148), ([5], [0], None, 1, 148), ([2048], [0], None, 32, 148), ([300, 1, 129, 4, 128], [7, 90, 0, 0, 64], None, 3, 20),
+    ([700], [1000], 100, 2, 7), ([64, 65], [63, 64], 16, 5, 148),
+])
+def test_the_work_list_holds_every_query_of_every_head_once(counts, starts, window, heads, ctas, monkeypatch):
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda t: t)
+    host, n, rows, at = kernels.latent_prefill_work(counts, starts, 4, window, heads, max_ctas=ctas)
+    long = [b for b, c in enumerate(counts) if c > 4]
+    assert (n == 0) == (not long) and n <= ctas
+    if not long:
+        assert rows == 0
+        return
+    w = host.numpy()
+    items = w[n + 1:at].reshape(-1, 4)
+    runs = w[at:].reshape(-1, 2)
+    assert w[0] == 0 and w[n] == len(items) and (np.diff(w[:n + 1]) >= 1).all() and len(runs) * 64 == rows
+    row_of = {(int(b), int(j)): i * 64 for i, (b, j) in enumerate(runs)}
+    seen = set()
+    for b, first, hn, row0 in items:
+        h, nt = int(hn) & 0xffff, int(hn) >> 16
+        assert nt in (1, 2) and counts[b] - first > (nt - 1) * 128
+        for i in range(nt):
+            assert (b, first + 128 * i, h) not in seen
+            seen.add((b, first + 128 * i, h))
+            p = starts[b] + first + 128 * i
+            last = p + min(128, counts[b] - first - 128 * i) - 1
+            lo = max(0, p - window + 1) if window else 0
+            for kt in range(lo // 64, last // 64 + 1):          # every key tile the kernel reads is a run of this portion
+                assert row_of[(int(b), kt * 64)] == row0 + kt * 64
+    assert seen == {(b, q, h) for b in long for q in range(0, counts[b], 128) for h in range(heads)}
+
+
+def _plain(q, rows, w_kv, heads, d, rd, dv, rank, start, window, scale, sink):
+    """float64: q [n, H, d + rd], rows [start + n, width]."""
+    n, end = q.shape[0], rows.shape[0]
+    k = (rows[:, :rank] @ w_kv[:heads * d].T).view(end, heads, d)
+    v = (rows[:, :rank] @ w_kv[heads * d:].T).view(end, heads, dv)
+    k = torch.cat([k, rows[:, None, rank:rank + rd].expand(end, heads, rd)], -1)
+    s = torch.einsum("ihd,jhd->hij", q, k) * scale
+    far = torch.arange(start, end)[:, None] - torch.arange(end)[None]
+    s = s.masked_fill((far < 0) | (far >= window if window else far < 0), -math.inf)
+    if sink is not None:
+        s = torch.cat([s, sink[:, None, None].expand(heads, n, 1)], -1)
+    return torch.einsum("hij,jhd->ihd", torch.softmax(s, -1)[..., :end], v)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,rd,dv,rank,tail", [(128, 64, 128, 512, 0), (128, 32, 128, 256, 0), (128, 0, 128, 64, 32), (64, 64, 64, 128, 0),
+                                               (64, 0, 64, 72, 0), (64, 8, 128, 64, 0), (128, 0, 64, 64, 0)])
+@pytest.mark.parametrize("counts,starts,window,heads,sink", [
+    ([5], [0], None, 1, False), ([127, 1, 129], [0, 40, 0], None, 3, True), ([128, 256, 257], [64, 0, 63], None, 2, False),
+    ([300, 6], [777, 130], 100, 2, True), ([64, 700], [3, 0], 64, 1, False), ([130], [1], 1, 2, False),
+])
+def test_rows_attention_agrees_with_plain_attention(d, rd, dv, rank, tail, counts, starts, window, heads, sink):
+    g = torch.Generator().manual_seed(d + 3 * rd + sum(counts))
+    bf = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    i32 = lambda a: torch.tensor(np.asarray(a), dtype=torch.int32, device=DEV)
+    width, ps, B, T = rank + rd + tail, 16, len(counts), sum(counts)
+    seqs = [bf(s + c, width) for s, c in zip(starts, counts)]
+    w_kv = (bf(heads * (d + dv), rank).float() * rank ** -0.5).bfloat16()
+    q_row = heads * (d + rd) + 8                                # queries in front of something else
+    q = bf(T, q_row)
+    per = max(-(-r.shape[0] // ps) for r in seqs)
+    table = torch.full((B, per), -1, dtype=torch.int32)
+    pages = torch.full((B * per + 1, ps, width), float("nan")).bfloat16()
+    order = torch.randperm(B * per + 1, generator=g).tolist()
+    for b, r in enumerate(seqs):
+        # pages that lie wholly in front of the window have been given back
+        gone = max(0, starts[b] - window + 1) // ps if window else 0
+        for p in range(gone, -(-r.shape[0] // ps)):
+            table[b, p] = order[b * per + p]
+            part = r[p * ps:(p + 1) * ps]
+            pages[table[b, p], :len(part)] = part
+    q_start, start_pos, err = i32(np.concatenate([[0], np.cumsum(counts)])), i32(starts), i32([0])
+    sinks = torch.randn(heads, generator=g) if sink else None
+    host, ctas, rows_n, at = kernels.latent_prefill_work(counts, starts, 4, window, heads)
+    work = host.to(DEV)
+    rows = torch.full((rows_n, width), float("nan"), dtype=torch.bfloat16, device=DEV)
+    kernels.latent_gather(rows, pages.to(DEV), work, at, q_start, start_pos, table.to(DEV), per, window, err)
+    kv = rows[:, :rank] @ w_kv.to(DEV).t()
+    out = torch.full((T, heads * dv), float("nan"), dtype=torch.bfloat16, device=DEV)
+    scale = (d + rd) ** -0.5
+    kernels.attn_rows_tc(out, q.to(DEV), q_row, kv, rows, work, ctas, q_start, start_pos, heads, d, rd, dv, rank, window, scale,
+                         sinks.to(DEV) if sink else None, err)
+    torch.cuda.synchronize()
+    assert int(err) == 0
+    at = 0
+    for b, (c, s) in enumerate(zip(counts, starts)):
+        got = out[at:at + c].double().cpu().view(c, heads, dv)
+        if c <= 4:
+            assert torch.isnan(got).all()                       # left to the kernel of the small portions
+        else:
+            ref = _plain(q[at:at + c, :heads * (d + rd)].double().view(c, heads, d + rd), seqs[b].double(), w_kv.double(), heads, d, rd,
+                         dv, rank, s, window, scale, sinks.double() if sink else None)
+            # keys, values, probabilities and the result are rounded to 8 bits: scores of size 1 move by 2^-9 each key
+            # channel's share, the result by 2^-9 of the largest value a few times over
+            assert (got - ref).abs().max() <= 4 * 2 ** -8 * max(1.0, ref.abs().max()), (b, (got - ref).abs().max())
+        at += c
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("design", ["dufitar", "napuzen"])
+def test_a_model_gives_the_same_logits_both_ways_and_for_mixed_steps(design, monkeypatch):
+    from xinfer_b200.engine.runner import ModelRunner, StepInput
+    from xinfer_b200.parts import latent_attention as part
+    d, H, rot = 64, 2, dict(dims=32, base=1000.0)
+    dense = dict(kind="dense", ff=128, limit=7.0)
+    if design == "dufitar":
+        m = dict(heads=H, dim=d, rot_dim=32, vdim=d, kv_rank=64, scale=0.1, mask=dict(size=150), rot=rot)
+        layers = [dict(type="latent_attention", mixer=m, mlp=dense), dict(type="latent_attention", mixer=dict(m, kv_from=0), mlp=dense)]
+        cfg = dict(architecture="Dufitar", vocab=300, width=128, norm=dict(eps=1e-6), residual_mult=0.5, embedding=dict(scale=2.0), layers=layers)
+    else:
+        one = dict(type="latent_attention", mlp=dense, mixer=dict(heads=H, dim=d, rot_dim=32, vdim=d, q_rank=96, kv_rank=64, scale=0.1, rot=rot))
+        two = dict(type="latent_attention_2", mlp=dense, mixer=dict(heads=H, dim=d, vdim=d, kv_rank=64, scale=0.1, mask=dict(size=100)))
+        cfg = dict(architecture="Napuzen", vocab=300, width=128, norm=dict(eps=1e-6), canon=dict(taps=4), logit_scale=0.8, layers=[one, two])
+    ids = np.random.default_rng(1).integers(0, 300, size=400)
+
+    def logits(rates):
+        monkeypatch.setattr(part, "ROWS_RATES", rates)
+        r = ModelRunner.random(cfg, 3, block_size=16, num_blocks=128, max_num_seqs=4, max_model_len=512)
+        before = kernels.launch_counts().get("attn_rows_tc", 0)
+        a, b = r.open_request(), r.open_request()
+        out = [r.step([StepInput(a, ids[:200], [7, 199])]).clone()]
+        out.append(r.step([StepInput(a, ids[200:201], [0]), StepInput(b, ids[:333], [332])]).clone())      # one token beside a prompt
+        out.append(r.step([StepInput(b, ids[333:400], [66]), StepInput(a, ids[201:204], [2])]).clone())     # portions behind cached tokens
+        r.check_errors()
+        return torch.cat(out).double(), kernels.launch_counts().get("attn_rows_tc", 0) - before
+    want, none = logits((1e30, 1.0, 1.0, 1e30, 1e30))         # attention over the rows themselves
+    got, some = logits((1e-9, 1e30, 1e30, 0.0, 0.0))         # on formed keys and values wherever they may be
+    assert none == 0 and some == 6
+    # two bfloat16 computations of the same numbers
+    assert (got - want).norm() <= 0.02 * want.norm()

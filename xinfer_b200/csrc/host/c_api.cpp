@@ -243,6 +243,80 @@ XB_API long long xb_attn_prefill_work(int B, const int* counts, const int* start
     return (long long)ctas + 1 + INTS * n_items;
 }
 
+// ---- work lists of the attention over keys and values formed for the step --------------------------
+// The step's portions of more than dec_max tokens: their visible rows lie one portion after the other, from the 64-key
+// tile of the first query's first key on, in runs of 64 rows.  Items are 256 (or 128) queries of one head; they go,
+// longest first, onto the CTA with the least work so far, and the cut into items that ends earlier is taken.
+// out: [ctas + 1] offsets (in items), 4 int32 per item (portion, first query of it, head | tiles of 128 queries << 16,
+// row of the position 0), then (portion, first position) of every run of 64 rows.  Returns the number of int32 written
+// (-1: capacity too small), the number of CTAs and of rows.
+XB_API long long xb_latent_prefill_work(int B, const int* counts, const int* starts, int dec_max, int window, int heads,
+                                        int max_ctas, int32_t* out, long long capacity, int* ctas_out, int* rows_out) {
+    // costs in sixths of a key tile of two query tiles, as for the kernel over pages
+    constexpr int QT = 128, KT = 64, TILE_OF_TWO = 6, TILE_OF_ONE = 4, START_UP = 18, INTS = 4;
+    struct Piece { int cost, b, first, nt, row0; };
+    std::vector<int32_t> runs;
+    std::vector<Piece> cuts[2];       // [0]: two query tiles per item where a portion has them, [1]: one
+    for (int b = 0; b < B; ++b) {
+        const int n = counts[b];
+        if (n <= dec_max) continue;
+        const int base = (window > 0 ? std::max(0, starts[b] - window + 1) : 0) / KT * KT, end = starts[b] + n;
+        const int row0 = (int)runs.size() / 2 * KT - base;
+        for (int j = base; j < end; j += KT) {
+            runs.push_back(b);
+            runs.push_back(j);
+        }
+        for (int c = 0; c < 2; ++c) {
+            for (int first = 0, nt; first < n; first += nt * QT) {
+                nt = c == 0 && n - first > QT ? 2 : 1;
+                const int p0 = starts[b] + first, last = p0 + std::min(nt * QT, n - first) - 1;
+                const int lo = (window > 0 ? std::max(0, p0 - window + 1) : 0) / KT;
+                cuts[c].push_back({(last / KT - lo + 1) * (nt == 2 ? TILE_OF_TWO : TILE_OF_ONE) + START_UP, b, first, nt, row0});
+            }
+        }
+    }
+    *ctas_out = 0;
+    *rows_out = (int)runs.size() / 2 * KT;
+    if (runs.empty() || heads <= 0 || heads > 65535) return 0;
+    std::vector<std::vector<int32_t>> lists[2];
+    long long longest[2] = {0, 0};
+    for (int c = 0; c < 2; ++c) {
+        std::stable_sort(cuts[c].begin(), cuts[c].end(), [](const Piece& x, const Piece& y) { return x.cost > y.cost; });
+        const int ctas = (int)std::min<long long>(max_ctas, (long long)cuts[c].size() * heads);
+        std::vector<std::pair<long long, int>> heap;
+        for (int i = 0; i < ctas; ++i) heap.emplace_back(0, i);
+        auto later = [](const std::pair<long long, int>& x, const std::pair<long long, int>& y) { return x > y; };
+        std::make_heap(heap.begin(), heap.end(), later);
+        lists[c].assign(ctas, {});
+        for (const Piece& p : cuts[c]) {
+            for (int h = 0; h < heads; ++h) {
+                std::pop_heap(heap.begin(), heap.end(), later);
+                auto& top = heap.back();
+                lists[c][top.second].insert(lists[c][top.second].end(), {p.b, p.first, h | p.nt << 16, p.row0});
+                top.first += p.cost;
+                longest[c] = std::max(longest[c], top.first);
+                std::push_heap(heap.begin(), heap.end(), later);
+            }
+        }
+    }
+    const int take = longest[1] < longest[0] ? 1 : 0;
+    const long long n_items = (long long)cuts[take].size() * heads;
+    const int ctas = (int)lists[take].size();
+    *ctas_out = ctas;
+    const long long used = ctas + 1 + INTS * n_items + (long long)runs.size();
+    if (used > capacity) return -1;
+    int32_t* items = out + ctas + 1;
+    int at = 0;
+    for (int c = 0; c < ctas; ++c) {
+        out[c] = at;
+        std::copy(lists[take][c].begin(), lists[take][c].end(), items + INTS * (long long)at);
+        at += (int)lists[take][c].size() / INTS;
+    }
+    out[ctas] = at;
+    std::copy(runs.begin(), runs.end(), items + INTS * n_items);
+    return used;
+}
+
 // ---- scheduler ---------------------------------------------------------------------------------
 struct SchedHandle {
     Scheduler sched;

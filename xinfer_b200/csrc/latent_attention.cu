@@ -18,11 +18,13 @@
 // rows another layer wrote).  q_lat[t, h] (strides given) is the head's query already carried into the latent
 // space; absent: the latent part of q_abs has been written already (by the product that formed it) and stays.  The first `rot` channels of a rotated part turn by position * inv_freq[pair] (pairs 2i, 2i+1), cos
 // and sin times rot_mag; the others pass.  `tail` further channels of a query row, behind the rotated part, are zero
-// (cached rows that carry a key part this layer does not read).  nh = 0: no queries are put together.  A second row of
+// (cached rows that carry a key part this layer does not read).  The rotated part of token t's head h goes to
+// q_abs + t * q_ts + h * q_hs + q_rot; q_abs may be the projection itself (the part is then rotated where it lies: `pairs`
+// only, a thread reads and writes the same pair).  nh = 0: no queries are put together.  A second row of
 // blocks (blockIdx.y = 1) norms the queries' own latent instead: cq[t] = the n_cq columns at cq_off, RMS-normed with
 // cq_w.
 template <typename T>
-__global__ void latent_prepare_kernel(T* __restrict__ q_abs, T* __restrict__ cache, const T* __restrict__ proj,
+__global__ void latent_prepare_kernel(T* q_abs, long long q_ts, long long q_hs, int q_rot, T* __restrict__ cache, const T* proj,
                                       long long row_len, int q_off, int kv_off, const T* __restrict__ q_lat,
                                       long long ql_ts, long long ql_hs, const float* __restrict__ norm_w,
                                       const float* __restrict__ inv_freq, const int* __restrict__ positions,
@@ -77,7 +79,7 @@ __global__ void latent_prepare_kernel(T* __restrict__ q_abs, T* __restrict__ cac
                 reinterpret_cast<const __nv_bfloat16*>(row) + q_off + (size_t)h * (d + rd) + d + 2 * pr);
             float2 v = __bfloat1622float2(in);
             if (2 * pr < rot) v = make_float2(fmaf(v.x, cs[pr], -v.y * sn[pr]), fmaf(v.y, cs[pr], v.x * sn[pr]));
-            *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(q_abs) + ((size_t)t * nh + h) * dk + rank + 2 * pr) =
+            *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(q_abs) + (size_t)t * q_ts + (size_t)h * q_hs + q_rot + 2 * pr) =
                 __floats2bfloat162_rn(v.x, v.y);
         }
     } else {
@@ -89,7 +91,7 @@ __global__ void latent_prepare_kernel(T* __restrict__ q_abs, T* __restrict__ cac
                 const float o = to_f32<T>(qr[e ^ 1]);
                 v = (e & 1) ? fmaf(v, cs[e >> 1], o * sn[e >> 1]) : fmaf(v, cs[e >> 1], -o * sn[e >> 1]);
             }
-            q_abs[((size_t)t * nh + h) * dk + rank + e] = from_f32<T>(v);
+            q_abs[(size_t)t * q_ts + (size_t)h * q_hs + q_rot + e] = from_f32<T>(v);
         }
     }
     if (kv_off < 0 || b < 0) return;
@@ -126,10 +128,15 @@ XB_EXPORT int xb_latent_prepare(int dtype, void* q_abs, void* cache, const void*
                                 const float* inv_freq, const int* positions, const int* req_of_token,
                                 const int* block_table, int table_stride, int tokens, int nh, int d, int rd, int rank,
                                 int rot, int page_size, int num_pages, float eps, float rot_mag, int tail, void* cq,
-                                int cq_off, int n_cq, const float* cq_w, int* err, cudaStream_t stream) {
+                                int cq_off, int n_cq, const float* cq_w, int in_place, int* err, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     // a layer that writes rows writes whole ones
     if (rot % 2 || rot > rd || (tail > 0 && kv_off >= 0)) return (int)cudaErrorInvalidValue;
+    // `in_place`: the rotated query parts stay in the projection's rows
+    if (in_place && (q_abs != nullptr || q_lat != nullptr || tail)) return (int)cudaErrorInvalidValue;
+    const long long q_ts = in_place ? row_len : (long long)nh * (rank + rd + tail), q_hs = in_place ? d + rd : rank + rd + tail;
+    const int q_rot = in_place ? d : rank;
+    if (in_place) q_abs = (char*)proj + (size_t)q_off * (dtype == XB_BF16 ? 2 : 4);
     const size_t smem = (size_t)rot * sizeof(float);
     if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
     const int work = q_lat != nullptr ? nh * (rank + rd) : (nh * rd > rank + rd ? nh * rd : rank + rd);
@@ -137,11 +144,12 @@ XB_EXPORT int xb_latent_prepare(int dtype, void* q_abs, void* cache, const void*
     // sum), so many resident blocks hide more than many threads per block
     const int threads = work >= 16384 ? 256 : 128;
 #define XB_GO(T)                                                                                                        \
-    latent_prepare_kernel<T><<<dim3(tokens, cq != nullptr ? 2 : 1), threads, smem, stream>>>((T*)q_abs, (T*)cache, (const T*)proj, row_len, q_off,  \
+    latent_prepare_kernel<T><<<dim3(tokens, cq != nullptr ? 2 : 1), threads, smem, stream>>>((T*)q_abs, q_ts, q_hs, q_rot, (T*)cache, (const T*)proj, row_len, q_off,  \
         kv_off, (const T*)q_lat, ql_ts, ql_hs, norm_w, inv_freq, positions, req_of_token, block_table, table_stride,   \
         nh, d, rd, rank, rot, page_size, num_pages, eps, rot_mag, pairs, tail, (T*)cq, cq_off, n_cq, cq_w, err)
     const int pairs = (dtype == XB_BF16 && !((row_len | q_off | d | rd | rank | tail) & 1) &&
                        !(((uintptr_t)proj | (uintptr_t)q_abs) & 3)) ? 1 : 0;
+    if (in_place && nh > 0 && !pairs) return (int)cudaErrorInvalidValue;
     if (dtype == XB_F32) XB_GO(float);
     else XB_GO(__nv_bfloat16);
 #undef XB_GO

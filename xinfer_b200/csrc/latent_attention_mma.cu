@@ -41,7 +41,7 @@ struct LatentMmaArgs {
     const float* sink;
     float* part_o;
     float* part_ml;
-    int num_entries, table_stride, nh, dk, rank, page_size, num_pages, window, parts, rg;
+    int num_entries, table_stride, nh, dk, rank, page_size, num_pages, window, parts, rg, most;
     float scale;
     int* err;
 };
@@ -69,7 +69,8 @@ __global__ void __launch_bounds__(64 * CW) attn_latent_mma_kernel(__nv_bfloat16*
     if (tid == 0) {
         int tile = blockIdx.x, found = -1;
         for (int b = 0; b < a.num_entries; ++b) {
-            const int rows = (a.q_start[b + 1] - a.q_start[b]) * H;
+            const int n = a.q_start[b + 1] - a.q_start[b];
+            const int rows = a.most > 0 && n > a.most ? 0 : n * H;    // a longer portion is another kernel's
             const int nt = (rows + R - 1) / R;
             if (tile < nt) { found = b; break; }
             tile -= nt;
@@ -391,20 +392,21 @@ XB_EXPORT int xb_attn_latent_mma_takes(int dk, int rank) {
 }
 
 // q [tokens, heads, dk], cache [pages, page_size, dk], out [tokens, heads, rank], all bfloat16.  `rg`: 16-row
-// groups per block (1 or 2).  `parts` > 1 needs part_o (tokens * heads * parts * rank floats) and part_ml
+// groups per block (1 or 2).  `most` > 0: portions of more tokens are left out, `tokens` counts those of the others.
+// `parts` > 1 (with every portion taken) needs part_o (tokens * heads * parts * rank floats) and part_ml
 // (tokens * heads * parts * 2 floats).
 XB_EXPORT int xb_attn_latent_mma(void* out, const void* q, const void* cache, const int* q_start, const int* start_pos,
                                  int num_entries, const int* block_table, int table_stride, int tokens, int nh, int dk,
                                  int rank, int page_size, int num_pages, int window, float scale, const float* sink, int rg,
-                                 int parts, float* part_o, float* part_ml, int* err, cudaStream_t stream) {
+                                 int most, int parts, float* part_o, float* part_ml, int* err, cudaStream_t stream) {
     if (tokens <= 0 || num_entries <= 0) return 0;
     if (!xb_attn_latent_mma_takes(dk, rank) || (rg != 1 && rg != 2) || parts < 1 || parts > 65535) return (int)cudaErrorInvalidValue;
-    if (parts > 1 && (part_o == nullptr || part_ml == nullptr)) return (int)cudaErrorInvalidValue;
+    if (parts > 1 && (part_o == nullptr || part_ml == nullptr || most > 0)) return (int)cudaErrorInvalidValue;
     LatentMmaArgs a;
     a.q_start = q_start; a.start_pos = start_pos; a.block_table = block_table; a.sink = sink;
     a.part_o = part_o; a.part_ml = part_ml;
     a.num_entries = num_entries; a.table_stride = table_stride; a.nh = nh; a.dk = dk; a.rank = rank;
-    a.page_size = page_size; a.num_pages = num_pages; a.window = window; a.parts = parts; a.rg = rg;
+    a.page_size = page_size; a.num_pages = num_pages; a.window = window; a.parts = parts; a.rg = rg; a.most = most;
     a.scale = scale; a.err = err;
     const int R = 16 * rg;
     // every entry's rows are cut into tiles of their own: at most one ragged tile per entry

@@ -1027,7 +1027,7 @@ def expert_router(choice, weight, h, w_router, correction, req_of_token, top: in
 
 # ---- attention over a cached latent ---------------------------------------------------------------------------------
 def latent_prepare(q_abs, cache, proj, q_off, kv_off, q_lat, norm_w, inv_freq, positions, req_of_token, block_table,
-                   table_stride, nh, d, rd, rank, rot, eps, rot_magnitude, err, *, tail: int = 0, query_latent=None):
+                   table_stride, nh, d, rd, rank, rot, eps, rot_magnitude, err, *, tail: int = 0, query_latent=None, in_place: bool = False):
     """Per token of the packed projection ``proj``: the query of every head as ``q_abs[t, h] = [q_lat[h, t] | rotated
     rd channels]`` (``q_lat`` ``[heads, T, rank]``: the plain query part carried into the latent space; None: the
     product that formed it has written it into ``q_abs`` already; ``nh`` 0: no queries), and, with
@@ -1035,17 +1035,21 @@ def latent_prepare(q_abs, cache, proj, q_off, kv_off, q_lat, norm_w, inv_freq, p
     (``cache`` ``[page, slot, rank + rd]``).  Rotation: pairs (2i, 2i + 1) of the first ``rot`` channels by
     ``position * inv_freq[i]``, cos and sin times ``rot_magnitude``.  ``tail``: further channels of the cached rows that
     this layer does not read; a query row ends in as many zeros.  ``query_latent`` = (out ``[T, n]``, column, weight):
-    out receives the n columns of ``proj`` from that column on, RMS-normed times the weight."""
+    out receives the n columns of ``proj`` from that column on, RMS-normed times the weight.  ``in_place``: the queries
+    stay in ``proj``, their rd channels are rotated where they lie (bfloat16; no ``q_abs``)."""
     T = proj.shape[0]
     width = rank + rd + tail
     _need(proj, "proj", None, (T, None))
-    if nh:
+    if in_place and (q_abs is not None or q_lat is not None or proj.dtype != torch.bfloat16 or q_off + nh * (d + rd) > proj.shape[1]):
+        raise KernelError("queries that stay in the projection are bfloat16 and have no other place")
+    if nh and not in_place:
         _need(q_abs, "q_abs", proj.dtype, (T, nh, width))
         if q_off + nh * (d + rd) > proj.shape[1]:
             raise KernelError("the queries lie outside the projection's rows")
     if q_lat is not None:
         _need(q_lat, "q_lat", proj.dtype, (nh, T, rank))
-    _need(cache, "cache", proj.dtype, (None, None, width))
+    if kv_off >= 0 or not in_place:
+        _need(cache, "cache", proj.dtype, (None, None, width))
     if rot:
         _need(inv_freq, "inv_freq", torch.float32, (rot // 2,))
     if kv_off >= 0:
@@ -1065,7 +1069,7 @@ def latent_prepare(q_abs, cache, proj, q_off, kv_off, q_lat, norm_w, inv_freq, p
         _ptr(q_lat), rank, T * rank, _ptr(norm_w), _ptr(inv_freq), positions.data_ptr(), req_of_token.data_ptr(),
         block_table.data_ptr(), int(table_stride), T, nh, d, rd, rank, int(rot), cache.shape[1], cache.shape[0], float(eps),
         float(rot_magnitude), int(tail), _ptr(cq), int(cq_off), cq.shape[1] if cq is not None else 0, _ptr(cq_w),
-        err.data_ptr(), _stream()), "latent_prepare")
+        int(bool(in_place)), err.data_ptr(), _stream()), "latent_prepare")
 
 
 def attn_latent_mma_takes(dk: int, rank: int) -> bool:
@@ -1074,13 +1078,14 @@ def attn_latent_mma_takes(dk: int, rank: int) -> bool:
 
 
 def attn_latent_mma(out, q, cache, q_start, start_pos, num_entries, block_table, table_stride, window, scale, sink, err, *,
-                    row_groups: int = 2, parts: int = 1, part_o=None, part_ml=None):
+                    row_groups: int = 2, parts: int = 1, part_o=None, part_ml=None, most: int = 0, tokens: Optional[int] = None):
     """Attention of every (token, head) row of ``q`` ``[T, heads, dk]`` over its request's cached rows
     (``cache`` ``[page, slot, dk]``; the first ``rank = out.shape[-1]`` channels of a row are its value), bfloat16 on
     tensor cores with float32 scores, softmax and sums.  ``sink`` (float32 per head or None): one more softmax entry
     of that score without a value.  ``row_groups``: 16-row groups per block (1 or 2).  ``parts`` > 1: every row's key
     tiles are dealt out to that many blocks and merged through ``part_o`` / ``part_ml`` (float32, T*heads*parts*rank
-    and T*heads*parts*2 elements)."""
+    and T*heads*parts*2 elements).  ``most`` > 0: the portions of more tokens are left out (their rows of ``out`` stay as
+    they are) and ``tokens`` is how many the others bring."""
     T, nh, dk = q.shape
     _need(q, "q", torch.bfloat16, (T, nh, dk))
     rank = out.shape[-1]
@@ -1095,9 +1100,71 @@ def attn_latent_mma(out, q, cache, q_start, start_pos, num_entries, block_table,
             raise KernelError("attention scratch buffers are too small for the number of key ranges")
     _ok(kernels_lib().xb_attn_latent_mma(
         out.data_ptr(), q.data_ptr(), cache.data_ptr(), q_start.data_ptr(), start_pos.data_ptr(), int(num_entries),
-        block_table.data_ptr(), int(table_stride), T, nh, dk, rank, cache.shape[1], cache.shape[0], int(window or 0),
-        float(scale), _ptr(sink), int(row_groups), int(parts), _ptr(part_o), _ptr(part_ml), err.data_ptr(), _stream()),
+        block_table.data_ptr(), int(table_stride), T if tokens is None else int(tokens), nh, dk, rank, cache.shape[1], cache.shape[0],
+        int(window or 0), float(scale), _ptr(sink), int(row_groups), int(most), int(parts), _ptr(part_o), _ptr(part_ml), err.data_ptr(), _stream()),
         "attn_latent_mma", 2 if parts > 1 else 1)
+
+
+def attn_rows_tc_takes(d: int, rd: int, dv: int, rank: int) -> bool:
+    """Whether ``attn_rows_tc`` takes these sizes."""
+    return bool(kernels_lib().xb_attn_rows_tc_takes(int(d), int(rd), int(dv), int(rank)))
+
+
+def latent_prefill_work(counts, starts, dec_max: int, window, heads: int, max_ctas: int = PREFILL_TC_MAX_CTAS, host_buffer=None):
+    """The work list of ``attn_rows_tc`` for a step whose entries bring ``counts`` tokens after ``starts`` cached ones
+    (host arrays): (pinned int32 host tensor, CTAs, rows the portions see, where the list of the rows' runs begins).  The
+    list holds what ``latent_gather`` needs, too.  ``host_buffer``: as in ``attn_prefill_work``."""
+    from .native import host_lib
+    counts = np.ascontiguousarray(counts, dtype=np.int32)
+    starts = np.ascontiguousarray(starts, dtype=np.int32)
+    long = counts > dec_max
+    tiles, keys = int(((counts[long] + 127) // 128).sum()), int(((starts + counts)[long] // 64 + 2).sum())
+    cap = max_ctas + 1 + 4 * tiles * heads + 2 * keys
+    host = host_buffer(cap) if host_buffer is not None else torch.empty(cap, dtype=torch.int32).pin_memory()
+    ctas, rows = ctypes.c_int(0), ctypes.c_int(0)
+    used = host_lib().xb_latent_prefill_work(len(counts), counts.ctypes.data, starts.ctypes.data, int(dec_max), int(window or 0),
+                                             int(heads), int(max_ctas), host.data_ptr(), cap, ctypes.byref(ctas), ctypes.byref(rows))
+    if used < 0:
+        raise KernelError("the work list does not fit its buffer")
+    return host[:max(int(used), 1)], int(ctas.value), int(rows.value), int(used) - rows.value // 32
+
+
+def latent_gather(out, pages, work, runs_at: int, q_start, start_pos, block_table, table_stride, window, err) -> None:
+    """The cached rows that the portions of a ``latent_prefill_work`` list see, one portion after the other, into ``out``
+    ``[rows, width]``; rows that no query of a portion sees are zeros."""
+    rows, width = out.shape
+    _need(out, "out", torch.bfloat16)
+    _need(pages, "pages", torch.bfloat16, (None, None, width))
+    _need(work, "work", torch.int32)
+    if width % 8 or rows % 64 or work.numel() < runs_at + rows // 32:
+        raise KernelError("gathered rows: a width that is no multiple of 8, or more rows than the work list names")
+    _ok(kernels_lib().xb_latent_gather(out.data_ptr(), pages.data_ptr(), work.data_ptr() + 4 * int(runs_at), rows, q_start.data_ptr(),
+                                       start_pos.data_ptr(), block_table.data_ptr(), int(table_stride), pages.shape[1], pages.shape[0],
+                                       int(window or 0), width, err.data_ptr(), _stream()), "latent_gather")
+
+
+def attn_rows_tc(out, q, q_row: int, kv, rows, work, ctas, q_start, start_pos, nh: int, d: int, rd: int, dv: int, rank: int,
+                 window, scale, sink, err) -> None:
+    """Attention of the portions of a ``latent_prefill_work`` list on tcgen05 (TMA-fed; scores, probabilities and
+    accumulators in tensor memory).  ``q``: rows of ``q_row`` elements whose first ``nh * (d + rd)`` are the heads'
+    queries; ``kv`` ``[n, nh * (d + dv)]``: all heads' keys, then all heads' values; ``rows`` ``[n, width]``: the gathered
+    rows, whose rd channels from ``rank`` on belong to every head's key.  ``out`` ``[T, nh * dv]`` receives the rows of the
+    list's portions; others stay as they are."""
+    n, width = rows.shape
+    T = out.shape[0]
+    _need(out, "out", torch.bfloat16, (T, nh * dv))
+    _need(q, "q", torch.bfloat16, (T, q_row))
+    _need(kv, "kv", torch.bfloat16, (n, nh * (d + dv)))
+    _need(rows, "rows", torch.bfloat16)
+    _need(work, "work", torch.int32)
+    if sink is not None:
+        _need(sink, "sink", torch.float32, (nh,))
+    if q_row < nh * (d + rd) or (ctas > 0 and work.numel() < ctas + 1):
+        raise KernelError("the queries or the work list are shorter than the call needs")
+    _ok(kernels_lib().xb_attn_rows_tc(
+        out.data_ptr(), nh * dv, q.data_ptr(), int(q_row), kv.data_ptr(), rows.data_ptr(), T, n, int(nh), int(d), int(rd), int(dv),
+        int(rank), width, q_start.data_ptr(), start_pos.data_ptr(), int(window or 0), float(scale), _ptr(sink), work.data_ptr(),
+        int(ctas), err.data_ptr(), _stream()), "attn_rows_tc")
 
 
 def gate_sigmoid(out, heads, gate):

@@ -107,7 +107,7 @@ def _plan(ctx, head_dim: int):
     return plan
 
 
-class _PinnedRing:
+class PinnedRing:
     """A few pinned staging buffers used in turn; one is reused only after the copy that read it has
     finished (pinning memory anew for every step would synchronise the device)."""
 
@@ -132,7 +132,7 @@ class _PinnedRing:
         self.events[self.i] = ev
 
 
-_work_ring = _PinnedRing()
+_work_ring = PinnedRing()
 
 
 def _prefill_work(ctx, nh: int, nkv: int, window, keep_first: int = 0):

@@ -16,7 +16,9 @@ Only the row ``[c | k_r]`` is cached.  Because ``q_h,plain . (W_uk,h c) = (W_uk,
 ``sum_j p_j W_uv,h c_j = W_uv,h sum_j p_j c_j``, the step carries each head's plain query part into the latent space
 (a batch of small products, one per head), runs attention with ONE key/value head over the cached rows themselves
 (kv_rank + rope_dim key channels, the first kv_rank of them the value) and maps the result through ``W_uv,h``
-afterwards: no key or value is ever formed per head, for prompts or for single tokens.  A layer with
+afterwards.  Long portions take the other way round, which needs fewer operations per query and key: the rows a portion
+sees are gathered, one product forms the keys and values of all heads, and ordinary attention runs on those
+(``rows_plan`` decides).  A layer with
 ``shares_cache`` has no ``W_dkv``: it reads the rows another layer wrote, with its own maps, queries, window and sink;
 where those rows carry a rotated key part that it does not use, its query rows are zero there.
 """
@@ -24,11 +26,13 @@ from __future__ import annotations
 
 from typing import List
 
+import numpy as np
 import torch
 
 from .. import kernels
 from ..config.plan import LatentAttentionSpec
 from ..weights.loader import WeightSpec
+from .attention_backend import PinnedRing
 from .base import CacheTensor, LayerCache, Mixer, PagedCacheNeed, StepContext, build_part, register_mixer
 from .linear import linear, stack_rows
 
@@ -47,11 +51,59 @@ USE_TENSOR_CORES = True
 # a step of single tokens deals every token's key tiles out to several blocks so that about one block per SM runs
 _DECODE_BLOCKS = 148
 _DECODE_MIN_TILES = 2
+_rows_ring = PinnedRing()
 
 
-def latent_attend(out, q, pages, ctx: StepContext, table, stride, page_size, window, scale, sink) -> None:
+# Portions of more tokens than this may run on keys and values formed for the step.
+ROWS_MIN_TOKENS = 4
+# ... as long as those take no more memory than this (in bytes)
+ROWS_MAX_BYTES = 1 << 30
+# What the two ways cost, for the choice between them: operations per microsecond of the attention over cached rows
+# (75 to 91 measured at ranks 256 and 512; a block of it walks over all keys of its 32 rows, at one SM's share of that
+# rate), of the products that form keys and values, and of the attention on those (780 measured at a prompt of 2,048
+# tokens and 32 heads, where the first way took 1,570 us and the second takes 55 + 18 us); beside that the second way is
+# a few microseconds shorter, as nothing is mapped in and out of the latent space - or as much longer, where the step's
+# small portions need the first way too.  Measured per layer (rank 512, 32 heads): 8 tokens after 3,000 cached ones 235 us
+# less the second way, 16 tokens alone 6 us less; 20 portions of 8 tokens after 1,000 cached ones 145 us less the first.
+ROWS_RATES = (75e6, 900e6, 700e6, -6.0, 20.0)
+ROWS_SMS = 148
+
+
+def rows_plan(ctx: StepContext, heads: int, d: int, rd: int, dv: int, rank: int, width: int, window):
+    """Whether (and how) the step's portions of more than ``ROWS_MIN_TOKENS`` tokens run on keys and values formed per
+    head: None, or (work list on the device, CTAs, rows, where the rows' runs begin in the list, tokens of the other
+    portions).  Decided once per step and shared by layers of the same sizes."""
+    key = ("latent_rows", heads, d, rd, dv, rank, width, window)
+    if key in ctx.scratch:
+        return ctx.scratch[key]
+    made = None
+    if not (ctx.fixed_shapes or ctx.all_single) and USE_TENSOR_CORES and ctx.dtype == torch.bfloat16 and width % 8 == 0 \
+            and kernels.attn_rows_tc_takes(d, rd, dv, rank) and kernels.attn_latent_mma_takes(width, rank):
+        counts = np.diff(ctx.h_q_start[: ctx.real_entries + 1]).astype(np.int64)
+        starts = ctx.h_start_pos[: ctx.real_entries].astype(np.int64)
+        long = counts > ROWS_MIN_TOKENS
+        n, before = counts[long], starts[long]
+        if window:
+            before = np.minimum(before, window)
+        keys, pairs = float((before + n).sum()), float((n * before + n * (n + 1) / 2).sum())
+        if window:
+            pairs = min(pairs, float(n.sum()) * window)
+        over_rows, form, over_heads, alone, beside = ROWS_RATES
+        first = 2 * (width + rank) / over_rows * max(pairs * heads, float((before + n).max(initial=0)) * 32 * ROWS_SMS)
+        second = (alone if long.all() else beside) + keys * heads * 2 * rank * (d + dv) / form + pairs * heads * 2 * (d + rd + dv) / over_heads
+        if len(n) and second < first and (keys + 64 * len(n)) * heads * (d + dv) * 2 <= ROWS_MAX_BYTES:
+            host, ctas, rows, runs_at = kernels.latent_prefill_work(counts, starts, ROWS_MIN_TOKENS, window, heads,
+                                                                    host_buffer=_rows_ring.take)
+            made = (host.to(ctx.positions.device, non_blocking=True), ctas, rows, runs_at, int(counts[~long].sum()))
+            _rows_ring.sent()
+    ctx.scratch[key] = made
+    return made
+
+
+def latent_attend(out, q, pages, ctx: StepContext, table, stride, page_size, window, scale, sink, small=None) -> None:
     """Attention of ``q`` ``[T, heads, dk]`` over the cached rows ``pages`` ``[page, slot, dk]`` into ``out``
-    ``[T, heads, rank]``: on tensor cores in bfloat16 where the sizes fit, else one warp per (token, head)."""
+    ``[T, heads, rank]``: on tensor cores in bfloat16 where the sizes fit, else one warp per (token, head).  ``small``:
+    only the portions of up to ``ROWS_MIN_TOKENS`` tokens, which bring that many."""
     T, H, dk = q.shape
     rank = out.shape[-1]
     if USE_TENSOR_CORES and q.dtype == torch.bfloat16 and kernels.attn_latent_mma_takes(dk, rank):
@@ -70,7 +122,8 @@ def latent_attend(out, q, pages, ctx: StepContext, table, stride, page_size, win
                 part_o = ctx.workspace.get("latent.part_o", (T * H * parts * rank,), torch.float32)
                 part_ml = ctx.workspace.get("latent.part_ml", (T * H * parts * 2,), torch.float32)
         kernels.attn_latent_mma(out, q, pages, ctx.q_start, ctx.start_pos, ctx.num_entries, table, stride, window, scale,
-                                sink, ctx.err, row_groups=rg, parts=parts, part_o=part_o, part_ml=part_ml)
+                                sink, ctx.err, row_groups=rg, parts=parts, part_o=part_o, part_ml=part_ml,
+                                most=0 if small is None else ROWS_MIN_TOKENS, tokens=small)
         return
     kernels.attention_plain(out, q, pages.view(pages.shape[0], 1, pages.shape[1], dk), None, ctx.positions,
                             ctx.req_of_token, table, stride, window, scale, ctx.err, sink=sink, value_dim=rank)
@@ -95,7 +148,7 @@ class LatentAttention(Mixer):
             raise ValueError("latent attention without a rotated part takes no rotary encoding")
         if spec.row_tail and not spec.shares_cache:
             raise ValueError("only a layer that reads another layer's rows can leave channels of them unread")
-        self.w_in = self.w_uq = self.w_uk = self.w_uv = self.w_o = self.norm_w = self.q_norm_w = self.sink = None
+        self.w_in = self.w_uq = self.w_kv = self.w_uk = self.w_uv = self.w_o = self.norm_w = self.q_norm_w = self.sink = None
 
     @classmethod
     def weight_specs(cls, spec: LatentAttentionSpec, prefix: str) -> List[WeightSpec]:
@@ -140,8 +193,10 @@ class LatentAttention(Mixer):
         self.w_in = stack_rows(parts)
         del parts
         H = s.num_heads
-        self.w_uk = operand(n[3]).view(H, s.head_dim, s.kv_rank)      # [head, plain channel, latent channel]
-        self.w_uv = operand(n[4]).view(H, s.v_head_dim, s.kv_rank)    # [head, value channel, latent channel]
+        # all heads' key maps, then all heads' value maps: one matrix for the keys and values of a long portion
+        self.w_kv = torch.cat([operand(n[3]), operand(n[4])])
+        self.w_uk = self.w_kv[:H * s.head_dim].view(H, s.head_dim, s.kv_rank)      # [head, plain channel, latent channel]
+        self.w_uv = self.w_kv[H * s.head_dim:].view(H, s.v_head_dim, s.kv_rank)    # [head, value channel, latent channel]
         self.w_o = operand(n[7])
         if s.sink:
             self.sink = store.get(p + n[5], self.device, torch.float32).float().contiguous()
@@ -149,6 +204,13 @@ class LatentAttention(Mixer):
     def cache_need(self) -> PagedCacheNeed:
         s = self.spec
         return PagedCacheNeed((("latent", CacheTensor((s.kv_rank + s.rope_dim + s.row_tail,), None, 0)),), s.cache_window)
+
+    def _plan(self, ctx: StepContext):
+        s = self.spec
+        return rows_plan(ctx, s.num_heads, s.head_dim, s.rope_dim, s.v_head_dim, s.kv_rank, s.kv_rank + s.rope_dim + s.row_tail, s.window)
+
+    def prepare_step(self, ctx: StepContext, cache: LayerCache) -> None:
+        self._plan(ctx)
 
     def forward(self, x, ctx: StepContext, cache: LayerCache, state=None, writes_cache: bool = True):
         s = self.spec
@@ -167,10 +229,10 @@ class LatentAttention(Mixer):
         rot = s.rope.rotary_dim if rd else 0
         inv_freq, magnitude = (self.position.frequencies(), s.rope.magnitude) if rd else (None, 1.0)
 
-        def prepare(q_abs, source, kv_off, query_latent=None):
+        def prepare(q_abs, source, kv_off, query_latent=None, in_place=False):
             kernels.latent_prepare(q_abs, pages, source, 0, kv_off, None, self.norm_w, inv_freq, ctx.positions, ctx.req_of_token,
-                                   table, stride, H if q_abs is not None else 0, d, rd, r, rot, s.norm_eps, magnitude, ctx.err,
-                                   tail=tail, query_latent=query_latent)
+                                   table, stride, H if q_abs is not None or in_place else 0, d, rd, r, rot, s.norm_eps, magnitude,
+                                   ctx.err, tail=0 if in_place or q_abs is None else tail, query_latent=query_latent, in_place=in_place)
         q_rows = proj
         if s.q_rank is not None:
             # the row to its page and the queries' own latent, then the queries
@@ -179,21 +241,37 @@ class LatentAttention(Mixer):
             kv_off = -1
             q_rows = ws.get("latent.queries", (T, H * (d + rd)), self.dtype)
             linear(q_rows, cq, self.w_uq, ctx.err)
-        # every head's plain query part carried into the latent space, q_lat[h] = q_plain[h] . W_uk,h, written
-        # straight into the front of the head's query row
-        q_plain = q_rows[:, :H * (d + rd)].view(T, H, d + rd)[:, :, :d].transpose(0, 1)          # [H, T, d] view
-        q_abs = ws.get("latent.q", (T, H, r + rd + tail), self.dtype)
-        batched_product(q_abs[:, :, :r].transpose(0, 1), q_plain, self.w_uk.transpose(1, 2))
-        if rd or tail or kv_off >= 0:
-            prepare(q_abs, q_rows, kv_off)
-        # one key/value head over the cached rows: keys are the whole row, values its first kv_rank channels
-        o_lat = ws.get("latent.o_lat", (T, H, r), self.dtype)
-        latent_attend(o_lat, q_abs, pages, ctx, table, stride, cache.page_size, s.window, s.scale, self.sink)
-        # back out of the latent space, head by head: o[h] = o_lat[h] . W_uv,h^T, written where the output
-        # projection reads it; the gate then works in place
         inner = ws.get("latent.inner", (T, H * dv), self.dtype)
         o_heads = inner.view(T, H, dv).transpose(0, 1)                                # [H, T, dv] view
-        batched_product(o_heads, o_lat.transpose(0, 1), self.w_uv)
+        plan = self._plan(ctx)
+        if plan is None or plan[4]:
+            # every head's plain query part carried into the latent space, q_lat[h] = q_plain[h] . W_uk,h, written
+            # straight into the front of the head's query row
+            q_plain = q_rows[:, :H * (d + rd)].view(T, H, d + rd)[:, :, :d].transpose(0, 1)          # [H, T, d] view
+            q_abs = ws.get("latent.q", (T, H, r + rd + tail), self.dtype)
+            batched_product(q_abs[:, :, :r].transpose(0, 1), q_plain, self.w_uk.transpose(1, 2))
+            if rd or tail or kv_off >= 0:
+                prepare(q_abs, q_rows, kv_off)
+                kv_off = -1
+            # one key/value head over the cached rows: keys are the whole row, values its first kv_rank channels
+            o_lat = ws.get("latent.o_lat", (T, H, r), self.dtype)
+            latent_attend(o_lat, q_abs, pages, ctx, table, stride, cache.page_size, s.window, s.scale, self.sink,
+                          plan[4] if plan is not None else None)
+            # back out of the latent space, head by head: o[h] = o_lat[h] . W_uv,h^T, written where the output
+            # projection reads it; the gate then works in place
+            batched_product(o_heads, o_lat.transpose(0, 1), self.w_uv)
+        if plan is not None:
+            # long portions: the keys and values of all heads for the rows they see, and attention on those (it writes
+            # its own tokens' rows of `inner`, whatever the other way left there)
+            work, ctas, n, runs_at, _ = plan
+            if rd or kv_off >= 0:
+                prepare(None, q_rows, kv_off, in_place=rd > 0)
+            rows = ws.get("latent.rows", (n, r + rd + tail), self.dtype)
+            kernels.latent_gather(rows, pages, work, runs_at, ctx.q_start, ctx.start_pos, table, stride, s.window, ctx.err)
+            kv = ws.get("latent.kv", (n, H * (d + dv)), self.dtype)
+            linear(kv, rows[:, :r], self.w_kv, ctx.err)
+            kernels.attn_rows_tc(inner, q_rows, q_rows.shape[1], kv, rows, work, ctas, ctx.q_start, ctx.start_pos, H, d, rd, dv, r,
+                                 s.window, s.scale, self.sink, ctx.err)
         if s.gate:
             kernels.gate_sigmoid(inner, o_heads, proj[:, at_gate:at_gate + (H if s.gate_per_head else H * dv)])
         out = ws.get("latent.out", (T, s.hidden), ctx.branch_dtype or self.dtype)
