@@ -317,6 +317,120 @@ XB_API long long xb_latent_prefill_work(int B, const int* counts, const int* sta
     return used;
 }
 
+// ---- work lists of the attention with talking heads over many tokens -------------------------------
+// All portions of the step, cut into blocks of 128 queries whose score tiles (128 queries x 32 keys of one head, from the
+// first query's first key on, aligned to 128 keys) lie one after the other: [head][32-key tile].  Blocks are taken in order
+// into chunks of at most cap_tiles tiles; a chunk is one pair of launches.  Per chunk: its blocks, the items of the first
+// launch (512 / heads queries of a block x a run of 128-key tiles) and of the second (a block x two heads of a key/value
+// head), each shared out longest first onto the CTA with the least work so far.
+// out: per chunk 6 int32 per block (portion, first query of it, first 32-key tile, 32-key tiles, first score tile, 0), then
+// [ctas + 1] offsets and 4 int32 per item (block, query tile, first 128-key tile, how many), then the same for the second
+// launch (block, first head, heads, 0).  chunks: 5 int32 per chunk: where its blocks, first and second list begin, CTAs of
+// both.  Returns the number of chunks, -1 where out or chunks are too small, -2 where one block has more than cap_tiles.
+namespace {
+struct WorkItem { long long cost; int32_t v[4]; };
+int share_items(std::vector<WorkItem>& items, int max_ctas, std::vector<int32_t>& out, long long* longest = nullptr) {
+    std::stable_sort(items.begin(), items.end(), [](const WorkItem& x, const WorkItem& y) { return x.cost > y.cost; });
+    const int ctas = (int)std::min<size_t>(max_ctas, items.size());
+    std::vector<std::vector<int32_t>> lists(ctas);
+    std::vector<std::pair<long long, int>> heap;
+    for (int i = 0; i < ctas; ++i) heap.emplace_back(0, i);
+    auto later = [](const std::pair<long long, int>& x, const std::pair<long long, int>& y) { return x > y; };
+    std::make_heap(heap.begin(), heap.end(), later);
+    if (longest) *longest = 0;
+    for (const WorkItem& it : items) {
+        std::pop_heap(heap.begin(), heap.end(), later);
+        auto& top = heap.back();
+        lists[top.second].insert(lists[top.second].end(), it.v, it.v + 4);
+        top.first += it.cost;
+        if (longest) *longest = std::max(*longest, top.first);
+        std::push_heap(heap.begin(), heap.end(), later);
+    }
+    int at = 0;
+    for (int c = 0; c < ctas; ++c) {
+        out.push_back(at);
+        at += (int)lists[c].size() / 4;
+    }
+    out.push_back(at);
+    for (const auto& l : lists) out.insert(out.end(), l.begin(), l.end());
+    return ctas;
+}
+}  // namespace
+
+XB_API int xb_talk_work(int B, const int* counts, const int* starts, int window, int heads, int kv_heads, int max_ctas,
+                        long long cap_tiles, int32_t* out, long long capacity, int32_t* chunks, int max_chunks,
+                        long long* used_out, long long* tiles_out) {
+    constexpr int ROWS = 128, KEYS = 128;
+    struct Block { int b, first, kb0, nkb, rows, p0; };
+    std::vector<Block> blocks;
+    auto first_key = [&](int p) { return window > 0 ? std::max(0, p - window + 1) : 0; };
+    for (int b = 0; b < B; ++b)
+        for (int first = 0; first < counts[b]; first += ROWS) {
+            const int p0 = starts[b] + first, rows = std::min(ROWS, counts[b] - first);
+            const int lo = first_key(p0) / KEYS, hi = (p0 + rows - 1) / KEYS;
+            blocks.push_back({b, first, lo * 4, (hi - lo + 1) * 4, rows, p0});
+        }
+    *used_out = *tiles_out = 0;
+    const int qn = 512 / heads, per = 128 / heads, rep = heads / kv_heads;
+    std::vector<int32_t> all;
+    int n_chunks = 0;
+    for (size_t at = 0; at < blocks.size();) {
+        size_t end = at;
+        long long tiles = 0;
+        while (end < blocks.size() && tiles + (long long)blocks[end].nkb * heads <= cap_tiles) tiles += (long long)blocks[end++].nkb * heads;
+        if (end == at) return -2;
+        if (n_chunks == max_chunks) return -1;
+        int32_t* ch = chunks + 5 * n_chunks++;
+        *tiles_out = std::max(*tiles_out, tiles);
+        ch[0] = (int32_t)all.size();
+        long long tile0 = 0, key_tiles = 0;
+        for (size_t i = at; i < end; ++i) {
+            const Block& k = blocks[i];
+            const int32_t rec[6] = {k.b, k.first, k.kb0, k.nkb, (int32_t)tile0, 0};
+            all.insert(all.end(), rec, rec + 6);
+            tile0 += (long long)k.nkb * heads;
+            key_tiles += (long long)(k.nkb / 4) * ((k.rows + qn - 1) / qn);
+        }
+        // runs of key tiles short enough to share them out evenly, long enough that the queries are not loaded often
+        const int run = (int)std::max<long long>(4, key_tiles / (4LL * max_ctas));
+        std::vector<WorkItem> one, two, singles;
+        for (size_t i = at; i < end; ++i) {
+            const Block& k = blocks[i];
+            for (int qt = 0; qt * qn < k.rows; ++qt) {
+                const int rows = std::min(qn, k.rows - qt * qn), p0 = k.p0 + qt * qn;
+                const int lo = first_key(p0) / KEYS, hi = (p0 + rows - 1) / KEYS;
+                const int batches = (std::min(rows, qn / 2) + per - 1) / per;      // of the warps that have most queries
+                for (int kt = lo; kt <= hi; kt += run) {
+                    const int n = std::min(run, hi - kt + 1);
+                    one.push_back({(long long)n * (1 + 4 * batches) + 3, {(int32_t)(i - at), qt, kt, n}});
+                }
+            }
+            const int n = (k.p0 + k.rows - 1) / 64 - first_key(k.p0) / 64 + 1;
+            for (int g = 0; g < kv_heads; ++g)
+                for (int h = 0; h < rep; h += 2) {
+                    const int nh = std::min(2, rep - h);
+                    two.push_back({(long long)n * (nh == 2 ? 6 : 4) + 18, {(int32_t)(i - at), g * rep + h, nh, 0}});
+                }
+            for (int h = 0; h < heads; ++h) singles.push_back({(long long)n * 4 + 18, {(int32_t)(i - at), h, 1, 0}});
+        }
+        ch[1] = (int32_t)all.size();
+        ch[3] = share_items(one, max_ctas, all);
+        ch[2] = (int32_t)all.size();
+        // items of two heads load a value tile once for both; where those are too few to fill the CTAs, one head each
+        long long longest[2];
+        std::vector<int32_t> lists[2];
+        const int n2 = share_items(two, max_ctas, lists[0], &longest[0]), n1 = share_items(singles, max_ctas, lists[1], &longest[1]);
+        const int take = longest[1] < longest[0] ? 1 : 0;
+        ch[4] = take ? n1 : n2;
+        all.insert(all.end(), lists[take].begin(), lists[take].end());
+        at = end;
+    }
+    *used_out = (long long)all.size();
+    if (*used_out > capacity) return -1;
+    std::copy(all.begin(), all.end(), out);
+    return n_chunks;
+}
+
 // ---- scheduler ---------------------------------------------------------------------------------
 struct SchedHandle {
     Scheduler sched;

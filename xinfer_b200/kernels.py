@@ -858,6 +858,66 @@ def attn_talking_mma(out, q, k_cache, v_cache, talk, q_start, start_pos, num_ent
         _ptr(part_o), _ptr(part_ml), err.data_ptr(), _stream()), "attn_talking_mma", 2 if parts > 1 else 1)
 
 
+TALK_TILE_FLOATS = 128 * 32     # a score tile of attn_talking_tc: 128 queries x 32 keys of one head
+
+
+def attn_talking_tc_takes(nh: int, nkv: int, d: int, dv: int, page_size: int) -> bool:
+    """Whether ``attn_talking_tc`` takes these sizes."""
+    return bool(kernels_lib().xb_attn_talking_tc_takes(int(nh), int(nkv), int(d), int(dv), int(page_size)))
+
+
+def talk_work(counts, starts, window, heads: int, kv_heads: int, cap_tiles: int, max_ctas: int = PREFILL_TC_MAX_CTAS, host_buffer=None):
+    """The work lists of ``attn_talking_tc`` for a step whose entries bring ``counts`` tokens after ``starts`` cached ones:
+    (pinned int32 host tensor, chunks as rows [blocks, first list, second list, CTAs of both], score tiles of the largest
+    chunk), or None where 128 queries alone have more than ``cap_tiles`` score tiles.  ``host_buffer``: as in
+    ``attn_prefill_work``."""
+    from .native import host_lib
+    counts = np.ascontiguousarray(counts, dtype=np.int32)
+    starts = np.ascontiguousarray(starts, dtype=np.int32)
+    ends = (starts + counts).astype(np.int64)
+    blocks = (counts.astype(np.int64) + 127) // 128
+    keys = (np.minimum(ends, counts + int(window)) if window else ends) // 128 + 2
+    per_block = -(-128 * heads // 512)
+    chunks = np.zeros((int(blocks.sum()), 5), dtype=np.int32)
+    cap = int((blocks * (6 + 4 * per_block * (keys // 4 + 1) + 4 * heads)).sum()) + 2 * (max_ctas + 1) * len(chunks)
+    host = host_buffer(cap) if host_buffer is not None else torch.empty(cap, dtype=torch.int32).pin_memory()
+    used, tiles = ctypes.c_longlong(0), ctypes.c_longlong(0)
+    n = host_lib().xb_talk_work(len(counts), counts.ctypes.data, starts.ctypes.data, int(window or 0), int(heads), int(kv_heads),
+                                int(max_ctas), int(cap_tiles), host.data_ptr(), cap, chunks.ctypes.data, len(chunks),
+                                ctypes.byref(used), ctypes.byref(tiles))
+    if n == -1:
+        raise KernelError("the work lists do not fit their buffer")
+    if n < 0:
+        return None
+    return host[:max(int(used.value), 1)], chunks[:n].tolist(), int(tiles.value)
+
+
+def attn_talking_tc(out, q, k_cache, v_cache, talk, scores, work, chunks, q_start, start_pos, block_table, table_stride, window,
+                    scale, sink, out_scale, err) -> None:
+    """``attn_talking`` for bfloat16 steps of many tokens: per chunk of ``talk_work`` one kernel forms the mixed float32
+    scores (tcgen05 products, mix on the FMA units) in ``scores`` and another one the softmax and the value sums (tcgen05).
+    ``talk``: the matrix in HOST memory (it travels with the launch)."""
+    T, nh, d = q.shape
+    _need(q, "q", torch.bfloat16, (T, nh, d))
+    _need(k_cache, "k_cache", torch.bfloat16, (None, None, None, d))
+    num_pages, nkv, ps, _ = k_cache.shape
+    dv = v_cache.shape[-1]
+    _need(v_cache, "v_cache", torch.bfloat16, (num_pages, nkv, ps, dv))
+    if out.dtype != torch.bfloat16 or out.shape != (T, nh * dv) or out.stride(1) != 1 or not out.is_cuda:
+        raise KernelError("out must be a bfloat16 view [T, heads * dv] with unit column stride")
+    if talk.is_cuda or talk.dtype != torch.float32 or talk.shape != (nh, nh) or not talk.is_contiguous():
+        raise KernelError("talk must be a contiguous float32 matrix [heads, heads] in host memory")
+    _need(scores, "scores", torch.float32)
+    _need(work, "work", torch.int32)
+    at = work.data_ptr()
+    for blocks, one, two, ctas1, ctas2 in chunks:
+        _ok(kernels_lib().xb_attn_talking_tc(
+            out.data_ptr(), int(out.stride(0)), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), talk.data_ptr(), scores.data_ptr(),
+            at + 4 * blocks, at + 4 * one, ctas1, at + 4 * two, ctas2, q_start.data_ptr(), start_pos.data_ptr(), block_table.data_ptr(),
+            int(table_stride), T, nh, nkv, d, dv, ps, num_pages, int(window or 0), float(scale), int(bool(sink)), float(out_scale),
+            err.data_ptr(), _stream()), "attn_talking_tc", 2)
+
+
 def gated_scan(y, zxg, bz, bx, state, q_start, slots, req_of_token, num_entries, out_scale, scratch=None):
     """The minGRU recurrence over a step's tokens: ``zxg`` float32 ``[T, 3 * width]`` (the z, x and g
     projections without biases), ``state`` float32 ``[slots, width]`` carried per request, ``y`` a view

@@ -61,6 +61,8 @@ def _declare_host(lib):
          [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p])
     _sig(lib, "xb_latent_prefill_work", c_longlong,
          [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p])
+    _sig(lib, "xb_talk_work", c_int,
+         [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p])
     _sig(lib, "xb_cm_log_freed", None, [c_void_p, c_int])
     _sig(lib, "xb_cm_drain_freed", c_int, [c_void_p, c_void_p, c_void_p, c_int])
     _sig(lib, "xb_assemble", c_longlong,
@@ -153,6 +155,9 @@ def _declare_kernels(lib):
     _sig(lib, "xb_attn_talking", I, [I, P, I, P, P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, I, F, I, F, I, I, P, P, P, P])
     _sig(lib, "xb_attn_talking_mma_tile", I, [I, I, I, I, I])
     _sig(lib, "xb_attn_talking_mma", I, [P, I, P, P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, I, F, I, F, I, I, P, P, P, P])
+    _sig(lib, "xb_attn_talking_tc_takes", I, [I, I, I, I, I])
+    _sig(lib, "xb_attn_talking_tc", I,
+         [P, L, P, P, P, P, P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, F, P, P])
     _sig(lib, "xb_gated_scan", I, [I, P, I, P, P, P, P, P, P, P, I, I, I, F, I, P, P])
     _sig(lib, "xb_polynorm", I, [I, P, P, P, I, I, F, P])
     _sig(lib, "xb_expert_route", I, [P, P, P, P, P, P, I, P, I, I, I, I, P, P])

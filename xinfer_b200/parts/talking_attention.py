@@ -30,6 +30,7 @@ import torch
 from .. import kernels
 from ..config.plan import AttentionSpec
 from ..weights.loader import WeightSpec
+from .attention_backend import PinnedRing
 from .base import CacheTensor, LayerCache, Mixer, PagedCacheNeed, StepContext, build_part, register_mixer
 from .linear import linear
 
@@ -42,6 +43,13 @@ _DECODE_BLOCKS = 148
 _DECODE_MIN_KEYS = 128
 # bfloat16: both products on tensor cores where the sizes allow; tests switch it off to compare the two forms
 USE_TENSOR_CORES = True
+# Scratch memory for the mixed scores of a step of many tokens (in bytes): more queries run one chunk after the other.
+# 2,048 tokens of 32 heads take 285 MB.  Cut to stay in the 126 MB L2 cache (3 chunks of 96 MB, 5 of 64 MB) a step of four
+# layers took 6.0 and 7.4 ms instead of 5.2: the launches of a chunk leave SMs idle.
+SCORES_BYTES = 320 << 20
+# Steps of many tokens on the two kernels that pass the mixed scores through memory; tests switch it off.
+USE_SCORES = True
+_work_ring = PinnedRing()
 # without a mix and a sink the attention is the ordinary one: use the kernels of the engine's attention backend
 USE_ATTENTION_BACKEND = True
 
@@ -59,7 +67,7 @@ class TalkingAttention(Mixer):
             raise ValueError("this attention needs a rotary position encoding that offers its frequencies")
         self.names = tuple(spec.names) if spec.names else _DEFAULT_NAMES
         self.w_qkv = self.w_o = self.talk = self.q_norm = self.k_norm = self.bias = self.b_o = None
-        self.sink_scores = self.taps = None
+        self.sink_scores = self.taps = self.talk_host = None
         if spec.value_from_key and spec.value_dim != spec.head_dim:
             raise ValueError(f"keys of {spec.head_dim} channels cannot double as values of {spec.value_dim}")
         if spec.chunk is not None and spec.window is not None:
@@ -128,6 +136,7 @@ class TalkingAttention(Mixer):
             self.sink_scores = store.get(p + s.sink_name, self.device, torch.float32).float().contiguous()
         if s.talking_heads:
             self.talk = store.get(p + n[4], self.device, torch.float32).float().contiguous()
+            self.talk_host = self.talk.cpu()
         if s.qk_norm and s.qk_norm_weight:
             qn, kn = s.qk_norm_names or _DEFAULT_NORM_NAMES
             self.q_norm = store.get(p + qn, self.device, torch.float32).float().contiguous()
@@ -165,6 +174,32 @@ class TalkingAttention(Mixer):
             attention_backend.prepare_step(ctx, self.dtype, s.num_heads, s.num_kv_heads, s.head_dim, cache.page_size,
                                            kernels.mask_code(s.window, s.chunk), ctx.strides[cache.group],
                                            keep_first=s.keep_first, dv=s.value_dim)
+
+        elif self._takes_scores(ctx, cache):
+            self._scores_work(ctx, cache)
+
+    def _takes_scores(self, ctx: StepContext, cache: LayerCache) -> bool:
+        """Heads that talk, in a bfloat16 step of more than single tokens, at sizes that the kernels take which pass the
+        mixed scores through memory.  (Their time is that of the FMA units' mix for whole blocks of queries: single tokens
+        are better off with their keys cut into ranges.)"""
+        s = self.spec
+        return (USE_TENSOR_CORES and USE_SCORES and s.talking_heads and self.dtype == torch.bfloat16
+                and not (ctx.all_single or ctx.fixed_shapes) and not self._changed_scores()
+                and kernels.attn_talking_tc_takes(s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, cache.page_size))
+
+    def _scores_work(self, ctx: StepContext, cache: LayerCache):
+        """The step's work lists for those kernels, made once and shared by layers of the same sizes; None: too many keys."""
+        s = self.spec
+        key = ("talk_work", s.num_heads, s.num_kv_heads, s.window)
+        if key not in ctx.scratch:
+            counts = ctx.h_q_start[1: ctx.real_entries + 1] - ctx.h_q_start[: ctx.real_entries]
+            made = kernels.talk_work(counts, ctx.h_start_pos[: ctx.real_entries], s.window, s.num_heads, s.num_kv_heads,
+                                     SCORES_BYTES // (4 * kernels.TALK_TILE_FLOATS), host_buffer=_work_ring.take)
+            if made is not None:
+                made = (made[0].to(ctx.positions.device, non_blocking=True), made[1], made[2])
+                _work_ring.sent()
+            ctx.scratch[key] = made
+        return ctx.scratch[key]
 
     # ---- the two halves ---------------------------------------------------------------------------
     def inner_width(self) -> int:
@@ -224,6 +259,14 @@ class TalkingAttention(Mixer):
                                     slope_exponent=s.distance_slope_exponent, chunk=s.chunk, keep_first=s.keep_first,
                                     out_scale=out_scale)
             return
+        if out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and self._takes_scores(ctx, cache):
+            made = self._scores_work(ctx, cache)
+            if made is not None:
+                work, chunks, tiles = made
+                scores = ws.get("tattn.scores", (tiles * kernels.TALK_TILE_FLOATS,), torch.float32)
+                kernels.attn_talking_tc(out, q, cache["k"], cache["v"], self.talk_host, scores, work, chunks, ctx.q_start, ctx.start_pos,
+                                        table, stride, s.window, s.scale, s.sink, out_scale, ctx.err)
+                return
         # queries per block: the longest portion decides (a step of single tokens takes one query per block
         # and cuts the keys instead); a replayed step must not look at its actual lengths
         single = ctx.all_single or ctx.fixed_shapes
