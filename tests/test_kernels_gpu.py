@@ -556,3 +556,21 @@ def test_attention_tiled_random_layouts_and_batches(seed):
                 entries.append((0, int(rng.integers(1, 300))))                              # the start of a prompt
         worst = attention_case(tiled_kernel, torch.bfloat16, nkv * G, nkv, d, ps, entries, window, seed=case)
         assert worst <= tol(torch.bfloat16, 2), (nkv * G, nkv, d, ps, window, entries, worst)
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 64, 65, 129, 300])
+@pytest.mark.parametrize("N,K", [(1, 4), (63, 12), (130, 68), (129, 1024), (1500, 100), (12800, 64)])
+def test_every_float32_product_forms_the_same_bits(M, N, K):
+    """Whichever kernel takes a product of float32 operands - by its rows, its size, the operands' alignment - adds the
+    same terms in the same order.  Operands that start off a 16-byte boundary run on the general kernel."""
+    from xinfer_b200 import kernels
+    a, w = rnd(M, K, seed=6), rnd(N, K, seed=7)
+
+    def shifted(t):
+        buf = torch.empty(t.numel() + 1, device=t.device)
+        buf[1:].copy_(t.flatten())
+        return buf[1:].view(t.shape)
+    one, two = torch.full((M, N), float("nan"), device=dev()), torch.full((M, N), float("nan"), device=dev())
+    kernels.gemm_plain(one, a, w)
+    kernels.gemm_plain(two, shifted(a), shifted(w))
+    assert torch.equal(one, two)
