@@ -152,3 +152,38 @@ def test_random_rows_and_options(seed):
         want = [plain.sample(logits[r], params[r].temperature, top_k=params[r].top_k, top_p=params[r].top_p, seed=seeds[r], draw=trial)
                 for r in range(rows)]
         assert got == want, (trial, vocab, rows, [(r, params[r]) for r in range(rows) if got[r] != want[r]][:3])
+
+
+@pytest.mark.parametrize("vocab", [4096, 4100, 32000, 151936])
+@pytest.mark.parametrize("kind", ["normal", "ties", "infinities", "nan"])
+def test_logits_read_four_at_a_time_give_the_tokens_of_those_read_one_by_one(vocab, kind):
+    """Rows on 16-byte boundaries are read four logits at a time and compared as floats; the same rows one element off
+    such a boundary are read one by one.  Few rows are cut into many chunks, many rows into long ones."""
+    from xinfer_b200.sampling import SamplingParams
+    from xinfer_b200.sampling.sampler import Sampler
+    dev = torch.device("cuda:0")
+    R = 80
+    g = torch.Generator().manual_seed(vocab)
+    x = torch.randn(R, vocab, generator=g) * 3
+    if kind == "ties":
+        x = (x * 2).round() / 2
+        x[x == 0] = -0.0
+        x[:, ::3] += 0.0
+    elif kind == "infinities":
+        x[:, ::2] = -float("inf")
+        x[::5] = -float("inf")
+        x[::5, vocab // 2:vocab // 2 + 40] = 1.0
+    elif kind == "nan":
+        x[:, ::7] = float("nan")
+    ways = [(0.0, None, None), (0.7, None, None), (0.6, 20, 0.95), (0.8, None, 0.9), (1.0, 64, None), (0.9, 200, 0.8), (0.9, 1000, None), (0.5, 1, None)]
+    params = [SamplingParams(temperature=t, top_k=k, top_p=p) for t, k, p in (ways[r % len(ways)] for r in range(R))]
+    for rows in (1, 3, R):
+        got = []
+        for off in (0, 1):
+            buf = torch.empty(rows * vocab + 1, device=dev)
+            logits = buf[off:off + rows * vocab].view(rows, vocab)
+            logits.copy_(x[:rows])
+            for first in range(0, 8 if rows < 8 else 1):
+                s = Sampler(dev, rows)
+                got.append(s.to_host(s.sample(logits, [params[first + r] for r in range(rows)], list(range(rows)), [5] * rows)).tolist())
+        assert got[:len(got) // 2] == got[len(got) // 2:]

@@ -45,27 +45,37 @@ class Sampler:
         R = logits.shape[0]
         if R > self.max_rows:
             raise ValueError(f"{R} rows exceed the sampler's capacity {self.max_rows}")
-        rec = self._params_np
+        # column by column: a value that all rows share is written once (requests of one batch often share their options)
+        params = params[:R]
+        n = len(params)
+        rec = self._params_np[:n]
+        own = params[:1] if all(p is params[0] for p in params) else params
+
+        def column(name, value):
+            vals = [value(p) for p in own]
+            rec[name] = vals[0] if len(vals) == 1 else vals
+        if n:
+            column("temperature", lambda p: 0.0 if p.greedy else float(p.temperature))
+            column("top_k", lambda p: int(p.top_k) if p.top_k and p.top_k > 0 else 0)
+            column("top_p", lambda p: float(p.top_p) if p.top_p is not None else 1.0)
+            column("frequency_penalty", lambda p: float(p.frequency_penalty or 0.0))
+            column("presence_penalty", lambda p: float(p.presence_penalty or 0.0))
+            s64 = np.array([int(s) & 0xFFFFFFFFFFFFFFFF for s in (seeds[r] for r in range(n))], dtype=np.uint64)
+            rec["seed_lo"], rec["seed_hi"] = s64 & np.uint64(0xFFFFFFFF), s64 >> np.uint64(32)
+            rec["draw"] = np.array([int(d) & 0xFFFFFFFF for d in (draws[r] for r in range(n))], dtype=np.uint32)
+            rec["history_offset"] = 0
+            rec["history_len"] = 0
         any_pen = False
         off = 0
-        for r, p in enumerate(params):
-            rec[r]["temperature"] = 0.0 if p.greedy else float(p.temperature)
-            rec[r]["top_k"] = int(p.top_k) if p.top_k and p.top_k > 0 else 0
-            rec[r]["top_p"] = float(p.top_p) if p.top_p is not None else 1.0
-            s = int(seeds[r]) & 0xFFFFFFFFFFFFFFFF
-            rec[r]["seed_lo"], rec[r]["seed_hi"] = s & 0xFFFFFFFF, s >> 32
-            rec[r]["draw"] = int(draws[r]) & 0xFFFFFFFF
-            rec[r]["frequency_penalty"] = float(p.frequency_penalty or 0.0)
-            rec[r]["presence_penalty"] = float(p.presence_penalty or 0.0)
-            rec[r]["history_offset"] = off
-            n = 0
-            if p.has_penalties and histories is not None:
-                h = list(histories[r])[-PENALTY_HISTORY:]
-                n = len(h)
-                self._hist_np[off:off + n] = h
-                any_pen = any_pen or n > 0
-            rec[r]["history_len"] = n
-            off += n
+        if histories is not None and any(p.has_penalties for p in own):
+            for r, p in enumerate(params):
+                rec[r]["history_offset"] = off
+                if p.has_penalties:
+                    h = list(histories[r])[-PENALTY_HISTORY:]
+                    self._hist_np[off:off + len(h)] = h
+                    any_pen = any_pen or len(h) > 0
+                    rec[r]["history_len"] = len(h)
+                    off += len(h)
         nb = R * kernels.SAMPLE_PARAMS.itemsize
         self._params_dev[:nb].copy_(self._params_host[:nb], non_blocking=True)
         if any_pen:
