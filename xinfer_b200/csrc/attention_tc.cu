@@ -586,7 +586,7 @@ attn_decode_plan_kernel(int* __restrict__ plan, int capacity, const int* __restr
                         const int* __restrict__ req_of_token, const int* __restrict__ q_start, int num_entries, int window,
                         int keep, int dec_max, int direct, int num_small, int min_tiles, int target_ctas, int nkv, int* err) {
     __shared__ int warp_sums[PLAN_THREADS / 32];
-    __shared__ int piece_tiles[PLAN_SORT_MAX];
+    __shared__ int piece_tiles[PLAN_SORT_MAX], piece_of[PLAN_SORT_MAX];    // of a piece: its tiles, its token * PLAN_SORT_MAX + index
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto block_scan = [&](int mine, int& before_me) -> int {   // exclusive prefix of `mine` over the threads; returns the total
         int incl = mine;
@@ -606,34 +606,29 @@ attn_decode_plan_kernel(int* __restrict__ plan, int capacity, const int* __restr
         }
         return total;
     };
-    constexpr int EACH_MAX = PLAN_TOKENS_MAX / PLAN_THREADS;
-    const int each = (num_small + PLAN_THREADS - 1) / PLAN_THREADS;
-    int tiles[EACH_MAX], tok[EACH_MAX], sum = 0, unused;
-#pragma unroll
-    for (int i = 0; i < EACH_MAX; ++i) {
-        const int z = (int)threadIdx.x * each + i;
-        tiles[i] = 0;
-        tok[i] = -1;
-        if (i < each && z < num_small) {
-            const int t = small_token(z, q_start, num_entries, dec_max, direct);
-            if (t >= 0 && req_of_token[t] >= 0) {
-                const int pos = positions[t];
-                const int lo = first_visible(pos, window);
-                tiles[i] = kept_tiles(keep, lo, KT) + pos / KT - lo / KT + 1;
-                tok[i] = t;
-            }
-        }
-        sum += tiles[i];
-    }
+    // Every thread takes `each` tokens in a row (one, in most steps).  The loops over them are not unrolled and a token's
+    // figures are formed again where they are needed, from the cache: the kernel runs once per step, so its time is that
+    // of fetching its code (14.6 -> 4.6 us at the start of a step with the short code).
+    const int each = (num_small + PLAN_THREADS - 1) / PLAN_THREADS, z0 = (int)threadIdx.x * each;
+    auto token_of = [&](int z, int& t, int& pos, int& lo) -> int {      // tiles of the z-th small token (0: none)
+        if (z >= num_small) return 0;
+        t = small_token(z, q_start, num_entries, dec_max, direct);
+        if (t < 0 || req_of_token[t] < 0) return 0;
+        pos = positions[t];
+        lo = first_visible(pos, window);
+        return kept_tiles(keep, lo, KT) + pos / KT - lo / KT + 1;
+    };
+    int sum = 0, unused, t, pos, lo;
+#pragma unroll 1
+    for (int i = 0; i < each; ++i) sum += token_of(z0 + i, t, pos, lo);
     const long long all_tiles = (long long)block_scan(sum, unused) * nkv;
-    // the share as an int (a larger one would cut nothing anyway), so that the divisions below are short ones:
-    // every thread of the block goes through them, most with nothing to divide
+    // the share as an int (a larger one would cut nothing anyway), so that the divisions below are short ones
     const int share = (int)max((long long)min_tiles, min((all_tiles + target_ctas - 1) / target_ctas, (long long)INT_MAX));
     int pieces = 0, at;
-#pragma unroll
-    for (int i = 0; i < EACH_MAX; ++i) {
-        if (tiles[i] == 0) continue;
-        pieces += max(1, tiles[i] / share);
+#pragma unroll 1
+    for (int i = 0; i < each; ++i) {
+        const int n = token_of(z0 + i, t, pos, lo);
+        if (n) pieces += max(1, n / share);
     }
     const int total = block_scan(pieces, at);
     if (threadIdx.x == 0) {
@@ -641,44 +636,46 @@ attn_decode_plan_kernel(int* __restrict__ plan, int capacity, const int* __restr
         if (total > capacity) atomicOr(err, XB_ERR_BAD_ROW);   // the plan was sized for fewer pieces
     }
     if (total > capacity) return;
-    // CTAs start in the order of the plan: the longest pieces first, so that no long one is left for the end
+    auto write = [&](int where, int z, int n, int j, int t, int pos, int lo) {
+        const int cz = max(1, n / share), sz = (n + cz - 1) / cz, ns = (n + sz - 1) / sz;   // tiles per piece; pieces that hold any
+        int* e = plan + PLAN_HEADER + (size_t)where * PLAN_ENTRY;
+        e[0] = t;
+        e[1] = req_of_token[t];
+        e[2] = pos;
+        e[3] = lo;
+        e[4] = j * sz;
+        e[5] = j * sz < n ? min(sz, n - j * sz) : 0;   // an empty piece (rounding): its CTA leaves
+        e[6] = (ns << 16) | j;
+        e[7] = z;
+    };
+    // CTAs start in the order of the plan: the longest pieces first, so that no long one is left for the end.  The pieces are
+    // placed by as many threads as there are pieces, whoever's token they belong to.
     const bool sorted = total <= PLAN_SORT_MAX;
-    if (sorted) {
-        int a = at;
-#pragma unroll
-        for (int i = 0; i < EACH_MAX; ++i) {
-            if (!tiles[i]) continue;
-            const int n = tiles[i], cz = max(1, n / share), sz = (n + cz - 1) / cz;
-            for (int j = 0; j < cz; ++j, ++a) piece_tiles[a] = j * sz < n ? min(sz, n - j * sz) : 0;
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < EACH_MAX; ++i) {
-        if (!tiles[i]) continue;
-        const int z = (int)threadIdx.x * each + i, t = tok[i], n = tiles[i];
-        const int cz = max(1, n / share);
-        const int sz = (n + cz - 1) / cz, ns = (n + sz - 1) / sz;   // tiles per piece; pieces that hold any
-        const int pos = positions[t];
-        const int lo = first_visible(pos, window);
+#pragma unroll 1
+    for (int i = 0; i < each; ++i) {
+        const int n = token_of(z0 + i, t, pos, lo);
+        if (!n) continue;
+        const int cz = max(1, n / share), sz = (n + cz - 1) / cz;
+#pragma unroll 1
         for (int j = 0; j < cz; ++j, ++at) {
-            int where = at;
-            if (sorted) {   // as many pieces are longer (or as long and earlier) as this one's place says
-                const int mine = piece_tiles[at];
-                where = 0;
-                for (int o = 0; o < total; ++o) where += (piece_tiles[o] > mine || (piece_tiles[o] == mine && o < at)) ? 1 : 0;
+            if (sorted) {
+                piece_tiles[at] = j * sz < n ? min(sz, n - j * sz) : 0;
+                piece_of[at] = (z0 + i) * PLAN_SORT_MAX + j;
+            } else {
+                write(at, z0 + i, n, j, t, pos, lo);
             }
-            int* e = plan + PLAN_HEADER + (size_t)where * PLAN_ENTRY;
-            const int i0 = j * sz;
-            e[0] = t;
-            e[1] = req_of_token[t];
-            e[2] = pos;
-            e[3] = lo;
-            e[4] = i0;
-            e[5] = i0 < n ? min(sz, n - i0) : 0;   // an empty piece (rounding): its CTA leaves
-            e[6] = (ns << 16) | j;
-            e[7] = z;
         }
+    }
+    if (!sorted) return;
+    __syncthreads();
+    for (int p = (int)threadIdx.x; p < total; p += PLAN_THREADS) {
+        // as many pieces are longer (or as long and earlier) as this one's place says
+        const int mine = piece_tiles[p], z = piece_of[p] / PLAN_SORT_MAX;
+        int where = 0;
+#pragma unroll 4
+        for (int o = 0; o < total; ++o) where += (piece_tiles[o] > mine || (piece_tiles[o] == mine && o < p)) ? 1 : 0;
+        const int n = token_of(z, t, pos, lo);
+        write(where, z, n, piece_of[p] % PLAN_SORT_MAX, t, pos, lo);
     }
 }
 
