@@ -1421,11 +1421,17 @@ def selective_scan(y, xbc, proj, dt_off, dt_bias, a_log, d_skip, state, q_start,
                                         _stream()), "selective_scan")
 
 
+def delta_scratch_floats(tokens: int, entries: int, heads: int, d: int) -> int:
+    """Elements of scratch that ``delta_rule`` needs for a step."""
+    return int(kernels_lib().xb_delta_prep_floats(int(tokens), int(entries), int(heads), int(d)))
+
+
 def delta_rule(o, qkv, proj, beta_off, ag, dt_bias, a_log, state, q_start, slots, num_entries, heads, kv_heads, d, dv,
-               unit_eps: float = 1e-6):
+               unit_eps: float = 1e-6, scratch=None):
     """The gated delta rule per (request, head): ``qkv`` float32 rows ``[q | k | v]`` (q and k per key head), beta =
     sigmoid(proj[:, beta_off + h]), decay per (head, key channel) from the front of ``ag`` rows; ``state``
-    ``[slots, heads, d, dv]``; ``o`` ``[T, heads * dv]`` before its norm and gate."""
+    ``[slots, heads, d, dv]``; ``o`` ``[T, heads * dv]`` before its norm and gate.  ``scratch``: float32, at least
+    ``delta_scratch_floats`` elements (default: made here)."""
     T = qkv.shape[0]
     _need(qkv, "qkv", torch.float32, (T, 2 * kv_heads * d + heads * dv))
     _need(proj, "proj", torch.float32, (T, None))
@@ -1434,10 +1440,15 @@ def delta_rule(o, qkv, proj, beta_off, ag, dt_bias, a_log, state, q_start, slots
     _need(dt_bias, "dt_bias", torch.float32, (heads * d,))
     _need(a_log, "a_log", torch.float32, (heads,))
     _need(state, "state", torch.float32, (None, heads, d, dv))
+    if scratch is None:
+        scratch = torch.empty(delta_scratch_floats(T, num_entries, heads, d), dtype=torch.float32, device=o.device)
+    _need(scratch, "scratch", torch.float32)
+    if scratch.numel() < delta_scratch_floats(T, num_entries, heads, d):
+        raise KernelError("the scratch of the delta rule is too small for the step")
     _ok(kernels_lib().xb_delta_rule(o.data_ptr(), qkv.data_ptr(), qkv.shape[1], proj.data_ptr(), proj.shape[1], int(beta_off),
                                     ag.data_ptr(), ag.shape[1], dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(),
-                                    q_start.data_ptr(), slots.data_ptr(), int(num_entries), heads, kv_heads, d, dv,
-                                    float(unit_eps), _stream()), "delta_rule")
+                                    q_start.data_ptr(), slots.data_ptr(), int(num_entries), T, heads, kv_heads, d, dv,
+                                    float(unit_eps), scratch.data_ptr(), _stream()), "delta_rule", 2)
 
 
 def linear_scan(o, proj, alpha, state, q_start, slots, num_entries, heads, d, dv, scale: float):
