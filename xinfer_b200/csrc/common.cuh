@@ -146,3 +146,17 @@ template <typename... KArgs, typename... Args>
 static inline int xb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     return xb_launch_opt(true, kernel, grid, block, smem, stream, args...);
 }
+// For the small kernels between the large ones: overlapped with their neighbours while the grid is no more than one block per
+// processor, as in decode steps, whose launches then hide each other's start-up.  In a prompt a kernel that starts early finds
+// its neighbour's blocks on most processors and crowds its own onto the others.  Such a kernel begins with pdl_overlap_few().
+constexpr unsigned long long XB_FEW_BLOCKS = 148;
+constexpr int XB_FEW_TOKENS = 8;            // a kernel that walks a request's tokens lets its successor start at this many or fewer
+__device__ __forceinline__ void pdl_overlap_few() {
+    if ((unsigned long long)gridDim.x * gridDim.y * gridDim.z <= XB_FEW_BLOCKS) pdl_launch_dependents();
+    pdl_wait();
+}
+template <typename... KArgs, typename... Args>
+static inline int xb_launch_few(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    const bool few = (unsigned long long)grid.x * grid.y * grid.z <= XB_FEW_BLOCKS;
+    return xb_launch_opt(few, kernel, grid, block, smem, stream, args...);
+}

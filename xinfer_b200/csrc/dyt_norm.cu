@@ -19,6 +19,7 @@ __global__ void dyt_kernel(TO* __restrict__ out, TX* sum_out, const TX* x, const
                            const float* __restrict__ b, float branch_scale, const float* __restrict__ b_alpha,
                            const float* __restrict__ b_w, const float* __restrict__ b_b, int nrows, int dim, int src_rows,
                            int* err) {
+    pdl_overlap_few();
     const float a = out ? alpha[0] : 0.f;
     const float ba = b_alpha ? b_alpha[0] : 0.f;
     for (int r = blockIdx.y; r < nrows; r += gridDim.y) {
@@ -49,7 +50,7 @@ static int dyt_launch(void* out, void* sum_out, const void* x, const void* branc
     const int threads = dim >= 1024 ? 256 : 128;
     int bx = (dim + threads * 4 - 1) / (threads * 4);
     if (bx < 1) bx = 1;
-    dyt_kernel<TX, TB, TO><<<dim3(bx, nrows < 65535 ? nrows : 65535), threads, 0, stream>>>((TO*)out, (TX*)sum_out, (const TX*)x, (const TB*)branch, rows,
+    xb_launch_few(dyt_kernel<TX, TB, TO>, dim3(dim3(bx, nrows < 65535 ? nrows : 65535)), dim3(threads), 0, stream, (TO*)out, (TX*)sum_out, (const TX*)x, (const TB*)branch, rows,
                                                                      alpha, w, b, branch_scale, b_alpha, b_w, b_b, nrows, dim,
                                                                      src_rows, err);
     return xb_launch_status();

@@ -44,6 +44,7 @@ expert_router_kernel(int* __restrict__ choice, float* __restrict__ weight, const
                      const int* __restrict__ req_of_token, float* __restrict__ gate, int tokens, int E, int K, int top,
                      int groups, int keep, int group_best, int softmax, int renorm, float renorm_eps, float weight_scale,
                      int vec4) {
+    pdl_overlap_few();
     extern __shared__ float sm[];
     const int rows = E + (gate != nullptr ? 1 : 0);      // rows of the matrix: the experts, then the gate's
     float* s_all = sm;                                   // [tokens of the block][rows] logits, then scores
@@ -215,7 +216,7 @@ XB_EXPORT int xb_expert_router(int dtype, int* choice, float* weight, const void
     const int rows = experts + (gate != nullptr ? 1 : 0);
     const int threads = 32 * (rows <= 8 ? 4 : (rows >= 2 * ROUTER_MAX_WARPS ? ROUTER_MAX_WARPS : (rows + 1) / 2));
 #define XB_ROUTER(T, N)                                                                                                   \
-    expert_router_kernel<T, N><<<blocks, threads, smem, stream>>>(choice, weight, (const T*)h, w_r, correction,    \
+    xb_launch_few(expert_router_kernel<T, N>, dim3(blocks), dim3(threads), smem, stream, choice, weight, (const T*)h, w_r, correction,    \
                                                                          req_of_token, gate, tokens, experts, K, top,     \
                                                                          groups, keep, group_best, softmax, renorm,       \
                                                                          renorm_eps, weight_scale, vec4)

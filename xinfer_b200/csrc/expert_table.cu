@@ -218,6 +218,7 @@ __global__ void expert_select_gate_kernel(T* __restrict__ act, const T* __restri
                                           const int* __restrict__ req_of_token, int top, int E, int F, int F_dense, int vocab,
                                           float weight, const float* __restrict__ weights,
                                           const float* __restrict__ dense_weight, int code, float p0, float p1, int* err) {
+    pdl_overlap_few();
     const int t = blockIdx.x, e = blockIdx.y;
     const T* gu_row = gu + (size_t)t * 2 * ((size_t)E * F + F_dense);
     T* act_row = act + (size_t)t * ((size_t)E * F + F_dense);
@@ -260,11 +261,11 @@ XB_EXPORT int xb_expert_select_gate(int dtype, void* act, const void* gu, const 
     const dim3 grid(tokens, experts + (F_dense > 0 ? 1 : 0));
     const float weight = 1.f / (float)top;
     if (dtype == XB_F32)
-        expert_select_gate_kernel<float><<<grid, 256, 0, stream>>>((float*)act, (const float*)gu, table, ids, sampled, num_sampled,
+        xb_launch_few(expert_select_gate_kernel<float>, dim3(grid), dim3(256), 0, stream, (float*)act, (const float*)gu, table, ids, sampled, num_sampled,
                                                                    req_of_token, top, experts, F, F_dense, vocab, weight,
                                                                    weights, dense_weight, code, p0, p1, err);
     else
-        expert_select_gate_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>((__nv_bfloat16*)act, (const __nv_bfloat16*)gu, table, ids,
+        xb_launch_few(expert_select_gate_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, (__nv_bfloat16*)act, (const __nv_bfloat16*)gu, table, ids,
                                                                            sampled, num_sampled, req_of_token, top, experts, F,
                                                                            F_dense, vocab, weight, weights, dense_weight, code,
                                                                            p0, p1, err);

@@ -32,6 +32,7 @@ __global__ void latent_prepare_kernel(T* q_abs, long long q_ts, long long q_hs, 
                                       int table_stride, int nh, int d, int rd, int rank, int rot, int page_size,
                                       int num_pages, float eps, float rot_mag, int pairs, int tail, T* __restrict__ cq,
                                       int cq_off, int n_cq, const float* __restrict__ cq_w, int* err) {
+    pdl_overlap_few();
     extern __shared__ float sm[];
     __shared__ float scratch[33];
     if (blockIdx.y == 1) {
@@ -144,7 +145,7 @@ XB_EXPORT int xb_latent_prepare(int dtype, void* q_abs, void* cache, const void*
     // sum), so many resident blocks hide more than many threads per block
     const int threads = work >= 16384 ? 256 : 128;
 #define XB_GO(T)                                                                                                        \
-    latent_prepare_kernel<T><<<dim3(tokens, cq != nullptr ? 2 : 1), threads, smem, stream>>>((T*)q_abs, q_ts, q_hs, q_rot, (T*)cache, (const T*)proj, row_len, q_off,  \
+    xb_launch_few(latent_prepare_kernel<T>, dim3(dim3(tokens, cq != nullptr ? 2 : 1)), dim3(threads), smem, stream, (T*)q_abs, q_ts, q_hs, q_rot, (T*)cache, (const T*)proj, row_len, q_off,  \
         kv_off, (const T*)q_lat, ql_ts, ql_hs, norm_w, inv_freq, positions, req_of_token, block_table, table_stride,   \
         nh, d, rd, rank, rot, page_size, num_pages, eps, rot_mag, pairs, tail, (T*)cq, cq_off, n_cq, cq_w, err)
     const int pairs = (dtype == XB_BF16 && !((row_len | q_off | d | rd | rank | tail) & 1) &&
@@ -177,6 +178,7 @@ __global__ void gate_sigmoid_kernel(T* out, const T* heads, long long h_ts, long
 __global__ void gate_sigmoid_bf16x8_kernel(__nv_bfloat16* out, const __nv_bfloat16* heads, long long h_ts,
                                            long long h_hs, const __nv_bfloat16* __restrict__ gate, long long g_ts, int nh,
                                            int dv, int tokens, int per_head) {
+    pdl_overlap_few();
     const int w = nh * dv;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (c >= w) return;
@@ -213,7 +215,7 @@ XB_EXPORT int xb_gate_sigmoid(int dtype, void* out, const void* heads, long long
         const int vecs = nh * dv / 8;
         const int threads = vecs >= 256 ? 256 : 64;
         const dim3 grid((unsigned)((vecs + threads - 1) / threads), (unsigned)(tokens < 65535 ? tokens : 65535));
-        gate_sigmoid_bf16x8_kernel<<<grid, threads, 0, stream>>>(
+        xb_launch_few(gate_sigmoid_bf16x8_kernel, dim3(grid), dim3(threads), 0, stream, 
             (__nv_bfloat16*)out, (const __nv_bfloat16*)heads, h_ts, h_hs, (const __nv_bfloat16*)gate, g_ts, nh, dv, tokens, per_head);
         return xb_launch_status();
     }

@@ -60,6 +60,7 @@ template <int MAXNT /* 8-column value tiles per warp */, int CW /* warps of a ro
 __global__ void __launch_bounds__(64 * CW) attn_latent_mma_kernel(__nv_bfloat16* __restrict__ out,
                                                               const __nv_bfloat16* __restrict__ q,
                                                               const __nv_bfloat16* __restrict__ cache, LatentMmaArgs a) {
+    pdl_overlap_few();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_entry, s_tile;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -365,6 +366,7 @@ __global__ void __launch_bounds__(64 * CW) attn_latent_mma_kernel(__nv_bfloat16*
 // out[row] = sum_p part_o[row, p] 2^(m_p - M) / sum_p l_p 2^(m_p - M),  M = max_p m_p  (maxima in the base-2 domain)
 __global__ void attn_latent_merge_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ part_o,
                                          const float* __restrict__ part_ml, int parts, int rank) {
+    pdl_overlap_few();
     const size_t row = blockIdx.x;
     float M = -INFINITY;
     for (int p = 0; p < parts; ++p) M = fmaxf(M, part_ml[(row * parts + p) * 2]);
@@ -420,7 +422,7 @@ XB_EXPORT int xb_attn_latent_mma(void* out, const void* q, const void* cache, co
 #define XB_GO(N, C)                                                                                                  \
     do {                                                                                                             \
         cudaFuncSetAttribute(attn_latent_mma_kernel<N, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-        attn_latent_mma_kernel<N, C><<<grid, block, smem, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)q,    \
+        xb_launch_few(attn_latent_mma_kernel<N, C>, dim3(grid), dim3(block), smem, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)q,    \
                                                                     (const __nv_bfloat16*)cache, a);                 \
     } while (0)
     if (cw == 8) {
@@ -434,6 +436,6 @@ XB_EXPORT int xb_attn_latent_mma(void* out, const void* q, const void* cache, co
 #undef XB_GO
     int rc = xb_launch_status();
     if (rc != 0 || parts == 1) return rc;
-    attn_latent_merge_kernel<<<(unsigned)((long long)tokens * nh), 128, 0, stream>>>((__nv_bfloat16*)out, part_o, part_ml, parts, rank);
+    xb_launch_few(attn_latent_merge_kernel, dim3((unsigned)((long long)tokens * nh)), dim3(128), 0, stream, (__nv_bfloat16*)out, part_o, part_ml, parts, rank);
     return xb_launch_status();
 }

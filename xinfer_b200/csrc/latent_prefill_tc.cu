@@ -59,6 +59,7 @@ __global__ void latent_gather_kernel(uint4* __restrict__ out, const uint4* __res
                                      int rows, const int* __restrict__ q_start, const int* __restrict__ start_pos,
                                      const int* __restrict__ table, int table_stride, int page_size, int num_pages, int window,
                                      int pieces, int* err) {
+    pdl_overlap_few();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     const int b = blocks[2 * (row >> 6)], j = blocks[2 * (row >> 6) + 1] + (row & 63);
@@ -433,7 +434,7 @@ XB_EXPORT int xb_latent_gather(void* out, const void* pages, const int* blocks, 
                                int window, int width, int* err, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (width % 8 || rows % 64 || page_size <= 0 || window < 0) return (int)cudaErrorInvalidValue;
-    latent_gather_kernel<<<(rows + 7) / 8, 256, 0, stream>>>((uint4*)out, (const uint4*)pages, blocks, rows, q_start, start_pos,
+    xb_launch_few(latent_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, (uint4*)out, (const uint4*)pages, blocks, rows, q_start, start_pos,
                                                              table, table_stride, page_size, num_pages, window, width / 8, err);
     return xb_launch_status();
 }

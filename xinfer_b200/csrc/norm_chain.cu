@@ -15,6 +15,7 @@ __global__ void rms_chain_kernel(TO* __restrict__ out, float* sum_out, const flo
                                  const int* __restrict__ rows, const float* __restrict__ w, const float* __restrict__ bw,
                                  const float* __restrict__ gain, int dim, int src_rows, float eps, float offset, float beps,
                                  float boffset, float bscale, int* err) {
+    pdl_overlap_few();
     __shared__ float scratch[33];
     extern __shared__ float srow[];
     const int r = blockIdx.x;
@@ -65,7 +66,7 @@ static int rms_chain_launch(void* out, float* sum_out, const float* x, const voi
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
     if (smem > 48 * 1024) cudaFuncSetAttribute(rms_chain_kernel<TB, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int threads = dim >= 2048 ? 512 : (dim >= 512 ? 256 : 128);
-    rms_chain_kernel<TB, TO><<<nrows, threads, smem, stream>>>((TO*)out, sum_out, x, (const TB*)branch, rows, w, bw, gain, dim,
+    xb_launch_few(rms_chain_kernel<TB, TO>, dim3(nrows), dim3(threads), smem, stream, (TO*)out, sum_out, x, (const TB*)branch, rows, w, bw, gain, dim,
                                                               src_rows, eps, offset, beps, boffset, bscale, err);
     return xb_launch_status();
 }
@@ -87,6 +88,7 @@ template <typename T>
 __global__ void dual_rms_sum_kernel(T* __restrict__ out, const T* __restrict__ l, const T* __restrict__ r,
                                     const float* __restrict__ wl, const float* __restrict__ wr, int dim, float eps,
                                     float offset, float sl, float sr) {
+    pdl_overlap_few();
     __shared__ float scratch[33];
     const size_t base = (size_t)blockIdx.x * dim;
     float a = 0.f, b = 0.f;
@@ -109,9 +111,9 @@ XB_EXPORT int xb_dual_rms_sum(int dtype, void* out, const void* l, const void* r
     if (rows <= 0) return 0;
     const int threads = dim >= 2048 ? 512 : (dim >= 512 ? 256 : 128);
     if (dtype == XB_F32)
-        dual_rms_sum_kernel<float><<<rows, threads, 0, stream>>>((float*)out, (const float*)l, (const float*)r, wl, wr, dim, eps, offset, sl, sr);
+        xb_launch_few(dual_rms_sum_kernel<float>, dim3(rows), dim3(threads), 0, stream, (float*)out, (const float*)l, (const float*)r, wl, wr, dim, eps, offset, sl, sr);
     else
-        dual_rms_sum_kernel<__nv_bfloat16><<<rows, threads, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)l,
+        xb_launch_few(dual_rms_sum_kernel<__nv_bfloat16>, dim3(rows), dim3(threads), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)l,
                                                                         (const __nv_bfloat16*)r, wl, wr, dim, eps, offset, sl, sr);
     return xb_launch_status();
 }
@@ -119,6 +121,7 @@ XB_EXPORT int xb_dual_rms_sum(int dtype, void* out, const void* l, const void* r
 // x[t, i] += bias[i]
 template <typename T>
 __global__ void add_bias_kernel(T* x, const float* __restrict__ bias, size_t n, int dim) {
+    pdl_overlap_few();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = from_f32<T>(to_f32<T>(x[i]) + bias[i % dim]);
 }
@@ -128,9 +131,9 @@ XB_EXPORT int xb_add_bias(int dtype, void* x, const float* bias, int rows, int d
     if (n == 0) return 0;
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (dtype == XB_F32)
-        add_bias_kernel<float><<<blocks, 256, 0, stream>>>((float*)x, bias, n, dim);
+        xb_launch_few(add_bias_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)x, bias, n, dim);
     else
-        add_bias_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)x, bias, n, dim);
+        xb_launch_few(add_bias_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)x, bias, n, dim);
     return xb_launch_status();
 }
 
@@ -138,6 +141,7 @@ XB_EXPORT int xb_add_bias(int dtype, void* x, const float* bias, int rows, int d
 template <typename TI, typename TO, int ACT>
 __global__ void swiglu_bias_kernel(TO* __restrict__ out, const TI* __restrict__ gu, const float* __restrict__ bias, int I,
                                    size_t n) {
+    pdl_overlap_few();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const size_t t = i / I;
@@ -152,9 +156,9 @@ static int swiglu_bias_launch(void* out, const void* gu, const float* bias, int 
     const size_t n = (size_t)rows * I;
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (act == XB_ACT_GELU_TANH)
-        swiglu_bias_kernel<TI, TO, XB_ACT_GELU_TANH><<<blocks, 256, 0, stream>>>((TO*)out, (const TI*)gu, bias, I, n);
+        xb_launch_few(swiglu_bias_kernel<TI, TO, XB_ACT_GELU_TANH>, dim3(blocks), dim3(256), 0, stream, (TO*)out, (const TI*)gu, bias, I, n);
     else
-        swiglu_bias_kernel<TI, TO, XB_ACT_SILU><<<blocks, 256, 0, stream>>>((TO*)out, (const TI*)gu, bias, I, n);
+        xb_launch_few(swiglu_bias_kernel<TI, TO, XB_ACT_SILU>, dim3(blocks), dim3(256), 0, stream, (TO*)out, (const TI*)gu, bias, I, n);
     return xb_launch_status();
 }
 

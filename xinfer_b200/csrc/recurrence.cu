@@ -32,6 +32,7 @@ __global__ void gated_scan_serial_kernel(T* __restrict__ y, int ldy, const float
                                          const float* __restrict__ bz, const float* __restrict__ bx,
                                          float* __restrict__ state, const int* __restrict__ q_start,
                                          const int* __restrict__ slots, int W, float out_scale) {
+    pdl_overlap_few();
     const int b = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int slot = slots[b];
@@ -62,6 +63,7 @@ constexpr int GS_CH = 32;
 __global__ void gated_scan_chunk_kernel(float* __restrict__ prodA, float* __restrict__ endB,
                                         const float* __restrict__ zxg, const float* __restrict__ bz,
                                         const float* __restrict__ bx, const int* __restrict__ req_of_token, int T, int W) {
+    pdl_overlap_few();
     const int k = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= W) return;
@@ -88,6 +90,7 @@ __global__ void gated_scan_chunk_kernel(float* __restrict__ prodA, float* __rest
 __global__ void gated_scan_starts_kernel(float* __restrict__ start, const float* __restrict__ prodA,
                                          const float* __restrict__ endB, float* __restrict__ state,
                                          const int* __restrict__ q_start, const int* __restrict__ slots, int W) {
+    pdl_overlap_few();
     const int b = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int slot = slots[b];
@@ -129,6 +132,7 @@ __global__ void gated_scan_finish_kernel(T* __restrict__ y, int ldy, const float
                                          const float* __restrict__ start, const float* __restrict__ prodA,
                                          const float* __restrict__ endB, const int* __restrict__ req_of_token,
                                          const int* __restrict__ q_start, int tokens, int W, float out_scale) {
+    pdl_overlap_few();
     const int t = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= W || t >= tokens) return;
@@ -152,25 +156,25 @@ XB_EXPORT int xb_gated_scan(int out_dtype, void* y, int ldy, const float* zxg, c
     if (!chunked || scratch == nullptr) {
         const dim3 grid(cx, num_entries);
         if (out_dtype == XB_F32)
-            gated_scan_serial_kernel<float><<<grid, threads, 0, stream>>>((float*)y, ldy, zxg, bz, bx, state, q_start, slots, W, out_scale);
+            xb_launch_few(gated_scan_serial_kernel<float>, dim3(grid), dim3(threads), 0, stream, (float*)y, ldy, zxg, bz, bx, state, q_start, slots, W, out_scale);
         else
-            gated_scan_serial_kernel<bf><<<grid, threads, 0, stream>>>((bf*)y, ldy, zxg, bz, bx, state, q_start, slots, W, out_scale);
+            xb_launch_few(gated_scan_serial_kernel<bf>, dim3(grid), dim3(threads), 0, stream, (bf*)y, ldy, zxg, bz, bx, state, q_start, slots, W, out_scale);
         return xb_launch_status();
     }
     float* prodA = scratch;
     float* endB = scratch + (size_t)tokens * W;
     float* start = scratch + 2 * (size_t)tokens * W;
     const int chunks = (tokens + GS_CH - 1) / GS_CH;
-    gated_scan_chunk_kernel<<<dim3(cx, chunks), threads, 0, stream>>>(prodA, endB, zxg, bz, bx, req_of_token, tokens, W);
+    xb_launch_few(gated_scan_chunk_kernel, dim3(dim3(cx, chunks)), dim3(threads), 0, stream, prodA, endB, zxg, bz, bx, req_of_token, tokens, W);
     int rc = xb_launch_status();
     if (rc) return rc;
-    gated_scan_starts_kernel<<<dim3(cx, num_entries), threads, 0, stream>>>(start, prodA, endB, state, q_start, slots, W);
+    xb_launch_few(gated_scan_starts_kernel, dim3(dim3(cx, num_entries)), dim3(threads), 0, stream, start, prodA, endB, state, q_start, slots, W);
     rc = xb_launch_status();
     if (rc) return rc;
     if (out_dtype == XB_F32)
-        gated_scan_finish_kernel<float><<<dim3(cx, tokens), threads, 0, stream>>>((float*)y, ldy, zxg, start, prodA, endB, req_of_token, q_start, tokens, W, out_scale);
+        xb_launch_few(gated_scan_finish_kernel<float>, dim3(dim3(cx, tokens)), dim3(threads), 0, stream, (float*)y, ldy, zxg, start, prodA, endB, req_of_token, q_start, tokens, W, out_scale);
     else
-        gated_scan_finish_kernel<bf><<<dim3(cx, tokens), threads, 0, stream>>>((bf*)y, ldy, zxg, start, prodA, endB, req_of_token, q_start, tokens, W, out_scale);
+        xb_launch_few(gated_scan_finish_kernel<bf>, dim3(dim3(cx, tokens)), dim3(threads), 0, stream, (bf*)y, ldy, zxg, start, prodA, endB, req_of_token, q_start, tokens, W, out_scale);
     return xb_launch_status();
 }
 
@@ -194,6 +198,7 @@ __device__ __forceinline__ void block_sum3(float& a, float& b, float& c, float* 
 template <typename T, int PER>
 __global__ void polynorm_kernel(T* __restrict__ out, const float* __restrict__ z, const float* __restrict__ coef, int F,
                                 float eps) {
+    pdl_overlap_few();
     __shared__ float scratch[96];
     const float* zr = z + (size_t)blockIdx.x * F;
     float v[PER];
@@ -248,9 +253,9 @@ __global__ void polynorm_long_kernel(T* __restrict__ out, const float* __restric
 
 template <typename T>
 static int polynorm_launch(void* out, const float* z, const float* coef, int rows, int F, float eps, cudaStream_t stream) {
-    if (F <= 4 * 256) polynorm_kernel<T, 4><<<rows, (F + 3) / 4 < 32 ? 32 : ((F + 3) / 4 + 31) / 32 * 32, 0, stream>>>((T*)out, z, coef, F, eps);
-    else if (F <= 8 * 512) polynorm_kernel<T, 8><<<rows, ((F + 7) / 8 + 31) / 32 * 32, 0, stream>>>((T*)out, z, coef, F, eps);
-    else if (F <= 16 * 1024) polynorm_kernel<T, 16><<<rows, ((F + 15) / 16 + 31) / 32 * 32, 0, stream>>>((T*)out, z, coef, F, eps);
+    if (F <= 4 * 256) xb_launch_few(polynorm_kernel<T, 4>, dim3(rows), dim3((F + 3) / 4 < 32 ? 32 : ((F + 3) / 4 + 31) / 32 * 32), 0, stream, (T*)out, z, coef, F, eps);
+    else if (F <= 8 * 512) xb_launch_few(polynorm_kernel<T, 8>, dim3(rows), dim3(((F + 7) / 8 + 31) / 32 * 32), 0, stream, (T*)out, z, coef, F, eps);
+    else if (F <= 16 * 1024) xb_launch_few(polynorm_kernel<T, 16>, dim3(rows), dim3(((F + 15) / 16 + 31) / 32 * 32), 0, stream, (T*)out, z, coef, F, eps);
     else polynorm_long_kernel<T><<<rows, 1024, 0, stream>>>((T*)out, z, coef, F, eps);
     return xb_launch_status();
 }

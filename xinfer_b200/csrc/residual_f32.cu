@@ -40,6 +40,7 @@ template <typename TB, typename TO>
 __global__ void rmsnorm_f32_kernel(TO* __restrict__ out, float* sum_out, const float* x, const TB* __restrict__ branch,
                                    const int* __restrict__ rows, const float* __restrict__ w, int dim, int src_rows,
                                    float eps, float offset, int* err) {
+    pdl_overlap_few();
     __shared__ float scratch[33];
     extern __shared__ float srow[];
     const int r = blockIdx.x;
@@ -75,7 +76,7 @@ static int rmsnorm_f32_launch(void* out, float* sum_out, const float* x, const v
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
     if (smem > 48 * 1024) cudaFuncSetAttribute(rmsnorm_f32_kernel<TB, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int threads = dim >= 2048 ? 512 : (dim >= 512 ? 256 : 128);
-    rmsnorm_f32_kernel<TB, TO><<<nrows, threads, smem, stream>>>((TO*)out, sum_out, x, (const TB*)branch, rows, w, dim, src_rows,
+    xb_launch_few(rmsnorm_f32_kernel<TB, TO>, dim3(nrows), dim3(threads), smem, stream, (TO*)out, sum_out, x, (const TB*)branch, rows, w, dim, src_rows,
                                                                 eps, offset, err);
     return xb_launch_status();
 }
@@ -93,6 +94,7 @@ XB_EXPORT int xb_rmsnorm_f32(int branch_dtype, int out_dtype, void* out, float* 
 
 template <typename TB>
 __global__ void add_f32_kernel(float* out, const float* x, const TB* branch, size_t n, float scale) {
+    pdl_overlap_few();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = scale == 1.f ? x[i] + to_f32<TB>(branch[i]) : fmaf(scale, to_f32<TB>(branch[i]), x[i]);
 }
@@ -101,8 +103,8 @@ XB_EXPORT int xb_add_f32(int branch_dtype, float* out, const float* x, const voi
     if (n <= 0) return 0;
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (branch_dtype == XB_F32)
-        add_f32_kernel<float><<<blocks, 256, 0, stream>>>(out, x, (const float*)branch, (size_t)n, scale);
+        xb_launch_few(add_f32_kernel<float>, dim3(blocks), dim3(256), 0, stream, out, x, (const float*)branch, (size_t)n, scale);
     else
-        add_f32_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(out, x, (const __nv_bfloat16*)branch, (size_t)n, scale);
+        xb_launch_few(add_f32_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, out, x, (const __nv_bfloat16*)branch, (size_t)n, scale);
     return xb_launch_status();
 }

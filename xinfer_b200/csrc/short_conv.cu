@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(128) conv_silu_run_kernel(TO* __restrict__ y, 
                                                             const int* __restrict__ req_of_token,
                                                             const int* __restrict__ q_start, const int* __restrict__ slots,
                                                             int C, int tokens, int run) {
+    pdl_overlap_few();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c >= C) return;
     float tap[K][V], b0[V], win[K > 1 ? K - 1 : 1][V];
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(128) conv_silu_run_kernel(TO* __restrict__ y, 
 template <typename T>
 __global__ void conv_state_kernel(T* __restrict__ state, const T* __restrict__ u, long long u_ld, int u_off,
                                   const int* __restrict__ q_start, const int* __restrict__ slots, int C, int K) {
+    pdl_overlap_few();
     const int b = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int slot = slots[b];
@@ -173,7 +175,7 @@ static int conv_silu_runs(TO* y, const float* u, long long u_ld, int u_off, cons
     const dim3 grid((tokens + run - 1) / run, cols);
 #define XB_CONV_K(KV)                                                                                                     \
     case KV:                                                                                                              \
-        conv_silu_run_kernel<TO, KV, V><<<grid, 128, 0, stream>>>(y, u, u_ld, u_off, taps, bias, state, req_of_token,    \
+        xb_launch_few(conv_silu_run_kernel<TO, KV, V>, dim3(grid), dim3(128), 0, stream, y, u, u_ld, u_off, taps, bias, state, req_of_token,    \
                                                                   q_start, slots, C, tokens, run);                       \
         return 1;
     switch (K) {
@@ -217,9 +219,9 @@ XB_EXPORT int xb_conv_state(int dtype, void* state, const void* u, long long u_l
     if (K > SC_MAX_TAPS) return (int)cudaErrorInvalidValue;
     const dim3 grid((C + 127) / 128, entries);
     if (dtype == XB_F32)
-        conv_state_kernel<float><<<grid, 128, 0, stream>>>((float*)state, (const float*)u, u_ld, u_off, q_start, slots, C, K);
+        xb_launch_few(conv_state_kernel<float>, dim3(grid), dim3(128), 0, stream, (float*)state, (const float*)u, u_ld, u_off, q_start, slots, C, K);
     else
-        conv_state_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>((__nv_bfloat16*)state, (const __nv_bfloat16*)u, u_ld, u_off,
+        xb_launch_few(conv_state_kernel<__nv_bfloat16>, dim3(grid), dim3(128), 0, stream, (__nv_bfloat16*)state, (const __nv_bfloat16*)u, u_ld, u_off,
                                                                    q_start, slots, C, K);
     return xb_launch_status();
 }

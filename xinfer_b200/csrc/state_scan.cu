@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(384, 1) selective_scan_kernel(float* __restric
                                                              float* __restrict__ state, const int* __restrict__ q_start,
                                                              const int* __restrict__ slots, int H, int P, int N, int G,
                                                              int TT, int stage, int cw, int vec) {
+    pdl_wait();
     extern __shared__ __align__(16) float scan_smem[];
     constexpr int CGW = 32 / DS, NP = DS * kRowsPad, NR = DS * kRows;
     const int b = blockIdx.x, h = blockIdx.y;
@@ -231,6 +232,7 @@ __global__ void __launch_bounds__(384, 1) selective_scan_kernel(float* __restric
     const int VT = cw * CGW * 2, c_base = blockIdx.z * VT;
     const int slot = slots[b];
     const int t0 = q_start[b], t1 = q_start[b + 1];
+    if (t1 - t0 <= XB_FEW_TOKENS) pdl_launch_dependents();
     if (slot < 0 || t1 <= t0) return;
     const int inner = H * P, g = h / (H / G);
     const int ntiles = (t1 - t0 + TT - 1) / TT;
@@ -374,6 +376,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(float* __restrict__ 
                                                             const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                                                             const int* __restrict__ q_start, int entries, int tokens, int H, int G,
                                                             int d, float unit_eps) {
+    pdl_overlap_few();
     const int lane = threadIdx.x & 31, h = blockIdx.y * 4 + (threadIdx.x >> 5);
     if (h >= H) return;
     int grp = blockIdx.x, b = 0, t = 0, n = 0;
@@ -504,6 +507,7 @@ __global__ void __launch_bounds__(384, 1) delta_rule_kernel(float* __restrict__ 
                                                          long long ldp, int beta_off, float* __restrict__ state,
                                                          const int* __restrict__ q_start, const int* __restrict__ slots, int tokens,
                                                          int H, int d, int dv, int TT, int stage, int cw, int vec) {
+    pdl_wait();
     extern __shared__ __align__(16) float scan_smem[];
     constexpr int CGW = 32 / DS, DP = DS * kRowsPad, NR = DS * kRows;
     const int b = blockIdx.x, h = blockIdx.y;
@@ -511,6 +515,7 @@ __global__ void __launch_bounds__(384, 1) delta_rule_kernel(float* __restrict__ 
     const int VT = cw * CGW * 2, c_base = blockIdx.z * VT;
     const int slot = slots[b];
     const int t0 = q_start[b], t1 = q_start[b + 1];
+    if (t1 - t0 <= XB_FEW_TOKENS) pdl_launch_dependents();
     if (slot < 0 || t1 <= t0) return;
     const int ntiles = (t1 - t0 + TT - 1) / TT;
     float* so = scan_smem + kStages * stage;
@@ -688,6 +693,7 @@ __global__ void __launch_bounds__(384, 1) linear_scan_kernel(float* __restrict__
                                                              float* __restrict__ state, const int* __restrict__ q_start,
                                                              const int* __restrict__ slots, int H, int d, int dv, float scale,
                                                              int TT, int stage, int cw, int vec) {
+    pdl_wait();
     extern __shared__ __align__(16) float scan_smem[];
     constexpr int CGW = 32 / DS, DP = DS * kRowsPad, NR = DS * kRows;
     const int b = blockIdx.x, h = blockIdx.y;
@@ -695,6 +701,7 @@ __global__ void __launch_bounds__(384, 1) linear_scan_kernel(float* __restrict__
     const int VT = cw * CGW * 2, c_base = blockIdx.z * VT;
     const int slot = slots[b];
     const int t0 = q_start[b], t1 = q_start[b + 1];
+    if (t1 - t0 <= XB_FEW_TOKENS) pdl_launch_dependents();
     if (slot < 0 || t1 <= t0) return;
     const int ntiles = (t1 - t0 + TT - 1) / TT;
     float* so = scan_smem + kStages * stage;
@@ -813,6 +820,7 @@ __global__ void __launch_bounds__(384, 1) matrix_memory_kernel(
     const float* __restrict__ bi, const float* __restrict__ bf, float cap, float* __restrict__ state_s,
     float* __restrict__ state_n, float* state_m, const int* __restrict__ q_start, const int* __restrict__ start_pos,
     const int* __restrict__ slots, int H, int d, int dv, float scale, float div_eps, int TT, int stage, int cw, int vec) {
+    pdl_wait();
     extern __shared__ __align__(16) float scan_smem[];
     constexpr int CGW = 32 / DS, DP = DS * kRowsPad, NR = DS * kRows;
     const int b = blockIdx.x, h = blockIdx.y;
@@ -820,6 +828,7 @@ __global__ void __launch_bounds__(384, 1) matrix_memory_kernel(
     const int VT = cw * CGW * 2, c_base = blockIdx.z * VT;
     const int slot = slots[b];
     const int t0 = q_start[b], t1 = q_start[b + 1];
+    if (t1 - t0 <= XB_FEW_TOKENS) pdl_launch_dependents();
     if (slot < 0 || t1 <= t0) return;
     const int ntiles = (t1 - t0 + TT - 1) / TT;
     float* so = scan_smem + kStages * stage;
@@ -1006,6 +1015,7 @@ __global__ void __launch_bounds__(kDecayChannels) low_rank_decay_kernel(float* _
                                                                         long long ldl, const float* __restrict__ w,
                                                                         const float* __restrict__ bias, int tokens, int C, int R,
                                                                         float inv_tau) {
+    pdl_overlap_few();
     __shared__ __align__(16) float sl[kDecayRanks][kDecayTokens];
     __shared__ float sw[kDecayRanks][kDecayChannels + 1];
     const int tb = blockIdx.x * kDecayTokens, nt = min(kDecayTokens, tokens - tb);
@@ -1097,7 +1107,7 @@ static inline int scan_smem_opt_in(K kernel, size_t bytes) {
     {                                                           \
         const int rc = scan_smem_opt_in(K, bytes);              \
         if (rc) return rc;                                      \
-        K<<<grid, threads, bytes, stream>>>(__VA_ARGS__);       \
+        xb_launch_few(K, dim3(grid), dim3(threads), bytes, stream, __VA_ARGS__); \
     }
 
 XB_EXPORT int xb_selective_scan(float* y, const float* xbc, int C, const float* proj, long long ldp, int dt_off,
@@ -1141,7 +1151,7 @@ XB_EXPORT int xb_delta_rule(float* o, const float* qkv, int Cq, const float* pro
     const bool fours = scan_aligned16(prep) && scan_aligned16(qkv) && scan_aligned16(ag) && scan_aligned16(dt_bias) && Cq % 4 == 0 &&
                        ldag % 4 == 0 && d % 4 == 0;
     const auto prepare = fours ? delta_prepare_kernel<4> : delta_prepare_kernel<1>;
-    prepare<<<dim3(tokens / 4 + entries, (H + 3) / 4), 128, 0, stream>>>(prep, qkv, Cq, ag, ldag, dt_bias, A_log, q_start, entries,
+    xb_launch_few(prepare, dim3(dim3(tokens / 4 + entries, (H + 3) / 4)), dim3(128), 0, stream, prep, qkv, Cq, ag, ldag, dt_bias, A_log, q_start, entries,
                                                                          tokens, H, G, d, unit_eps);
     const int rc0 = xb_launch_status();
     if (rc0) return rc0;
@@ -1197,7 +1207,7 @@ XB_EXPORT int xb_low_rank_decay(float* alpha, const float* low, long long ldl, c
     const int cols = (C + kDecayChannels - 1) / kDecayChannels;
     if (R < 1 || !(tau > 0.f) || cols > 65535) return (int)cudaErrorInvalidValue;
     const dim3 grid((tokens + kDecayTokens - 1) / kDecayTokens, cols);
-    low_rank_decay_kernel<<<grid, kDecayChannels, 0, stream>>>(alpha, low, ldl, w, bias, tokens, C, R, 1.f / tau);
+    xb_launch_few(low_rank_decay_kernel, dim3(grid), dim3(kDecayChannels), 0, stream, alpha, low, ldl, w, bias, tokens, C, R, 1.f / tau);
     return xb_launch_status();
 }
 
@@ -1211,6 +1221,7 @@ template <typename TO>
 __global__ void gated_head_norm_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ gate,
                                        long long ldg, int g_off, const float* __restrict__ w, int w_len, int W, int part,
                                        float eps, int mode, const float* __restrict__ div, long long ldo, float out_scale) {
+    pdl_overlap_few();
     __shared__ float scratch[33];
     const int t = blockIdx.x, c0 = blockIdx.y * part;
     const float* yr = y + (size_t)t * W + c0;
@@ -1247,6 +1258,7 @@ __global__ void __launch_bounds__(256) gated_head_norm_warp_kernel(TO* __restric
                                                                    const float* __restrict__ w, int w_len, int W, int part,
                                                                    float eps, int mode, const float* __restrict__ div,
                                                                    long long ldo, float out_scale, long long units) {
+    pdl_overlap_few();
     const int lane = threadIdx.x & 31;
     const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (unit >= units) return;
@@ -1288,7 +1300,7 @@ static void gated_head_norm_launch(TO* out, const float* y, const float* gate, l
     const int warps = 8;
     const unsigned blocks = (unsigned)((units + warps - 1) / warps);
 #define XB_HEAD_NORM_NV(NVV)                                                                                              \
-    gated_head_norm_warp_kernel<TO, NVV><<<blocks, warps * 32, 0, stream>>>(out, y, gate, ldg, g_off, w, w_len, W, part, \
+    xb_launch_few(gated_head_norm_warp_kernel<TO, NVV>, dim3(blocks), dim3(warps * 32), 0, stream, out, y, gate, ldg, g_off, w, w_len, W, part, \
                                                                             eps, mode, div, ldo, out_scale, units)
     if (part <= 32) XB_HEAD_NORM_NV(1);
     else if (part <= 64) XB_HEAD_NORM_NV(2);
@@ -1298,7 +1310,7 @@ static void gated_head_norm_launch(TO* out, const float* y, const float* gate, l
     else {
         const dim3 grid(tokens, W / part);
         const int threads = part >= 1024 ? 256 : 128;
-        gated_head_norm_kernel<TO><<<grid, threads, 0, stream>>>(out, y, gate, ldg, g_off, w, w_len, W, part, eps, mode, div, ldo,
+        xb_launch_few(gated_head_norm_kernel<TO>, dim3(grid), dim3(threads), 0, stream, out, y, gate, ldg, g_off, w, w_len, W, part, eps, mode, div, ldo,
                                                              out_scale);
     }
 #undef XB_HEAD_NORM_NV

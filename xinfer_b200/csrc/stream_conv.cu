@@ -71,6 +71,7 @@ __device__ __forceinline__ void store_channels(__nv_bfloat16* p, const float (&v
 
 template <typename TO, int K, int V>
 __global__ void __launch_bounds__(kThreads) stream_conv_kernel(TO* __restrict__ out, StreamConvArgs a) {
+    pdl_overlap_few();
     __shared__ float part[(kMaxRun + kMaxTaps) * kSegments];
     __shared__ float inv_of[kMaxRun + kMaxTaps];
     const int C = a.C;
@@ -242,7 +243,7 @@ template <typename TO, int V>
 int launch_taps(TO* out, const StreamConvArgs& a, int K, dim3 grid, cudaStream_t stream) {
 #define XB_TAPS(KV)                                                        \
     case KV:                                                               \
-        stream_conv_kernel<TO, KV, V><<<grid, kThreads, 0, stream>>>(out, a); \
+        xb_launch_few(stream_conv_kernel<TO, KV, V>, dim3(grid), dim3(kThreads), 0, stream, out, a); \
         return xb_launch_status();
     switch (K) {
         XB_TAPS(1) XB_TAPS(2) XB_TAPS(3) XB_TAPS(4) XB_TAPS(5) XB_TAPS(6) XB_TAPS(7) XB_TAPS(8)

@@ -73,6 +73,7 @@ __global__ void qkv_prepare_kernel(T* __restrict__ q_out, T* __restrict__ k_cach
                                    long long v_off, const float* __restrict__ taps, int K, T* conv_state,
                                    const int* __restrict__ q_start, const int* __restrict__ slots, int keep_state,
                                    float value_eps, int* err) {
+    pdl_overlap_few();
     extern __shared__ float sm[];
     __shared__ float red2[2][32];
     const int half = rot / 2;
@@ -553,7 +554,7 @@ XB_EXPORT int xb_qkv_prepare(int dtype, void* q_out, void* k_cache, void* v_cach
         if (done) return xb_launch_status();
     }
 #define XB_PREPARE(T, CONV)                                                                                               \
-    qkv_prepare_kernel<T, CONV><<<dim3(tokens, spread), threads, smem, stream>>>(                                                      \
+    xb_launch_few(qkv_prepare_kernel<T, CONV>, dim3(dim3(tokens, spread)), dim3(threads), smem, stream,                                                       \
         (T*)q_out, (T*)k_cache, (T*)v_cache, (const T*)qkv, q_w, k_w, inv_freq, positions, req_of_token, block_table,    \
         table_stride, nh, nkv, d, dv, rot, interleaved, norm_mode, page_size, num_pages, eps, write_kv, vec4, rot_mag,   \
         bias, temp_coef, temp_every, row_len, v_off, taps, K, (T*)conv_state, q_start, slots, keep_state, value_eps, err)
@@ -786,6 +787,7 @@ template <typename T>
 __global__ void attn_talking_merge_kernel(T* __restrict__ out, const float* __restrict__ part_o,
                                           const float* __restrict__ part_ml, int H, int dv, int parts, int ldo,
                                           float out_scale) {
+    pdl_overlap_few();
     extern __shared__ float fy[];          // [parts] factors, then the sum
     const int t = blockIdx.x, h = blockIdx.y;
     const float* ml = part_ml + (size_t)t * parts * H * 2 + 2 * h;
@@ -820,7 +822,7 @@ template <typename T>
 static int talking_merge_launch(void* out, const float* part_o, const float* part_ml, int tokens, int H, int dv, int parts,
                                 int ldo, float out_scale, cudaStream_t stream) {
     const int threads = dv >= 128 ? 128 : (dv >= 64 ? 64 : 32);
-    attn_talking_merge_kernel<T><<<dim3(tokens, H), threads, (parts + 1) * sizeof(float), stream>>>((T*)out, part_o, part_ml, H, dv,
+    xb_launch_few(attn_talking_merge_kernel<T>, dim3(dim3(tokens, H)), dim3(threads), (parts + 1) * sizeof(float), stream, (T*)out, part_o, part_ml, H, dv,
                                                                                                   parts, ldo, out_scale);
     return xb_launch_status();
 }

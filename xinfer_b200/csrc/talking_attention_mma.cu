@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(TM_THREADS) attn_talking_mma_kernel(__nv_bfloa
                                                                       const __nv_bfloat16* __restrict__ k_cache,
                                                                       const __nv_bfloat16* __restrict__ v_cache,
                                                                       TalkMmaArgs a) {
+    pdl_overlap_few();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_entry, s_tile;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -389,7 +390,7 @@ static int talk_mma_launch(void* out, const void* q, const void* kc, const void*
                            cudaStream_t stream) {
     typedef __nv_bfloat16 bf;
     cudaFuncSetAttribute(attn_talking_mma_kernel<MAXH, DVT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attn_talking_mma_kernel<MAXH, DVT><<<grid, TM_THREADS, smem, stream>>>((bf*)out, (const bf*)q, (const bf*)kc, (const bf*)vc, a);
+    xb_launch_few(attn_talking_mma_kernel<MAXH, DVT>, dim3(grid), dim3(TM_THREADS), smem, stream, (bf*)out, (const bf*)q, (const bf*)kc, (const bf*)vc, a);
     return xb_launch_status();
 }
 

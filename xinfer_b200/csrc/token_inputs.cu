@@ -92,6 +92,7 @@ XB_EXPORT int xb_embed_sum(int table_dtype, float* out, const void* table, const
 // prev_state[slot of entry b] = the entry's last token of this step
 __global__ void prev_store_kernel(int* __restrict__ prev_state, const int* __restrict__ ids, const int* __restrict__ sampled,
                                   int num_sampled, const int* __restrict__ q_start, const int* __restrict__ slots, int entries) {
+    pdl_overlap_few();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= entries) return;
     const int slot = slots[b];
@@ -103,7 +104,7 @@ __global__ void prev_store_kernel(int* __restrict__ prev_state, const int* __res
 XB_EXPORT int xb_prev_store(int* prev_state, const int* ids, const int* sampled, int num_sampled, const int* q_start,
                             const int* slots, int entries, cudaStream_t stream) {
     if (entries <= 0) return 0;
-    prev_store_kernel<<<(entries + 127) / 128, 128, 0, stream>>>(prev_state, ids, sampled, num_sampled, q_start, slots, entries);
+    xb_launch_few(prev_store_kernel, dim3((entries + 127) / 128), dim3(128), 0, stream, prev_state, ids, sampled, num_sampled, q_start, slots, entries);
     return xb_launch_status();
 }
 
@@ -111,6 +112,7 @@ template <typename T>
 __global__ void token_gate_kernel(T* __restrict__ out, const T* __restrict__ u, const T* __restrict__ table, int table_ld,
                                   int col0, const int* __restrict__ ids, const int* __restrict__ sampled, int num_sampled,
                                   const int* __restrict__ req_of_token, int dim, int vocab, size_t n, int* err) {
+    pdl_overlap_few();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int t = (int)(i / dim), j = (int)(i % dim);
@@ -131,10 +133,10 @@ XB_EXPORT int xb_token_gate(int dtype, void* out, const void* u, const void* tab
     if (n == 0) return 0;
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (dtype == XB_F32)
-        token_gate_kernel<float><<<blocks, 256, 0, stream>>>((float*)out, (const float*)u, (const float*)table, table_ld, col0, ids,
+        xb_launch_few(token_gate_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)out, (const float*)u, (const float*)table, table_ld, col0, ids,
                                                             sampled, num_sampled, req_of_token, dim, vocab, n, err);
     else
-        token_gate_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)u,
+        xb_launch_few(token_gate_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)u,
                                                                     (const __nv_bfloat16*)table, table_ld, col0, ids, sampled,
                                                                     num_sampled, req_of_token, dim, vocab, n, err);
     return xb_launch_status();
