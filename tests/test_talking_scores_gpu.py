@@ -134,6 +134,7 @@ def test_a_model_gives_the_same_logits_both_ways_and_for_mixed_steps(monkeypatch
     def logits(on, nbytes):
         monkeypatch.setattr(part, "USE_SCORES", on)
         monkeypatch.setattr(part, "SCORES_BYTES", nbytes)
+        monkeypatch.setattr(part, "SCORES_MIN_US", 0.0)
         r = ModelRunner.random(cfg, 3, block_size=16, num_blocks=128, max_num_seqs=4, max_model_len=512)
         before = kernels.launch_counts().get("attn_talking_tc", 0)
         a, b = r.open_request(), r.open_request()
@@ -148,3 +149,16 @@ def test_a_model_gives_the_same_logits_both_ways_and_for_mixed_steps(monkeypatch
     assert none == 0 and some == 12 and more > some
     # two bfloat16 computations of the same numbers
     assert (got - want).norm() <= 0.02 * want.norm() and (again - got).norm() <= 1e-3 * got.norm()
+
+
+@pytest.mark.parametrize("heads,counts,starts,window,pays", [
+    (32, [100] * 8, [0] * 8, None, False), (32, [400, 400], [0, 0], None, True), (16, [400, 400], [0, 0], None, True),
+    (16, [100] * 8, [0] * 8, None, False), (32, [20], [0], None, False), (32, [2048], [0], None, True), (32, [2048], [0], 64, True),
+    (32, [64, 1], [0, 3000], None, True), (32, [64, 1], [0, 3000], 64, False), (8, [5], [0], None, False)])
+def test_short_steps_stay_on_the_kernel_that_holds_all_heads(heads, counts, starts, window, pays):
+    from types import SimpleNamespace as N
+    from xinfer_b200.parts.talking_attention import TalkingAttention
+    layer = N(spec=N(num_heads=heads, window=window))
+    ctx = N(max_context=max(a + b for a, b in zip(counts, starts)), real_tokens=sum(counts), real_entries=len(counts),
+            h_q_start=np.concatenate([[0], np.cumsum(counts)]), h_start_pos=np.asarray(starts))
+    assert TalkingAttention._scores_pay(layer, ctx) == pays

@@ -61,11 +61,13 @@ ROWS_MAX_BYTES = 1 << 30
 # What the two ways cost, for the choice between them: operations per microsecond of the attention over cached rows
 # (75 to 91 measured at ranks 256 and 512; a block of it walks over all keys of its 32 rows, at one SM's share of that
 # rate), of the products that form keys and values, and of the attention on those (780 measured at a prompt of 2,048
-# tokens and 32 heads, where the first way took 1,570 us and the second takes 55 + 18 us); beside that the second way is
-# a few microseconds shorter, as nothing is mapped in and out of the latent space - or as much longer, where the step's
-# small portions need the first way too.  Measured per layer (rank 512, 32 heads): 8 tokens after 3,000 cached ones 235 us
-# less the second way, 16 tokens alone 6 us less; 20 portions of 8 tokens after 1,000 cached ones 145 us less the first.
-ROWS_RATES = (75e6, 900e6, 700e6, -6.0, 20.0)
+# tokens and 32 heads, where the first way took 1,570 us and the second takes 55 + 18 us); beside that what the second way
+# costs the host, which a short prompt waits for: its work list and launches, more where the step's small portions need the
+# first way too.  Measured per layer on the device (rank 512, 32 heads): 8 tokens after 3,000 cached ones 235 us less the second
+# way, 16 tokens alone 6 us less; 20 portions of 8 tokens after 1,000 cached ones 145 us less the first.  Measured as steps of
+# four layers, first and second way: 8 prompts of 100 tokens 1,463 and 1,683 us at 16 heads of rank 256, 1,810 and 2,067 us at
+# 32 heads of rank 512; 2 prompts of 400 tokens 1,202 and 1,388 us, 2,100 and 2,009 us.
+ROWS_RATES = (75e6, 900e6, 700e6, 60.0, 90.0)
 ROWS_SMS = 148
 
 
@@ -77,7 +79,9 @@ def rows_plan(ctx: StepContext, heads: int, d: int, rd: int, dv: int, rank: int,
     if key in ctx.scratch:
         return ctx.scratch[key]
     made = None
-    if not (ctx.fixed_shapes or ctx.all_single) and USE_TENSOR_CORES and ctx.dtype == torch.bfloat16 and width % 8 == 0 \
+    # (no more pairs than tokens times the longest context: most short steps are decided by this alone)
+    most = ctx.max_context * max(ctx.real_tokens * heads, 32 * ROWS_SMS)
+    if not (ctx.fixed_shapes or ctx.all_single) and 2 * (width + rank) * most > ROWS_RATES[0] * ROWS_RATES[3] and USE_TENSOR_CORES and ctx.dtype == torch.bfloat16 and width % 8 == 0 \
             and kernels.attn_rows_tc_takes(d, rd, dv, rank) and kernels.attn_latent_mma_takes(width, rank):
         counts = np.diff(ctx.h_q_start[: ctx.real_entries + 1]).astype(np.int64)
         starts = ctx.h_start_pos[: ctx.real_entries].astype(np.int64)

@@ -47,6 +47,13 @@ USE_TENSOR_CORES = True
 # 2,048 tokens of 32 heads take 285 MB.  Cut to stay in the 126 MB L2 cache (3 chunks of 96 MB, 5 of 64 MB) a step of four
 # layers took 6.0 and 7.4 ms instead of 5.2: the launches of a chunk leave SMs idle.
 SCORES_BYTES = 320 << 20
+# ... and only where the kernel that holds all heads in a block would take longer than SCORES_MIN_US: it walks a key for four
+# queries in about 0.53 us at 32 heads (0.3 at 16), the blocks share 148 processors, and the longest row of blocks is walked in
+# order.  Below that the two launches, their start-up and their work list cost more than they save: steps of four layers, that
+# kernel and the two, 8 prompts of 100 tokens (53 us by this rule) 2,478 and 2,553 us at 32 heads, 2 prompts of 400 tokens
+# (212 us) 3,668 and 3,451 us; at 16 heads (27 and 106 us) 1,451 and 1,535 us, 1,613 and 1,377 us.
+SCORES_MIN_US = 80.0
+SCORES_KEY_US = 0.0166          # a key, four queries, per head
 # Steps of many tokens on the two kernels that pass the mixed scores through memory; tests switch it off.
 USE_SCORES = True
 _work_ring = PinnedRing()
@@ -187,14 +194,31 @@ class TalkingAttention(Mixer):
                 and not (ctx.all_single or ctx.fixed_shapes) and not self._changed_scores()
                 and kernels.attn_talking_tc_takes(s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, cache.page_size))
 
+    def _scores_pay(self, ctx: StepContext) -> bool:
+        """Whether blocks that hold all heads would take longer than SCORES_MIN_US over the step."""
+        s = self.spec
+        key_us = SCORES_KEY_US * s.num_heads
+        keys = ctx.max_context if not s.window else min(ctx.max_context, s.window + 4)
+        blocks = ctx.real_tokens / 4 + ctx.real_entries
+        if key_us * max(keys, blocks * keys / 148) <= SCORES_MIN_US:       # (the work below is no more than this)
+            return False
+        counts = ctx.h_q_start[1: ctx.real_entries + 1] - ctx.h_q_start[: ctx.real_entries]
+        walked = ctx.h_start_pos[: ctx.real_entries] + (counts + 1) * 0.5
+        if s.window:
+            walked = walked.clip(max=s.window + 4)
+        return key_us * max(keys, float((walked * ((counts + 3) // 4)).sum()) / 148) > SCORES_MIN_US
+
     def _scores_work(self, ctx: StepContext, cache: LayerCache):
-        """The step's work lists for those kernels, made once and shared by layers of the same sizes; None: too many keys."""
+        """The step's work lists for those kernels, made once and shared by layers of the same sizes; None: too many keys,
+        or too few to pay."""
         s = self.spec
         key = ("talk_work", s.num_heads, s.num_kv_heads, s.window)
         if key not in ctx.scratch:
-            counts = ctx.h_q_start[1: ctx.real_entries + 1] - ctx.h_q_start[: ctx.real_entries]
-            made = kernels.talk_work(counts, ctx.h_start_pos[: ctx.real_entries], s.window, s.num_heads, s.num_kv_heads,
-                                     SCORES_BYTES // (4 * kernels.TALK_TILE_FLOATS), host_buffer=_work_ring.take)
+            made = None
+            if self._scores_pay(ctx):
+                counts = ctx.h_q_start[1: ctx.real_entries + 1] - ctx.h_q_start[: ctx.real_entries]
+                made = kernels.talk_work(counts, ctx.h_start_pos[: ctx.real_entries], s.window, s.num_heads, s.num_kv_heads,
+                                         SCORES_BYTES // (4 * kernels.TALK_TILE_FLOATS), host_buffer=_work_ring.take)
             if made is not None:
                 made = (made[0].to(ctx.positions.device, non_blocking=True), made[1], made[2])
                 _work_ring.sent()
