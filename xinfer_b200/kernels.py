@@ -39,7 +39,7 @@ def _need(t: torch.Tensor, name: str, dtype=None, shape=None) -> None:
         ok = t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype == dtype)
     except AttributeError:
         ok = False
-    if ok and shape is not None:
+    if ok and shape is not None and t.shape != shape:       # (equal as a whole: no dimension was left open)
         ts = t.shape
         if len(ts) != len(shape):
             ok = False
