@@ -1,5 +1,6 @@
 """Kernels that start before their predecessor has ended read and write nothing before its end: chains of dependent launches,
 at grids and portions on both sides of the rule, give the numbers of launches with a synchronisation between them."""
+import numpy as np
 import pytest
 import torch
 
@@ -39,3 +40,26 @@ def test_a_chain_of_scans_carries_its_state(tokens):
         return torch.stack(out), state
     for got, want in zip(chain(False), chain(True)):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("d,dv", [(64, 64), (64, 128), (128, 64)])
+def test_attention_with_room_beside_it_runs_in_front_of_a_product_of_few_tokens(d, dv):
+    # Both allocate tensor memory, and at these sizes a processor has shared memory for a block of each.
+    H, rank, T, start = 40, 64, 8, 700
+    g = torch.Generator(device="cuda:0").manual_seed(d + dv)
+    bf = lambda *s: torch.randn(*s, generator=g, device="cuda:0").bfloat16()
+    i32 = lambda a: torch.tensor(np.asarray(a), dtype=torch.int32, device="cuda:0")
+    host, ctas, n, _ = kernels.latent_prefill_work([T], [start], 4, None, H)
+    work, q, kv, rows, w = host.to("cuda:0"), bf(T, H * d), bf(n, H * (d + dv)), bf(n, rank), bf(512, H * dv)
+    q_start, start_pos, err = i32([0, T]), i32([start]), i32([0])
+
+    def chain(wait):
+        out, y = torch.zeros(T, H * dv, dtype=torch.bfloat16, device="cuda:0"), [torch.empty(T, 512, device="cuda:0") for _ in range(20)]
+        for one in y:
+            kernels.attn_rows_tc(out, q, H * d, kv, rows, work, ctas, q_start, start_pos, H, d, 0, dv, rank, None, d ** -0.5, None, err)
+            if wait:
+                torch.cuda.synchronize()
+            assert kernels.gemm_skinny_tc(one, out, w, err)
+        torch.cuda.synchronize()
+        return torch.stack(y)
+    assert torch.equal(chain(False), chain(True)) and int(err) == 0

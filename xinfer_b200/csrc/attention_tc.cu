@@ -126,7 +126,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const uint32_t q_full = bars + 208, bar_o = bars + 216, q_empty = bars + 224;
     volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 240);  // tmem, -, -, dead
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
 
     // what follows until the wait reads only what the host sent before the step's first kernel
     const int ctas = (int)gridDim.x;
@@ -148,6 +147,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (*reinterpret_cast<volatile int*>(err) & XB_ERR_WAIT) item_end = item_begin;
     __syncthreads();
     if (item_end <= item_begin || (base & 1023u)) {
+        pdl_launch_dependents();
         pdl_wait();   // a kernel that depends on this one may rely on every block having waited
         return;
     }
@@ -160,6 +160,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = words[0];
+    pdl_launch_dependents();   // only now: see pdl_launch_dependents on tensor memory
     pdl_wait();   // q and the new keys and values come from the kernel before
 
     const int box_rows = ps < KT ? ps : KT;
@@ -730,7 +731,6 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 4 * RING_BARS + 72);  // tmem, dead, last, skip
     int* s_pages = reinterpret_cast<int*>(smem_raw + BAR_OFF + 4 * RING_BARS + 96);   // this range's part of the block table
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
 
     // what this CTA works on: the plan was written by the step's first kernel, before any kernel that runs
     // under programmatic dependent launch could have started
@@ -779,6 +779,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = words[0];
+    pdl_launch_dependents();   // only now: see pdl_launch_dependents on tensor memory
     const uint32_t tmem_s = tmem, tmem_o = tmem + 128;
 
     if (warp == 1 || warp == 3) {

@@ -91,9 +91,8 @@ gemm_skinny_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const int iters = k_end > k_begin ? (k_end - k_begin + TILE_K - 1) / TILE_K : 0;
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[16]), accum = smem_u32(&bars[32]);
     const uint32_t tmem_cols = mp < 32 ? 32u : (uint32_t)mp;
-    pdl_launch_dependents();
 
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 32) {       // (the first warp allocates meanwhile)
         for (int s = 0; s < stages; ++s) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 1);
@@ -109,6 +108,7 @@ gemm_skinny_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
+    pdl_launch_dependents();   // only now: see pdl_launch_dependents on tensor memory
 
     if (threadIdx.x == 0) {
         // ---- producer: stream W and x tiles -------------------------------------------------------

@@ -98,7 +98,6 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t q_full = bars + 224, q_empty = bars + 232;
     volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 240);   // tensor memory, dead
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
 
     const int ctas = (int)gridDim.x;
     const int item_begin = work[blockIdx.x];
@@ -123,6 +122,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (*reinterpret_cast<volatile int*>(err) & XB_ERR_WAIT) item_end = item_begin;   // an earlier CTA gave up
     __syncthreads();
     if (item_end <= item_begin || (base & 1023u)) {
+        pdl_launch_dependents();
         pdl_wait();
         return;
     }
@@ -131,6 +131,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = words[0];
+    pdl_launch_dependents();    // only now: see pdl_launch_dependents on tensor memory
     pdl_wait();
 
     auto item_at = [&](int k) { return item_of(items + (size_t)k * ITEM_INTS, q_start, start_pos, window); };

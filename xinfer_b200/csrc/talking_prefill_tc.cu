@@ -121,7 +121,6 @@ talk_scores_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const uint32_t k_full0 = bars, k_empty0 = bars + 16, d_full = bars + 32, d_empty = bars + 40, q_full = bars + 48, q_empty = bars + 56;
     volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + L::BAR_OFF + 64);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rep = H / nkv;
-    pdl_launch_dependents();
     const int ctas = (int)gridDim.x;
     const int item_begin = work[blockIdx.x];
     int item_end = work[blockIdx.x + 1];
@@ -142,6 +141,7 @@ talk_scores_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (*reinterpret_cast<volatile int*>(err) & XB_ERR_WAIT) item_end = item_begin;
     __syncthreads();
     if (item_end <= item_begin || (base & 1023u)) {
+        pdl_launch_dependents();
         pdl_wait();
         return;
     }
@@ -150,6 +150,7 @@ talk_scores_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = words[0];
+    pdl_launch_dependents();    // only now: see pdl_launch_dependents on tensor memory
     pdl_wait();     // queries and new keys come from the kernel before; the tiles were read by the one before that
 
     if (warp < 8) {
@@ -360,7 +361,6 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* __
     const uint32_t s_full0 = bars + 96, s_empty0 = bars + 96 + 16 * S_STAGES;
     volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 240);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
     const int ctas = (int)gridDim.x;
     const int item_begin = work[blockIdx.x];
     int item_end = work[blockIdx.x + 1];
@@ -384,6 +384,7 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* __
     if (*reinterpret_cast<volatile int*>(err) & XB_ERR_WAIT) item_end = item_begin;
     __syncthreads();
     if (item_end <= item_begin || (base & 1023u)) {
+        pdl_launch_dependents();
         pdl_wait();
         return;
     }
@@ -392,6 +393,7 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* __
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = words[0];
+    pdl_launch_dependents();    // only now: see pdl_launch_dependents on tensor memory
     pdl_wait();
 
     struct Item {
