@@ -82,12 +82,18 @@ __device__ __forceinline__ pair2 pr_mul(pair2 a, pair2 b) {
     return d;
 }
 constexpr int kPairs = kRows / 2;
-// Whether a group of four tokens is whole: its code then has no branch between the tokens, and the loads of one can overlap the
-// arithmetic of another.
-template <bool B>
-struct Whole {
-    static constexpr bool value = B;
+// A group of N tokens that are worked on together.  Whole: its code then has no branch between the tokens, and the loads of one
+// can overlap the arithmetic of another.
+template <int N, bool WHOLE>
+struct Group {
+    static constexpr int tokens = N;
+    static constexpr bool whole = WHOLE;
 };
+// Where no request brings more than this many tokens the kernels take them one by one: there is no chain to hide, and the code
+// needs 128 registers instead of 140 to 166, with which two blocks of eight warps fit a processor.  256 requests of one token, 8
+// heads of 64 x 64 states: linear 42 -> 27 us, selective 43 -> 28 us; 32 requests of five tokens, 13 -> 11 us.  (At 40 tokens groups
+// of four are 1.1 to 1.2 times as fast.)  The sums are the same bits either way.
+constexpr int kFewTokens = 16;
 
 // The feeding warps' walk over the tiles, in step with the computing warps (one block barrier per tile): while tile t is
 // worked on, the copies of t + 2 are asked for, t + 1 has landed and is finished, and the results of t - 1 leave: the copies have
@@ -216,8 +222,8 @@ __device__ __forceinline__ void stage_cols(float* dst, const float* src, int c_b
 // xbc[t] = [x: H*P | B: G*N | C: G*N] after the short convolution; dt is column dt_off + h of proj[t] (before
 // the bias and the softplus).  state [slots, H, N, P].  y [T, H*P].  Shared memory: three stages of
 // B[TT][NP] C[TT][NP] x[TT][VT] dt[TT] dec[TT], then two tiles y[TT][VT].  `cw` of the block's warps compute.
-template <int DS>
-__global__ void __launch_bounds__(384, 1) selective_scan_kernel(float* __restrict__ y, const float* __restrict__ xbc, int C,
+template <int DS, bool FEW>
+__global__ void __launch_bounds__(FEW ? 256 : 384, FEW ? 2 : 1) selective_scan_kernel(float* __restrict__ y, const float* __restrict__ xbc, int C,
                                                              const float* __restrict__ proj, long long ldp, int dt_off,
                                                              const float* __restrict__ dt_bias,
                                                              const float* __restrict__ A_log, const float* __restrict__ Dv,
@@ -298,12 +304,14 @@ __global__ void __launch_bounds__(384, 1) selective_scan_kernel(float* __restric
         float* out = sy + (tile & 1) * TT * VT + cl;
         const int nt = min(TT, t1 - t0 - tile * TT);
         // four tokens at a time: the state's updates of one token hide the sums over the row groups of the others
-        auto group = [&](int tt, auto whole) {
-            float v[8];
+        auto group = [&](int tt, auto grp) {
+            constexpr int NG = decltype(grp)::tokens;
+            constexpr bool whole = decltype(grp)::whole;
+            float v[2 * NG];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < NG; ++k) {
                 v[2 * k] = v[2 * k + 1] = 0.f;
-                if (!decltype(whole)::value && tt + k >= nt) continue;
+                if (!whole && tt + k >= nt) continue;
                 const float dt = sdt[tt + k], dec = sdt[TT + tt + k];
                 const float2 xv = *reinterpret_cast<const float2*>(sx + (tt + k) * VT);
                 const pair2 d0 = pr_make(dt * xv.x, dt * xv.x), d1 = pr_make(dt * xv.y, dt * xv.y), keep = pr_make(dec, dec);
@@ -321,18 +329,22 @@ __global__ void __launch_bounds__(384, 1) selective_scan_kernel(float* __restric
                 v[2 * k + 1] = pr_sum(a1);
             }
             int first;
-            const int n = fold_many<DS, 8>(v, ds, first);
-            if (fold_writes<DS, 8>(ds)) {
+            const int n = fold_many<DS, 2 * NG>(v, ds, first);
+            if (fold_writes<DS, 2 * NG>(ds)) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 2 * NG; ++i) {
                     const int k = (first + i) >> 1, c = (first + i) & 1;
-                    if (i < n && (decltype(whole)::value || tt + k < nt)) out[(tt + k) * VT + c] = fmaf(Dh, sx[(tt + k) * VT + c], v[i]);
+                    if (i < n && (whole || tt + k < nt)) out[(tt + k) * VT + c] = fmaf(Dh, sx[(tt + k) * VT + c], v[i]);
                 }
             }
         };
-        int done = 0;
-        for (; done + 4 <= nt; done += 4) group(done, Whole<true>{});
-        if (done < nt) group(done, Whole<false>{});
+        if constexpr (FEW) {
+            for (int tt = 0; tt < nt; ++tt) group(tt, Group<1, true>{});
+        } else {
+            int done = 0;
+            for (; done + 4 <= nt; done += 4) group(done, Group<4, true>{});
+            if (done < nt) group(done, Group<4, false>{});
+        }
         __syncthreads();
     }
 #pragma unroll
@@ -684,11 +696,173 @@ __global__ void __launch_bounds__(384, 1) delta_rule_kernel(float* __restrict__ 
     }
 }
 
+// The delta rule where every request brings few tokens (delta_few): one at a time, with unit vectors and decays formed by the
+// feeding warps, since a launch in front of it costs more than it saves.  With gS the decayed state, o = (gS)^T q + u (k . q).
+// Shared memory: three stages of q[TT][DP] k[TT][DP] g[TT][DP] v[TT][VT] beta[TT] kq[TT], then two tiles o[TT][VT].
+// One token of 16 heads of 128 x 128, 1 and 8 requests: 15 and 26 us with the kernel in front, 11 and 18 us so.  A small state's
+// chain is short beside that kernel: 8 heads of 64 x 64, 32 requests of five tokens 28 and 15 us, eight of 40 tokens 28 and 20 us, one
+// of 128 tokens 48 and 47 us, of 600 tokens 161 and 185 us; of 128 x 128, eight of 40 tokens 52 and 65 us.
+constexpr int kFewTokensSmall = 96;
+static inline bool delta_few(int longest, int d) { return longest <= (d <= 64 ? kFewTokensSmall : kFewTokens); }
+template <int DS>
+__global__ void __launch_bounds__(384, 1) delta_few_kernel(float* __restrict__ o, const float* __restrict__ qkv, int Cq,
+                                                        const float* __restrict__ proj, long long ldp, int beta_off,
+                                                        const float* __restrict__ ag, long long ldag,
+                                                        const float* __restrict__ dt_bias, const float* __restrict__ A_log,
+                                                        float* __restrict__ state, const int* __restrict__ q_start,
+                                                        const int* __restrict__ slots, int H, int G, int d, int dv,
+                                                        float unit_eps, int TT, int stage, int cw, int vec) {
+    pdl_wait();
+    extern __shared__ __align__(16) float scan_smem[];
+    constexpr int CGW = 32 / DS, DP = DS * kRowsPad, NR = DS * kRows;
+    const int b = blockIdx.x, h = blockIdx.y;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int VT = cw * CGW * 2, c_base = blockIdx.z * VT;
+    const int slot = slots[b];
+    const int t0 = q_start[b], t1 = q_start[b + 1];
+    if (t1 - t0 <= XB_FEW_TOKENS) pdl_launch_dependents();
+    if (slot < 0 || t1 <= t0) return;
+    const int kvh = h / (H / G);
+    const int ntiles = (t1 - t0 + TT - 1) / TT;
+    float* so = scan_smem + kStages * stage;
+    if (w >= cw) {
+        // feeding warps: warp `pi` of `pw` takes tokens pi, pi + pw, ... of every tile
+        const int pi = w - cw, pw = (blockDim.x >> 5) - cw;
+        const float A = expf(A_log[h]);
+        const float qk_scale = 1.f / sqrtf((float)d);
+        const float* bias = dt_bias + (size_t)h * d;
+        auto bring = [&](int tile) {
+            float* sq = scan_smem + (tile % kStages) * stage;
+            float* sk = sq + TT * DP;
+            float* sg = sk + TT * DP;
+            float* sv = sg + TT * DP;
+            float* sbeta = sv + TT * VT;
+            const int tb = t0 + tile * TT, nt = min(TT, t1 - tb);
+            for (int tt = pi; tt < nt; tt += pw) {
+                const float* row = qkv + (size_t)(tb + tt) * Cq;
+                stage_rows(sq + tt * DP, row + kvh * d, d, NR, lane, vec);
+                stage_rows(sk + tt * DP, row + (G + kvh) * d, d, NR, lane, vec);
+                stage_rows(sg + tt * DP, ag + (size_t)(tb + tt) * ldag + h * d, d, NR, lane, vec);
+                stage_cols(sv + tt * VT, row + 2 * G * d + h * dv, c_base, dv, VT, lane, vec);
+                if (lane == 0) scan_cp4(sbeta + tt, proj + (size_t)(tb + tt) * ldp + beta_off + h);
+            }
+        };
+        auto finish = [&](int tile) {
+            float* sq = scan_smem + (tile % kStages) * stage;
+            float* sk = sq + TT * DP;
+            float* sg = sk + TT * DP;
+            float* sbeta = sg + TT * DP + TT * VT;
+            const int nt = min(TT, t1 - t0 - tile * TT);
+            scan_cp_land();
+            for (int tt = pi; tt < nt; tt += pw) {
+                float* q = sq + tt * DP;
+                float* k = sk + tt * DP;
+                float* gd = sg + tt * DP;
+                float qq = 0.f, kk = 0.f;
+                for (int j = lane; j < d; j += 32) {
+                    const int at = padded_row(j);
+                    qq = fmaf(q[at], q[at], qq);
+                    kk = fmaf(k[at], k[at], kk);
+                }
+                qq = warp_total(qq);
+                kk = warp_total(kk);
+                const float qs = qk_scale / sqrtf(qq + unit_eps), ks = 1.f / sqrtf(kk + unit_eps);
+                float kq = 0.f;
+                for (int j = lane; j < d; j += 32) {
+                    const int at = padded_row(j);
+                    const float qn = q[at] * qs, kn = k[at] * ks;
+                    q[at] = qn;
+                    k[at] = kn;
+                    kq = fmaf(kn, qn, kq);
+                    gd[at] = expf(-A * softplus_f32(gd[at] + bias[j]));
+                }
+                kq = warp_total(kq);
+                if (lane == 0) {
+                    sbeta[TT + tt] = kq;
+                    sbeta[tt] = sigmoid_exact(sbeta[tt]);
+                }
+            }
+        };
+        auto leave = [&](int tile) {
+            const float* src = so + (tile & 1) * TT * VT;
+            const int tb = t0 + tile * TT, nt = min(TT, t1 - tb);
+            for (int tt = pi; tt < nt; tt += pw)
+                for (int c = lane; c < VT; c += 32)
+                    if (c_base + c < dv) o[((size_t)(tb + tt) * H + h) * dv + c_base + c] = src[tt * VT + c];
+        };
+        feed(ntiles, bring, finish, leave);
+        leave(ntiles - 1);
+        return;
+    }
+    const int ds = lane / CGW, cl = (w * CGW + lane % CGW) * 2, v0 = c_base + cl;
+    float S0[kRows], S1[kRows];
+    float* st = state + ((size_t)slot * H + h) * d * dv;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        const int j = ds * kRows + r;
+        S0[r] = j < d && v0 < dv ? st[(size_t)j * dv + v0] : 0.f;
+        S1[r] = j < d && v0 + 1 < dv ? st[(size_t)j * dv + v0 + 1] : 0.f;
+    }
+    __syncthreads();
+    for (int tile = 0; tile < ntiles; ++tile) {
+        const float* sq = scan_smem + (tile % kStages) * stage + ds * kRowsPad;
+        const float* sk = sq + TT * DP;
+        const float* sg = sk + TT * DP;
+        const float* sv = scan_smem + (tile % kStages) * stage + 3 * TT * DP;
+        const float* sbeta = sv + TT * VT;
+        sv += cl;
+        float* out = so + (tile & 1) * TT * VT + cl;
+        const int nt = min(TT, t1 - t0 - tile * TT);
+        for (int tt = 0; tt < nt; ++tt, sq += DP, sk += DP, sg += DP, sv += VT, out += VT) {
+            const float beta = sbeta[tt];
+            const float2 vv = *reinterpret_cast<const float2*>(sv);
+            const float4* qp = reinterpret_cast<const float4*>(sq);
+            const float4* kp = reinterpret_cast<const float4*>(sk);
+            const float4* gp = reinterpret_cast<const float4*>(sg);
+            float kr[kRows], a[4] = {0.f, 0.f, 0.f, 0.f};     // (gS)^T k and (gS)^T q of the two columns
+#pragma unroll
+            for (int i = 0; i < kRows / 4; ++i) {
+                const float4 g4 = gp[i], k4 = kp[i], q4 = qp[i];
+                const float ge[4] = {g4.x, g4.y, g4.z, g4.w}, ke[4] = {k4.x, k4.y, k4.z, k4.w}, qe[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int r = 4 * i + e;
+                    S0[r] *= ge[e];
+                    S1[r] *= ge[e];
+                    a[0] = fmaf(S0[r], ke[e], a[0]);
+                    a[1] = fmaf(S1[r], ke[e], a[1]);
+                    a[2] = fmaf(S0[r], qe[e], a[2]);
+                    a[3] = fmaf(S1[r], qe[e], a[3]);
+                    kr[r] = ke[e];
+                }
+            }
+#pragma unroll
+            for (int bit = 16; bit >= CGW; bit >>= 1)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] += __shfl_xor_sync(0xffffffffu, a[i], bit);
+            const float u0 = beta * (vv.x - a[0]), u1 = beta * (vv.y - a[1]);
+#pragma unroll
+            for (int r = 0; r < kRows; ++r) {
+                S0[r] = fmaf(kr[r], u0, S0[r]);
+                S1[r] = fmaf(kr[r], u1, S1[r]);
+            }
+            if (ds == 0) *reinterpret_cast<float2*>(out) = make_float2(fmaf(u0, sbeta[TT + tt], a[2]), fmaf(u1, sbeta[TT + tt], a[3]));
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        const int j = ds * kRows + r;
+        if (j < d && v0 < dv) st[(size_t)j * dv + v0] = S0[r];
+        if (j < d && v0 + 1 < dv) st[(size_t)j * dv + v0 + 1] = S1[r];
+    }
+}
+
 // proj[t] holds q (H*d from column 0), k (H*d behind it) and v (H*dv behind that) of a token; alpha[t] the decay of
 // every (head, key channel).  state [slots, H, d, dv].  o [T, H*dv] = scale * S^T q after the token's own write.  Shared
 // memory: three stages of q[TT][DP] k[TT][DP] alpha[TT][DP] v[TT][VT], then two tiles o[TT][VT].
-template <int DS>
-__global__ void __launch_bounds__(384, 1) linear_scan_kernel(float* __restrict__ o, const float* __restrict__ proj,
+template <int DS, bool FEW>
+__global__ void __launch_bounds__(FEW ? 256 : 384, FEW ? 2 : 1) linear_scan_kernel(float* __restrict__ o, const float* __restrict__ proj,
                                                              long long ldp, const float* __restrict__ alpha,
                                                              float* __restrict__ state, const int* __restrict__ q_start,
                                                              const int* __restrict__ slots, int H, int d, int dv, float scale,
@@ -752,12 +926,14 @@ __global__ void __launch_bounds__(384, 1) linear_scan_kernel(float* __restrict__
         const float* sv = scan_smem + (tile % kStages) * stage + 3 * TT * DP + cl;
         float* out = so + (tile & 1) * TT * VT + cl;
         const int nt = min(TT, t1 - t0 - tile * TT);
-        auto group = [&](int tt, auto whole) {      // four tokens at a time, as in selective_scan_kernel
-            float v[8];
+        auto group = [&](int tt, auto grp) {        // as in selective_scan_kernel
+            constexpr int NG = decltype(grp)::tokens;
+            constexpr bool whole = decltype(grp)::whole;
+            float v[2 * NG];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < NG; ++k) {
                 v[2 * k] = v[2 * k + 1] = 0.f;
-                if (!decltype(whole)::value && tt + k >= nt) continue;
+                if (!whole && tt + k >= nt) continue;
                 const float2 vv = *reinterpret_cast<const float2*>(sv + (tt + k) * VT);
                 pair2 q[kPairs], kv[kPairs], a0 = 0ull, a1 = 0ull;
                 load_pairs(sq + (tt + k) * DP, q);
@@ -776,18 +952,22 @@ __global__ void __launch_bounds__(384, 1) linear_scan_kernel(float* __restrict__
                 v[2 * k + 1] = pr_sum(a1);
             }
             int first;
-            const int n = fold_many<DS, 8>(v, ds, first);
-            if (fold_writes<DS, 8>(ds)) {
+            const int n = fold_many<DS, 2 * NG>(v, ds, first);
+            if (fold_writes<DS, 2 * NG>(ds)) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 2 * NG; ++i) {
                     const int k = (first + i) >> 1, c = (first + i) & 1;
-                    if (i < n && (decltype(whole)::value || tt + k < nt)) out[(tt + k) * VT + c] = scale * v[i];
+                    if (i < n && (whole || tt + k < nt)) out[(tt + k) * VT + c] = scale * v[i];
                 }
             }
         };
-        int done = 0;
-        for (; done + 4 <= nt; done += 4) group(done, Whole<true>{});
-        if (done < nt) group(done, Whole<false>{});
+        if constexpr (FEW) {
+            for (int tt = 0; tt < nt; ++tt) group(tt, Group<1, true>{});
+        } else {
+            int done = 0;
+            for (; done + 4 <= nt; done += 4) group(done, Group<4, true>{});
+            if (done < nt) group(done, Group<4, false>{});
+        }
         __syncthreads();
     }
 #pragma unroll
@@ -814,7 +994,7 @@ __global__ void __launch_bounds__(384, 1) linear_scan_kernel(float* __restrict__
 // Shared memory: three stages of q[TT][DP] k[TT][DP] v[TT][VT] a[TT] b[TT] e^(-m')[TT], then two tiles o[TT][VT].  Besides
 // the computing and the feeding warps there is one (warp `cw`) that carries n where the block has the head's first
 // columns; the first feeding warp works out the gates, a lane per token, and walks m over the tile.
-template <int DS>
+template <int DS, bool FEW>
 __global__ void __launch_bounds__(384, 1) matrix_memory_kernel(
     float* __restrict__ o, float* __restrict__ div, const float* __restrict__ proj, long long ldp, int gate_off,
     const float* __restrict__ bi, const float* __restrict__ bf, float cap, float* __restrict__ state_s,
@@ -957,12 +1137,14 @@ __global__ void __launch_bounds__(384, 1) matrix_memory_kernel(
         sv += cl;
         float* out = so + (tile & 1) * TT * VT + cl;
         const int nt = min(TT, t1 - t0 - tile * TT);
-        auto group = [&](int tt, auto whole) {      // four tokens at a time, as in selective_scan_kernel
-            float v[8];
+        auto group = [&](int tt, auto grp) {        // as in selective_scan_kernel
+            constexpr int NG = decltype(grp)::tokens;
+            constexpr bool whole = decltype(grp)::whole;
+            float v[2 * NG];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < NG; ++k) {
                 v[2 * k] = v[2 * k + 1] = 0.f;
-                if (!decltype(whole)::value && tt + k >= nt) continue;
+                if (!whole && tt + k >= nt) continue;
                 const float2 vv = *reinterpret_cast<const float2*>(sv + (tt + k) * VT);
                 pair2 q[kPairs], kv[kPairs], a0 = 0ull, a1 = 0ull;
                 load_pairs(sq + (tt + k) * DP, q);
@@ -980,18 +1162,22 @@ __global__ void __launch_bounds__(384, 1) matrix_memory_kernel(
                 v[2 * k + 1] = pr_sum(a1);
             }
             int first;
-            const int n = fold_many<DS, 8>(v, ds, first);
-            if (fold_writes<DS, 8>(ds)) {
+            const int n = fold_many<DS, 2 * NG>(v, ds, first);
+            if (fold_writes<DS, 2 * NG>(ds)) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 2 * NG; ++i) {
                     const int k = (first + i) >> 1, c = (first + i) & 1;
-                    if (i < n && (decltype(whole)::value || tt + k < nt)) out[(tt + k) * VT + c] = scale * v[i];
+                    if (i < n && (whole || tt + k < nt)) out[(tt + k) * VT + c] = scale * v[i];
                 }
             }
         };
-        int done = 0;
-        for (; done + 4 <= nt; done += 4) group(done, Whole<true>{});
-        if (done < nt) group(done, Whole<false>{});
+        if constexpr (FEW) {
+            for (int tt = 0; tt < nt; ++tt) group(tt, Group<1, true>{});
+        } else {
+            int done = 0;
+            for (; done + 4 <= nt; done += 4) group(done, Group<4, true>{});
+            if (done < nt) group(done, Group<4, false>{});
+        }
         __syncthreads();
     }
 #pragma unroll
@@ -1067,10 +1253,10 @@ static inline int scan_row_groups(int rows) {
 // Computing warps per block: enough to cover the columns (at most 8), fewer (down to 2) while the grid would
 // leave a third of the processors idle.  Every block of a head repeats the feeding warps' work, so column tiles
 // are not cut finer than that.
-static inline int scan_warps(int cols, int ds, long long heads_total) {
+static inline int scan_warps(int cols, int ds, long long heads_total, int most = 8) {
     const int per_warp = (32 / ds) * 2;
     int warps = 1;
-    while (warps < 8 && warps * per_warp < cols) warps *= 2;
+    while (warps < most && warps * per_warp < cols) warps *= 2;
     auto blocks = [&](int n) { return heads_total * ((cols + n * per_warp - 1) / (n * per_warp)); };
     while (warps > 2 && blocks(warps) < 100 && blocks(warps / 2) <= 148) warps /= 2;      // (a block fills an SM)
     return warps;
@@ -1094,14 +1280,29 @@ static inline int scan_smem_opt_in(K kernel, size_t bytes) {
     return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-#define XB_SCAN_DISPATCH(KERNEL, DSV, ...)                                                       \
+#define XB_SCAN_DISPATCH(KERNEL, DSV, ...)                                                      \
     switch (DSV) {                                                                              \
-        case 1: XB_SCAN_LAUNCH(KERNEL<1>, __VA_ARGS__) break;                                   \
-        case 2: XB_SCAN_LAUNCH(KERNEL<2>, __VA_ARGS__) break;                                   \
-        case 4: XB_SCAN_LAUNCH(KERNEL<4>, __VA_ARGS__) break;                                   \
-        case 8: XB_SCAN_LAUNCH(KERNEL<8>, __VA_ARGS__) break;                                   \
-        case 16: XB_SCAN_LAUNCH(KERNEL<16>, __VA_ARGS__) break;                                 \
-        default: XB_SCAN_LAUNCH(KERNEL<32>, __VA_ARGS__) break;                                 \
+        case 1: XB_SCAN_LAUNCH((KERNEL<1>), __VA_ARGS__) break;                                 \
+        case 2: XB_SCAN_LAUNCH((KERNEL<2>), __VA_ARGS__) break;                                 \
+        case 4: XB_SCAN_LAUNCH((KERNEL<4>), __VA_ARGS__) break;                                 \
+        case 8: XB_SCAN_LAUNCH((KERNEL<8>), __VA_ARGS__) break;                                 \
+        case 16: XB_SCAN_LAUNCH((KERNEL<16>), __VA_ARGS__) break;                               \
+        default: XB_SCAN_LAUNCH((KERNEL<32>), __VA_ARGS__) break;                               \
+    }
+#define XB_SCAN_DISPATCH_FEW(KERNEL, DSV, FEW, ...)                                             \
+    switch ((DSV) * 2 + ((FEW) ? 1 : 0)) {                                                      \
+        case 2: XB_SCAN_LAUNCH((KERNEL<1, false>), __VA_ARGS__) break;                          \
+        case 3: XB_SCAN_LAUNCH((KERNEL<1, true>), __VA_ARGS__) break;                           \
+        case 4: XB_SCAN_LAUNCH((KERNEL<2, false>), __VA_ARGS__) break;                          \
+        case 5: XB_SCAN_LAUNCH((KERNEL<2, true>), __VA_ARGS__) break;                           \
+        case 8: XB_SCAN_LAUNCH((KERNEL<4, false>), __VA_ARGS__) break;                          \
+        case 9: XB_SCAN_LAUNCH((KERNEL<4, true>), __VA_ARGS__) break;                           \
+        case 16: XB_SCAN_LAUNCH((KERNEL<8, false>), __VA_ARGS__) break;                         \
+        case 17: XB_SCAN_LAUNCH((KERNEL<8, true>), __VA_ARGS__) break;                          \
+        case 32: XB_SCAN_LAUNCH((KERNEL<16, false>), __VA_ARGS__) break;                        \
+        case 33: XB_SCAN_LAUNCH((KERNEL<16, true>), __VA_ARGS__) break;                         \
+        case 65: XB_SCAN_LAUNCH((KERNEL<32, true>), __VA_ARGS__) break;                         \
+        default: XB_SCAN_LAUNCH((KERNEL<32, false>), __VA_ARGS__) break;                        \
     }
 #define XB_SCAN_LAUNCH(K, ...)                                  \
     {                                                           \
@@ -1110,13 +1311,15 @@ static inline int scan_smem_opt_in(K kernel, size_t bytes) {
         xb_launch_few(K, dim3(grid), dim3(threads), bytes, stream, __VA_ARGS__); \
     }
 
+// `longest`, here and below: tokens of the request that brings most, as far as the caller knows; only the choice between the
+// forms of a kernel depends on it.
 XB_EXPORT int xb_selective_scan(float* y, const float* xbc, int C, const float* proj, long long ldp, int dt_off,
                                 const float* dt_bias, const float* A_log, const float* Dv, float* state, const int* q_start,
-                                const int* slots, int entries, int H, int P, int N, int G, cudaStream_t stream) {
+                                const int* slots, int entries, int longest, int H, int P, int N, int G, cudaStream_t stream) {
     if (entries <= 0) return 0;
     if (N < 1 || N > 32 * kRows || P < 1 || G < 1 || H % G || H > 65535) return (int)cudaErrorInvalidValue;
     const int ds = scan_row_groups(N);
-    const int warps = scan_warps(P, ds, (long long)entries * H);
+    const int warps = scan_warps(P, ds, (long long)entries * H, longest <= kFewTokens ? 4 : 8);
     const int vt = warps * (32 / ds) * 2;
     int tt, stage;
     size_t bytes;
@@ -1124,27 +1327,39 @@ XB_EXPORT int xb_selective_scan(float* y, const float* xbc, int C, const float* 
     const dim3 grid(entries, H, (P + vt - 1) / vt);
     const int threads = (warps + 4) * 32;  // four feeding warps
     const int vec = scan_aligned16(xbc) && C % 4 == 0 && P % 4 == 0 && N % 4 == 0 && vt % 4 == 0;
-    XB_SCAN_DISPATCH(selective_scan_kernel, ds, y, xbc, C, proj, ldp, dt_off, dt_bias, A_log, Dv, state, q_start, slots, H, P, N,
+    XB_SCAN_DISPATCH_FEW(selective_scan_kernel, ds, longest <= kFewTokens, y, xbc, C, proj, ldp, dt_off, dt_bias, A_log, Dv, state, q_start, slots, H, P, N,
                      G, tt, stage, warps, vec)
     return xb_launch_status();
 }
 
-// Floats of `prep` for that many tokens and entries.
-XB_EXPORT long long xb_delta_prep_floats(int tokens, int entries, int H, int d) {
-    return (long long)tokens * H * 3 * d + (long long)(tokens / 4 + entries + 1) * H * (d + 16);
+// Floats of `prep` for that many tokens and entries (none where every request brings few).
+XB_EXPORT long long xb_delta_prep_floats(int tokens, int entries, int longest, int H, int d) {
+    return delta_few(longest, d) ? 0 : (long long)tokens * H * 3 * d + (long long)(tokens / 4 + entries + 1) * H * (d + 16);
 }
 
 XB_EXPORT int xb_delta_rule(float* o, const float* qkv, int Cq, const float* proj, long long ldp, int beta_off, const float* ag,
                             long long ldag, const float* dt_bias, const float* A_log, float* state, const int* q_start,
-                            const int* slots, int entries, int tokens, int H, int G, int d, int dv, float unit_eps, float* prep,
-                            cudaStream_t stream) {
+                            const int* slots, int entries, int tokens, int longest, int H, int G, int d, int dv, float unit_eps,
+                            float* prep, cudaStream_t stream) {
     if (entries <= 0 || tokens <= 0) return 0;
-    if (d < 1 || d > 32 * kRows || dv < 1 || G < 1 || H % G || H > 65535 || !prep) return (int)cudaErrorInvalidValue;
+    const bool few = delta_few(longest, d);
+    if (d < 1 || d > 32 * kRows || dv < 1 || G < 1 || H % G || H > 65535 || (!few && !prep)) return (int)cudaErrorInvalidValue;
     const int ds = scan_row_groups(d);
     const int warps = scan_warps(dv, ds, (long long)entries * H);
     const int vt = warps * (32 / ds) * 2;
     int tt, stage;
     size_t bytes;
+    if (few) {
+        scan_tile(3, ds, vt, tt, stage, bytes);
+        const dim3 grid(entries, H, (dv + vt - 1) / vt);
+        // the unit vectors and decays are the feeding warps' work: eight of them where the block has room, else four
+        const int threads = (warps + (warps <= 4 ? 8 : 4)) * 32;
+        const int vec = scan_aligned16(qkv) && scan_aligned16(ag) && Cq % 4 == 0 && ldag % 4 == 0 && d % 4 == 0 && dv % 4 == 0 &&
+                        vt % 4 == 0;
+        XB_SCAN_DISPATCH(delta_few_kernel, ds, o, qkv, Cq, proj, ldp, beta_off, ag, ldag, dt_bias, A_log, state, q_start, slots, H,
+                         G, d, dv, unit_eps, tt, stage, warps, vec)
+        return xb_launch_status();
+    }
     scan_tile(3, ds, vt, tt, stage, bytes, 5 + ds * kRowsPad / 4);      // beta, A and B, a quarter of a row vector
     if (tt < 4) return (int)cudaErrorInvalidValue;                       // (a tile holds whole groups of four tokens)
     // every request adds at most one group of fewer than four tokens
@@ -1165,11 +1380,11 @@ XB_EXPORT int xb_delta_rule(float* o, const float* qkv, int Cq, const float* pro
 }
 
 XB_EXPORT int xb_linear_scan(float* o, const float* proj, long long ldp, const float* alpha, float* state, const int* q_start,
-                             const int* slots, int entries, int H, int d, int dv, float scale, cudaStream_t stream) {
+                             const int* slots, int entries, int longest, int H, int d, int dv, float scale, cudaStream_t stream) {
     if (entries <= 0) return 0;
     if (d < 1 || d > 32 * kRows || dv < 1 || H < 1 || H > 65535) return (int)cudaErrorInvalidValue;
     const int ds = scan_row_groups(d);
-    const int warps = scan_warps(dv, ds, (long long)entries * H);
+    const int warps = scan_warps(dv, ds, (long long)entries * H, longest <= kFewTokens ? 4 : 8);
     const int vt = warps * (32 / ds) * 2;
     int tt, stage;
     size_t bytes;
@@ -1177,13 +1392,13 @@ XB_EXPORT int xb_linear_scan(float* o, const float* proj, long long ldp, const f
     const dim3 grid(entries, H, (dv + vt - 1) / vt);
     const int threads = (warps + 4) * 32;  // four feeding warps: they only copy
     const int vec = scan_aligned16(proj) && scan_aligned16(alpha) && ldp % 4 == 0 && d % 4 == 0 && dv % 4 == 0 && vt % 4 == 0;
-    XB_SCAN_DISPATCH(linear_scan_kernel, ds, o, proj, ldp, alpha, state, q_start, slots, H, d, dv, scale, tt, stage, warps, vec)
+    XB_SCAN_DISPATCH_FEW(linear_scan_kernel, ds, longest <= kFewTokens, o, proj, ldp, alpha, state, q_start, slots, H, d, dv, scale, tt, stage, warps, vec)
     return xb_launch_status();
 }
 
 XB_EXPORT int xb_matrix_memory(float* o, float* div, const float* proj, long long ldp, int gate_off, const float* bi,
                                const float* bf, float cap, float* state_s, float* state_n, float* state_m, const int* q_start,
-                               const int* start_pos, const int* slots, int entries, int H, int d, int dv, float scale,
+                               const int* start_pos, const int* slots, int entries, int longest, int H, int d, int dv, float scale,
                                float div_eps, cudaStream_t stream) {
     if (entries <= 0) return 0;
     if (d < 1 || d > 32 * kRows || dv < 1 || H < 1 || H > 65535 || !(cap > 0.f)) return (int)cudaErrorInvalidValue;
@@ -1196,7 +1411,7 @@ XB_EXPORT int xb_matrix_memory(float* o, float* div, const float* proj, long lon
     const dim3 grid(entries, H, (dv + vt - 1) / vt);
     const int threads = (warps + 1 + (warps == 8 ? 3 : 4)) * 32;   // the warp of n, then three or four feeding warps
     const int vec = scan_aligned16(proj) && ldp % 4 == 0 && d % 4 == 0 && dv % 4 == 0 && vt % 4 == 0;
-    XB_SCAN_DISPATCH(matrix_memory_kernel, ds, o, div, proj, ldp, gate_off, bi, bf, cap, state_s, state_n, state_m, q_start,
+    XB_SCAN_DISPATCH_FEW(matrix_memory_kernel, ds, longest <= kFewTokens, o, div, proj, ldp, gate_off, bi, bf, cap, state_s, state_n, state_m, q_start,
                      start_pos, slots, H, d, dv, scale, div_eps, tt, stage, warps, vec)
     return xb_launch_status();
 }

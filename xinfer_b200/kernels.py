@@ -1403,10 +1403,17 @@ def conv_silu(y, u, u_off, taps, bias, state, req_of_token, q_start, slots, num_
                               int(num_entries), C, K, _stream()), "conv_state")
 
 
+def _longest(longest: Optional[int], tokens: int, entries: int) -> int:
+    """Tokens of the request that brings most; by default as many as one could bring beside others of one token.  Only the
+    choice between the forms of a scan depends on it, never what it computes."""
+    return int(longest) if longest is not None else max(1, tokens - max(int(entries), 1) + 1)
+
+
 def selective_scan(y, xbc, proj, dt_off, dt_bias, a_log, d_skip, state, q_start, slots, num_entries, heads, head_dim, n_state,
-                   groups):
+                   groups, longest: Optional[int] = None):
     """S <- exp(-exp(a_log) dt) S + dt B x^T, y = S^T C + d_skip x per (request, head); ``xbc`` float32 rows
-    ``[x | B | C]``, dt = softplus(proj[:, dt_off + h] + dt_bias); ``state`` ``[slots, heads, n_state, head_dim]``."""
+    ``[x | B | C]``, dt = softplus(proj[:, dt_off + h] + dt_bias); ``state`` ``[slots, heads, n_state, head_dim]``.
+    ``longest``: see ``_longest``."""
     T = xbc.shape[0]
     inner = heads * head_dim
     _need(xbc, "xbc", torch.float32, (T, inner + 2 * groups * n_state))
@@ -1417,21 +1424,22 @@ def selective_scan(y, xbc, proj, dt_off, dt_bias, a_log, d_skip, state, q_start,
     _need(state, "state", torch.float32, (None, heads, n_state, head_dim))
     _ok(kernels_lib().xb_selective_scan(y.data_ptr(), xbc.data_ptr(), xbc.shape[1], proj.data_ptr(), proj.shape[1], int(dt_off),
                                         dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(),
-                                        q_start.data_ptr(), slots.data_ptr(), int(num_entries), heads, head_dim, n_state, groups,
+                                        q_start.data_ptr(), slots.data_ptr(), int(num_entries), _longest(longest, T, num_entries),
+                                        heads, head_dim, n_state, groups,
                                         _stream()), "selective_scan")
 
 
-def delta_scratch_floats(tokens: int, entries: int, heads: int, d: int) -> int:
-    """Elements of scratch that ``delta_rule`` needs for a step."""
-    return int(kernels_lib().xb_delta_prep_floats(int(tokens), int(entries), int(heads), int(d)))
+def delta_scratch_floats(tokens: int, entries: int, heads: int, d: int, longest: Optional[int] = None) -> int:
+    """Elements of scratch that ``delta_rule`` needs for a step (0: none, where every request brings few tokens)."""
+    return int(kernels_lib().xb_delta_prep_floats(int(tokens), int(entries), _longest(longest, tokens, entries), int(heads), int(d)))
 
 
 def delta_rule(o, qkv, proj, beta_off, ag, dt_bias, a_log, state, q_start, slots, num_entries, heads, kv_heads, d, dv,
-               unit_eps: float = 1e-6, scratch=None):
+               unit_eps: float = 1e-6, scratch=None, longest: Optional[int] = None):
     """The gated delta rule per (request, head): ``qkv`` float32 rows ``[q | k | v]`` (q and k per key head), beta =
     sigmoid(proj[:, beta_off + h]), decay per (head, key channel) from the front of ``ag`` rows; ``state``
     ``[slots, heads, d, dv]``; ``o`` ``[T, heads * dv]`` before its norm and gate.  ``scratch``: float32, at least
-    ``delta_scratch_floats`` elements (default: made here)."""
+    ``delta_scratch_floats`` elements (default: made here).  ``longest``: see ``_longest``."""
     T = qkv.shape[0]
     _need(qkv, "qkv", torch.float32, (T, 2 * kv_heads * d + heads * dv))
     _need(proj, "proj", torch.float32, (T, None))
@@ -1440,21 +1448,24 @@ def delta_rule(o, qkv, proj, beta_off, ag, dt_bias, a_log, state, q_start, slots
     _need(dt_bias, "dt_bias", torch.float32, (heads * d,))
     _need(a_log, "a_log", torch.float32, (heads,))
     _need(state, "state", torch.float32, (None, heads, d, dv))
-    if scratch is None:
-        scratch = torch.empty(delta_scratch_floats(T, num_entries, heads, d), dtype=torch.float32, device=o.device)
-    _need(scratch, "scratch", torch.float32)
-    if scratch.numel() < delta_scratch_floats(T, num_entries, heads, d):
-        raise KernelError("the scratch of the delta rule is too small for the step")
+    longest = _longest(longest, T, num_entries)
+    need = delta_scratch_floats(T, num_entries, heads, d, longest)
+    if need and scratch is None:
+        scratch = torch.empty(need, dtype=torch.float32, device=o.device)
+    if need:
+        _need(scratch, "scratch", torch.float32)
+        if scratch.numel() < need:
+            raise KernelError("the scratch of the delta rule is too small for the step")
     _ok(kernels_lib().xb_delta_rule(o.data_ptr(), qkv.data_ptr(), qkv.shape[1], proj.data_ptr(), proj.shape[1], int(beta_off),
                                     ag.data_ptr(), ag.shape[1], dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(),
-                                    q_start.data_ptr(), slots.data_ptr(), int(num_entries), T, heads, kv_heads, d, dv,
-                                    float(unit_eps), scratch.data_ptr(), _stream()), "delta_rule", 2)
+                                    q_start.data_ptr(), slots.data_ptr(), int(num_entries), T, longest, heads, kv_heads, d, dv,
+                                    float(unit_eps), _ptr(scratch if need else None), _stream()), "delta_rule", 2 if need else 1)
 
 
-def linear_scan(o, proj, alpha, state, q_start, slots, num_entries, heads, d, dv, scale: float):
+def linear_scan(o, proj, alpha, state, q_start, slots, num_entries, heads, d, dv, scale: float, longest: Optional[int] = None):
     """Gated linear attention per (request, head): S <- diag(alpha) S + k v^T, o = scale * S^T q after the token's own
     write.  ``proj`` float32 rows ``[q | k | v | ...]``, ``alpha`` float32 ``[T, heads * d]``, ``state``
-    ``[slots, heads, d, dv]``; ``o`` ``[T, heads * dv]`` before its norm and gate."""
+    ``[slots, heads, d, dv]``; ``o`` ``[T, heads * dv]`` before its norm and gate.  ``longest``: see ``_longest``."""
     T = proj.shape[0]
     _need(proj, "proj", torch.float32, (T, None))
     if proj.shape[1] < heads * (2 * d + dv):
@@ -1463,7 +1474,8 @@ def linear_scan(o, proj, alpha, state, q_start, slots, num_entries, heads, d, dv
     _need(o, "o", torch.float32, (T, heads * dv))
     _need(state, "state", torch.float32, (None, heads, d, dv))
     _ok(kernels_lib().xb_linear_scan(o.data_ptr(), proj.data_ptr(), proj.shape[1], alpha.data_ptr(), state.data_ptr(),
-                                     q_start.data_ptr(), slots.data_ptr(), int(num_entries), heads, d, dv, float(scale),
+                                     q_start.data_ptr(), slots.data_ptr(), int(num_entries), _longest(longest, T, num_entries),
+                                     heads, d, dv, float(scale),
                                      _stream()), "linear_scan")
 
 
@@ -1550,13 +1562,13 @@ def gated_head_norm(out, y, gate, g_off, weight, part, eps, gate_after: bool, si
 
 
 def matrix_memory(o, div, proj, gate_off, b_in, b_forget, cap: float, state, q_start, start_pos, slots, num_entries, heads, d,
-                  dv, scale: float, div_eps: float):
+                  dv, scale: float, div_eps: float, longest: Optional[int] = None):
     """A matrix memory with exponential gates per (request, head): with the log gates i = cap tanh((z_i + b_in) / cap) and
     f = logsigmoid(cap tanh((z_f + b_forget) / cap)) and the running maximum m' = max(f + m, i),
     S <- e^(f + m - m') S + e^(i - m') k v^T, n likewise with k alone; ``o`` ``[T, heads * dv]`` = scale S^T q and ``div``
     ``[T, heads]`` = max(|scale n . q|, e^(-m')) + div_eps, both after the token's own write.  ``proj`` float32 rows
     ``[q | k | v | ...]`` with z_i and z_f (heads each) from column ``gate_off``.  ``state``: "S" ``[slots, heads, d, dv]``,
-    "n" ``[slots, heads, d]`` and "m" ``[slots, heads, 2, 2]``, all zero at a request's start."""
+    "n" ``[slots, heads, d]`` and "m" ``[slots, heads, 2, 2]``, all zero at a request's start.  ``longest``: see ``_longest``."""
     T = proj.shape[0]
     _need(proj, "proj", torch.float32, (T, None))
     if proj.shape[1] < max(heads * (2 * d + dv), gate_off + 2 * heads) or gate_off < 0:
@@ -1572,7 +1584,8 @@ def matrix_memory(o, div, proj, gate_off, b_in, b_forget, cap: float, state, q_s
     _ok(kernels_lib().xb_matrix_memory(o.data_ptr(), div.data_ptr(), proj.data_ptr(), proj.shape[1], int(gate_off),
                                        b_in.data_ptr(), b_forget.data_ptr(), float(cap), state["S"].data_ptr(),
                                        state["n"].data_ptr(), state["m"].data_ptr(), q_start.data_ptr(), start_pos.data_ptr(),
-                                       slots.data_ptr(), int(num_entries), heads, d, dv, float(scale), float(div_eps),
+                                       slots.data_ptr(), int(num_entries), _longest(longest, T, num_entries), heads, d, dv,
+                                       float(scale), float(div_eps),
                                        _stream()), "matrix_memory")
 
 

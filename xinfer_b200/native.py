@@ -133,14 +133,14 @@ def _declare_kernels(lib):
     _sig(lib, "xb_token_gate", I, [I, P, P, P, I, I, P, P, I, P, I, I, I, P, P])
     _sig(lib, "xb_conv_silu", I, [I, P, P, L, I, P, P, P, P, P, P, I, I, I, P])
     _sig(lib, "xb_conv_state", I, [I, P, P, L, I, P, P, I, I, I, P])
-    _sig(lib, "xb_selective_scan", I, [P, P, I, P, L, I, P, P, P, P, P, P, I, I, I, I, I, P])
-    _sig(lib, "xb_delta_rule", I, [P, P, I, P, L, I, P, L, P, P, P, P, P, I, I, I, I, I, I, F, P, P])
-    _sig(lib, "xb_delta_prep_floats", c_longlong, [I, I, I, I])
-    _sig(lib, "xb_linear_scan", I, [P, P, L, P, P, P, P, I, I, I, I, F, P])
+    _sig(lib, "xb_selective_scan", I, [P, P, I, P, L, I, P, P, P, P, P, P, I, I, I, I, I, I, P])
+    _sig(lib, "xb_delta_rule", I, [P, P, I, P, L, I, P, L, P, P, P, P, P, I, I, I, I, I, I, I, F, P, P])
+    _sig(lib, "xb_delta_prep_floats", c_longlong, [I, I, I, I, I])
+    _sig(lib, "xb_linear_scan", I, [P, P, L, P, P, P, P, I, I, I, I, I, F, P])
     _sig(lib, "xb_low_rank_decay", I, [P, P, L, P, P, I, I, I, F, P])
     _sig(lib, "xb_stream_conv", I, [I, P, P, P, P, P, P, P, P, P, P, I, I, I, F, F, F, I, P])
     _sig(lib, "xb_gated_head_norm", I, [I, P, P, P, L, I, P, I, I, I, I, F, I, P, L, F, P])
-    _sig(lib, "xb_matrix_memory", I, [P, P, P, L, I, P, P, F, P, P, P, P, P, P, I, I, I, I, F, F, P])
+    _sig(lib, "xb_matrix_memory", I, [P, P, P, L, I, P, P, F, P, P, P, P, P, P, I, I, I, I, I, F, F, P])
     _sig(lib, "xb_stream_mix", I, [I, I, P, P, P, L, L, P, P, P, P, P, P, I, I, I, I, F, F, P, P])
     _sig(lib, "xb_dyt_norm", I, [I, I, I, P, P, P, P, P, P, P, P, F, P, P, P, I, I, I, P, P])
     _sig(lib, "xb_latent_prepare", I,

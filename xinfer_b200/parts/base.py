@@ -100,6 +100,17 @@ class StepContext:
     # (float32 where the model keeps a float32 stream); None: the engine's dtype
     branch_dtype: Optional[torch.dtype] = None
 
+    def longest_portion(self) -> int:
+        """Tokens of the entry that brings most (a replayed step brings one of each)."""
+        if self.all_single or self.fixed_shapes:
+            return 1
+        if self.h_q_start is None or self.real_entries < 1:
+            return max(1, self.num_tokens)
+        if "longest_portion" not in self.scratch:
+            starts = self.h_q_start[: self.real_entries + 1]
+            self.scratch["longest_portion"] = int((starts[1:] - starts[:-1]).max(initial=1))
+        return self.scratch["longest_portion"]
+
 
 @dataclass(frozen=True)
 class CacheTensor:

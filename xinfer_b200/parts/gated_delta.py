@@ -102,9 +102,11 @@ class GatedDelta(Mixer):
         kernels.conv_silu(qkv, proj, 0, self.taps, None, state.get("conv"), ctx.req_of_token, ctx.q_start, ctx.slots,
                           ctx.num_entries)
         o = ws.get("gdelta.o", (T, self.vw), torch.float32)
+        longest = ctx.longest_portion()
+        need = kernels.delta_scratch_floats(T, ctx.num_entries, H, s.head_dim, longest)
         kernels.delta_rule(o, qkv, proj, C, ag, self.dt_bias, self.a_log, state["S"], ctx.q_start, ctx.slots, ctx.num_entries,
                            H, s.kv_heads, s.head_dim, s.v_head_dim, s.unit_eps,
-                           ws.get("gdelta.prep", (kernels.delta_scratch_floats(T, ctx.num_entries, H, s.head_dim),), torch.float32))
+                           ws.get("gdelta.prep", (need,), torch.float32) if need else None, longest)
         gated = ws.get("gdelta.gated", (T, self.vw), self.dtype)
         kernels.gated_head_norm(gated, o, ag, H * s.head_dim, self.norm_w, s.v_head_dim, s.eps, gate_after=True)
         out = ws.get("gdelta.out", (T, s.hidden), ctx.branch_dtype or self.dtype)

@@ -73,7 +73,8 @@ class GatedLinearAttention(Mixer):
         alpha = ws.get("gla.alpha", (T, self.qk), torch.float32)
         kernels.low_rank_decay(alpha, proj[:, at:at + self.w_decay.shape[1]], self.w_decay, self.decay_bias, s.tau)
         o = ws.get("gla.o", (T, self.vw), torch.float32)
-        kernels.linear_scan(o, proj, alpha, state["S"], ctx.q_start, ctx.slots, ctx.num_entries, H, d, dv, d ** -0.5)
+        kernels.linear_scan(o, proj, alpha, state["S"], ctx.q_start, ctx.slots, ctx.num_entries, H, d, dv, d ** -0.5,
+                            ctx.longest_portion())
         gated = ws.get("gla.gated", (T, self.vw), self.dtype)
         kernels.gated_head_norm(gated, o, proj, 2 * self.qk + self.vw, self.norm_w, dv, s.eps, gate_after=True, silu_gate=True)
         out = ws.get("gla.out", (T, s.hidden), ctx.branch_dtype or self.dtype)

@@ -76,7 +76,7 @@ class MatrixMemory(Mixer):
         o = ws.get("memory.o", (T, self.vw), torch.float32)
         div = ws.get("memory.div", (T, H), torch.float32)
         kernels.matrix_memory(o, div, proj, 2 * self.qk + 2 * self.vw, self.b_in, self.b_forget, s.gate_cap, state, ctx.q_start,
-                              ctx.start_pos, ctx.slots, ctx.num_entries, H, d, dv, d ** -0.5, s.divisor_eps)
+                              ctx.start_pos, ctx.slots, ctx.num_entries, H, d, dv, d ** -0.5, s.divisor_eps, ctx.longest_portion())
         kernels.gated_head_norm(out, o, proj, 2 * self.qk + self.vw, self.norm_w, dv, s.eps, gate_after=True, div=div,
                                 out_scale=out_scale)
 

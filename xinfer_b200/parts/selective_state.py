@@ -79,7 +79,7 @@ class SelectiveState(Mixer):
                           ctx.slots, ctx.num_entries)
         y = ws.get("sstate.y", (T, inner), torch.float32)
         kernels.selective_scan(y, xbc, proj, inner + C, self.dt_bias, self.a_log, self.d_skip, state["S"], ctx.q_start,
-                               ctx.slots, ctx.num_entries, s.heads, s.head_dim, s.state, s.groups)
+                               ctx.slots, ctx.num_entries, s.heads, s.head_dim, s.state, s.groups, ctx.longest_portion())
         gated = ws.get("sstate.gated", (T, inner), self.dtype)
         kernels.gated_head_norm(gated, y, proj, 0, self.norm_w, inner // s.norm_groups, s.eps, gate_after=False)
         out = ws.get("sstate.out", (T, s.hidden), ctx.branch_dtype or self.dtype)
