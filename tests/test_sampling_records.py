@@ -34,17 +34,25 @@ def _field_by_field(rec, params, seeds, draws, histories, hist):
 
 
 @pytest.mark.filterwarnings("ignore:overflow encountered")
-@pytest.mark.parametrize("rows", [[], [0], [1, 2, 8], list(range(len(ROWS))), [5, 5, 6, 7, 5]])
+@pytest.mark.parametrize("rows", [[], [0], [1, 2, 8], list(range(len(ROWS))), [5, 5, 6, 7, 5], [1] * 15, [1] * 16, [4] * 20, [5] * 20,
+                                  [1] * 19 + [8, 2]])
 @pytest.mark.parametrize("with_histories", [False, True])
 def test_records_hold_what_every_row_asked_for(rows, with_histories):
     params = [ROWS[i] for i in rows]
-    seeds, draws = [-1, 0, 2 ** 63, 7, 2 ** 40 + 5, 1, 2, 3, 4][:len(rows)], [2 ** 32 + 3, 0, -1, 5, 6, 7, 8, 9, 10][:len(rows)]
+    seeds, draws = ([-1, 0, 2 ** 63, 7, 2 ** 40 + 5, 1, -2 ** 62] * 4)[:len(rows)], ([2 ** 32 + 3, 0, -1, 5, 6] * 5)[:len(rows)]
     histories = [list(range(i, i + (PENALTY_HISTORY + 9 if i % 2 else 3))) for i in range(len(rows))] if with_histories else None
     made = []
     for fill in (fill_records, _field_by_field):
-        rec, hist = np.full(16, 255, dtype=np.uint8).repeat(40).view(kernels.SAMPLE_PARAMS).copy(), np.zeros(16 * PENALTY_HISTORY, dtype=np.int32)
+        rec, hist = np.full(24 * 40, 255, dtype=np.uint8).view(kernels.SAMPLE_PARAMS), np.zeros(24 * PENALTY_HISTORY, dtype=np.int32)
         made.append((fill(rec, params, seeds, draws, histories, hist), rec.tobytes(), hist.tobytes()))
     assert made[0] == made[1]
+
+
+def test_seeds_that_fit_64_signed_bits_and_others_are_filled_alike():
+    for seeds in ([2 ** 63] * 16, [2 ** 63 - 1] * 16, [-2 ** 63] * 16, [-2 ** 63 - 1] * 16, [0, 2 ** 64 + 9] * 8):
+        rec = np.zeros(16, dtype=kernels.SAMPLE_PARAMS)
+        fill_records(rec, [SHARED] * 16, seeds, [1] * 16, None, np.zeros(1, dtype=np.int32))
+        assert [int(r["seed_lo"]) | int(r["seed_hi"]) << 32 for r in rec] == [s & (2 ** 64 - 1) for s in seeds]
 
 
 def test_a_number_that_no_field_holds_is_refused():
