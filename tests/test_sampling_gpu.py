@@ -187,3 +187,27 @@ def test_logits_read_four_at_a_time_give_the_tokens_of_those_read_one_by_one(voc
                 s = Sampler(dev, rows)
                 got.append(s.to_host(s.sample(logits, [params[first + r] for r in range(rows)], list(range(rows)), [5] * rows)).tolist())
         assert got[:len(got) // 2] == got[len(got) // 2:]
+
+
+def test_calls_that_nobody_waits_for_keep_their_own_options():
+    from xinfer_b200.sampling import Sampler, SamplingParams
+    # The device is busy when the calls are made, so that none of their copies has begun when the next call is prepared.
+    R, V, calls = 3, 512, 40
+    g = torch.Generator(device="cuda:0").manual_seed(1)
+    logits = torch.randn(R, V, generator=g, device="cuda:0") * 3
+    ask = [dict(params=[SamplingParams(temperature=0.2 + 0.3 * i, frequency_penalty=0.5 * (i % 3))] * R, seeds=[i, i + 1, 2 ** 40 + i], draws=[i] * R,
+                histories=[list(range(i * 7, i * 7 + 40))] * R) for i in range(calls)]
+
+    def run(busy):
+        sampler = Sampler("cuda:0", R)
+        copies = [logits.clone() for _ in ask]
+        torch.cuda.synchronize()
+        if busy:
+            torch.cuda._sleep(200_000_000)      # about a tenth of a second
+        out = []
+        for one, rows in zip(ask, copies):
+            out.append(sampler.sample(rows, one["params"], one["seeds"], one["draws"], one["histories"]).clone())
+            if not busy:
+                torch.cuda.synchronize()
+        return torch.stack(out).cpu()
+    assert torch.equal(run(True), run(False))

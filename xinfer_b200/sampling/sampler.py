@@ -60,6 +60,44 @@ def fill_records(records: np.ndarray, params: Sequence[SamplingParams], seeds, d
     return off
 
 
+class _PinnedSet:
+    """Where one call's records and counted tokens lie on the host until they have been copied."""
+
+    def __init__(self, max_rows: int, record_bytes: int):
+        self.params = torch.zeros(max_rows * record_bytes, dtype=torch.uint8, pin_memory=True)
+        self.params_np = self.params.numpy().view(kernels.SAMPLE_PARAMS)
+        self.hist = self.hist_np = None
+
+    def history(self, max_rows: int) -> np.ndarray:
+        if self.hist is None:
+            self.hist = torch.zeros(max_rows * PENALTY_HISTORY, dtype=torch.int32, pin_memory=True)
+            self.hist_np = self.hist.numpy()
+        return self.hist_np
+
+
+class _PinnedSets:
+    """Pinned sets used in turn by calls that nobody may have waited for.  Half of them are taken again only after the copies that
+    read them have been made: one event per half, since recording and asking one for every call took a tenth of its time."""
+
+    def __init__(self, max_rows: int, record_bytes: int, half: int = 8):
+        self.sets = [_PinnedSet(max_rows, record_bytes) for _ in range(2 * half)]
+        self.copied = [torch.cuda.Event(), torch.cuda.Event()]
+        self.half, self.at = half, 0
+
+    def take(self) -> _PinnedSet:
+        """A set that no copy reads any more."""
+        if self.at % self.half == 0:
+            self.copied[self.at // self.half].synchronize()
+        return self.sets[self.at]
+
+    def sent(self) -> None:
+        """The set last taken has been handed to its copies."""
+        self.at += 1
+        if self.at % self.half == 0:
+            self.copied[self.at // self.half - 1].record()
+            self.at %= 2 * self.half
+
+
 class Sampler:
     def __init__(self, device, max_rows: int, out_dev: Optional[torch.Tensor] = None,
                  err_word: Optional[torch.Tensor] = None):
@@ -70,17 +108,14 @@ class Sampler:
         self.max_rows = max_rows
         self.err_word = err_word
         rec = kernels.SAMPLE_PARAMS.itemsize
-        self._params_host = torch.zeros(max_rows * rec, dtype=torch.uint8, pin_memory=True)
+        self._pinned = _PinnedSets(max_rows, rec)
         self._params_dev = torch.zeros(max_rows * rec, dtype=torch.uint8, device=device)
-        self._hist_host = torch.zeros(max_rows * PENALTY_HISTORY, dtype=torch.int32, pin_memory=True)
         self._hist_dev = torch.zeros(max_rows * PENALTY_HISTORY, dtype=torch.int32, device=device)
         self._out_dev = out_dev if out_dev is not None else torch.zeros(max_rows + 1, dtype=torch.int32, device=device)
         if self._out_dev.numel() < max_rows + 1 or self._out_dev.dtype != torch.int32:
             raise ValueError("the sampler's output buffer must hold max_rows + 1 int32")
         self._out_host = torch.zeros(max_rows + 1, dtype=torch.int32, pin_memory=True)
         self._scratch = torch.zeros(kernels.sample_scratch_bytes(max_rows), dtype=torch.uint8, device=device)
-        self._params_np = self._params_host.numpy().view(kernels.SAMPLE_PARAMS)
-        self._hist_np = self._hist_host.numpy()
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int],
                draws: Sequence[int], histories: Optional[Sequence[Sequence[int]]] = None) -> torch.Tensor:
@@ -90,12 +125,14 @@ class Sampler:
         R = logits.shape[0]
         if R > self.max_rows:
             raise ValueError(f"{R} rows exceed the sampler's capacity {self.max_rows}")
-        off = fill_records(self._params_np, params[:R], seeds, draws, histories, self._hist_np)
+        mine = self._pinned.take()
+        off = fill_records(mine.params_np, params[:R], seeds, draws, histories, mine.history(self.max_rows) if histories is not None else None)
         any_pen = off > 0
         nb = R * kernels.SAMPLE_PARAMS.itemsize
-        self._params_dev[:nb].copy_(self._params_host[:nb], non_blocking=True)
+        self._params_dev[:nb].copy_(mine.params[:nb], non_blocking=True)
         if any_pen:
-            self._hist_dev[:off].copy_(self._hist_host[:off], non_blocking=True)
+            self._hist_dev[:off].copy_(mine.hist[:off], non_blocking=True)
+        self._pinned.sent()
         if tracing.ENABLED:
             tracing.push("sample")
         kernels.sample(self._out_dev, logits, self._params_dev, self._hist_dev, any_pen, self._scratch, self.err_word,
