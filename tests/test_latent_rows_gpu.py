@@ -143,3 +143,33 @@ def test_a_model_gives_the_same_logits_both_ways_and_for_mixed_steps(design, mon
     assert none == 0 and some == 6
     # two bfloat16 computations of the same numbers
     assert (got - want).norm() <= 0.02 * want.norm()
+
+
+@pytest.mark.parametrize("counts,starts,window,most", [([1], [0], None, 4), ([5, 4, 300], [7, 900, 40], None, 4), ([5, 4, 300, 1], [7, 900, 40, 0], 33, 4),
+                                                       ([2, 2], [9, 9], 1, 0)])
+def test_the_sums_over_portions(counts, starts, window, most):
+    got = kernels.portion_sums(np.concatenate([[0], np.cumsum(counts)]), starts, len(counts), most, window)
+    for part, at in ((lambda n: n > most, 0), (lambda n: n <= most, 5)):
+        them = [(n, s if not window else min(s, window)) for n, s in zip(counts, starts) if part(n)]
+        pairs = [n * s + n * (n + 1) / 2 for n, s in them]
+        if window:
+            pairs = [min(p, n * window) for p, (n, _) in zip(pairs, them)]
+        assert got[at:at + 5] == [len(them), sum(n for n, _ in them), sum(n + s for n, s in them), sum(pairs),
+                                  max([n + s for n, s in them], default=0)]
+
+
+# What was measured as steps of four layers: which way was the faster one (heads, rank; portions; requests that decode at a context).
+@pytest.mark.parametrize("heads,rank,prompts,live,context,pays", [
+    (32, 512, [(0, 2048)], 0, 0, True), (32, 512, [(3000, 300)], 0, 0, True), (32, 512, [(2000, 16)], 0, 0, True), (16, 256, [(3000, 300)], 0, 0, True),
+    (32, 512, [(0, 1275), (0, 632)], 0, 0, True), (16, 256, [(0, 100)] * 8, 0, 0, False), (32, 512, [(0, 30)], 32, 1000, False),
+    (32, 512, [(0, 512)], 4, 500, False), (32, 512, [(0, 512)], 16, 1000, False), (32, 512, [(0, 200)], 24, 2000, False),
+    (32, 512, [(0, 512)], 48, 3000, False), (32, 512, [(0, 100)], 8, 4000, False), (32, 512, [(1000, 40)] * 3, 4, 200, False),
+    (32, 512, [(0, 2048)], 4, 500, True), (32, 512, [(0, 6)], 8, 1000, False)])
+def test_the_way_that_was_measured_to_be_faster_is_taken(heads, rank, prompts, live, context, pays):
+    from types import SimpleNamespace as N
+    from xinfer_b200.parts.latent_attention import rows_pay
+    counts, starts = [1] * live + [n for _, n in prompts], [context] * live + [s for s, _ in prompts]
+    ctx = N(max_context=max(a + b for a, b in zip(counts, starts)), real_tokens=sum(counts), real_entries=len(counts),
+            h_q_start=np.concatenate([[0], np.cumsum(counts)]), h_start_pos=np.asarray(starts))
+    got = rows_pay(ctx, heads, 128, rank // 8, 128, rank, rank + rank // 8, None)
+    assert got == (live if pays else None)

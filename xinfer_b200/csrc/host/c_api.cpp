@@ -243,6 +243,22 @@ XB_API long long xb_attn_prefill_work(int B, const int* counts, const int* start
     return (long long)ctas + 1 + INTS * n_items;
 }
 
+// What a step's portions bring and see, of those of more than `most` tokens and of the others:
+// out[0..4]: portions, tokens, keys seen, pairs of query and key, longest walk of a query over keys; out[5..9]: of the others.
+XB_API void xb_portion_sums(int B, const int* q_start, const int* starts, int most, int window, double* out) {
+    for (int i = 0; i < 10; ++i) out[i] = 0;
+    for (int b = 0; b < B; ++b) {
+        const double n = q_start[b + 1] - q_start[b], before = window > 0 ? std::min(starts[b], window) : starts[b];
+        double* o = out + (n > most ? 0 : 5), pairs = n * before + n * (n + 1) / 2;
+        if (window > 0) pairs = std::min(pairs, n * window);
+        o[0] += 1;
+        o[1] += n;
+        o[2] += before + n;
+        o[3] += pairs;
+        o[4] = std::max(o[4], before + n);
+    }
+}
+
 // ---- work lists of the attention over keys and values formed for the step --------------------------
 // The step's portions of more than dec_max tokens: their visible rows lie one portion after the other, from the 64-key
 // tile of the first query's first key on, in runs of 64 rows.  Items are 256 (or 128) queries of one head; they go,

@@ -1170,6 +1170,18 @@ def attn_rows_tc_takes(d: int, rd: int, dv: int, rank: int) -> bool:
     return bool(kernels_lib().xb_attn_rows_tc_takes(int(d), int(rd), int(dv), int(rank)))
 
 
+def portion_sums(q_start, starts, entries: int, most: int, window) -> list:
+    """[portions, tokens, keys they see, pairs of query and key, longest walk of a query over keys] of a step's portions of more
+    than ``most`` tokens, then the same five of the others.  ``q_start`` and ``starts``: host arrays of a step."""
+    from .native import host_lib
+    q_start, starts = np.ascontiguousarray(q_start, dtype=np.int32), np.ascontiguousarray(starts, dtype=np.int32)
+    if len(q_start) <= entries or len(starts) < entries:
+        raise KernelError("the step has fewer entries than that")
+    out = (ctypes.c_double * 10)()
+    host_lib().xb_portion_sums(int(entries), q_start.ctypes.data, starts.ctypes.data, int(most), int(window or 0), out)
+    return list(out)
+
+
 def latent_prefill_work(counts, starts, dec_max: int, window, heads: int, max_ctas: int = PREFILL_TC_MAX_CTAS, host_buffer=None):
     """The work list of ``attn_rows_tc`` for a step whose entries bring ``counts`` tokens after ``starts`` cached ones
     (host arrays): (pinned int32 host tensor, CTAs, rows the portions see, where the list of the rows' runs begins).  The

@@ -59,6 +59,7 @@ def _declare_host(lib):
     _sig(lib, "xb_cm_consistent", c_int, [c_void_p, c_char_p, c_int])
     _sig(lib, "xb_attn_prefill_work", c_longlong,
          [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p])
+    _sig(lib, "xb_portion_sums", None, [c_int, c_void_p, c_void_p, c_int, c_int, c_void_p])
     _sig(lib, "xb_latent_prefill_work", c_longlong,
          [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p])
     _sig(lib, "xb_talk_work", c_int,

@@ -26,7 +26,6 @@ from __future__ import annotations
 
 from typing import List
 
-import numpy as np
 import torch
 
 from .. import kernels
@@ -63,12 +62,32 @@ ROWS_MAX_BYTES = 1 << 30
 # rate), of the products that form keys and values, and of the attention on those (780 measured at a prompt of 2,048
 # tokens and 32 heads, where the first way took 1,570 us and the second takes 55 + 18 us); beside that what the second way
 # costs the host, which a short prompt waits for: its work list and launches, more where the step's small portions need the
-# first way too.  Measured per layer on the device (rank 512, 32 heads): 8 tokens after 3,000 cached ones 235 us less the second
-# way, 16 tokens alone 6 us less; 20 portions of 8 tokens after 1,000 cached ones 145 us less the first.  Measured as steps of
-# four layers, first and second way: 8 prompts of 100 tokens 1,463 and 1,683 us at 16 heads of rank 256, 1,810 and 2,067 us at
-# 32 heads of rank 512; 2 prompts of 400 tokens 1,202 and 1,388 us, 2,100 and 2,009 us.
+# first way too - which then takes what it takes for those, whose longest walk is often the longest of all.  Measured per layer
+# on the device (rank 512, 32 heads): 8 tokens after 3,000 cached ones 235 us less the second way, 16 tokens alone 6 us less; 20
+# portions of 8 tokens after 1,000 cached ones 145 us less the first.  Measured as steps of four layers, first and second way: 8
+# prompts of 100 tokens 1,463 and 1,683 us at 16 heads of rank 256, 1,810 and 2,067 us at 32 heads of rank 512; 2 prompts of 400
+# tokens 1,202 and 1,388 us, 2,100 and 2,009 us; beside requests that decode (32 heads of rank 512) 512 tokens and 48 requests at
+# 3,000 cached ones 2,585 and 2,949 us, three times 40 tokens after 1,000 and four requests at 200 1,239 and 1,489 us.
 ROWS_RATES = (75e6, 900e6, 700e6, 60.0, 90.0)
 ROWS_SMS = 148
+
+
+def rows_pay(ctx: StepContext, heads: int, d: int, rd: int, dv: int, rank: int, width: int, window):
+    """Whether the step's portions of more than ``ROWS_MIN_TOKENS`` tokens are better off on keys and values formed per head:
+    None, or the tokens of the other portions."""
+    over_rows, form, over_heads, alone, beside = ROWS_RATES
+    ops = 2 * (width + rank)
+    # (no more pairs than tokens times the longest context: most short steps are decided by this alone)
+    if ops * ctx.max_context * max(ctx.real_tokens * heads, 32 * ROWS_SMS) <= over_rows * alone:
+        return None
+    many, _, keys, pairs, walk, others, tokens, _, o_pairs, o_walk = kernels.portion_sums(ctx.h_q_start, ctx.h_start_pos, ctx.real_entries,
+                                                                                      ROWS_MIN_TOKENS, window)
+    if not many or (keys + 64 * many) * heads * (d + dv) * 2 > ROWS_MAX_BYTES:
+        return None
+    first = ops / over_rows * max((pairs + o_pairs) * heads, max(walk, o_walk) * 32 * ROWS_SMS)
+    second = ops / over_rows * max(o_pairs * heads, o_walk * 32 * ROWS_SMS) + (beside if others else alone) \
+        + keys * heads * 2 * rank * (d + dv) / form + pairs * heads * 2 * (d + rd + dv) / over_heads
+    return int(tokens) if second < first else None
 
 
 def rows_plan(ctx: StepContext, heads: int, d: int, rd: int, dv: int, rank: int, width: int, window):
@@ -79,26 +98,14 @@ def rows_plan(ctx: StepContext, heads: int, d: int, rd: int, dv: int, rank: int,
     if key in ctx.scratch:
         return ctx.scratch[key]
     made = None
-    # (no more pairs than tokens times the longest context: most short steps are decided by this alone)
-    most = ctx.max_context * max(ctx.real_tokens * heads, 32 * ROWS_SMS)
-    if not (ctx.fixed_shapes or ctx.all_single) and 2 * (width + rank) * most > ROWS_RATES[0] * ROWS_RATES[3] and USE_TENSOR_CORES and ctx.dtype == torch.bfloat16 and width % 8 == 0 \
+    if not (ctx.fixed_shapes or ctx.all_single) and USE_TENSOR_CORES and ctx.dtype == torch.bfloat16 and width % 8 == 0 \
             and kernels.attn_rows_tc_takes(d, rd, dv, rank) and kernels.attn_latent_mma_takes(width, rank):
-        counts = np.diff(ctx.h_q_start[: ctx.real_entries + 1]).astype(np.int64)
-        starts = ctx.h_start_pos[: ctx.real_entries].astype(np.int64)
-        long = counts > ROWS_MIN_TOKENS
-        n, before = counts[long], starts[long]
-        if window:
-            before = np.minimum(before, window)
-        keys, pairs = float((before + n).sum()), float((n * before + n * (n + 1) / 2).sum())
-        if window:
-            pairs = min(pairs, float(n.sum()) * window)
-        over_rows, form, over_heads, alone, beside = ROWS_RATES
-        first = 2 * (width + rank) / over_rows * max(pairs * heads, float((before + n).max(initial=0)) * 32 * ROWS_SMS)
-        second = (alone if long.all() else beside) + keys * heads * 2 * rank * (d + dv) / form + pairs * heads * 2 * (d + rd + dv) / over_heads
-        if len(n) and second < first and (keys + 64 * len(n)) * heads * (d + dv) * 2 <= ROWS_MAX_BYTES:
-            host, ctas, rows, runs_at = kernels.latent_prefill_work(counts, starts, ROWS_MIN_TOKENS, window, heads,
-                                                                    host_buffer=_rows_ring.take)
-            made = (host.to(ctx.positions.device, non_blocking=True), ctas, rows, runs_at, int(counts[~long].sum()))
+        small = rows_pay(ctx, heads, d, rd, dv, rank, width, window)
+        if small is not None:
+            starts = ctx.h_q_start[: ctx.real_entries + 1]
+            host, ctas, rows, runs_at = kernels.latent_prefill_work(starts[1:] - starts[:-1], ctx.h_start_pos[: ctx.real_entries],
+                                                                    ROWS_MIN_TOKENS, window, heads, host_buffer=_rows_ring.take)
+            made = (host.to(ctx.positions.device, non_blocking=True), ctas, rows, runs_at, small)
             _rows_ring.sent()
     ctx.scratch[key] = made
     return made
