@@ -173,3 +173,23 @@ def test_the_way_that_was_measured_to_be_faster_is_taken(heads, rank, prompts, l
             h_q_start=np.concatenate([[0], np.cumsum(counts)]), h_start_pos=np.asarray(starts))
     got = rows_pay(ctx, heads, 128, rank // 8, 128, rank, rank + rank // 8, None)
     assert got == (live if pays else None)
+
+
+def _one_portion(T, heads, d, dv, rank, g):
+    """What ``attn_rows_tc`` takes for a prompt of T tokens: (work, CTAs, q, kv, rows, q_start, start_pos, err)."""
+    host, ctas, n, _ = kernels.latent_prefill_work([T], [0], 4, None, heads)
+    bf = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
+    i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    return host.to(DEV), ctas, bf(T, heads * d), bf(n, heads * (d + dv)), bf(n, rank), i32(0, T), i32(0), i32(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("key", [0, 3, 7, 38, 63, 64, 130])
+def test_a_key_that_is_not_a_number_shows_in_every_query_that_sees_it(key):
+    T, H, d, dv, rank = 200, 2, 64, 64, 64
+    work, ctas, q, kv, rows, q_start, start_pos, err = _one_portion(T, H, d, dv, rank, torch.Generator().manual_seed(key))
+    out = torch.zeros(T, H * dv, dtype=torch.bfloat16, device=DEV)
+    kv[key, :H * d] = float("nan")           # the keys of both heads; the values stay numbers
+    kernels.attn_rows_tc(out, q, H * d, kv, rows, work, ctas, q_start, start_pos, H, d, 0, dv, rank, None, d ** -0.5, None, err)
+    bad = torch.isnan(out)
+    assert int(err) == 0 and bad[key:].all() and not bad[:key].any()

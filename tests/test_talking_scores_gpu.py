@@ -162,3 +162,28 @@ def test_short_steps_stay_on_the_kernel_that_holds_all_heads(heads, counts, star
     ctx = N(max_context=max(a + b for a, b in zip(counts, starts)), real_tokens=sum(counts), real_entries=len(counts),
             h_q_start=np.concatenate([[0], np.cumsum(counts)]), h_start_pos=np.asarray(starts))
     assert TalkingAttention._scores_pay(layer, ctx) == pays
+
+
+def _prompt(T, H, G, d, dv, g, vary=1.0):
+    """A prompt of T tokens on pages of 16: (q, keys, values, table, work lists, scratch, the rest of the arguments)."""
+    bf = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    i32 = lambda a: torch.tensor(np.asarray(a), dtype=torch.int32, device=DEV)
+    n = -(-T // 16)
+    host, chunks, tiles = kernels.talk_work([T], [0], None, H, G, 1 << 16)
+    scores = torch.empty(tiles * kernels.TALK_TILE_FLOATS, device=DEV)
+    return ((vary * bf(T, H, d)).to(DEV), bf(n, G, 16, d).to(DEV), bf(n, G, 16, dv).to(DEV), i32([range(n)]), (host.to(DEV), chunks), scores,
+            (i32([0, T]), i32([0])), i32([0]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("key", [0, 3, 7, 38, 63, 64, 130])
+def test_a_key_that_is_not_a_number_shows_in_every_query_that_sees_it(key):
+    T, H, G, d, dv = 200, 8, 4, 64, 64
+    g = torch.Generator().manual_seed(key)
+    q, k, v, table, (work, chunks), scores, (q_start, start_pos), err = _prompt(T, H, G, d, dv, g)
+    k[key // 16, :, key % 16] = float("nan")
+    talk = torch.randn(H, H, generator=g)
+    out = torch.zeros(T, H * dv, dtype=torch.bfloat16, device=DEV)
+    kernels.attn_talking_tc(out, q, k, v, talk, scores, work, chunks, q_start, start_pos, table, table.shape[1], None, d ** -0.5, True, 1.0, err)
+    bad = torch.isnan(out)
+    assert int(err) == 0 and bad[key:].all() and not bad[:key].any()

@@ -344,9 +344,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     for (int c = 0; c < 8; c += 2)
                         unpack2(fma2(pack2(sc[c8 * 8 + c], sc[c8 * 8 + c + 1]), scale2, mneg2), x[c], x[c + 1]);
 #pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        if ((c & 3) != 3) e[c] = ex2(x[c]);
-                    ex2_poly2(x[3], x[7], e[3], e[7]);
+                    for (int c = 0; c < 8; ++c) e[c] = ex2(x[c]);
                     sum_a = add2(sum_a, add2(pack2(e[0], e[1]), pack2(e[2], e[3])));
                     sum_b = add2(sum_b, add2(pack2(e[4], e[5]), pack2(e[6], e[7])));
                     pk[c8 * 4] = pack_bf16(e[0], e[1]);
