@@ -187,3 +187,18 @@ def test_a_key_that_is_not_a_number_shows_in_every_query_that_sees_it(key):
     kernels.attn_talking_tc(out, q, k, v, talk, scores, work, chunks, q_start, start_pos, table, table.shape[1], None, d ** -0.5, True, 1.0, err)
     bad = torch.isnan(out)
     assert int(err) == 0 and bad[key:].all() and not bad[:key].any()
+
+
+@pytest.mark.gpu
+def test_weights_are_divided_by_their_own_sum():
+    # Values that are all one: the result is the sum of the rounded weights over what it is divided by, times the factor.  The
+    # factor lies 2^-14 above the middle between two bfloat16 numbers, so that a quotient that is off by more than that rounds to
+    # the lower one (weights that are summed before they are rounded: by up to 2^-9); float32 sums of 200 terms are off by 2^-20.
+    T, H, G, d, dv = 200, 8, 4, 64, 64
+    g = torch.Generator().manual_seed(5)
+    q, k, v, table, (work, chunks), scores, (q_start, start_pos), err = _prompt(T, H, G, d, dv, g, vary=2.0)
+    out = torch.zeros(T, H * dv, dtype=torch.bfloat16, device=DEV)
+    factor = 1.0 + 2.0 ** -8 + 2.0 ** -14
+    kernels.attn_talking_tc(out, q, k, torch.ones_like(v), torch.eye(H), scores, work, chunks, q_start, start_pos, table, table.shape[1], None,
+                            d ** -0.5, False, factor, err)
+    assert int(err) == 0 and (out == 1.0 + 2.0 ** -7).all()

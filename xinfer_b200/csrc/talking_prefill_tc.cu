@@ -12,8 +12,9 @@
 //                           work item.  Bound by reading the tiles: 4 bytes per pair and head, 280 MB at 2,048 tokens.
 //
 // 2,048 tokens: 1,890 us -> 135 + 64 us with 32 heads, 1,088 us -> 51 + 43 us with 16.
-// Nothing is rounded that was not before: the mixed scores leave as float32.  Steps whose tiles would not fit the scratch
-// memory run as several pairs of launches over fewer queries each.
+// What is rounded is what talking_attention_mma.cu rounds: the weights, once, in front of their product with the values, and it
+// is the rounded ones that are summed; the mixed scores leave as float32.  Steps whose tiles would not fit the scratch memory run
+// as several pairs of launches over fewer queries each.
 #include "attention_common.cuh"
 #include "tc_common.cuh"
 
@@ -595,12 +596,16 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* __
                     for (int c = 0; c < 8; c += 2) unpack2(add2(pack2(sc[c8 * 8 + c], sc[c8 * 8 + c + 1]), mneg2), x[c], x[c + 1]);
 #pragma unroll
                     for (int c = 0; c < 8; ++c) e[c] = ex2(x[c]);
-                    sum_a = add2(sum_a, add2(pack2(e[0], e[1]), pack2(e[2], e[3])));
-                    sum_b = add2(sum_b, add2(pack2(e[4], e[5]), pack2(e[6], e[7])));
-                    pk[c8 * 4] = pack_bf16(e[0], e[1]);
-                    pk[c8 * 4 + 1] = pack_bf16(e[2], e[3]);
-                    pk[c8 * 4 + 2] = pack_bf16(e[4], e[5]);
-                    pk[c8 * 4 + 3] = pack_bf16(e[6], e[7]);
+                    // the sum is that of the weights as the product sees them
+                    f32x2 w[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint32_t two = pack_bf16(e[2 * c], e[2 * c + 1]);
+                        pk[c8 * 4 + c] = two;
+                        w[c] = pack2(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u));
+                    }
+                    sum_a = add2(sum_a, add2(w[0], w[1]));
+                    sum_b = add2(sum_b, add2(w[2], w[3]));
                 }
                 float s0, s1, s2, s3;
                 unpack2(sum_a, s0, s1);
