@@ -58,3 +58,28 @@ def test_successors_start_only_once_tensor_memory_is_allocated(path):
         for at in starts:
             leaves = re.match(r"pdl_launch_dependents\(\);\s*pdl_wait\(\);\s*return;", body[at:])
             assert at > allocated or leaves, f"{name} lets its successor start before it has allocated tensor memory"
+
+
+# Pointers that may be declared __restrict__ in a kernel that waits for its predecessor: weights and what the host sent before the
+# step, which no kernel writes; and plain outputs, whose values come from loads behind the wait.
+SENT = set("""rows w b b_alpha b_w b_b w_r correction req_of_token table ids positions q_start slots start_pos block_table norm_w inv_freq
+              cq_w sink blocks work bw gain wl wr bias bz bx coef taps dt_bias A_log Dv bi bf q_w k_w dense_weight""".split())
+OUTPUTS = set("out y o act prep scores alpha div q_out k_cache v_cache cq choice weight gate prodA endB start cache prev_state".split())
+
+
+@pytest.mark.parametrize("path", [f for f in FILES if re.search(r"pdl_(wait|overlap_few)\(\)", open(f).read())], ids=os.path.basename)
+def test_what_a_predecessor_writes_is_not_promised_to_stay(path):
+    # A pointer to const with __restrict__ says that its data does not change while the kernel runs, and one that is read and
+    # written that nobody else does: their loads may then be moved in front of the wait.
+    for name, params, body in kernels_of(path):
+        if not re.search(r"pdl_(wait|overlap_few)\(\)", body):
+            continue
+        for p in params.split(","):
+            if "__restrict__" not in p:
+                continue
+            word = re.findall(r"\w+", p)[-1]
+            if "const" in p.split("*")[0].split():
+                ok = word in SENT or (name, word) == ("dyt_kernel", "alpha")
+            else:
+                ok = word in OUTPUTS
+            assert ok, f"{name}: {' '.join(p.split())}"

@@ -318,13 +318,13 @@ attn_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __rest
 // ------------------------------------------------------------------------------------------------
 template <int DP>
 __global__ void __launch_bounds__(128)
-attn_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
-                   const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc,
-                   const __nv_bfloat16* __restrict__ vc, const int* __restrict__ positions,
+attn_decode_kernel(__nv_bfloat16* __restrict__ out, float* part_o, float* part_ml,
+                   const __nv_bfloat16* q, const __nv_bfloat16* kc,
+                   const __nv_bfloat16* vc, const int* __restrict__ positions,
                    const int* __restrict__ req_of_token, const int* __restrict__ q_start, int num_entries,
                    const int* __restrict__ block_table, int table_stride, int nh, int nkv, int d, int ps,
                    int ps_shift, int num_pages, int window, float scale_log2, int dec_max, int direct, int split,
-                   int num_splits, int page_cap, int* __restrict__ tickets, int* err) {
+                   int num_splits, int page_cap, int* tickets, int* err) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr int NT = 128;

@@ -696,11 +696,11 @@ template <int DP, bool EXT>
 __global__ void __launch_bounds__(128, 2)
 attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
-                      float* __restrict__ part_o, float* __restrict__ part_ml, const int* __restrict__ plan,
+                      float* part_o, float* part_ml, const int* plan,
                       const int* __restrict__ block_table, int table_stride, int nh, int nkv, int dv, long long ldo, int ps,
                       int ps_shift, int num_pages, int keep, float scale_log2_in, float softcap, float slope_exp,
                       const float* __restrict__ sink, float out_scale, int dec_max,
-                      int splits_max, int page_cap, int* __restrict__ tickets, int* err) {
+                      int splits_max, int page_cap, int* tickets, int* err) {
     constexpr int HALVES = DP / 64, DEC_STAGES = dec_stages(DP);
     if (!EXT) {     // as for the prefill kernel
         softcap = slope_exp = 0.f;

@@ -112,6 +112,8 @@ static inline int xb_launch_status() { return (int)cudaGetLastError(); }
 // kernel before it in the stream is still running; it calls pdl_wait() before it touches anything
 // that kernel may have written (or still reads), and pdl_launch_dependents() as early as it likes
 // to let the kernel after it do the same.  Both are no-ops in a kernel launched the plain way.
+// What a predecessor writes is read through pointers without __restrict__: that word promises that nobody else writes there
+// while the kernel runs, so that the compiler may load in front of the wait.
 // A kernel that allocates tensor memory lets the next one start only once every thread block has its columns (and a block
 // that allocates none, where it leaves): the next kernel's blocks hold theirs while they wait for this grid's end, so a block
 // of this grid that still waited for columns on the same processor would wait for ever, and so would they.

@@ -14,7 +14,7 @@
 #include "common.cuh"
 
 template <typename TX, typename TB, typename TO>
-__global__ void dyt_kernel(TO* __restrict__ out, TX* sum_out, const TX* x, const TB* __restrict__ branch,
+__global__ void dyt_kernel(TO* __restrict__ out, TX* sum_out, const TX* x, const TB* branch,
                            const int* __restrict__ rows, const float* __restrict__ alpha, const float* __restrict__ w,
                            const float* __restrict__ b, float branch_scale, const float* __restrict__ b_alpha,
                            const float* __restrict__ b_w, const float* __restrict__ b_b, int nrows, int dim, int src_rows,

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_bf16_kernel(__nv_bfloat16* __res
 constexpr int SWIGLU_THREADS = 128;
 template <int SWIGLU_UNROLL, int ACT>
 __global__ void __launch_bounds__(SWIGLU_THREADS)
-swiglu_bf16_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ gu, int inter, int tokens, float p0,
+swiglu_bf16_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* gu, int inter, int tokens, float p0,
                    float p1) {
     pdl_launch_dependents();
     pdl_wait();
@@ -139,7 +139,7 @@ swiglu_bf16_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restr
 constexpr int SG_THREADS = 128, SG_U = 4;
 template <int ACT>
 __global__ void __launch_bounds__(SG_THREADS)
-swiglu_rows_bf16_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ gu, int inter, int tokens, float p0,
+swiglu_rows_bf16_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* gu, int inter, int tokens, float p0,
                         float p1) {
     pdl_launch_dependents();
     pdl_wait();
@@ -184,7 +184,7 @@ swiglu_rows_bf16_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __
 // A group of LPH lanes owns one (token, head); the arithmetic is that of qk_rope.cuh.  What does not
 // depend on the projection (positions, pages, weights, angles) is fetched before the wait for its producer.
 template <int LPH>
-__global__ void qk_norm_rope_write_bf16_kernel(const xbqk::QkArgs A, const __nv_bfloat16* __restrict__ qkv, int tokens, int* err) {
+__global__ void qk_norm_rope_write_bf16_kernel(const xbqk::QkArgs A, const __nv_bfloat16* qkv, int tokens, int* err) {
     pdl_launch_dependents();
     const int total_heads = A.nh + 2 * A.nkv;
     const int groups_per_block = blockDim.x / LPH;

@@ -39,7 +39,7 @@ __device__ __forceinline__ void router_load4<__nv_bfloat16>(const __nv_bfloat16*
 
 template <typename T, int ROUTER_TOKENS>
 __global__ void __launch_bounds__(ROUTER_MAX_WARPS * 32)
-expert_router_kernel(int* __restrict__ choice, float* __restrict__ weight, const T* __restrict__ h,
+expert_router_kernel(int* __restrict__ choice, float* __restrict__ weight, const T* h,
                      const float* __restrict__ w_r, const float* __restrict__ correction,
                      const int* __restrict__ req_of_token, float* __restrict__ gate, int tokens, int E, int K, int top,
                      int groups, int keep, int group_best, int softmax, int renorm, float renorm_eps, float weight_scale,

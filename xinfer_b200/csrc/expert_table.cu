@@ -213,10 +213,10 @@ XB_EXPORT int xb_expert_gemm(int in_dtype, int out_dtype, void* y, const void* a
 // Behind the experts a row may hold one more gated feed-forward, F_dense wide, that every token runs, with a weight per
 // token (dense_weight):  act[t, E * F + f] = dense_weight[t] * act(gu[t, E*2F + f], gu[t, E*2F + F_dense + f]).
 template <typename T>
-__global__ void expert_select_gate_kernel(T* __restrict__ act, const T* __restrict__ gu, const int* __restrict__ table,
-                                          const int* __restrict__ ids, const int* __restrict__ sampled, int num_sampled,
+__global__ void expert_select_gate_kernel(T* __restrict__ act, const T* gu, const int* __restrict__ table,
+                                          const int* __restrict__ ids, const int* sampled, int num_sampled,
                                           const int* __restrict__ req_of_token, int top, int E, int F, int F_dense, int vocab,
-                                          float weight, const float* __restrict__ weights,
+                                          float weight, const float* weights,
                                           const float* __restrict__ dense_weight, int code, float p0, float p1, int* err) {
     pdl_overlap_few();
     const int t = blockIdx.x, e = blockIdx.y;

@@ -13,7 +13,7 @@
 // ------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void embedding_kernel(T* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids,
-                                 const int* __restrict__ sampled, int num_sampled, int hidden, int vocab, float scale,
+                                 const int* sampled, int num_sampled, int hidden, int vocab, float scale,
                                  int* err) {
     pdl_launch_dependents();
     pdl_wait();

@@ -25,7 +25,7 @@
 // cq_w.
 template <typename T>
 __global__ void latent_prepare_kernel(T* q_abs, long long q_ts, long long q_hs, int q_rot, T* __restrict__ cache, const T* proj,
-                                      long long row_len, int q_off, int kv_off, const T* __restrict__ q_lat,
+                                      long long row_len, int q_off, int kv_off, const T* q_lat,
                                       long long ql_ts, long long ql_hs, const float* __restrict__ norm_w,
                                       const float* __restrict__ inv_freq, const int* __restrict__ positions,
                                       const int* __restrict__ req_of_token, const int* __restrict__ block_table,
@@ -176,7 +176,7 @@ __global__ void gate_sigmoid_kernel(T* out, const T* heads, long long h_ts, long
 // eight bfloat16 elements per thread with 16-byte accesses (dv and every stride a multiple of 8, pointers aligned);
 // grid (pieces of a token's row, tokens)
 __global__ void gate_sigmoid_bf16x8_kernel(__nv_bfloat16* out, const __nv_bfloat16* heads, long long h_ts,
-                                           long long h_hs, const __nv_bfloat16* __restrict__ gate, long long g_ts, int nh,
+                                           long long h_hs, const __nv_bfloat16* gate, long long g_ts, int nh,
                                            int dv, int tokens, int per_head) {
     pdl_overlap_few();
     const int w = nh * dv;

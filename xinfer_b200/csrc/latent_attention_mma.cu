@@ -58,8 +58,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 
 template <int MAXNT /* 8-column value tiles per warp */, int CW /* warps of a row group: 4 or 8 */>
 __global__ void __launch_bounds__(64 * CW) attn_latent_mma_kernel(__nv_bfloat16* __restrict__ out,
-                                                              const __nv_bfloat16* __restrict__ q,
-                                                              const __nv_bfloat16* __restrict__ cache, LatentMmaArgs a) {
+                                                              const __nv_bfloat16* q,
+                                                              const __nv_bfloat16* cache, LatentMmaArgs a) {
     pdl_overlap_few();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_entry, s_tile;
@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(64 * CW) attn_latent_mma_kernel(__nv_bfloat16*
 }
 
 // out[row] = sum_p part_o[row, p] 2^(m_p - M) / sum_p l_p 2^(m_p - M),  M = max_p m_p  (maxima in the base-2 domain)
-__global__ void attn_latent_merge_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ part_o,
-                                         const float* __restrict__ part_ml, int parts, int rank) {
+__global__ void attn_latent_merge_kernel(__nv_bfloat16* __restrict__ out, const float* part_o,
+                                         const float* part_ml, int parts, int rank) {
     pdl_overlap_few();
     const size_t row = blockIdx.x;
     float M = -INFINITY;

@@ -55,7 +55,7 @@ __device__ __forceinline__ Item item_of(const int* __restrict__ it, const int* _
 }
 
 // One warp per row of the gathered buffer.  blocks: (portion, first position) of every run of 64 rows.
-__global__ void latent_gather_kernel(uint4* __restrict__ out, const uint4* __restrict__ pages, const int* __restrict__ blocks,
+__global__ void latent_gather_kernel(uint4* __restrict__ out, const uint4* pages, const int* __restrict__ blocks,
                                      int rows, const int* __restrict__ q_start, const int* __restrict__ start_pos,
                                      const int* __restrict__ table, int table_stride, int page_size, int num_pages, int window,
                                      int pieces, int* err) {

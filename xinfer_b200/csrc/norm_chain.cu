@@ -11,7 +11,7 @@
 #include "common.cuh"
 
 template <typename TB, typename TO>
-__global__ void rms_chain_kernel(TO* __restrict__ out, float* sum_out, const float* x, const TB* __restrict__ branch,
+__global__ void rms_chain_kernel(TO* __restrict__ out, float* sum_out, const float* x, const TB* branch,
                                  const int* __restrict__ rows, const float* __restrict__ w, const float* __restrict__ bw,
                                  const float* __restrict__ gain, int dim, int src_rows, float eps, float offset, float beps,
                                  float boffset, float bscale, int* err) {
@@ -85,7 +85,7 @@ XB_EXPORT int xb_rms_chain(int branch_dtype, int out_dtype, void* out, float* su
 
 // out = sl * l * rsqrt(mean(l^2) + eps) * (offset + wl) + sr * r * rsqrt(mean(r^2) + eps) * (offset + wr), row by row
 template <typename T>
-__global__ void dual_rms_sum_kernel(T* __restrict__ out, const T* __restrict__ l, const T* __restrict__ r,
+__global__ void dual_rms_sum_kernel(T* __restrict__ out, const T* l, const T* r,
                                     const float* __restrict__ wl, const float* __restrict__ wr, int dim, float eps,
                                     float offset, float sl, float sr) {
     pdl_overlap_few();
@@ -139,7 +139,7 @@ XB_EXPORT int xb_add_bias(int dtype, void* x, const float* bias, int rows, int d
 
 // out[t, i] = act(gu[t, i] + bias[i]) * (gu[t, I + i] + bias[I + i])    (float32 arithmetic, exact exponential)
 template <typename TI, typename TO, int ACT>
-__global__ void swiglu_bias_kernel(TO* __restrict__ out, const TI* __restrict__ gu, const float* __restrict__ bias, int I,
+__global__ void swiglu_bias_kernel(TO* __restrict__ out, const TI* gu, const float* __restrict__ bias, int I,
                                    size_t n) {
     pdl_overlap_few();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -28,9 +28,9 @@ __device__ __forceinline__ void gate_and_candidate(const float* __restrict__ row
 }
 
 template <typename T>
-__global__ void gated_scan_serial_kernel(T* __restrict__ y, int ldy, const float* __restrict__ zxg,
+__global__ void gated_scan_serial_kernel(T* __restrict__ y, int ldy, const float* zxg,
                                          const float* __restrict__ bz, const float* __restrict__ bx,
-                                         float* __restrict__ state, const int* __restrict__ q_start,
+                                         float* state, const int* __restrict__ q_start,
                                          const int* __restrict__ slots, int W, float out_scale) {
     pdl_overlap_few();
     const int b = blockIdx.y;
@@ -61,7 +61,7 @@ constexpr int GS_CH = 32;
 // results are stored per row range as "value and product up to the end of the row's piece within the
 // chunk" at the piece's last row.
 __global__ void gated_scan_chunk_kernel(float* __restrict__ prodA, float* __restrict__ endB,
-                                        const float* __restrict__ zxg, const float* __restrict__ bz,
+                                        const float* zxg, const float* __restrict__ bz,
                                         const float* __restrict__ bx, const int* __restrict__ req_of_token, int T, int W) {
     pdl_overlap_few();
     const int k = blockIdx.y;
@@ -87,8 +87,8 @@ __global__ void gated_scan_chunk_kernel(float* __restrict__ prodA, float* __rest
 // pass 2 + 3: per (entry, channel) walk over the entry's chunk ends to find each chunk's start value, then
 // every row's state is  S_t = prodA[t] * start(piece of t) + endB[t]; one thread per (row, channel) would
 // need the start values, so they are kept per chunk piece in `start` ([rows, W] at the piece's first row).
-__global__ void gated_scan_starts_kernel(float* __restrict__ start, const float* __restrict__ prodA,
-                                         const float* __restrict__ endB, float* __restrict__ state,
+__global__ void gated_scan_starts_kernel(float* __restrict__ start, const float* prodA,
+                                         const float* endB, float* state,
                                          const int* __restrict__ q_start, const int* __restrict__ slots, int W) {
     pdl_overlap_few();
     const int b = blockIdx.y;
@@ -128,9 +128,9 @@ __global__ void gated_scan_starts_kernel(float* __restrict__ start, const float*
 }
 
 template <typename T>
-__global__ void gated_scan_finish_kernel(T* __restrict__ y, int ldy, const float* __restrict__ zxg,
-                                         const float* __restrict__ start, const float* __restrict__ prodA,
-                                         const float* __restrict__ endB, const int* __restrict__ req_of_token,
+__global__ void gated_scan_finish_kernel(T* __restrict__ y, int ldy, const float* zxg,
+                                         const float* start, const float* prodA,
+                                         const float* endB, const int* __restrict__ req_of_token,
                                          const int* __restrict__ q_start, int tokens, int W, float out_scale) {
     pdl_overlap_few();
     const int t = blockIdx.y;
@@ -196,7 +196,7 @@ __device__ __forceinline__ void block_sum3(float& a, float& b, float& c, float* 
 
 // PER values of the row per thread stay in registers between the sums and the result (F <= PER * threads).
 template <typename T, int PER>
-__global__ void polynorm_kernel(T* __restrict__ out, const float* __restrict__ z, const float* __restrict__ coef, int F,
+__global__ void polynorm_kernel(T* __restrict__ out, const float* z, const float* __restrict__ coef, int F,
                                 float eps) {
     pdl_overlap_few();
     __shared__ float scratch[96];

@@ -37,7 +37,7 @@ XB_EXPORT int xb_embedding_f32(int table_dtype, float* out, const void* table, c
 //   out = s * rsqrt(mean(s^2) + eps) * (offset + w)     in TO
 // sum_out (float32, nullable) receives s; it may be x itself when no rows are gathered.
 template <typename TB, typename TO>
-__global__ void rmsnorm_f32_kernel(TO* __restrict__ out, float* sum_out, const float* x, const TB* __restrict__ branch,
+__global__ void rmsnorm_f32_kernel(TO* __restrict__ out, float* sum_out, const float* x, const TB* branch,
                                    const int* __restrict__ rows, const float* __restrict__ w, int dim, int src_rows,
                                    float eps, float offset, int* err) {
     pdl_overlap_few();

@@ -61,9 +61,9 @@ __device__ __forceinline__ void store_run<__nv_bfloat16, 4>(__nv_bfloat16* dst, 
 // per thread.  Where a run meets another request's first token the registers are filled again as above.  Taps are added
 // in the same order as in conv_silu_kernel, so both give the same bits.
 template <typename TO, int K, int V>
-__global__ void __launch_bounds__(128) conv_silu_run_kernel(TO* __restrict__ y, const float* __restrict__ u, long long u_ld,
+__global__ void __launch_bounds__(128) conv_silu_run_kernel(TO* __restrict__ y, const float* u, long long u_ld,
                                                             int u_off, const float* __restrict__ taps,
-                                                            const float* __restrict__ bias, const float* __restrict__ state,
+                                                            const float* __restrict__ bias, const float* state,
                                                             const int* __restrict__ req_of_token,
                                                             const int* __restrict__ q_start, const int* __restrict__ slots,
                                                             int C, int tokens, int run) {
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(128) conv_silu_run_kernel(TO* __restrict__ y, 
 }
 
 template <typename T>
-__global__ void conv_state_kernel(T* __restrict__ state, const T* __restrict__ u, long long u_ld, int u_off,
+__global__ void conv_state_kernel(T* state, const T* u, long long u_ld, int u_off,
                                   const int* __restrict__ q_start, const int* __restrict__ slots, int C, int K) {
     pdl_overlap_few();
     const int b = blockIdx.y;

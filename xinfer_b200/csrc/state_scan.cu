@@ -223,11 +223,11 @@ __device__ __forceinline__ void stage_cols(float* dst, const float* src, int c_b
 // the bias and the softplus).  state [slots, H, N, P].  y [T, H*P].  Shared memory: three stages of
 // B[TT][NP] C[TT][NP] x[TT][VT] dt[TT] dec[TT], then two tiles y[TT][VT].  `cw` of the block's warps compute.
 template <int DS, bool FEW>
-__global__ void __launch_bounds__(FEW ? 256 : 384, FEW ? 2 : 1) selective_scan_kernel(float* __restrict__ y, const float* __restrict__ xbc, int C,
-                                                             const float* __restrict__ proj, long long ldp, int dt_off,
+__global__ void __launch_bounds__(FEW ? 256 : 384, FEW ? 2 : 1) selective_scan_kernel(float* __restrict__ y, const float* xbc, int C,
+                                                             const float* proj, long long ldp, int dt_off,
                                                              const float* __restrict__ dt_bias,
                                                              const float* __restrict__ A_log, const float* __restrict__ Dv,
-                                                             float* __restrict__ state, const int* __restrict__ q_start,
+                                                             float* state, const int* __restrict__ q_start,
                                                              const int* __restrict__ slots, int H, int P, int N, int G,
                                                              int TT, int stage, int cw, int vec) {
     pdl_wait();
@@ -383,8 +383,8 @@ __device__ __forceinline__ const float* delta_group(const float* prep, long long
 // V = 4: a lane takes four neighbouring channels with 16-byte accesses, where the rows allow it (2,048 tokens of 32 heads of
 // 128: 136 -> 94 us).
 template <int V>
-__global__ void __launch_bounds__(128) delta_prepare_kernel(float* __restrict__ prep, const float* __restrict__ qkv, int Cq,
-                                                            const float* __restrict__ ag, long long ldag,
+__global__ void __launch_bounds__(128) delta_prepare_kernel(float* __restrict__ prep, const float* qkv, int Cq,
+                                                            const float* ag, long long ldag,
                                                             const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                                                             const int* __restrict__ q_start, int entries, int tokens, int H, int G,
                                                             int d, float unit_eps) {
@@ -514,9 +514,9 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(float* __restrict__ 
 // Shared memory: three stages of Gq[TT][DP] Gk[TT][DP] Ek[TT][DP] v[TT][VT] beta[TT] A, B[TT/4][16] G_3[TT/4][DP], then two
 // tiles o[TT][VT].
 template <int DS>
-__global__ void __launch_bounds__(384, 1) delta_rule_kernel(float* __restrict__ o, const float* __restrict__ prep,
-                                                         const float* __restrict__ vals, int ldv, const float* __restrict__ proj,
-                                                         long long ldp, int beta_off, float* __restrict__ state,
+__global__ void __launch_bounds__(384, 1) delta_rule_kernel(float* __restrict__ o, const float* prep,
+                                                         const float* vals, int ldv, const float* proj,
+                                                         long long ldp, int beta_off, float* state,
                                                          const int* __restrict__ q_start, const int* __restrict__ slots, int tokens,
                                                          int H, int d, int dv, int TT, int stage, int cw, int vec) {
     pdl_wait();
@@ -705,11 +705,11 @@ __global__ void __launch_bounds__(384, 1) delta_rule_kernel(float* __restrict__ 
 constexpr int kFewTokensSmall = 96;
 static inline bool delta_few(int longest, int d) { return longest <= (d <= 64 ? kFewTokensSmall : kFewTokens); }
 template <int DS>
-__global__ void __launch_bounds__(384, 1) delta_few_kernel(float* __restrict__ o, const float* __restrict__ qkv, int Cq,
-                                                        const float* __restrict__ proj, long long ldp, int beta_off,
-                                                        const float* __restrict__ ag, long long ldag,
+__global__ void __launch_bounds__(384, 1) delta_few_kernel(float* __restrict__ o, const float* qkv, int Cq,
+                                                        const float* proj, long long ldp, int beta_off,
+                                                        const float* ag, long long ldag,
                                                         const float* __restrict__ dt_bias, const float* __restrict__ A_log,
-                                                        float* __restrict__ state, const int* __restrict__ q_start,
+                                                        float* state, const int* __restrict__ q_start,
                                                         const int* __restrict__ slots, int H, int G, int d, int dv,
                                                         float unit_eps, int TT, int stage, int cw, int vec) {
     pdl_wait();
@@ -862,9 +862,9 @@ __global__ void __launch_bounds__(384, 1) delta_few_kernel(float* __restrict__ o
 // every (head, key channel).  state [slots, H, d, dv].  o [T, H*dv] = scale * S^T q after the token's own write.  Shared
 // memory: three stages of q[TT][DP] k[TT][DP] alpha[TT][DP] v[TT][VT], then two tiles o[TT][VT].
 template <int DS, bool FEW>
-__global__ void __launch_bounds__(FEW ? 256 : 384, FEW ? 2 : 1) linear_scan_kernel(float* __restrict__ o, const float* __restrict__ proj,
-                                                             long long ldp, const float* __restrict__ alpha,
-                                                             float* __restrict__ state, const int* __restrict__ q_start,
+__global__ void __launch_bounds__(FEW ? 256 : 384, FEW ? 2 : 1) linear_scan_kernel(float* __restrict__ o, const float* proj,
+                                                             long long ldp, const float* alpha,
+                                                             float* state, const int* __restrict__ q_start,
                                                              const int* __restrict__ slots, int H, int d, int dv, float scale,
                                                              int TT, int stage, int cw, int vec) {
     pdl_wait();
@@ -996,9 +996,9 @@ __global__ void __launch_bounds__(FEW ? 256 : 384, FEW ? 2 : 1) linear_scan_kern
 // columns; the first feeding warp works out the gates, a lane per token, and walks m over the tile.
 template <int DS, bool FEW>
 __global__ void __launch_bounds__(384, 1) matrix_memory_kernel(
-    float* __restrict__ o, float* __restrict__ div, const float* __restrict__ proj, long long ldp, int gate_off,
-    const float* __restrict__ bi, const float* __restrict__ bf, float cap, float* __restrict__ state_s,
-    float* __restrict__ state_n, float* state_m, const int* __restrict__ q_start, const int* __restrict__ start_pos,
+    float* __restrict__ o, float* __restrict__ div, const float* proj, long long ldp, int gate_off,
+    const float* __restrict__ bi, const float* __restrict__ bf, float cap, float* state_s,
+    float* state_n, float* state_m, const int* __restrict__ q_start, const int* __restrict__ start_pos,
     const int* __restrict__ slots, int H, int d, int dv, float scale, float div_eps, int TT, int stage, int cw, int vec) {
     pdl_wait();
     extern __shared__ __align__(16) float scan_smem[];
@@ -1197,7 +1197,7 @@ __global__ void __launch_bounds__(384, 1) matrix_memory_kernel(
 // column range of wider float32 rows.  A block takes a tile of tokens and 128 channels, a thread one channel of all its
 // tokens; both operands pass through shared memory, so that memory is read in order; r in order for every output.
 constexpr int kDecayTokens = 16, kDecayRanks = 16, kDecayChannels = 128;
-__global__ void __launch_bounds__(kDecayChannels) low_rank_decay_kernel(float* __restrict__ alpha, const float* __restrict__ low,
+__global__ void __launch_bounds__(kDecayChannels) low_rank_decay_kernel(float* __restrict__ alpha, const float* low,
                                                                         long long ldl, const float* __restrict__ w,
                                                                         const float* __restrict__ bias, int tokens, int C, int R,
                                                                         float inv_tau) {
@@ -1433,9 +1433,9 @@ XB_EXPORT int xb_low_rank_decay(float* alpha, const float* low, long long ldl, c
 // gate is column g_off + c of a wider float32 row.  div (nullable): every y of a part is first divided by div[t, part].
 // out's rows lie ldo apart and receive out_scale times the result.
 template <typename TO>
-__global__ void gated_head_norm_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ gate,
+__global__ void gated_head_norm_kernel(TO* __restrict__ out, const float* y, const float* gate,
                                        long long ldg, int g_off, const float* __restrict__ w, int w_len, int W, int part,
-                                       float eps, int mode, const float* __restrict__ div, long long ldo, float out_scale) {
+                                       float eps, int mode, const float* div, long long ldo, float out_scale) {
     pdl_overlap_few();
     __shared__ float scratch[33];
     const int t = blockIdx.x, c0 = blockIdx.y * part;
@@ -1468,10 +1468,10 @@ __global__ void gated_head_norm_kernel(TO* __restrict__ out, const float* __rest
 // The same for parts of at most 32 * NV channels: a warp per (token, part) keeps its channels in registers, one pass
 // over memory, sums by shuffles; a block's warps take neighbouring parts of a token.
 template <typename TO, int NV>
-__global__ void __launch_bounds__(256) gated_head_norm_warp_kernel(TO* __restrict__ out, const float* __restrict__ y,
-                                                                   const float* __restrict__ gate, long long ldg, int g_off,
+__global__ void __launch_bounds__(256) gated_head_norm_warp_kernel(TO* __restrict__ out, const float* y,
+                                                                   const float* gate, long long ldg, int g_off,
                                                                    const float* __restrict__ w, int w_len, int W, int part,
-                                                                   float eps, int mode, const float* __restrict__ div,
+                                                                   float eps, int mode, const float* div,
                                                                    long long ldo, float out_scale, long long units) {
     pdl_overlap_few();
     const int lane = threadIdx.x & 31;

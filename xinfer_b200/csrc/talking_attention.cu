@@ -64,7 +64,7 @@ __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, const fl
 
 template <typename T, bool CONV>
 __global__ void qkv_prepare_kernel(T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                   const T* __restrict__ qkv, const float* __restrict__ q_w, const float* __restrict__ k_w,
+                                   const T* qkv, const float* __restrict__ q_w, const float* __restrict__ k_w,
                                    const float* __restrict__ inv_freq, const int* __restrict__ positions,
                                    const int* __restrict__ req_of_token, const int* __restrict__ block_table,
                                    int table_stride, int nh, int nkv, int d, int dv, int rot, int interleaved, int norm_mode,
@@ -784,8 +784,8 @@ __global__ void __launch_bounds__(TA_THREADS) attn_talking_kernel(T* __restrict_
 // out[t, h] = out_scale * sum_y e^(m_y - m) o_y / sum_y e^(m_y - m) l_y  over the `parts` key ranges of token t.
 // One block per (token, head): the ranges' factors once into shared memory, then a thread per column.
 template <typename T>
-__global__ void attn_talking_merge_kernel(T* __restrict__ out, const float* __restrict__ part_o,
-                                          const float* __restrict__ part_ml, int H, int dv, int parts, int ldo,
+__global__ void attn_talking_merge_kernel(T* __restrict__ out, const float* part_o,
+                                          const float* part_ml, int H, int dv, int parts, int ldo,
                                           float out_scale) {
     pdl_overlap_few();
     extern __shared__ float fy[];          // [parts] factors, then the sum

@@ -67,9 +67,9 @@ __host__ __device__ inline TalkMmaSmem talk_mma_smem(int H, int G, int d, int dv
 
 template <int MAXH, int DVT /* 8-column tiles of a value head */>
 __global__ void __launch_bounds__(TM_THREADS) attn_talking_mma_kernel(__nv_bfloat16* __restrict__ out,
-                                                                      const __nv_bfloat16* __restrict__ q,
-                                                                      const __nv_bfloat16* __restrict__ k_cache,
-                                                                      const __nv_bfloat16* __restrict__ v_cache,
+                                                                      const __nv_bfloat16* q,
+                                                                      const __nv_bfloat16* k_cache,
+                                                                      const __nv_bfloat16* v_cache,
                                                                       TalkMmaArgs a) {
     pdl_overlap_few();
     extern __shared__ __align__(16) unsigned char smraw[];

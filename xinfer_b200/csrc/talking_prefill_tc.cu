@@ -349,7 +349,7 @@ constexpr uint32_t V_SCORES = 2 * TILE_FLOATS * 4;       // one head's scores of
 
 template <int DVC>
 __global__ void __launch_bounds__(V_THREADS)
-talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* __restrict__ scores, __nv_bfloat16* __restrict__ out,
+talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* scores, __nv_bfloat16* __restrict__ out,
                       long long ldo, const int* __restrict__ blocks, const int* __restrict__ work, const int* __restrict__ q_start,
                       const int* __restrict__ start_pos, const int* __restrict__ block_table, int table_stride, int nh, int nkv,
                       int ps, int ps_shift, int num_pages, int window, int sink, float out_scale, int* err) {

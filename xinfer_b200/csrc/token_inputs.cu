@@ -90,7 +90,7 @@ XB_EXPORT int xb_embed_sum(int table_dtype, float* out, const void* table, const
 }
 
 // prev_state[slot of entry b] = the entry's last token of this step
-__global__ void prev_store_kernel(int* __restrict__ prev_state, const int* __restrict__ ids, const int* __restrict__ sampled,
+__global__ void prev_store_kernel(int* __restrict__ prev_state, const int* __restrict__ ids, const int* sampled,
                                   int num_sampled, const int* __restrict__ q_start, const int* __restrict__ slots, int entries) {
     pdl_overlap_few();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -109,8 +109,8 @@ XB_EXPORT int xb_prev_store(int* prev_state, const int* ids, const int* sampled,
 }
 
 template <typename T>
-__global__ void token_gate_kernel(T* __restrict__ out, const T* __restrict__ u, const T* __restrict__ table, int table_ld,
-                                  int col0, const int* __restrict__ ids, const int* __restrict__ sampled, int num_sampled,
+__global__ void token_gate_kernel(T* __restrict__ out, const T* u, const T* __restrict__ table, int table_ld,
+                                  int col0, const int* __restrict__ ids, const int* sampled, int num_sampled,
                                   const int* __restrict__ req_of_token, int dim, int vocab, size_t n, int* err) {
     pdl_overlap_few();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
