@@ -193,3 +193,31 @@ def test_a_key_that_is_not_a_number_shows_in_every_query_that_sees_it(key):
     kernels.attn_rows_tc(out, q, H * d, kv, rows, work, ctas, q_start, start_pos, H, d, 0, dv, rank, None, d ** -0.5, None, err)
     bad = torch.isnan(out)
     assert int(err) == 0 and bad[key:].all() and not bad[:key].any()
+
+
+@pytest.mark.gpu
+def test_a_full_device_keeps_to_the_rows_and_a_growing_context_moves_its_scratch_rarely(monkeypatch):
+    from xinfer_b200.engine.runner import ModelRunner, StepInput
+    from xinfer_b200.parts import latent_attention as part
+    from xinfer_b200.parts.base import Workspace
+    m = dict(heads=2, dim=64, rot_dim=32, vdim=64, kv_rank=64, scale=0.1, rot=dict(dims=32, base=1000.0))
+    cfg = dict(architecture="Dufitar", vocab=300, width=128, norm=dict(eps=1e-6), residual_mult=0.5, embedding=dict(scale=2.0),
+               layers=[dict(type="latent_attention", mixer=m, mlp=dict(kind="dense", ff=128, limit=7.0))])
+    ids = np.random.default_rng(1).integers(0, 300, size=1000)
+    monkeypatch.setattr(part, "ROWS_RATES", (1e-9, 1e30, 1e30, 0.0, 0.0))
+
+    def logits():
+        r = ModelRunner.random(cfg, 3, block_size=16, num_blocks=128, max_num_seqs=4, max_model_len=1024)
+        before, a, out, places = kernels.launch_counts().get("attn_rows_tc", 0), r.open_request(), [], []
+        for at in range(0, 1000, 40):
+            out.append(r.step([StepInput(a, ids[at:at + 40], [39])]).clone())
+            buf = r.workspace._bufs.get("latent.kv")
+            places.append(None if buf is None else (buf.data_ptr(), buf.numel()))
+        r.check_errors()
+        return torch.cat(out).double(), kernels.launch_counts().get("attn_rows_tc", 0) - before, places
+    got, some, places = logits()
+    assert some == 25 and len(set(places)) == 5                 # 64, 128, 256, 512 and 1,024 rows
+    monkeypatch.setattr(Workspace, "reserve", lambda *a: False)
+    want, none, places = logits()
+    assert none == 0 and set(places) == {None}
+    assert (got - want).norm() <= 0.02 * want.norm()             # two bfloat16 computations of the same numbers

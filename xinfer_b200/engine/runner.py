@@ -314,7 +314,8 @@ class ModelRunner:
             token_bytes[g] += needs[pos].bytes_per_token(self.dtype)
         if num_blocks is None:
             free, _ = torch.cuda.mem_get_info(self.device)
-            budget = int(free * kv_fraction)
+            # (beside the share the parts keep what their scratch may grow to)
+            budget = max(min(int(free * kv_fraction), free - self.model.context_scratch_bytes()), 0)
             total = sum(token_bytes) * self.block_size or 1
             num_blocks = max(budget // total, 1)
             # no group needs more pages than every request at full length

@@ -115,6 +115,17 @@ class DecoderModel:
             out.append(mixer.cache_need() if mixer is not None else None)
         return out
 
+    def context_scratch_bytes(self) -> int:
+        """What the parts' workspace whose size follows the context may take, in bytes (buffers of one name are shared)."""
+        most: Dict[str, int] = {}
+        parts = [p for block in self.blocks for p in block.all_parts()]
+        while parts:
+            part = parts.pop()
+            parts += part.children()
+            for name, n in part.context_scratch().items():
+                most[name] = max(most.get(name, 0), int(n))
+        return sum(most.values())
+
     def state_need_of_model(self):
         """Per-request state that belongs to no layer: the token before, for the pair embedding."""
         if self.plan.pair_embedding is not None:

@@ -23,6 +23,7 @@ class Workspace:
         self.device = device
         self._bufs: Dict[str, torch.Tensor] = {}
         self._views: Dict[tuple, torch.Tensor] = {}   # (name, shape, dtype) -> view of the buffer
+        self._refused: Dict[str, int] = {}            # bytes that the device had no room for (``reserve``)
         self.frozen = False
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
@@ -48,12 +49,38 @@ class Workspace:
         self._views[key] = view
         return view
 
+    def reserve(self, name: str, n: int, dtype: torch.dtype, most: int) -> bool:
+        """Make sure that ``get`` will find ``n`` elements in this buffer, whose contents are undefined: for scratch whose size
+        follows the context, which would otherwise grow a little with nearly every step.  It grows to powers of two, to
+        ``most`` elements (or ``n``) at most, and the old buffer goes first.  False: the device has no room for it; whoever asks
+        has another way."""
+        buf = self._bufs.get(name)
+        if buf is not None and buf.dtype == dtype and buf.numel() >= n:
+            return True
+        if self.frozen and buf is not None:
+            raise RuntimeError(f"workspace buffer '{name}' would have to grow while a CUDA graph uses it")
+        size = dtype.itemsize
+        if n * size >= self._refused.get(name, n * size + 1):
+            return False
+        del buf
+        self._bufs.pop(name, None)
+        self._views = {k: v for k, v in self._views.items() if k[0] != name}
+        for cap in (max(n, min(int(most), 1 << max(0, n - 1).bit_length())), n):
+            try:
+                self._bufs[name] = torch.empty(max(cap, 1), dtype=dtype, device=self.device)
+                return True
+            except torch.OutOfMemoryError:
+                pass
+        self._refused[name] = n * size
+        return False
+
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._bufs.values())
 
     def clear(self) -> None:
         """Zero every buffer (their addresses stay): counters and tickets that kernels keep at zero
         between launches are zero again after a step that did not run to its end."""
+        self._refused.clear()
         for b in self._bufs.values():
             b.zero_()
 
@@ -197,6 +224,11 @@ class Part:
 
     def load(self, store: WeightStore) -> None:
         pass
+
+    def context_scratch(self) -> Dict[str, int]:
+        """Workspace whose size follows the context of a step and not its tokens: name -> bytes at most.  The page pool leaves
+        room for it."""
+        return {}
 
     def children(self) -> Sequence["Part"]:
         """Parts that this one is made of and that hold weights of their own."""

@@ -105,8 +105,13 @@ def rows_plan(ctx: StepContext, heads: int, d: int, rd: int, dv: int, rank: int,
             starts = ctx.h_q_start[: ctx.real_entries + 1]
             host, ctas, rows, runs_at = kernels.latent_prefill_work(starts[1:] - starts[:-1], ctx.h_start_pos[: ctx.real_entries],
                                                                     ROWS_MIN_TOKENS, window, heads, host_buffer=_rows_ring.take)
-            made = (host.to(ctx.positions.device, non_blocking=True), ctas, rows, runs_at, small)
-            _rows_ring.sent()
+            # (a device that is full to the brim keeps to the first way)
+            ws, per_row = ctx.workspace, heads * (d + dv)
+            most = ROWS_MAX_BYTES // (2 * per_row)
+            if ws.reserve("latent.rows", rows * width, torch.bfloat16, most * width) \
+                    and ws.reserve("latent.kv", rows * per_row, torch.bfloat16, most * per_row):
+                made = (host.to(ctx.positions.device, non_blocking=True), ctas, rows, runs_at, small)
+                _rows_ring.sent()
     ctx.scratch[key] = made
     return made
 
@@ -211,6 +216,13 @@ class LatentAttention(Mixer):
         self.w_o = operand(n[7])
         if s.sink:
             self.sink = store.get(p + n[5], self.device, torch.float32).float().contiguous()
+
+    def context_scratch(self):
+        s = self.spec
+        if self.dtype != torch.bfloat16:
+            return {}
+        rows = ROWS_MAX_BYTES // (2 * s.num_heads * (s.head_dim + s.v_head_dim))
+        return {"latent.kv": ROWS_MAX_BYTES, "latent.rows": 2 * rows * (s.kv_rank + s.rope_dim + s.row_tail)}
 
     def cache_need(self) -> PagedCacheNeed:
         s = self.spec

@@ -149,6 +149,9 @@ class TalkingAttention(Mixer):
             self.q_norm = store.get(p + qn, self.device, torch.float32).float().contiguous()
             self.k_norm = store.get(p + kn, self.device, torch.float32).float().contiguous()
 
+    def context_scratch(self):
+        return {"tattn.scores": SCORES_BYTES} if self.spec.talking_heads and self.dtype == torch.bfloat16 else {}
+
     def cache_need(self) -> PagedCacheNeed:
         s = self.spec
         return PagedCacheNeed((("k", CacheTensor((s.num_kv_heads, s.head_dim), None, 1)),
@@ -219,6 +222,9 @@ class TalkingAttention(Mixer):
                 counts = ctx.h_q_start[1: ctx.real_entries + 1] - ctx.h_q_start[: ctx.real_entries]
                 made = kernels.talk_work(counts, ctx.h_start_pos[: ctx.real_entries], s.window, s.num_heads, s.num_kv_heads,
                                          SCORES_BYTES // (4 * kernels.TALK_TILE_FLOATS), host_buffer=_work_ring.take)
+            # (a device that is full to the brim keeps to the kernel that holds all heads)
+            if made is not None and not ctx.workspace.reserve("tattn.scores", made[2] * kernels.TALK_TILE_FLOATS, torch.float32, SCORES_BYTES // 4):
+                made = None
             if made is not None:
                 made = (made[0].to(ctx.positions.device, non_blocking=True), made[1], made[2])
                 _work_ring.sent()
