@@ -7,6 +7,8 @@ may hold both).  Everything else (float32, other head sizes) runs on the plain k
 """
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import torch
 
@@ -107,9 +109,11 @@ def _plan(ctx, head_dim: int):
     return plan
 
 
-class PinnedRing:
+class PinnedRing(threading.local):
     """A few pinned staging buffers used in turn; one is reused only after the copy that read it has
-    finished (pinning memory anew for every step would synchronise the device)."""
+    finished (pinning memory anew for every step would synchronise the device).  Every thread has its own:
+    engines in several threads share the module that holds the ring, and another thread's ``take`` between a
+    thread's ``take`` and ``sent`` would leave the wrong buffer marked as being read."""
 
     def __init__(self, depth: int = 4):
         self.bufs = [None] * depth
