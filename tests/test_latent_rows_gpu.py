@@ -221,3 +221,21 @@ def test_a_full_device_keeps_to_the_rows_and_a_growing_context_moves_its_scratch
     want, none, places = logits()
     assert none == 0 and set(places) == {None}
     assert (got - want).norm() <= 0.02 * want.norm()             # two bfloat16 computations of the same numbers
+
+
+@pytest.mark.gpu
+def test_a_work_list_that_was_cut_off_is_refused():
+    T, H, d, dv, rank = 300, 2, 64, 64, 64
+    work, ctas, q, kv, rows, q_start, start_pos, err = _one_portion(T, H, d, dv, rank, torch.Generator().manual_seed(1))
+    _, _, n, at = kernels.latent_prefill_work([T], [0], 4, None, H)
+    out = torch.zeros(T, H * dv, dtype=torch.bfloat16, device=DEV)
+
+    def run(work, kv=kv, rows=rows, at=at):
+        kernels.attn_rows_tc(out, q, H * d, kv, rows, work, ctas, q_start, start_pos, H, d, 0, dv, rank, None, 0.1, None, err, at)
+    for bad in (dict(work=work[:-1].contiguous()), dict(work=work[:ctas + 1].contiguous()), dict(work=work[:-4].contiguous()),
+                dict(work=work, kv=kv[:-64].contiguous(), rows=rows[:-64].contiguous(), at=None), dict(work=work[:-1].contiguous(), at=None)):
+        with pytest.raises(kernels.KernelError):
+            run(**bad)
+    run(work)
+    run(work, at=None)
+    assert int(err) == 0

@@ -202,3 +202,18 @@ def test_weights_are_divided_by_their_own_sum():
     kernels.attn_talking_tc(out, q, k, torch.ones_like(v), torch.eye(H), scores, work, chunks, q_start, start_pos, table, table.shape[1], None,
                             d ** -0.5, False, factor, err)
     assert int(err) == 0 and (out == 1.0 + 2.0 ** -7).all()
+
+
+@pytest.mark.gpu
+def test_scratch_and_work_lists_that_are_too_short_are_refused():
+    T, H, G, d, dv = 300, 8, 4, 64, 64
+    q, k, v, table, (work, chunks), scores, (q_start, start_pos), err = _prompt(T, H, G, d, dv, torch.Generator().manual_seed(2))
+    out = torch.zeros(T, H * dv, dtype=torch.bfloat16, device=DEV)
+
+    def run(work=work, chunks=chunks, scores=scores):
+        kernels.attn_talking_tc(out, q, k, v, torch.eye(H), scores, work, chunks, q_start, start_pos, table, table.shape[1], None, 0.1, True, 1.0, err)
+    for bad in (dict(work=work[:-1].contiguous()), dict(scores=scores[:-1].contiguous()), dict(chunks=list(chunks))):
+        with pytest.raises(kernels.KernelError):
+            run(**bad)
+    run()
+    assert int(err) == 0

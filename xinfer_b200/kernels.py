@@ -866,6 +866,15 @@ def attn_talking_tc_takes(nh: int, nkv: int, d: int, dv: int, page_size: int) ->
     return bool(kernels_lib().xb_attn_talking_tc_takes(int(nh), int(nkv), int(d), int(dv), int(page_size)))
 
 
+class TalkChunks(list):
+    """The chunks of a ``talk_work`` list (rows of five numbers), with the score tiles that the largest one needs and the length of
+    the list."""
+
+    def __init__(self, rows, tiles: int, ints: int):
+        super().__init__(rows)
+        self.tiles, self.ints = int(tiles), int(ints)
+
+
 def talk_work(counts, starts, window, heads: int, kv_heads: int, cap_tiles: int, max_ctas: int = PREFILL_TC_MAX_CTAS, host_buffer=None):
     """The work lists of ``attn_talking_tc`` for a step whose entries bring ``counts`` tokens after ``starts`` cached ones:
     (pinned int32 host tensor, chunks as rows [blocks, first list, second list, CTAs of both], score tiles of the largest
@@ -889,7 +898,7 @@ def talk_work(counts, starts, window, heads: int, kv_heads: int, cap_tiles: int,
         raise KernelError("the work lists do not fit their buffer")
     if n < 0:
         return None
-    return host[:max(int(used.value), 1)], chunks[:n].tolist(), int(tiles.value)
+    return host[:max(int(used.value), 1)], TalkChunks(chunks[:n].tolist(), tiles.value, used.value), int(tiles.value)
 
 
 def attn_talking_tc(out, q, k_cache, v_cache, talk, scores, work, chunks, q_start, start_pos, block_table, table_stride, window,
@@ -909,6 +918,8 @@ def attn_talking_tc(out, q, k_cache, v_cache, talk, scores, work, chunks, q_star
         raise KernelError("talk must be a contiguous float32 matrix [heads, heads] in host memory")
     _need(scores, "scores", torch.float32)
     _need(work, "work", torch.int32)
+    if not isinstance(chunks, TalkChunks) or work.numel() < chunks.ints or scores.numel() < chunks.tiles * TALK_TILE_FLOATS:
+        raise KernelError("the work list or the scratch for the scores is shorter than the chunks of its talk_work need")
     at = work.data_ptr()
     for blocks, one, two, ctas1, ctas2 in chunks:
         _ok(kernels_lib().xb_attn_talking_tc(
@@ -1216,12 +1227,12 @@ def latent_gather(out, pages, work, runs_at: int, q_start, start_pos, block_tabl
 
 
 def attn_rows_tc(out, q, q_row: int, kv, rows, work, ctas, q_start, start_pos, nh: int, d: int, rd: int, dv: int, rank: int,
-                 window, scale, sink, err) -> None:
+                 window, scale, sink, err, runs_at: Optional[int] = None) -> None:
     """Attention of the portions of a ``latent_prefill_work`` list on tcgen05 (TMA-fed; scores, probabilities and
     accumulators in tensor memory).  ``q``: rows of ``q_row`` elements whose first ``nh * (d + rd)`` are the heads'
     queries; ``kv`` ``[n, nh * (d + dv)]``: all heads' keys, then all heads' values; ``rows`` ``[n, width]``: the gathered
     rows, whose rd channels from ``rank`` on belong to every head's key.  ``out`` ``[T, nh * dv]`` receives the rows of the
-    list's portions; others stay as they are."""
+    list's portions; others stay as they are.  ``runs_at``: as ``latent_prefill_work`` returned it, to check the list with."""
     n, width = rows.shape
     T = out.shape[0]
     _need(out, "out", torch.bfloat16, (T, nh * dv))
@@ -1231,7 +1242,9 @@ def attn_rows_tc(out, q, q_row: int, kv, rows, work, ctas, q_start, start_pos, n
     _need(work, "work", torch.int32)
     if sink is not None:
         _need(sink, "sink", torch.float32, (nh,))
-    if q_row < nh * (d + rd) or (ctas > 0 and work.numel() < ctas + 1):
+    items = work.numel() - n // 32 - (ctas + 1) if runs_at is None else int(runs_at) - (ctas + 1)       # four numbers each
+    if q_row < nh * (d + rd) or width < rank + rd or n % 64 or (ctas > 0 and (
+            items < 4 * ctas or items % 4 or work.numel() < ctas + 1 + items + n // 32)):
         raise KernelError("the queries or the work list are shorter than the call needs")
     _ok(kernels_lib().xb_attn_rows_tc(
         out.data_ptr(), nh * dv, q.data_ptr(), int(q_row), kv.data_ptr(), rows.data_ptr(), T, n, int(nh), int(d), int(rd), int(dv),

@@ -294,7 +294,7 @@ class LatentAttention(Mixer):
             kv = ws.get("latent.kv", (n, H * (d + dv)), self.dtype)
             linear(kv, rows[:, :r], self.w_kv, ctx.err)
             kernels.attn_rows_tc(inner, q_rows, q_rows.shape[1], kv, rows, work, ctas, ctx.q_start, ctx.start_pos, H, d, rd, dv, r,
-                                 s.window, s.scale, self.sink, ctx.err)
+                                 s.window, s.scale, self.sink, ctx.err, runs_at)
         if s.gate:
             kernels.gate_sigmoid(inner, o_heads, proj[:, at_gate:at_gate + (H if s.gate_per_head else H * dv)])
         out = ws.get("latent.out", (T, s.hidden), ctx.branch_dtype or self.dtype)
