@@ -6,9 +6,10 @@
 // costs 2 rank (d + dv) per head and key, once for all queries of the step, so it pays from a few dozen queries on.
 // The tensor cores bound the kernel at long prompts, the exponentials of the softmax beside them.  It replaces the
 // mma.sync kernel over the rows for portions of more than four tokens: at rank 512, 32 heads and a prompt of 2,048
-// tokens 1,570 us (91 TFLOP/s) before, now 55 us for the attention (782 TFLOP/s of its 43 GFLOP), 18 us for the product
-// that forms keys and values and 4 us for the gathering, without the 33 us of maps into and out of the latent space; at
-// rank 256 and 16 heads 626 us before, 37 + 9 us now.
+// tokens 1,570 us (91 TFLOP/s) before, now 55 us for the attention where the product has just left keys and values in the L2
+// cache (782 TFLOP/s of its 43 GFLOP; 66 us after a flush), 18 us for the product that forms them and 4 us for the gathering,
+// without the 33 us of maps into and out of the latent space; at rank 256 and 16 heads 626 us before, 37 + 9 us now (47 us
+// after a flush).
 //
 //   latent_gather_kernel   the rows a step's portions can see, out of their pages, in runs of 64 rows per portion that
 //                          begin at a multiple of 64 positions; rows no query of the portion sees are zeros.  The matrix
@@ -16,6 +17,9 @@
 //   attn_rows_tc_kernel    128 or 256 queries of one head per work item against that head's keys and values: tcgen05.mma
 //                          with scores, probabilities and accumulators in tensor memory, TMA-fed rings, one softmax row
 //                          per thread.  Two tiles of 128 queries share every key/value tile.
+//
+// A value that is no number reaches every query of its tile of 128, those in front of it too (0 x NaN), as in the kernel over
+// pages; the kernel over the cached rows kept it to its block of 32 (query, head) rows.
 #include "attention_common.cuh"
 #include "tc_common.cuh"
 
@@ -96,7 +100,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t k_full0 = bars, k_empty0 = bars + 32, v_full0 = bars + 64, v_empty0 = bars + 96;
     const uint32_t s_ready0 = bars + 128, pv_done0 = bars + 160, p_ready0 = bars + 192, o_done0 = bars + 208;
     const uint32_t q_full = bars + 224, q_empty = bars + 232;
-    volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 240);   // tensor memory, dead
+    volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 240);   // where tensor memory begins
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     const int ctas = (int)gridDim.x;
@@ -105,7 +109,6 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int* const items = work + ctas + 1;
     if (threadIdx.x == 0) {
         if (base & 1023u) atomicOr(err, XB_ERR_WAIT);
-        words[1] = 0;
         for (int i = 0; i < 16; ++i) mbar_init(bars + 8 * i, 1);            // k_full, k_empty, v_full, v_empty
         for (int i = 0; i < 4; ++i) {
             mbar_init(s_ready0 + 8 * i, 1);
@@ -148,7 +151,6 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const int last = w.nt == 2 ? w.hi[1] : w.hi[0];
             for (int kt = w.lo[0]; kt <= last; ++kt) {
                 if (rounds && !__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1u, err))) {
-                    words[1] = 1;
                     ok = false;
                     break;
                 }
@@ -233,7 +235,6 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 }
             }
         }
-        if (!ok) words[1] = 1;
     } else if (warp == 11) {
         // ---- O += P V of both tiles: P in tensor memory over the scores it came from, V MN-major
         const bool leader = lane == 0;
@@ -275,7 +276,6 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 }
             }
         }
-        if (!ok) words[1] = 1;
     } else if (warp < 8) {
         // ---- softmax: one query per thread
         const int i = warp >> 2, r = (int)threadIdx.x & 127;
@@ -406,7 +406,6 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             // these reads of O come before this tile's next announcement, and so before the product that overwrites it
         }
-        if (!alive) words[1] = 1;
     }
     tc_fence_before();
     __syncthreads();

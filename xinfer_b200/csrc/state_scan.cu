@@ -1250,9 +1250,9 @@ static inline int scan_row_groups(int rows) {
     return ds;
 }
 
-// Computing warps per block: enough to cover the columns (at most 8), fewer (down to 2) while the grid would
-// leave a third of the processors idle.  Every block of a head repeats the feeding warps' work, so column tiles
-// are not cut finer than that.
+// Computing warps per block: enough to cover the columns (at most 8; 4 where two blocks are to share a processor), fewer (down to
+// 2) while the grid would leave a third of the processors idle and the finer one still runs as one block per processor.  Every
+// block of a head repeats the feeding warps' copies, so column tiles are not cut finer than that.
 static inline int scan_warps(int cols, int ds, long long heads_total, int most = 8) {
     const int per_warp = (32 / ds) * 2;
     int warps = 1;

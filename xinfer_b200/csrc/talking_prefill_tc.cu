@@ -14,7 +14,8 @@
 // 2,048 tokens: 1,890 us -> 135 + 64 us with 32 heads, 1,088 us -> 51 + 43 us with 16.
 // What is rounded is what talking_attention_mma.cu rounds: the weights, once, in front of their product with the values, and it
 // is the rounded ones that are summed; the mixed scores leave as float32.  Steps whose tiles would not fit the scratch memory run
-// as several pairs of launches over fewer queries each.
+// as several pairs of launches over fewer queries each.  A value that is no number reaches every query of its tile of 128, those in
+// front of it too (0 x NaN); it was every query of a tile of 16.
 #include "attention_common.cuh"
 #include "tc_common.cuh"
 
@@ -96,7 +97,7 @@ constexpr int S_THREADS = 384;
 constexpr int S_MIX_REGS = 224, S_AUX_REGS = 56;
 constexpr int S_KEYS = 128;
 
-// The matrix, times the scale and log2(e): a kernel parameter, so that an entry is an operand of the constant bank.
+// The matrix, times the scale and log2(e).  It travels with the launch and is copied to shared memory, where the mix reads it.
 template <int H>
 struct TalkMatrix {
     float t[H * H];
