@@ -60,35 +60,29 @@ def fill_records(records: np.ndarray, params: Sequence[SamplingParams], seeds, d
     return off
 
 
-class _PinnedSet:
-    """Where one call's records and counted tokens lie on the host until they have been copied."""
-
-    def __init__(self, max_rows: int, record_bytes: int):
-        self.params = torch.zeros(max_rows * record_bytes, dtype=torch.uint8, pin_memory=True)
-        self.params_np = self.params.numpy().view(kernels.SAMPLE_PARAMS)
-        self.hist = self.hist_np = None
-
-    def history(self, max_rows: int) -> np.ndarray:
-        if self.hist is None:
-            self.hist = torch.zeros(max_rows * PENALTY_HISTORY, dtype=torch.int32, pin_memory=True)
-            self.hist_np = self.hist.numpy()
-        return self.hist_np
-
-
 class _PinnedSets:
-    """Pinned sets used in turn by calls that nobody may have waited for.  Half of them are taken again only after the copies that
-    read them have been made: one event per half, since recording and asking one for every call took a tenth of its time."""
+    """Where calls' records and counted tokens lie on the host until they have been copied, for calls that nobody may have waited
+    for: sets used in turn.  Half of them are taken again only after the copies that read them have been made: one event per
+    half, since recording and asking one for every call took a tenth of its time."""
 
     def __init__(self, max_rows: int, record_bytes: int, half: int = 8):
-        self.sets = [_PinnedSet(max_rows, record_bytes) for _ in range(2 * half)]
+        self.params = torch.zeros((2 * half, max_rows * record_bytes), dtype=torch.uint8, pin_memory=True)
+        self.max_rows, self.hist = max_rows, None
+        self.sets = [None] * (2 * half)         # (bytes, the same as records, counted tokens, the same as an array), made when needed
         self.copied = [torch.cuda.Event(), torch.cuda.Event()]
         self.half, self.at = half, 0
 
-    def take(self) -> _PinnedSet:
-        """A set that no copy reads any more."""
+    def take(self, counts_tokens: bool):
+        """A set that no copy reads any more: (bytes, the same as records, counted tokens, the same as an array; None without)."""
         if self.at % self.half == 0:
             self.copied[self.at // self.half].synchronize()
-        return self.sets[self.at]
+        mine = self.sets[self.at]
+        if mine is None or (counts_tokens and mine[2] is None):
+            if counts_tokens and self.hist is None:
+                self.hist = torch.zeros((2 * self.half, self.max_rows * PENALTY_HISTORY), dtype=torch.int32, pin_memory=True)
+            params, hist = self.params[self.at], self.hist[self.at] if self.hist is not None else None
+            mine = self.sets[self.at] = (params, params.numpy().view(kernels.SAMPLE_PARAMS), hist, hist.numpy() if hist is not None else None)
+        return mine
 
     def sent(self) -> None:
         """The set last taken has been handed to its copies."""
@@ -125,13 +119,13 @@ class Sampler:
         R = logits.shape[0]
         if R > self.max_rows:
             raise ValueError(f"{R} rows exceed the sampler's capacity {self.max_rows}")
-        mine = self._pinned.take()
-        off = fill_records(mine.params_np, params[:R], seeds, draws, histories, mine.history(self.max_rows) if histories is not None else None)
+        params_host, records, hist_host, hist = self._pinned.take(histories is not None)
+        off = fill_records(records, params[:R], seeds, draws, histories, hist)
         any_pen = off > 0
         nb = R * kernels.SAMPLE_PARAMS.itemsize
-        self._params_dev[:nb].copy_(mine.params[:nb], non_blocking=True)
+        self._params_dev[:nb].copy_(params_host[:nb], non_blocking=True)
         if any_pen:
-            self._hist_dev[:off].copy_(mine.hist[:off], non_blocking=True)
+            self._hist_dev[:off].copy_(hist_host[:off], non_blocking=True)
         self._pinned.sent()
         if tracing.ENABLED:
             tracing.push("sample")
