@@ -239,3 +239,38 @@ def test_a_work_list_that_was_cut_off_is_refused():
     run(work)
     run(work, at=None)
     assert int(err) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("key,channel,value", [(0, 0, math.nan), (100, 71, math.inf), (127, 3, -math.inf), (128, 8, math.nan), (190, 70, math.nan),
+                                               (250, 9, math.inf), (449, 5, math.nan)])
+@pytest.mark.parametrize("window", [None, 70])
+def test_a_row_that_is_not_finite_reaches_only_the_queries_that_see_it(key, channel, value, window):
+    H, d, rd, dv, rank, ps, start, n = 3, 64, 8, 64, 72, 16, 150, 300
+    g = torch.Generator().manual_seed(key)
+    i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    end, width = start + n, rank + rd
+    rows_in, q = torch.randn(end, width, generator=g).bfloat16(), torch.randn(n, H * (d + rd), generator=g).bfloat16().to(DEV)
+    w_kv = (torch.randn(H * (d + dv), rank, generator=g) * rank ** -0.5).bfloat16().to(DEV)
+    per = -(-end // ps)
+    host, ctas, total, at = kernels.latent_prefill_work([n], [start], 4, window, H)
+    work, q_start, start_pos, err, table = host.to(DEV), i32(0, n), i32(start), i32(0), torch.arange(per, dtype=torch.int32, device=DEV).view(1, per)
+
+    def run(rows_in):
+        pages = torch.zeros(per * ps, width, dtype=torch.bfloat16)
+        pages[:end] = rows_in
+        rows, bad = torch.empty(total, width, dtype=torch.bfloat16, device=DEV), torch.full((total // 32,), -1, dtype=torch.int32, device=DEV)
+        kernels.latent_gather(rows, pages.to(DEV).view(per, ps, width), work, at, q_start, start_pos, table, per, window, err, rank=rank, bad=bad)
+        out = torch.zeros(n, H * dv, dtype=torch.bfloat16, device=DEV)
+        kernels.attn_rows_tc(out, q, H * (d + rd), rows[:, :rank] @ w_kv.t(), rows, work, ctas, q_start, start_pos, H, d, rd, dv, rank, window,
+                             (d + rd) ** -0.5, None, err, at, bad)
+        assert int(err) == 0
+        return out.cpu(), bad.cpu()
+    clean, none = run(rows_in)
+    assert not none.any() and torch.isfinite(clean).all()
+    rows_in[key, channel] = value
+    got, bad = run(rows_in)
+    first = max(0, start - window + 1) if window else 0
+    assert sum(bin(int(b) & 0xFFFFFFFF).count("1") for b in bad) == (1 if key >= first else 0)
+    sees = torch.tensor([key <= start + i and (window is None or key > start + i - window) for i in range(n)])
+    assert torch.isnan(got[sees]).all() and torch.equal(got[~sees], clean[~sees])

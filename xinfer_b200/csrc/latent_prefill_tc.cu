@@ -18,8 +18,9 @@
 //                          with scores, probabilities and accumulators in tensor memory, TMA-fed rings, one softmax row
 //                          per thread.  Two tiles of 128 queries share every key/value tile.
 //
-// A value that is no number reaches every query of its tile of 128, those in front of it too (0 x NaN), as in the kernel over
-// pages; the kernel over the cached rows kept it to its block of 32 (query, head) rows.
+// A cached row whose latent holds an infinity or no number must not reach queries that do not see it (a weight of 0 times its
+// values would): the gathering kernel leaves zeros in its place and marks it, and the attention makes the result of every query
+// that sees it no number.
 #include "attention_common.cuh"
 #include "tc_common.cuh"
 
@@ -58,14 +59,15 @@ __device__ __forceinline__ Item item_of(const int* __restrict__ it, const int* _
     return w;
 }
 
-// One warp per row of the gathered buffer.  blocks: (portion, first position) of every run of 64 rows.
+// One warp per row of the gathered buffer, eight rows a block.  blocks: (portion, first position) of every run of 64 rows.  `bad`
+// (a bit per row): rows whose first `checked` pieces hold something that is not finite; they are gathered as zeros.
 __global__ void latent_gather_kernel(uint4* __restrict__ out, const uint4* pages, const int* __restrict__ blocks,
                                      int rows, const int* __restrict__ q_start, const int* __restrict__ start_pos,
                                      const int* __restrict__ table, int table_stride, int page_size, int num_pages, int window,
-                                     int pieces, int* err) {
+                                     int pieces, int checked, unsigned char* bad, int* err) {
     pdl_overlap_few();
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= rows) return;
+    __shared__ int s_off[8];
+    const int warp = threadIdx.x >> 5, row = blockIdx.x * 8 + warp, lane = threadIdx.x & 31;      // rows: a multiple of 64
     const int b = blocks[2 * (row >> 6)], j = blocks[2 * (row >> 6) + 1] + (row & 63);
     const int start = start_pos[b], end = start + q_start[b + 1] - q_start[b];
     const uint4* src = nullptr;
@@ -77,7 +79,21 @@ __global__ void latent_gather_kernel(uint4* __restrict__ out, const uint4* pages
             src = pages + ((size_t)page * page_size + j % page_size) * pieces;
         }
     }
+    bool off = false;
+    if (bad != nullptr && src != nullptr)
+        for (int c = lane; c < checked; c += 32) off |= bf16_not_finite(src[c]);
+    if (__any_sync(0xffffffffu, off)) src = nullptr, off = true;
     for (int c = lane; c < pieces; c += 32) out[(size_t)row * pieces + c] = src ? src[c] : make_uint4(0, 0, 0, 0);
+    if (bad != nullptr) {
+        if (lane == 0) s_off[warp] = off ? 1 << warp : 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int bits = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) bits |= s_off[i];
+            bad[blockIdx.x] = (unsigned char)bits;
+        }
+    }
 }
 
 // NKC: 64-channel pieces of a key (the last one is the part all heads share when TAIL), DVC: of a value.
@@ -90,7 +106,8 @@ __global__ void __launch_bounds__(THREADS)
 attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                     const __grid_constant__ CUtensorMap map_tail, __nv_bfloat16* __restrict__ out, long long ldo,
                     const int* __restrict__ q_start, const int* __restrict__ start_pos, int nh, int rank, int window,
-                    float scale_log2, const float* __restrict__ sink, const int* __restrict__ work, int* err) {
+                    float scale_log2, const float* __restrict__ sink, const int* __restrict__ work, const unsigned long long* bad,
+                    int* err) {
     constexpr int D = 64 * (NKC - (TAIL ? 1 : 0)), DV = 64 * DVC;
     constexpr uint32_t Q_ONE = NKC * QT * 128, Q_BYTES = 2 * Q_ONE;
     constexpr uint32_t PIECE = KT * 128, K_BYTES = NKC * PIECE, STAGE_BYTES = (NKC + DVC) * PIECE;
@@ -293,6 +310,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             float m_ref = -INFINITY, l = 0.f;
             for (int kt = lo; kt <= hi; ++kt, ++th) {
                 const int sb = th & 1, key0 = kt * KT;
+                const unsigned long long off = bad != nullptr ? bad[(w.row0 + key0) / KT] : 0ull;
                 if (!__all_sync(0xffffffffu, mbar_wait(my_s_ready + 8 * sb, (th >> 1) & 1, err))) {
                     alive = false;
                     break;
@@ -315,6 +333,13 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     for (int c = 0; c < 64; ++c) {
                         const int j = key0 + c;
                         sc[c] = (j <= my_pos && j <= last_key && j >= my_lo) ? sc[c] : -INFINITY;
+                    }
+                }
+                if (off != 0ull) {      // (rare) rows of the tile that were not finite: no number for the queries that see them
+#pragma unroll
+                    for (int c = 0; c < 64; ++c) {
+                        const int j = key0 + c;
+                        if (((off >> c) & 1ull) && j <= my_pos && j <= last_key && j >= my_lo) sc[c] = NAN;
                     }
                 }
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -414,26 +439,27 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
 template <int NKC, int DVC, bool TAIL>
 int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mt, void* out, long long ldo, const int* q_start,
-           const int* start_pos, int nh, int rank, int window, float sl2, const float* sink, const int* work, int ctas, int* err,
-           cudaStream_t stream) {
+           const int* start_pos, int nh, int rank, int window, float sl2, const float* sink, const int* work, int ctas,
+           const unsigned long long* bad, int* err, cudaStream_t stream) {
     constexpr size_t smem = (size_t)2 * NKC * QT * 128 + (size_t)STAGES * (NKC + DVC) * KT * 128 + 1024;
     const auto kernel = attn_rows_tc_kernel<NKC, DVC, TAIL>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return xb_launch(kernel, dim3(ctas), dim3(THREADS), smem, stream, mq, mkv, mt, (__nv_bfloat16*)out, ldo, q_start, start_pos,
-                     nh, rank, window, sl2, sink, work, err);
+                     nh, rank, window, sl2, sink, work, bad, err);
 }
 
 }  // namespace
 
 // Rows of `width` bfloat16 (a multiple of 8) from their pages [pages, page_size, width] into out [rows, width], rows a
-// multiple of 64: run i of 64 rows holds portion blocks[2 i]'s positions from blocks[2 i + 1] on.
+// multiple of 64: run i of 64 rows holds portion blocks[2 i]'s positions from blocks[2 i + 1] on.  `bad` (rows / 8 bytes, or none):
+// see latent_gather_kernel; `rank` channels are looked at.
 XB_EXPORT int xb_latent_gather(void* out, const void* pages, const int* blocks, int rows, const int* q_start,
                                const int* start_pos, const int* table, int table_stride, int page_size, int num_pages,
-                               int window, int width, int* err, cudaStream_t stream) {
+                               int window, int width, int rank, void* bad, int* err, cudaStream_t stream) {
     if (rows <= 0) return 0;
-    if (width % 8 || rows % 64 || page_size <= 0 || window < 0) return (int)cudaErrorInvalidValue;
-    xb_launch_few(latent_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, (uint4*)out, (const uint4*)pages, blocks, rows, q_start, start_pos,
-                                                             table, table_stride, page_size, num_pages, window, width / 8, err);
+    if (width % 8 || rows % 64 || page_size <= 0 || window < 0 || rank % 8 || rank < 0 || rank > width) return (int)cudaErrorInvalidValue;
+    xb_launch_few(latent_gather_kernel, dim3(rows / 8), dim3(256), 0, stream, (uint4*)out, (const uint4*)pages, blocks, rows, q_start, start_pos,
+                  table, table_stride, page_size, num_pages, window, width / 8, rank / 8, (unsigned char*)bad, err);
     return xb_launch_status();
 }
 
@@ -445,14 +471,14 @@ XB_EXPORT int xb_attn_rows_tc_takes(int d, int rd, int dv, int rank) {
 // q: head h of token t at q + t * q_ts + h * (d + rd) [d + rd]; kv [rows, nh * (d + dv)]: all heads' keys, then all
 // heads' values; tail [rows, width]: channels rank .. rank + rd - 1 are the key part all heads share; out: head h of
 // token t at out + t * ldo + h * dv.  `work` comes from xb_latent_prefill_work (host library) for the same step, heads
-// and window.  Returns cudaErrorNotSupported, having done nothing, for sizes or strides it does not take.
+// and window; `bad` from xb_latent_gather (or none).  Returns cudaErrorNotSupported, having done nothing, for sizes or strides it does not take.
 XB_EXPORT int xb_attn_rows_tc(void* out, long long ldo, const void* q, long long q_ts, const void* kv, const void* tail,
                               int tokens, int rows, int nh, int d, int rd, int dv, int rank, int width, const int* q_start,
                               const int* start_pos, int window, float scale, const float* sink, const int* work, int ctas,
-                              int* err, cudaStream_t stream) {
+                              const void* bad, int* err, cudaStream_t stream) {
     if (ctas <= 0) return 0;
     if (!xb_attn_rows_tc_takes(d, rd, dv, rank) || nh <= 0 || nh > 65535 || q_ts % 8 || width % 8 || width < rank + rd || ldo % 8 ||
-        rows % 64 || window < 0 || (((uintptr_t)out | (uintptr_t)q | (uintptr_t)kv | (uintptr_t)tail) & 15))
+        rows % 64 || window < 0 || (((uintptr_t)out | (uintptr_t)q | (uintptr_t)kv | (uintptr_t)tail) & 15) || ((uintptr_t)bad & 7))
         return (int)cudaErrorNotSupported;
     CUtensorMap mq, mkv, mt;
     const long long qd[3] = {d + rd, nh, tokens}, qs[2] = {d + rd, q_ts};
@@ -464,7 +490,7 @@ XB_EXPORT int xb_attn_rows_tc(void* out, long long ldo, const void* q, long long
         !tensor_map_bf16(&mt, tail, 2, td, ts, tb))
         return (int)cudaErrorNotSupported;
     const float sl2 = scale * 1.4426950408889634f;
-#define XB_GO(N, V, T) return launch<N, V, T>(mq, mkv, mt, out, ldo, q_start, start_pos, nh, rank, window, sl2, sink, work, ctas, err, stream)
+#define XB_GO(N, V, T) return launch<N, V, T>(mq, mkv, mt, out, ldo, q_start, start_pos, nh, rank, window, sl2, sink, work, ctas, (const unsigned long long*)bad, err, stream)
     if (d == 128) {
         if (dv == 128) { if (rd) XB_GO(3, 2, true); else XB_GO(2, 2, false); }
         if (rd) XB_GO(3, 1, true); else XB_GO(2, 1, false);

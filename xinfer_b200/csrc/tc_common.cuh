@@ -266,6 +266,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Whether one of the eight bfloat16 numbers is an infinity or no number.
+__device__ __forceinline__ bool bf16_not_finite(const uint4& v) {
+    auto two = [](uint32_t w) { return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u; };
+    return two(v.x) || two(v.y) || two(v.z) || two(v.w);
+}
+
 // ---- host: tensor maps -------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,

@@ -1212,27 +1212,35 @@ def latent_prefill_work(counts, starts, dec_max: int, window, heads: int, max_ct
     return host[:max(int(used), 1)], int(ctas.value), int(rows.value), int(used) - rows.value // 32
 
 
-def latent_gather(out, pages, work, runs_at: int, q_start, start_pos, block_table, table_stride, window, err) -> None:
+def latent_gather(out, pages, work, runs_at: int, q_start, start_pos, block_table, table_stride, window, err, *, rank: int = 0,
+                  bad=None) -> None:
     """The cached rows that the portions of a ``latent_prefill_work`` list see, one portion after the other, into ``out``
-    ``[rows, width]``; rows that no query of a portion sees are zeros."""
+    ``[rows, width]``; rows that no query of a portion sees are zeros.  ``bad`` (int32, ``rows / 32``): a bit for every row whose
+    first ``rank`` channels are not all finite; it is zeros in ``out``."""
     rows, width = out.shape
     _need(out, "out", torch.bfloat16)
     _need(pages, "pages", torch.bfloat16, (None, None, width))
     _need(work, "work", torch.int32)
     if width % 8 or rows % 64 or work.numel() < runs_at + rows // 32:
         raise KernelError("gathered rows: a width that is no multiple of 8, or more rows than the work list names")
+    if bad is not None:
+        _need(bad, "bad", torch.int32)
+        if bad.numel() < rows // 32 or rank % 8 or not 0 < rank <= width:
+            raise KernelError("marked rows: fewer bits than rows, or a rank that is no multiple of 8")
     _ok(kernels_lib().xb_latent_gather(out.data_ptr(), pages.data_ptr(), work.data_ptr() + 4 * int(runs_at), rows, q_start.data_ptr(),
                                        start_pos.data_ptr(), block_table.data_ptr(), int(table_stride), pages.shape[1], pages.shape[0],
-                                       int(window or 0), width, err.data_ptr(), _stream()), "latent_gather")
+                                       int(window or 0), width, int(rank) if bad is not None else 0, _ptr(bad), err.data_ptr(),
+                                       _stream()), "latent_gather")
 
 
 def attn_rows_tc(out, q, q_row: int, kv, rows, work, ctas, q_start, start_pos, nh: int, d: int, rd: int, dv: int, rank: int,
-                 window, scale, sink, err, runs_at: Optional[int] = None) -> None:
+                 window, scale, sink, err, runs_at: Optional[int] = None, bad=None) -> None:
     """Attention of the portions of a ``latent_prefill_work`` list on tcgen05 (TMA-fed; scores, probabilities and
     accumulators in tensor memory).  ``q``: rows of ``q_row`` elements whose first ``nh * (d + rd)`` are the heads'
     queries; ``kv`` ``[n, nh * (d + dv)]``: all heads' keys, then all heads' values; ``rows`` ``[n, width]``: the gathered
     rows, whose rd channels from ``rank`` on belong to every head's key.  ``out`` ``[T, nh * dv]`` receives the rows of the
-    list's portions; others stay as they are.  ``runs_at``: as ``latent_prefill_work`` returned it, to check the list with."""
+    list's portions; others stay as they are.  ``runs_at``: as ``latent_prefill_work`` returned it, to check the list with.
+    ``bad``: the rows that ``latent_gather`` marked; a query that sees one has no number for a result."""
     n, width = rows.shape
     T = out.shape[0]
     _need(out, "out", torch.bfloat16, (T, nh * dv))
@@ -1242,6 +1250,10 @@ def attn_rows_tc(out, q, q_row: int, kv, rows, work, ctas, q_start, start_pos, n
     _need(work, "work", torch.int32)
     if sink is not None:
         _need(sink, "sink", torch.float32, (nh,))
+    if bad is not None:
+        _need(bad, "bad", torch.int32)
+        if bad.numel() < n // 32:
+            raise KernelError("fewer marks than gathered rows")
     items = work.numel() - n // 32 - (ctas + 1) if runs_at is None else int(runs_at) - (ctas + 1)       # four numbers each
     if q_row < nh * (d + rd) or width < rank + rd or n % 64 or (ctas > 0 and (
             items < 4 * ctas or items % 4 or work.numel() < ctas + 1 + items + n // 32)):
@@ -1249,7 +1261,7 @@ def attn_rows_tc(out, q, q_row: int, kv, rows, work, ctas, q_start, start_pos, n
     _ok(kernels_lib().xb_attn_rows_tc(
         out.data_ptr(), nh * dv, q.data_ptr(), int(q_row), kv.data_ptr(), rows.data_ptr(), T, n, int(nh), int(d), int(rd), int(dv),
         int(rank), width, q_start.data_ptr(), start_pos.data_ptr(), int(window or 0), float(scale), _ptr(sink), work.data_ptr(),
-        int(ctas), err.data_ptr(), _stream()), "attn_rows_tc")
+        int(ctas), _ptr(bad), err.data_ptr(), _stream()), "attn_rows_tc")
 
 
 def gate_sigmoid(out, heads, gate):

@@ -109,7 +109,8 @@ def rows_plan(ctx: StepContext, heads: int, d: int, rd: int, dv: int, rank: int,
             ws, per_row = ctx.workspace, heads * (d + dv)
             most = ROWS_MAX_BYTES // (2 * per_row)
             if ws.reserve("latent.rows", rows * width, torch.bfloat16, most * width) \
-                    and ws.reserve("latent.kv", rows * per_row, torch.bfloat16, most * per_row):
+                    and ws.reserve("latent.kv", rows * per_row, torch.bfloat16, most * per_row) \
+                    and ws.reserve("latent.bad", rows // 32, torch.int32, most // 32):
                 made = (host.to(ctx.positions.device, non_blocking=True), ctas, rows, runs_at, small)
                 _rows_ring.sent()
     ctx.scratch[key] = made
@@ -290,11 +291,12 @@ class LatentAttention(Mixer):
             if rd or kv_off >= 0:
                 prepare(None, q_rows, kv_off, in_place=rd > 0)
             rows = ws.get("latent.rows", (n, r + rd + tail), self.dtype)
-            kernels.latent_gather(rows, pages, work, runs_at, ctx.q_start, ctx.start_pos, table, stride, s.window, ctx.err)
+            bad = ws.get("latent.bad", (n // 32,), torch.int32)
+            kernels.latent_gather(rows, pages, work, runs_at, ctx.q_start, ctx.start_pos, table, stride, s.window, ctx.err, rank=r, bad=bad)
             kv = ws.get("latent.kv", (n, H * (d + dv)), self.dtype)
             linear(kv, rows[:, :r], self.w_kv, ctx.err)
             kernels.attn_rows_tc(inner, q_rows, q_rows.shape[1], kv, rows, work, ctas, ctx.q_start, ctx.start_pos, H, d, rd, dv, r,
-                                 s.window, s.scale, self.sink, ctx.err, runs_at)
+                                 s.window, s.scale, self.sink, ctx.err, runs_at, bad)
         if s.gate:
             kernels.gate_sigmoid(inner, o_heads, proj[:, at_gate:at_gate + (H if s.gate_per_head else H * dv)])
         out = ws.get("latent.out", (T, s.hidden), ctx.branch_dtype or self.dtype)
