@@ -190,6 +190,36 @@ def test_a_key_that_is_not_a_number_shows_in_every_query_that_sees_it(key):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("key,channel,value", [(0, 0, math.nan), (63, 5, math.inf), (64, 63, -math.inf), (130, 8, math.nan), (190, 17, math.inf),
+                                               (199, 40, math.nan)])
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("H,G,dv", [(16, 8, 128), (8, 8, 64)])
+def test_a_value_that_is_not_finite_reaches_only_the_queries_that_see_it(H, G, dv, window, key, channel, value):
+    T, d = 200, 64
+    g = torch.Generator().manual_seed(key)
+    q, k, v, table, _, _, (q_start, start_pos), err = _prompt(T, H, G, d, dv, g)
+    host, chunks, tiles = kernels.talk_work([T], [0], window, H, G, 1 << 16)
+    work, scores = host.to(DEV), torch.empty(tiles * kernels.TALK_TILE_FLOATS, device=DEV)
+    talk = torch.randn(H, H, generator=g) * H ** -0.5
+
+    def run():
+        out = torch.zeros(T, H, dv, dtype=torch.bfloat16, device=DEV)
+        kernels.attn_talking_tc(out.view(T, H * dv), q, k, v, talk, scores, work, chunks, q_start, start_pos, table, table.shape[1], window,
+                                d ** -0.5, True, 1.0, err)
+        return out
+    v[key // 16, 1, key % 16, channel] = 0
+    want = run()
+    v[key // 16, 1, key % 16, channel] = value
+    got = run()
+    sees = torch.zeros_like(want, dtype=torch.bool)
+    sees[key:key + (window or T), H // G: 2 * (H // G), channel] = True
+    # (a query of a tile that every query sees whole may turn a weight too small for bfloat16 times infinity into no number)
+    assert int(err) == 0 and not torch.isfinite(got[sees]).any() and torch.equal(got[~sees], want[~sees])
+    if value == value:
+        assert not (got[sees] == -value).any()
+
+
+@pytest.mark.gpu
 def test_weights_are_divided_by_their_own_sum():
     # Values that are all one: the result is the sum of the rounded weights over what it is divided by, times the factor.  The
     # factor lies 2^-14 above the middle between two bfloat16 numbers, so that a quotient that is off by more than that rounds to

@@ -14,8 +14,9 @@
 // 2,048 tokens: 1,890 us -> 135 + 64 us with 32 heads, 1,088 us -> 51 + 43 us with 16.
 // What is rounded is what talking_attention_mma.cu rounds: the weights, once, in front of their product with the values, and it
 // is the rounded ones that are summed; the mixed scores leave as float32.  Steps whose tiles would not fit the scratch memory run
-// as several pairs of launches over fewer queries each.  A value that is no number reaches every query of its tile of 128, those in
-// front of it too (0 x NaN); it was every query of a tile of 16.
+// as several pairs of launches over fewer queries each.  A value that is not finite must not reach queries that do not see it (a
+// weight of 0 times it would): in tiles that some query sees in part it is a 0 for the product, and is added to the results of the
+// queries that see it.
 #include "attention_common.cuh"
 #include "tc_common.cuh"
 
@@ -341,16 +342,49 @@ talk_scores_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 // tiles of 16 KB lie side by side in memory and come as one bulk copy into one of three stages; a thread reads its row, whose 16-byte pieces the
 // kernel before has laid out XOR-ed with row & 7.  The roles and waits are those of the prefill kernel over pages, with
 // scores from shared memory in place of a product.
-//   warps 0..3, 4..7 softmax of the two heads, warp 8 loads score tiles, warp 10 value pages, warp 11 issues O += P V.
+//   warps 0..3, 4..7 softmax of the two heads, warp 8 loads score tiles, warp 10 value pages, warp 9 clears in them what must not
+//   meet a weight of 0, warp 11 issues O += P V.
 // Tensor memory: P of head A at 0 and 32, of head B at 64 and 96 (two buffers each); O at 128 and 256.
 constexpr int V_THREADS = 384;
 constexpr int V_KEYS = 64;
 constexpr int S_STAGES = 3, V_STAGES = 2;       // of scores (64 KB each) and of values (16 KB)
 constexpr uint32_t V_SCORES = 2 * TILE_FLOATS * 4;       // one head's scores of a stage
 
+// Whether some of the queries from position p0 on do not see all of the 64 keys from key0 on; edge_lo: the first key that the last
+// of them sees.
+__device__ __forceinline__ bool seen_in_part(int key0, int p0, int edge_lo) { return key0 + V_KEYS - 1 > p0 || key0 < edge_lo; }
+
+// An element of a value row that holds an infinity or no number.
+__device__ __forceinline__ bool bf16_bits_not_finite(uint32_t b) { return (b & 0x7f80u) == 0x7f80u; }
+
+// (Rare.)  To one query's result of one head: the values that are not finite, of the keys from `first` to `last` (those it sees) in
+// tiles that were cleared of them.
+__device__ __noinline__ void add_not_finite(__nv_bfloat16* dst, const __nv_bfloat16* vc, const int* table, int nkv, int g, int ps, int ps_shift,
+                                            int num_pages, int dv, int first, int last, int p0, int edge_lo, float out_scale) {
+    for (int j = first; j <= last; ++j) {
+        const int key0 = j / V_KEYS * V_KEYS;
+        if (!seen_in_part(key0, p0, edge_lo)) {
+            j = key0 + V_KEYS - 1;
+            continue;
+        }
+        const int page = table[j >> ps_shift];
+        if (page < 0 || page >= num_pages) continue;
+        const uint4* row = reinterpret_cast<const uint4*>(vc + ((size_t)(page * nkv + g) * ps + (j & (ps - 1))) * dv);
+        for (int c8 = 0; c8 < dv / 8; ++c8) {
+            const uint4 v = row[c8];
+            if (!bf16_not_finite(v)) continue;
+            for (int c = 0; c < 8; ++c) {
+                const uint32_t w = c < 2 ? v.x : c < 4 ? v.y : c < 6 ? v.z : v.w, b = (c & 1) ? w >> 16 : w & 0xffffu;
+                if (bf16_bits_not_finite(b))
+                    dst[c8 * 8 + c] = __float2bfloat16(__bfloat162float(dst[c8 * 8 + c]) + out_scale * __uint_as_float(b << 16));
+            }
+        }
+    }
+}
+
 template <int DVC>
 __global__ void __launch_bounds__(V_THREADS)
-talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* scores, __nv_bfloat16* __restrict__ out,
+talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const __nv_bfloat16* vc, const float* scores, __nv_bfloat16* __restrict__ out,
                       long long ldo, const int* __restrict__ blocks, const int* __restrict__ work, const int* __restrict__ q_start,
                       const int* __restrict__ start_pos, const int* __restrict__ block_table, int table_stride, int nh, int nkv,
                       int ps, int ps_shift, int num_pages, int window, int sink, float out_scale, int* err) {
@@ -360,8 +394,10 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
     const uint32_t base = smem_u32(smem_raw), bars = base + BAR_OFF;
     // v_full[stage] v_empty[stage] pv_done[head][2] p_ready[head] o_done[head] s_full[head][stage] s_empty[head][stage]
     const uint32_t v_full0 = bars, v_empty0 = bars + 16, pv_done0 = bars + 32, p_ready0 = bars + 64, o_done0 = bars + 80;
-    const uint32_t s_full0 = bars + 96, s_empty0 = bars + 96 + 16 * S_STAGES;
+    const uint32_t s_full0 = bars + 96, s_empty0 = bars + 96 + 16 * S_STAGES, v_clear0 = bars + 96 + 32 * S_STAGES;      // v_clear[stage]
+    volatile uint32_t* marks = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 112 + 32 * S_STAGES);      // of four items in turn
     volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem_raw + BAR_OFF + 240);
+    static_assert(112 + 32 * S_STAGES + 16 <= 240, "room for the barriers");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ctas = (int)gridDim.x;
     const int item_begin = work[blockIdx.x];
@@ -380,6 +416,7 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
         for (int i = 0; i < 2; ++i) {
             mbar_init(p_ready0 + 8 * i, 128);
             mbar_init(o_done0 + 8 * i, 1);
+            mbar_init(v_clear0 + 8 * i, 32);
         }
         mbar_init_fence();
     }
@@ -485,6 +522,52 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
                 }
             }
         }
+    } else if (warp == 9) {
+        // ---- values that must not meet a weight of 0, in tiles that some query sees in part: rows that no query of the block
+        // sees (their pages were not loaded, or hold anything) become zeros, and so do elements that are not finite; whether
+        // there were any of those is the item's mark.  The product waits for this warp at every tile.
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int k = item_begin; k < item_end && ok; ++k) {
+            const Item w = item_at(k);
+            const int edge_lo = first_visible(w.blk.p0 + QB_ROWS - 1, window);
+            bool any = false;
+            if (lane == 0) marks[k & 3] = 0;
+            for (int kt = w.lo; kt <= w.hi; ++kt) {
+                if (!__all_sync(0xffffffffu, mbar_wait(v_full0 + 8 * s, ph, err))) {
+                    ok = false;
+                    break;
+                }
+                const int key0 = kt * V_KEYS;
+                if (seen_in_part(key0, w.blk.p0, edge_lo)) {
+                    uint4* tile = reinterpret_cast<uint4*>(smem_raw + V_OFF + s * V_BYTES);
+#pragma unroll 4
+                    for (int i = lane; i < (int)V_BYTES / 16; i += 32) {       // a row is 8 pieces of 16 bytes, in any order
+                        const int j = key0 + ((i >> 3) & (V_KEYS - 1));
+                        const bool out_of = j < w.first_key || j > w.last_key;
+                        uint4 v = tile[i];
+                        if (out_of) {
+                            tile[i] = make_uint4(0, 0, 0, 0);
+                        } else if (bf16_not_finite(v)) {
+                            auto clear = [](uint32_t x) {
+                                return (bf16_bits_not_finite(x) ? 0u : x & 0xffffu) | (bf16_bits_not_finite(x >> 16) ? 0u : x & 0xffff0000u);
+                            };
+                            tile[i] = make_uint4(clear(v.x), clear(v.y), clear(v.z), clear(v.w));
+                            any = true;
+                        }
+                    }
+                    fence_async_shared();
+                    any = __any_sync(0xffffffffu, any);
+                    if (any && lane == 0) marks[k & 3] = 1;
+                }
+                mbar_arrive(v_clear0 + 8 * s);
+                if (++s == V_STAGES) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
     } else if (warp == 11) {
         // ---- O += P V
         const bool leader = lane == 0;
@@ -496,7 +579,7 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
         for (int k = item_begin; k < item_end && ok; ++k) {
             const Item w = item_at(k);
             for (int kt = w.lo; kt <= w.hi && ok; ++kt) {
-                ok = __all_sync(0xffffffffu, mbar_wait(v_full0 + 8 * s, ph, err, true));
+                ok = __all_sync(0xffffffffu, mbar_wait(v_clear0 + 8 * s, ph, err, true));
                 const uint64_t dv = dv0 + (uint64_t)((s * V_BYTES) >> 4);
 #pragma unroll
                 for (int hd = 0; hd < 2; ++hd) {
@@ -530,19 +613,16 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
         const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
         const uint32_t tmem_p = tmem + (uint32_t)(hd * 64) + lane_addr, tmem_o = tmem + (uint32_t)(128 + hd * 128) + lane_addr;
         const uint32_t my_p_ready = p_ready0 + 8 * hd, my_pv_done = pv_done0 + 16 * hd;
-        int th = 0, vt = 0, done = 0;      // key tiles of this head, of all items, items of this head
+        int th = 0, done = 0;      // key tiles of this head, items of this head
         uint32_t ss = 0, sph = 0;           // stage of this head's next scores, parity of the rounds
         bool alive = true;
         for (int k = item_begin; k < item_end && alive; ++k) {
             const Item w = item_at(k);
-            if (hd >= w.nhd) {
-                vt += w.hi - w.lo + 1;
-                continue;
-            }
+            if (hd >= w.nhd) continue;
             const int p0 = w.blk.p0, my_pos = p0 + r, last_key = w.last_key, lo = w.lo, hi = w.hi;
             const int my_lo = first_visible(my_pos, window), edge_lo = first_visible(p0 + QB_ROWS - 1, window);
             float m_ref = sink ? 0.f : -INFINITY, l = sink ? 1.f : 0.f;      // the silent entry: score 0
-            for (int kt = lo; kt <= hi; ++kt, ++th, ++vt) {
+            for (int kt = lo; kt <= hi; ++kt, ++th) {
                 const int sb = th & 1, key0 = kt * V_KEYS;
                 if (!__all_sync(0xffffffffu, mbar_wait(s_full0 + 8 * (S_STAGES * hd + ss), sph, err))) {
                     alive = false;
@@ -563,7 +643,7 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
                     ss = 0;
                     sph ^= 1u;
                 }
-                if (key0 + V_KEYS - 1 > p0 || key0 + V_KEYS - 1 > last_key || key0 < edge_lo) {
+                if (seen_in_part(key0, p0, edge_lo)) {
 #pragma unroll
                     for (int c = 0; c < 64; ++c) {
                         const int j = key0 + c;
@@ -614,24 +694,6 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
                 l = l * corr + ((s0 + s1) + (s2 + s3));
                 // P's buffer was read two tiles ago: by the product whose end was waited for one tile ago, or one before it
                 tmem_st32_u(tmem_p + sb * 32, pk);
-                // value rows that no query of the block sees become zeros (the tiles at the ends of the range); the second
-                // head's product is issued after the first's, so it sees them too
-                if (hd == 0 && (key0 < w.first_key || key0 + V_KEYS - 1 > last_key)) {
-                    const int st = vt & 1;
-                    if (!__all_sync(0xffffffffu, mbar_wait(v_full0 + 8 * st, (vt >> 1) & 1, err))) {
-                        alive = false;
-                        break;
-                    }
-                    if (r < V_KEYS && (key0 + r < w.first_key || key0 + r > last_key)) {
-#pragma unroll
-                        for (int f = 0; f < DVC; ++f) {
-                            uint4* vr = reinterpret_cast<uint4*>(smem_raw + V_OFF + st * V_BYTES + f * PIECE + r * 128);
-#pragma unroll
-                            for (int c8 = 0; c8 < 8; ++c8) vr[c8] = make_uint4(0, 0, 0, 0);
-                        }
-                    }
-                    fence_async_shared();
-                }
                 // the product before must be complete before O is touched, and before this tile is announced
                 if (kt > lo && !__all_sync(0xffffffffu, mbar_wait(my_pv_done + 8 * (sb ^ 1), ((th - 1) >> 1) & 1, err))) {
                     alive = false;
@@ -676,6 +738,9 @@ talk_values_tc_kernel(const __grid_constant__ CUtensorMap map_v, const float* sc
                         }
                     }
                 }
+                if (marks[k & 3] != 0 && r < w.blk.rows)        // (the item's tiles have all been looked at: its products are done)
+                    add_not_finite(dst, vc, block_table + (size_t)w.blk.b * table_stride, nkv, w.g, ps, ps_shift, num_pages, DV, my_lo, my_pos, p0,
+                                   edge_lo, out_scale);
             }
         }
     }
@@ -697,13 +762,13 @@ int launch_scores(const CUtensorMap& mq, const CUtensorMap& mk, float* scores, c
                      stride, nkv, ps, shift, num_pages, window, err);
 }
 template <int DVC>
-int launch_values(const CUtensorMap& mv, const float* scores, void* out, long long ldo, const int* blocks, const int* work, int ctas,
+int launch_values(const CUtensorMap& mv, const void* vc, const float* scores, void* out, long long ldo, const int* blocks, const int* work, int ctas,
                   const int* q_start, const int* start_pos, const int* table, int stride, int nh, int nkv, int ps, int shift,
                   int num_pages, int window, int sink, float out_scale, int* err, cudaStream_t stream) {
     constexpr size_t smem = (size_t)S_STAGES * 2 * V_SCORES + V_STAGES * DVC * V_KEYS * 128 + 256;
     const auto kernel = talk_values_tc_kernel<DVC>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return xb_launch(kernel, dim3(ctas), dim3(V_THREADS), smem, stream, mv, scores, (__nv_bfloat16*)out, ldo, blocks, work, q_start,
+    return xb_launch(kernel, dim3(ctas), dim3(V_THREADS), smem, stream, mv, (const __nv_bfloat16*)vc, scores, (__nv_bfloat16*)out, ldo, blocks, work, q_start,
                      start_pos, table, stride, nh, nkv, ps, shift, num_pages, window, sink, out_scale, err);
 }
 
@@ -748,7 +813,7 @@ XB_EXPORT int xb_attn_talking_tc(void* out, long long ldo, const void* q, const 
 #undef XB_SH
 #undef XB_S
     if (rc != 0) return rc;
-#define XB_V(N) launch_values<N>(mv, scores, out, ldo, blocks, work2, ctas2, q_start, start_pos, table, stride, nh, nkv, ps, shift, num_pages, window, sink, out_scale, err, stream)
+#define XB_V(N) launch_values<N>(mv, vc, scores, out, ldo, blocks, work2, ctas2, q_start, start_pos, table, stride, nh, nkv, ps, shift, num_pages, window, sink, out_scale, err, stream)
     return dv == 128 ? XB_V(2) : XB_V(1);
 #undef XB_V
 }
