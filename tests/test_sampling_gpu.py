@@ -211,3 +211,25 @@ def test_calls_that_nobody_waits_for_keep_their_own_options():
                 torch.cuda.synchronize()
         return torch.stack(out).cpu()
     assert torch.equal(run(True), run(False))
+
+
+def test_calls_inside_a_graph_leave_no_event_to_wait_for():
+    from xinfer_b200.sampling import Sampler, SamplingParams
+    # 10 captured calls pass the point at which a half of the pinned sets is marked, and the calls after it come round to it again
+    R, V = 3, 512
+    g = torch.Generator(device="cuda:0").manual_seed(2)
+    logits, other = (torch.randn(R, V, generator=g, device="cuda:0") * 3 for _ in range(2))
+    sampler, params = Sampler("cuda:0", R), [SamplingParams(temperature=0.8)] * R
+    want = sampler.sample(logits, params, [1, 2, 3], [0] * R).clone()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        for _ in range(10):
+            kept = sampler.sample(logits, params, [1, 2, 3], [0] * R)
+    graph.replay()
+    assert torch.equal(kept, want)
+    eager = [sampler.sample(other, params, [i, 2, 3], [0] * R).clone() for i in range(20)]
+    plain = Sampler("cuda:0", R)
+    assert all(torch.equal(a, plain.sample(other, params, [i, 2, 3], [0] * R)) for i, a in enumerate(eager))
+    torch.cuda.synchronize()

@@ -63,7 +63,9 @@ def fill_records(records: np.ndarray, params: Sequence[SamplingParams], seeds, d
 class _PinnedSets:
     """Where calls' records and counted tokens lie on the host until they have been copied, for calls that nobody may have waited
     for: sets used in turn.  Half of them are taken again only after the copies that read them have been made: one event per
-    half, since recording and asking one for every call took a tenth of its time."""
+    half, since recording and asking one for every call took a tenth of its time.  A call that a CUDA graph captures neither waits
+    nor records (its copies have not been made, and an event of the graph cannot be waited for): the graph copies from the set of
+    that call whenever it is replayed."""
 
     def __init__(self, max_rows: int, record_bytes: int, half: int = 8):
         self.params = torch.zeros((2 * half, max_rows * record_bytes), dtype=torch.uint8, pin_memory=True)
@@ -74,7 +76,7 @@ class _PinnedSets:
 
     def take(self, counts_tokens: bool):
         """A set that no copy reads any more: (bytes, the same as records, counted tokens, the same as an array; None without)."""
-        if self.at % self.half == 0:
+        if self.at % self.half == 0 and not torch.cuda.is_current_stream_capturing():
             self.copied[self.at // self.half].synchronize()
         mine = self.sets[self.at]
         if mine is None or (counts_tokens and mine[2] is None):
@@ -88,7 +90,8 @@ class _PinnedSets:
         """The set last taken has been handed to its copies."""
         self.at += 1
         if self.at % self.half == 0:
-            self.copied[self.at // self.half - 1].record()
+            if not torch.cuda.is_current_stream_capturing():
+                self.copied[self.at // self.half - 1].record()
             self.at %= 2 * self.half
 
 
