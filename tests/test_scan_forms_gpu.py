@@ -47,3 +47,22 @@ def test_both_forms_give_the_same(H, d, dv, counts):
     tol = (24 + max(counts)) * 2.0 ** -24 * d ** 0.5
     for a, b in zip(few[-2:], many[-2:]):
         assert torch.isfinite(a).all() and (a - b).abs().max() <= 2 * tol * (1 + b.abs().max())
+
+
+def test_a_full_device_takes_the_tokens_of_the_delta_rule_one_by_one(monkeypatch):
+    from gulipel_models import TINY_G
+    from xinfer_b200.engine.runner import ModelRunner, StepInput
+    from xinfer_b200.parts.base import Workspace
+    cfg, seed, ps = TINY_G["G1"]
+    ids = np.random.default_rng(1).integers(0, cfg["vocab"], size=200)
+
+    def logits():
+        r = ModelRunner.random(cfg, seed, dtype="f32", block_size=ps, num_blocks=400 // ps + 2, max_num_seqs=2, max_model_len=400)
+        out = r.step([StepInput(r.open_request(), ids, [9, 198, 199])]).clone()
+        r.check_errors()
+        return out.double(), "gdelta.prep" in r.workspace._bufs
+    got, scratch = logits()
+    monkeypatch.setattr(Workspace, "reserve", lambda *a: False)
+    want, none = logits()
+    assert scratch and not none
+    assert (got - want).norm() <= 1e-4 * want.norm()        # float32 sums in another order, through the layers behind them

@@ -104,6 +104,8 @@ class GatedDelta(Mixer):
         o = ws.get("gdelta.o", (T, self.vw), torch.float32)
         longest = ctx.longest_portion()
         need = kernels.delta_scratch_floats(T, ctx.num_entries, H, s.head_dim, longest)
+        if need and not ws.reserve("gdelta.prep", need, torch.float32, need):
+            longest, need = 1, 0        # (no room on the device: the form that takes one token at a time needs none)
         kernels.delta_rule(o, qkv, proj, C, ag, self.dt_bias, self.a_log, state["S"], ctx.q_start, ctx.slots, ctx.num_entries,
                            H, s.kv_heads, s.head_dim, s.v_head_dim, s.unit_eps,
                            ws.get("gdelta.prep", (need,), torch.float32) if need else None, longest)
