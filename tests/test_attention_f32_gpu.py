@@ -1,0 +1,105 @@
+"""The tiled float32 attention: every change of scores and mask against 64 bits, tiles that hold several requests, and the
+same bits for a token whatever runs beside it."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from test_kernels_gpu import dev, err_word, make_cache, meta, rnd
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, k, v, start, scale, window=None, keep_first=0, chunk=None, sink=None, softcap=None, slope_exponent=None, out_scale=1.0):
+    n, nh, _ = q.shape
+    out = torch.zeros(n, nh, v.shape[2], dtype=torch.float64)
+    for i in range(n):
+        p = start + i
+        lo = max(0, p - window + 1) if window else 0
+        if chunk:
+            lo = max(lo, p // chunk * chunk)
+        seen = [j for j in range(p + 1) if j >= lo or j < keep_first]
+        for h in range(nh):
+            g = h // (nh // k.shape[1])
+            s = (k[seen, g] @ q[i, h]) * scale
+            if softcap:
+                s = softcap * torch.tanh(s / softcap)
+            if slope_exponent:
+                s = s - 2.0 ** (-slope_exponent * (h + 1) / nh) * (p - torch.tensor(seen, dtype=torch.float64))
+            if sink is not None:
+                s = torch.cat([s, sink[h:h + 1]])
+            w = torch.softmax(s, 0)[: len(seen)]
+            out[i, h] = out_scale * (w @ v[seen, g])
+    return out
+
+
+# nh, nkv, d, dv, page, entries, what changes
+CASES = [
+    (16, 8, 128, 128, 16, [(0, 45), (31, 1), (32, 1), (0, 1), (95, 33)], {}),
+    (6, 2, 100, 36, 8, [(0, 7), (64, 9)], dict(softcap=3.0)),
+    (20, 1, 4, 8, 16, [(0, 34), (63, 2)], dict(sink=True)),
+    (8, 8, 64, 128, 4, [(130, 40), (0, 3)], dict(window=37, keep_first=5)),
+    (8, 8, 64, 64, 16, [(130, 40), (5, 3)], dict(window=3, keep_first=70)),
+    (4, 2, 32, 32, 16, [(60, 70), (0, 1)], dict(chunk=48, slope_exponent=8.0)),
+    (12, 4, 80, 80, 32, [(200, 1), (0, 19)], dict(window=33, out_scale=0.5)),
+]
+
+
+@pytest.mark.parametrize("nh,nkv,d,dv,ps,entries,kw", CASES)
+def test_tiles_against_64_bits_and_one_token_alone(nh, nkv, d, dv, ps, entries, kw):
+    from xinfer_b200 import kernels
+    pages = sum((s + c + ps - 1) // ps for s, c in entries) + 3
+    pos, req, table, stride, table_np = meta(entries, ps, pages, 3)
+    kc, _ = make_cache(pages, nkv, ps, d, torch.float32)
+    vc, _ = make_cache(pages, nkv, ps, dv, torch.float32)
+    kc.fill_(float("nan"))       # keys that nobody has written, and values that a mask hides, reach no sum
+    vc.fill_(float("nan"))
+    T = sum(c for _, c in entries)
+    q = rnd(T, nh, d, seed=9)
+    ks, vs = [], []
+    for b, (s, c) in enumerate(entries):
+        ks.append(rnd(s + c, nkv, d, seed=20 + b))
+        vs.append(rnd(s + c, nkv, dv, seed=40 + b))
+        for j in range(s + c):
+            kc[table_np[b, j // ps], :, j % ps] = ks[b][j]
+            vc[table_np[b, j // ps], :, j % ps] = vs[b][j]
+    scale, e = 1.0 / math.sqrt(d), err_word()
+    args = dict(kw)
+    if args.pop("sink", None):
+        args["sink"] = rnd(nh, seed=7)
+
+    def run(rows):
+        out = torch.full((len(rows), nh, dv), float("nan"), device=dev())
+        window = args.get("window")
+        kernels.attention_plain(out, q[rows].contiguous(), kc, vc, pos[rows].contiguous(), req[rows].contiguous(), table, stride,
+                                window, scale, e, **{k: v for k, v in args.items() if k != "window"})
+        return out
+
+    out = run(list(range(T)))
+    assert int(e) == 0
+    t0 = 0
+    for b, (s, c) in enumerate(entries):
+        ref = reference(q[t0:t0 + c].double().cpu(), ks[b].double().cpu(), vs[b].double().cpu(), s, scale,
+                        **{k: v.double().cpu() if isinstance(v, torch.Tensor) else v for k, v in args.items()})
+        diff = (out[t0:t0 + c].double().cpu() - ref).abs().max().item()
+        assert diff <= 2e-5, (b, diff)       # (the bound of the plain kernel's own test)
+        t0 += c
+    for t in sorted({0, T // 2, T - 1}):
+        assert torch.equal(run([t])[0], out[t]), "a token's bits changed with what ran beside it"
+
+
+def test_a_padding_token_gives_zeros_and_a_bad_page_is_reported():
+    from xinfer_b200 import kernels
+    nh, nkv, d, ps = 4, 2, 32, 16
+    kc, vc = make_cache(4, nkv, ps, d, torch.float32)
+    q = rnd(3, nh, d)
+    table = torch.tensor([[0, 9], [1, 2]], dtype=torch.int32, device=dev())     # page 9 does not exist
+    out = torch.full((3, nh, d), float("nan"), device=dev())
+    e = err_word()
+    kernels.attention_plain(out, q, kc, vc, torch.tensor([3, 5, 0], dtype=torch.int32, device=dev()),
+                            torch.tensor([0, 1, -1], dtype=torch.int32, device=dev()), table, 2, None, 0.2, e)
+    assert int(e) == 0 and torch.isfinite(out).all() and torch.count_nonzero(out[2]) == 0
+    kernels.attention_plain(out, q, kc, vc, torch.tensor([20, 5, 0], dtype=torch.int32, device=dev()),
+                            torch.tensor([0, 1, -1], dtype=torch.int32, device=dev()), table, 2, None, 0.2, e)
+    assert int(e) == kernels.ERR_BAD_PAGE and torch.isfinite(out).all()

@@ -5,6 +5,7 @@
 // output element is reduced in an order that depends only on that element (its row, its key
 // range), never on what else is in the batch, so float32 results are bit-identical however the
 // tokens were cut into steps.
+#include "attention_f32.h"
 #include "common.cuh"
 
 // ------------------------------------------------------------------------------------------
@@ -593,7 +594,7 @@ XB_EXPORT int xb_qk_norm_rope_write(
 }
 
 // ------------------------------------------------------------------------------------------
-// Plain attention over the paged cache.  One warp per (token, head); keys are visited in
+// Plain attention over the paged cache (float32 heads of up to 128 channels: attention_f32.cu).  One warp per (token, head); keys are visited in
 // position order with a running maximum, so a query's result depends only on its own position
 // and the keys before it.  Scores, softmax and the value sum are float32.
 //   keys seen by a query at position p:  max(0, p - window + 1) .. p   (window <= 0: from 0)
@@ -717,10 +718,15 @@ XB_EXPORT int xb_attention_plain(int dtype, void* out, const void* q, long long 
                                  int d, int dv, int page_size, int num_pages, int window, int keep, float scale, float softcap,
                                  float slope_exp, int chunk, long long ldo, float out_scale, int* err, cudaStream_t stream) {
     if (tokens <= 0) return 0;
-    if (dtype == XB_F32)
+    if (dtype == XB_F32) {
+        const XbAttentionF32 p = {(float*)out, (const float*)q, (const float*)k_cache, (const float*)v_cache, sink, positions,
+                                  req_of_token, block_table, err, q_ts, q_hs, ldo, k_stride, v_stride, table_stride, tokens, nh,
+                                  nkv, d, dv, page_size, num_pages, window, keep, chunk, scale, softcap, slope_exp, out_scale};
+        if (xb_attention_f32_takes(p)) return xb_attention_f32(p, stream);
         return attention_plain_launch<float>(out, q, q_ts, q_hs, k_cache, v_cache, k_stride, v_stride, sink, positions,
                                              req_of_token, block_table,
                                              table_stride, tokens, nh, nkv, d, dv, page_size, num_pages, window, keep, scale, softcap, slope_exp, chunk, ldo, out_scale, err, stream);
+    }
     return attention_plain_launch<__nv_bfloat16>(out, q, q_ts, q_hs, k_cache, v_cache, k_stride, v_stride, sink, positions,
                                                  req_of_token, block_table,
                                                  table_stride, tokens, nh, nkv, d, dv, page_size, num_pages, window, keep, scale, softcap, slope_exp, chunk, ldo, out_scale, err, stream);
