@@ -7,6 +7,7 @@
 // tokens were cut into steps.
 #include "attention_f32.h"
 #include "common.cuh"
+#include "gemm_f32_tc.h"
 
 // ------------------------------------------------------------------------------------------
 // Embedding gather: out[t, :] = table[ids[t], :].  An id -1 - i stands for sampled[i], the id a
@@ -147,7 +148,8 @@ XB_EXPORT int xb_add(int dtype, void* out, const void* x, const void* branch, lo
 }
 
 // ------------------------------------------------------------------------------------------
-// Plain matrix product  out[M, N] = a[M, K] . w[N, K]^T  with float32 FMA accumulation.
+// Plain matrix product  out[M, N] = a[M, K] . w[N, K]^T  with float32 FMA accumulation, for operands or results in bfloat16
+// (all in float32: gemm_f32_tc.cu).
 // 64x64 tile, 16-deep panels, 256 threads with 4x4 outputs each.  Every output sums its panels' terms in
 // order and the panels' sums in order, so a row's result does not depend on M.
 // ------------------------------------------------------------------------------------------
@@ -213,227 +215,6 @@ __global__ void gemm_plain_kernel(TO* __restrict__ out, const TA* __restrict__ a
     }
 }
 
-// The same product for float32 operands whose rows start on 16-byte boundaries (K a multiple of 4): the sums above in the
-// same order - a panel's 16 terms by fused multiply-adds, then the panels - so every output has the same bits whichever
-// kernel forms it, and a row's result still does not depend on M.  What bounds the kernel above is shared memory: two
-// values loaded per 2 multiply-adds of a thread.  Here a thread holds TM x TN outputs (and as many panel sums), multiplied
-// two at a time, and the next panel is in registers while this one is summed.  Two layers of the 0.6B
-// sizes at 451 tokens (28 GFLOP) take 1,400 us, 24 TFLOP/s in the larger tiles and 16 in the smaller ones, of 74 at the
-// FMA units' rate; what is left is the last wave (192 blocks on 148 SMs) and waiting for shared memory.
-// Tiles of 128 x 128 (8 x 8 outputs per thread) where they fill the SMs, else 64 x 64 (8 x 4, 128 threads; 4 x 4 with 256
-// was 4 % slower).
-__device__ __forceinline__ unsigned long long gm_pack(float a, float b) {
-    unsigned long long v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-    return v;
-}
-__device__ __forceinline__ void gm_unpack(unsigned long long v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long gm_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long gm_add(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ w, int M, int N, int K) {
-    constexpr int BK = 16, THREADS = (BM / TM) * (BN / TN), LDA = BM + 4, LDW = BN + 4;
-    constexpr int NA = BM * BK / 4 / THREADS, NW = BN * BK / 4 / THREADS;
-    __shared__ __align__(16) float sa[2][BK][LDA];
-    __shared__ __align__(16) float sw[2][BK][LDW];
-    // a warp covers 4 x 8 threads' outputs: its loads of a row of A or W are 64 or 128 different bytes
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, across = BN / TN / 8;
-    const int tx = warp % across * 8 + lane % 8, ty = warp / across * 4 + lane / 8;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float4 ra[NA], rw[NW];
-    auto fetch = [&](int k0) {          // four lanes to the 64 bytes a row has in the panel
-#pragma unroll
-        for (int i = 0; i < NA; ++i) {
-            const int idx = tid + i * THREADS, gm = m0 + idx / 4, gk = k0 + idx % 4 * 4;
-            ra[i] = gm < M && gk < K ? *reinterpret_cast<const float4*>(a + (size_t)gm * K + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int i = 0; i < NW; ++i) {
-            const int idx = tid + i * THREADS, gn = n0 + idx / 4, gk = k0 + idx % 4 * 4;
-            rw[i] = gn < N && gk < K ? *reinterpret_cast<const float4*>(w + (size_t)gn * K + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    auto stage = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) {
-            const int idx = tid + i * THREADS, r = idx / 4, c = idx % 4 * 4;
-            sa[buf][c][r] = ra[i].x; sa[buf][c + 1][r] = ra[i].y; sa[buf][c + 2][r] = ra[i].z; sa[buf][c + 3][r] = ra[i].w;
-        }
-#pragma unroll
-        for (int i = 0; i < NW; ++i) {
-            const int idx = tid + i * THREADS, r = idx / 4, c = idx % 4 * 4;
-            sw[buf][c][r] = rw[i].x; sw[buf][c + 1][r] = rw[i].y; sw[buf][c + 2][r] = rw[i].z; sw[buf][c + 3][r] = rw[i].w;
-        }
-    };
-    // a thread's rows: ty * 4 .. + 3 of every BM / (TM / 4) rows; its columns likewise
-    constexpr int HA = TM / 4, HW = TN / 4;
-    unsigned long long acc[TM][TN / 2];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
-    fetch(0);
-    stage(0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += BK, buf ^= 1) {
-        const bool more = k0 + BK < K;
-        if (more) fetch(k0 + BK);
-        unsigned long long part[TM][TN / 2];
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN / 2; ++j) part[i][j] = 0ull;
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float av[TM];
-            unsigned long long wv[TN / 2];
-#pragma unroll
-            for (int u = 0; u < HA; ++u) {
-                const float4 v = *reinterpret_cast<const float4*>(&sa[buf][kk][u * (BM / HA) + ty * 4]);
-                av[u * 4] = v.x; av[u * 4 + 1] = v.y; av[u * 4 + 2] = v.z; av[u * 4 + 3] = v.w;
-            }
-#pragma unroll
-            for (int u = 0; u < HW; ++u) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&sw[buf][kk][u * (BN / HW) + tx * 4]);
-                wv[u * 2] = v.x; wv[u * 2 + 1] = v.y;
-            }
-#pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                const unsigned long long a2 = gm_pack(av[i], av[i]);
-#pragma unroll
-                for (int j = 0; j < TN / 2; ++j) part[i][j] = gm_fma(a2, wv[j], part[i][j]);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN / 2; ++j) acc[i][j] = gm_add(acc[i][j], part[i][j]);
-        if (more) stage(buf ^ 1);
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + (i / 4) * (BM / HA) + ty * 4 + i % 4;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int u = 0; u < HW; ++u) {
-            const int gn = n0 + u * (BN / HW) + tx * 4;
-            float v[4];
-            gm_unpack(acc[i][u * 2], v[0], v[1]);
-            gm_unpack(acc[i][u * 2 + 1], v[2], v[3]);
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (gn + c < N) out[(size_t)gm * N + gn + c] = v[c];
-        }
-    }
-}
-
-// Few rows (decode steps, the head of a prompt): bound by reading W once.  A thread forms the outputs of one column for all
-// BM rows; panels of 64 terms of 128 rows of W come through a ring of shared-memory stages, the rows of A are broadcast.
-// The sums are formed as above.  The head of the 0.6B sizes for two rows (622 MB) takes
-// 108 us, 5,760 GB/s.
-template <int BM>
-__global__ void __launch_bounds__(128) gemm_f32_rows_kernel(float* __restrict__ out, const float* __restrict__ a,
-                                                            const float* __restrict__ w, int M, int N, int K) {
-    constexpr int BN = 128, BK = 64, STAGES = 3, LDW = BK + 4;     // rows 4 floats apart from a multiple of 32 banks
-    extern __shared__ __align__(16) float gm_smem[];               // STAGES x (W [BN][LDW], A [BM][BK])
-    constexpr int STAGE = BN * LDW + BM * BK;
-    const int tid = threadIdx.x, n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
-    const int panels = (K + BK - 1) / BK;
-    auto bring = [&](int p) {
-        if (p < panels) {
-            float* dw = gm_smem + (p % STAGES) * STAGE;
-            float* da = dw + BN * LDW;
-            const int k0 = p * BK;
-            for (int idx = tid; idx < BN * BK / 4; idx += 128) {
-                const int r = idx / (BK / 4), c = idx % (BK / 4) * 4, gn = n0 + r, gk = k0 + c;
-                const bool in = gn < N && gk < K;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dw + r * LDW + c)),
-                             "l"(in ? w + (size_t)gn * K + gk : w), "r"(in ? 16 : 0) : "memory");
-            }
-            for (int idx = tid; idx < BM * BK / 4; idx += 128) {
-                const int r = idx / (BK / 4), c = idx % (BK / 4) * 4, gm = m0 + r, gk = k0 + c;
-                const bool in = gm < M && gk < K;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(da + r * BK + c)),
-                             "l"(in ? a + (size_t)gm * K + gk : a), "r"(in ? 16 : 0) : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    float acc[BM];
-#pragma unroll
-    for (int i = 0; i < BM; ++i) acc[i] = 0.f;
-    bring(0);
-    bring(1);
-    for (int p = 0; p < panels; ++p) {
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        __syncthreads();                 // the panel has landed, and the one before it has been read by everyone
-        bring(p + 2);
-        const float* dw = gm_smem + (p % STAGES) * STAGE;
-        const float* da = dw + BN * LDW;
-        const float4* wr = reinterpret_cast<const float4*>(dw + tid * LDW);
-#pragma unroll 1
-        for (int k = 0; k < BK && p * BK + k < K; k += 16) {
-            float part[BM];
-#pragma unroll
-            for (int i = 0; i < BM; ++i) part[i] = 0.f;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float4 v = wr[k / 4 + c];
-#pragma unroll
-                for (int i = 0; i < BM; ++i) {
-                    const float4 u = *reinterpret_cast<const float4*>(da + i * BK + k + c * 4);
-                    part[i] = fmaf(u.x, v.x, part[i]);
-                    part[i] = fmaf(u.y, v.y, part[i]);
-                    part[i] = fmaf(u.z, v.z, part[i]);
-                    part[i] = fmaf(u.w, v.w, part[i]);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < BM; ++i) acc[i] += part[i];
-        }
-    }
-    if (n0 + tid < N) {
-#pragma unroll
-        for (int i = 0; i < BM; ++i)
-            if (m0 + i < M) out[(size_t)(m0 + i) * N + n0 + tid] = acc[i];
-    }
-}
-
-template <int BM>
-static int gemm_f32_rows_launch(float* out, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
-    constexpr int smem = 3 * (128 * 68 + BM * 64) * 4;
-    cudaFuncSetAttribute(gemm_f32_rows_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    gemm_f32_rows_kernel<BM><<<dim3((N + 127) / 128, (M + BM - 1) / BM), 128, smem, stream>>>(out, a, w, M, N, K);
-    return xb_launch_status();
-}
-
-static int gemm_f32_launch(float* out, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
-    if (M <= 1) return gemm_f32_rows_launch<1>(out, a, w, M, N, K, stream);
-    if (M <= 2) return gemm_f32_rows_launch<2>(out, a, w, M, N, K, stream);
-    if (M <= 4) return gemm_f32_rows_launch<4>(out, a, w, M, N, K, stream);
-    if (M <= 8) return gemm_f32_rows_launch<8>(out, a, w, M, N, K, stream);
-    const long long large = (long long)((M + 127) / 128) * ((N + 127) / 128);
-    if (M > 64 && large >= 96)
-        gemm_f32_kernel<128, 128, 8, 8><<<dim3((N + 127) / 128, (M + 127) / 128), 256, 0, stream>>>(out, a, w, M, N, K);
-    else
-        gemm_f32_kernel<64, 64, 8, 4><<<dim3((N + 63) / 64, (M + 63) / 64), 128, 0, stream>>>(out, a, w, M, N, K);
-    return xb_launch_status();
-}
-
 template <typename TA, typename TW, typename TO>
 static int gemm_plain_launch(void* out, const void* a, const void* w, int M, int N, int K, cudaStream_t stream) {
     dim3 grid((N + 63) / 64, (M + 63) / 64);
@@ -443,12 +224,11 @@ static int gemm_plain_launch(void* out, const void* a, const void* w, int M, int
 
 // a_dtype / w_dtype / out_dtype are element type codes.
 XB_EXPORT int xb_gemm_plain(int a_dtype, int w_dtype, int out_dtype, void* out, const void* a,
-                            const void* w, int M, int N, int K, cudaStream_t stream) {
+                            const void* w, int M, int N, int K, int* err, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     typedef __nv_bfloat16 bf;
     const int code = a_dtype * 4 + w_dtype * 2 + out_dtype;
-    if (code == 0 && K > 0 && K % 4 == 0 && !(((uintptr_t)a | (uintptr_t)w) & 15) && (M + 63) / 64 <= 65535)
-        return gemm_f32_launch((float*)out, (const float*)a, (const float*)w, M, N, K, stream);
+    if (code == 0 && K > 0) return xb_gemm_f32_tc((float*)out, (const float*)a, (const float*)w, M, N, K, err, stream);
     switch (code) {
         case 0: return gemm_plain_launch<float, float, float>(out, a, w, M, N, K, stream);
         case 1: return gemm_plain_launch<float, float, bf>(out, a, w, M, N, K, stream);

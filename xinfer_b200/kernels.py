@@ -257,15 +257,27 @@ def dyt_norm(out, x, alpha, weight, bias, err, *, branch=None, branch_scale: flo
                                   err.data_ptr(), _stream()), "dyt_norm")
 
 
-def gemm_plain(out, a, w):
-    """out[M, N] = a[M, K] . w[N, K]^T with float32 FMA accumulation (no tensor cores)."""
+_err_words: dict = {}
+
+
+def _own_err_word(device) -> torch.Tensor:
+    """The error word of calls that bring none."""
+    if device not in _err_words:
+        _err_words[device] = torch.zeros(1, dtype=torch.int32, device=device)
+    return _err_words[device]
+
+
+def gemm_plain(out, a, w, err=None):
+    """out[M, N] = a[M, K] . w[N, K]^T in float32: of float32 operands and result on the tensor cores, in three bfloat16 parts of
+    each number, else by float32 FMA.  ``err``: the step's device error word."""
     M, K = a.shape
     N = w.shape[0]
     _need(a, "a", None, (M, K))
     _need(w, "w", None, (N, K))
     _need(out, "out", None, (M, N))
     _ok(kernels_lib().xb_gemm_plain(dtype_code(a.dtype), dtype_code(w.dtype), dtype_code(out.dtype), out.data_ptr(),
-                                    a.data_ptr(), w.data_ptr(), M, N, K, _stream()), "gemm_plain")
+                                    a.data_ptr(), w.data_ptr(), M, N, K,
+                                    (err if err is not None else _own_err_word(out.device)).data_ptr(), _stream()), "gemm_plain")
 
 
 def rope_table(cos_t, sin_t, inv_freq):

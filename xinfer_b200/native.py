@@ -94,7 +94,7 @@ def _declare_kernels(lib):
     _sig(lib, "xb_logits_post", I, [P, L, F, F, P])
     _sig(lib, "xb_rmsnorm", I, [I, P, P, P, P, P, P, I, I, I, F, F, P, P])
     _sig(lib, "xb_add", I, [I, P, P, P, L, F, P])
-    _sig(lib, "xb_gemm_plain", I, [I, I, I, P, P, P, I, I, I, P])
+    _sig(lib, "xb_gemm_plain", I, [I, I, I, P, P, P, I, I, I, P, P])
     _sig(lib, "xb_rope_table", I, [P, P, P, I, I, P])
     _sig(lib, "xb_qk_norm_rope_write", I,
          [I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P])

@@ -1,6 +1,6 @@
 """Dense projection ``y = x . W^T`` with ``W`` stored ``[out, in]`` (src/models/layers/linear.rs:76-124).
 
-float32: the engine's own FMA kernel (true 32-bit, no tensor-core mode).  bfloat16: the engine's
+float32: the engine's own kernel (true 32-bit results; on the tensor cores in parts of bfloat16).  bfloat16: the engine's
 tcgen05 kernel for steps of few tokens, else the library matrix product, as in the reference
 (cuBLAS through its tensor library); see ``gemm_backend``.  Both write float32 accumulators
 straight into a float32 ``out`` (the logits).
@@ -28,7 +28,7 @@ def linear(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, err: Option
             # row's logits are the same numbers whichever kernel the size of the batch selects
             torch.mm(x, weight.t(), out_dtype=torch.float32, out=out)
         return out
-    kernels.gemm_plain(out, x, weight)
+    kernels.gemm_plain(out, x, weight, err)
     return out
 
 
