@@ -1,0 +1,47 @@
+"""All layers by one native call against the parts one by one: the same kernels, so the same bits, for every kind of step."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hidden,heads,kv_heads,dim,inter,layers,window,page", [
+    (64, 4, 2, 16, 72, 1, None, 8), (256, 8, 2, 64, 640, 3, None, 16), (1024, 16, 8, 128, 3072, 2, 40, 16), (2056, 3, 3, 112, 520, 2, None, 32)])
+def test_every_kind_of_step_gives_the_same_bits(hidden, heads, kv_heads, dim, inter, layers, window, page, monkeypatch):
+    from xinfer_b200 import kernels
+    from xinfer_b200.engine.runner import ModelRunner, StepInput
+    from xinfer_b200.models import dense_layers
+    cfg = dict(architectures=["Qwen3ForCausalLM"], vocab_size=300, hidden_size=hidden, intermediate_size=inter, num_hidden_layers=layers,
+               num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=dim, rms_norm_eps=1e-6, rope_theta=10000.0,
+               max_position_embeddings=2048, tie_word_embeddings=False, sliding_window=window)
+    rng = np.random.default_rng(5)
+    ids = lambda n: rng.integers(0, 300, size=n, dtype=np.int32)
+    # portions of the step's requests, some of which go on from the step before
+    script = [[(0, 1), (1, 33), (2, 300)], [(0, 5), (1, 1), (2, 1)], [(0, 1), (1, 1), (2, 1)], [(0, 1), (1, 1), (2, 1)], [(3, 32)], [(4, 4), (0, 2)]]
+    tokens = [[ids(n) for _, n in step] for step in script]
+
+    def run(native):
+        monkeypatch.setattr(dense_layers, "ENABLED", native)
+        r = ModelRunner.random(cfg, 7, dtype="bf16", block_size=page, num_blocks=64, max_num_seqs=5, max_model_len=512)
+        slots = [r.open_request() for _ in range(5)]
+        before, out = kernels.launch_counts(), []
+        for i, (step, toks) in enumerate(zip(script, tokens)):
+            out.append(r.step([StepInput(slots[b], t, range(len(t))) for (b, n), t in zip(step, toks)], allow_graph=i == 3).clone())
+        r.check_errors()
+        return torch.cat(out), {k: n - before.get(k, 0) for k, n in kernels.launch_counts().items() if n > before.get(k, 0)}
+
+    a, count_a = run(True)
+    b, count_b = run(False)
+    count_a.pop("rope_table", None)         # (kept from the first run)
+    assert torch.equal(a, b) and count_a == count_b
+
+
+def test_other_stacks_keep_to_the_parts():
+    from xinfer_b200.engine.runner import ModelRunner
+    cfg = dict(architectures=["Qwen3ForCausalLM"], vocab_size=300, hidden_size=64, intermediate_size=64, num_hidden_layers=1, num_attention_heads=2,
+               num_key_value_heads=1, head_dim=160, rms_norm_eps=1e-6, rope_theta=10000.0, max_position_embeddings=64, tie_word_embeddings=True)
+    opts = dict(block_size=16, num_blocks=8, max_num_seqs=1, max_model_len=64)
+    assert ModelRunner.random(cfg, 1, dtype="bf16", **opts).model.dense is None          # heads of more than 128 values
+    assert ModelRunner.random(dict(cfg, head_dim=64), 1, dtype="f32", **opts).model.dense is None
+    assert ModelRunner.random(dict(cfg, head_dim=64), 1, dtype="bf16", **opts).model.dense is not None

@@ -734,6 +734,41 @@ def attn_prefill_tc(out, q, k_cache, v_cache, q_start, start_pos, block_table, t
     return True
 
 
+def dense_layers(step_type, bufs, nums, reals, library, layers):
+    """The layers of a pre-norm stack, queued by one native call.  ``step_type``: the ctypes mirror of the native step; ``bufs``
+    (tensors), ``nums``, ``reals`` and ``library`` (addresses): its fields by name; ``layers``: for each w_qkv, w_o, w_gate_up,
+    w_down, the weights of the two norms, q and k norm weights (or None), key pages, value pages."""
+    T, H, nh, nkv, d, I = (nums[k] for k in ("tokens", "hidden", "nh", "nkv", "d", "inter"))
+    bf, width = torch.bfloat16, (nums["nh"] + 2 * nums["nkv"]) * nums["d"]
+    for name, shape in (("x", (T, H)), ("h", (T, H)), ("qkv", (T, width)), ("q", (T, nh, d)), ("o", (T, nh, d)), ("attn_out", (T, H)),
+                        ("gate_up", (T, 2 * I)), ("act", (T, I)), ("ffn_out", (T, H))):
+        _need(bufs[name], name, bf, shape)
+    pages = layers[0][8].shape
+    table = (ctypes.c_void_p * (10 * len(layers)))()
+    at = 0
+    for ts in layers:
+        for t, name, dtype, shape in zip(ts, ("w_qkv", "w_o", "w_gate_up", "w_down", "norm", "norm", "q norm", "k norm", "k pages", "v pages"),
+                                         (bf, bf, bf, bf, torch.float32, torch.float32, torch.float32, torch.float32, bf, bf),
+                                         ((width, H), (H, nh * d), (2 * I, H), (H, I), (H,), (H,), (d,), (d,), pages, pages)):
+            if t is not None:
+                _need(t, name, dtype, shape)
+                table[at] = t.data_ptr()
+            at += 1
+    lib, done = kernels_lib(), ctypes.c_int(0)
+    if lib.xb_dense_step_size() != ctypes.sizeof(step_type):
+        raise KernelError("the native step and its mirror differ in size")
+    step = step_type(**{k: t.data_ptr() for k, t in bufs.items()}, **nums, **reals, **library)
+    n = len(layers)
+    rc = lib.xb_dense_layers(ctypes.byref(step), table, n, ctypes.byref(done), _stream())
+    _ok(rc, "rmsnorm_bf16", 2 * n)
+    _ok(0, "qk_norm_rope_write_bf16", n)
+    _ok(0, "swiglu_rows_bf16" if T >= nums["many_rows"] else "swiglu_bf16", n)
+    for name, count in (("gemm_skinny_tc", 4 * n - done.value), ("attn_prefill_tc", n if nums["prefill_ctas"] else 0),
+                        ("attn_decode_tc", n if nums["small"] else 0)):
+        if count:
+            _ok(0, name, count)
+
+
 # ---- attention with talking heads and a sink; gated recurrence; polynomial activation; table experts ----
 def qkv_prepare(q_out, k_cache, v_cache, qkv, q_w, k_w, inv_freq, positions, req_of_token, block_table, table_stride,
                 nh, nkv, d, dv, rot, interleaved, norm_mode, eps, write_kv, err, rot_magnitude: float = 1.0, bias=None,

@@ -18,6 +18,7 @@ from ..parts import Block, LayerCache, StepContext, build_part, part_class
 from ..parts.block import Addend, Stream, fused_norm, stream_chain
 from ..parts.linear import linear
 from ..weights.loader import WeightSpec, WeightStore
+from .dense_layers import DenseLayers
 
 
 def model_weight_specs(plan: ModelPlan) -> List[WeightSpec]:
@@ -54,6 +55,7 @@ class DecoderModel:
         self.final_norm = build_part("norm", plan.final_norm, plan.final_norm_name, dtype, self.device)
         # the residual stream's dtype: the engine's, or float32 where the plan says so
         self.stream_dtype = torch.float32 if plan.residual_dtype == "float32" else dtype
+        self.dense = DenseLayers.of(plan, self.blocks, dtype, self.stream_dtype)     # all layers by one native call, where it knows them
         self.embed = None
         self.head = None
         self.pair_table = self.pos_table = None
@@ -149,7 +151,8 @@ class DecoderModel:
         x = ws.get("model.x", (T, H), self.stream_dtype)
         ctx.branch_dtype = self.stream_dtype
         # what mixers decide once per step from its metadata, before the step's first kernel
-        for pos, run in enumerate(self.plan.runs):
+        whole = self.dense is not None and self.dense.takes(ctx, caches)
+        for pos, run in enumerate(self.plan.runs[:1] if whole else self.plan.runs):      # (alike, over one group of pages)
             mixer = self.blocks[run.block].mixer
             if mixer is not None:
                 mixer.prepare_step(ctx, caches[pos if run.cache_from is None else run.cache_from])
@@ -178,7 +181,9 @@ class DecoderModel:
             # runs that add the embedding's output again: it is kept apart from the stream that the blocks change
             x0 = ws.get("model.x0", (T, H), self.stream_dtype)
             x0.copy_(x)
-        for pos, run in enumerate(self.plan.runs):
+        if whole:
+            stream.pending.append(Addend(self.dense.forward(x, ctx, caches)))
+        for pos, run in enumerate(() if whole else self.plan.runs):
             if run.add_input:
                 stream.pending.append(Addend(x0))      # summed by whoever reads the stream next
             src = pos if run.cache_from is None else run.cache_from

@@ -31,6 +31,8 @@ def host_lib():
 def kernels_lib():
     """CUDA kernels for sm_100a."""
     global _kernels
+    if _kernels is not None:
+        return _kernels
     with _lock:
         if _kernels is None:
             from .csrc.build import build_kernels
@@ -95,6 +97,8 @@ def _declare_kernels(lib):
     _sig(lib, "xb_rmsnorm", I, [I, P, P, P, P, P, P, I, I, I, F, F, P, P])
     _sig(lib, "xb_add", I, [I, P, P, P, L, F, P])
     _sig(lib, "xb_gemm_plain", I, [I, I, I, P, P, P, I, I, I, P, P])
+    _sig(lib, "xb_dense_step_size", I, [])
+    _sig(lib, "xb_dense_layers", I, [P, P, I, P, P])
     _sig(lib, "xb_rope_table", I, [P, P, P, I, I, P])
     _sig(lib, "xb_qk_norm_rope_write", I,
          [I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P])
