@@ -12,6 +12,7 @@
 // storage types.  Also here: the kernel that prepares a step's queries, keys and values (rotation,
 // per-head norm before or after it, page write) with heads of different key and value sizes.
 #include "common.cuh"
+#include "qk_rope.cuh"
 
 // ------------------------------------------------------------------------------------------
 // qkv[t] = [heads x d | kv_heads x d | kv_heads x dv].  Per q/k head, in this order:
@@ -507,6 +508,146 @@ static bool qkv_conv_runs(T* q_out, T* k_cache, T* v_cache, const T* qkv, long l
 #undef XB_RUNS
 }
 
+// ------------------------------------------------------------------------------------------
+// The same in bfloat16 for many tokens, where heads are of 16 to 128 channels in sixteens, a rotation turns neighbours or the
+// halves of whole heads, and there is neither a convolution nor a norm over values or whole projections: a warp per token (or
+// per share of a token's heads, while there are few).  Eight lanes take a head, a lane sixteen channels: eight from either half, so
+// that both of a pair are its own; eight heads are in flight at once.  What bounded the kernel above (a block per token,
+// a warp's heads one after the other through shared memory) was latency, and a form with a lane per four channels the
+// instructions that every head costs beside its channels (172 a head): 2,048 tokens of 32 + 2 x 8 heads of 128 channels,
+// 50 MB: 52 us, 36 us, here 20.
+// ------------------------------------------------------------------------------------------
+constexpr int kTokenHeads = 2;      // heads of a group of eight lanes in flight
+__global__ void __launch_bounds__(256) qkv_prepare_tokens_kernel(
+    __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, const __nv_bfloat16* qkv,
+    const float* __restrict__ q_w, const float* __restrict__ k_w, const float* __restrict__ inv_freq, const int* __restrict__ positions,
+    const int* __restrict__ req_of_token, const int* __restrict__ block_table, int table_stride, int tokens, int nh, int nkv, int d, int dv,
+    int rot, int interleaved, int norm_mode, int page_size, int num_pages, float eps, int write_kv, float rot_mag, const float* __restrict__ bias,
+    float temp_coef, int temp_every, long long row_len, long long v_off, int* err) {
+    using xbqk::Pack8;
+    pdl_overlap_few();
+    __shared__ float2 angles[8][64];          // cos and sin of a warp's token
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = lane >> 3, li = lane & 7, t = blockIdx.x * 8 + warp;
+    if (t >= tokens) return;
+    const __nv_bfloat16* row = qkv + (size_t)t * row_len;
+    const int heads = nh + 2 * nkv, share = (heads + (int)gridDim.y - 1) / (int)gridDim.y;
+    const int begin = blockIdx.y * share, end = min(begin + share, heads);
+    Pack8 ra[kTokenHeads], rb[kTokenHeads];
+    auto fetch = [&](int h0) {
+#pragma unroll
+        for (int u = 0; u < kTokenHeads; ++u) {
+            const int h = h0 + u * 4 + group, half = (h < nh + nkv ? d : dv) / 16;
+            ra[u] = rb[u] = Pack8{};
+            if (h < end && li < half) {
+                const Pack8* p = reinterpret_cast<const Pack8*>(row + (h < nh + nkv ? (long long)h * d : v_off + (long long)(h - nh - nkv) * dv));
+                ra[u] = p[li];
+                rb[u] = p[li + half];
+            }
+        }
+    };
+    fetch(begin);                             // in flight while the angles are formed
+    const int pos = positions[t], b = req_of_token[t];
+    long long kv_row = -1;
+    if (write_kv && b >= 0) {
+        const int page = block_table[(size_t)b * table_stride + pos / page_size];
+        if (page < 0 || page >= num_pages) {
+            if (lane == 0 && blockIdx.y == 0) atomicOr(err, XB_ERR_BAD_PAGE);
+        } else {
+            kv_row = (long long)page * nkv * page_size + (pos % page_size);
+        }
+    }
+    if (inv_freq) {
+        for (int j = lane; j < rot / 2; j += 32) {
+            float sn, cs;
+            sincosf((float)pos * inv_freq[j], &sn, &cs);
+            angles[warp][j] = make_float2(cs * rot_mag, sn * rot_mag);
+        }
+        __syncwarp();
+    }
+    const float q_mul = temp_every > 0 ? 1.f + temp_coef * logf((float)((pos + 1) / temp_every) + 1.f) : 1.f;
+    for (int h0 = begin; h0 < end; h0 += 4 * kTokenHeads) {
+        if (h0 > begin) fetch(h0);
+#pragma unroll
+        for (int u = 0; u < kTokenHeads; ++u) {
+            const int h = h0 + u * 4 + group;
+            const bool is_q = h < nh, is_v = h >= nh + nkv;
+            const int half = (is_v ? dv : d) / 16;
+            const bool live = h < end && li < half;
+            float v[2][8];
+            xbqk::unpack8(ra[u], v[0]);
+            xbqk::unpack8(rb[u], v[1]);
+            if (bias && live) {
+                const float* bh = bias + (is_v ? v_off + (long long)(h - nh - nkv) * dv : (long long)h * d);
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int e = 0; e < 8; e += 4) {
+                        const float4 w = *reinterpret_cast<const float4*>(bh + (li + s * half) * 8 + e);
+                        v[s][e] += w.x, v[s][e + 1] += w.y, v[s][e + 2] += w.z, v[s][e + 3] += w.w;
+                    }
+            }
+            auto normed = [&]() {             // (of values too, whose results nobody takes: the sums are over all lanes of a group)
+                float ss = 0.f;
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) ss += v[s][e] * v[s][e];
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                if (is_v) return;
+                const float inv = 1.f / sqrtf(ss / (float)d + eps);
+                const float* nw = is_q ? q_w : k_w;
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int e = 0; e < 8; e += 4) {
+                        const float4 w = nw && live ? *reinterpret_cast<const float4*>(nw + (li + s * half) * 8 + e) : make_float4(1.f, 1.f, 1.f, 1.f);
+                        v[s][e] = v[s][e] * inv * w.x, v[s][e + 1] = v[s][e + 1] * inv * w.y;
+                        v[s][e + 2] = v[s][e + 2] * inv * w.z, v[s][e + 3] = v[s][e + 3] * inv * w.w;
+                    }
+            };
+            if (norm_mode == 1) normed();
+            if (inv_freq && live && !is_v) {
+                if (interleaved) {
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+#pragma unroll
+                        for (int e = 0; e < 8; e += 2) {
+                            const int i = (li + s * half) * 8 + e;
+                            if (i < rot) {
+                                const float2 a = angles[warp][i / 2];
+                                const float x = v[s][e], y = v[s][e + 1];
+                                v[s][e] = x * a.x - y * a.y;
+                                v[s][e + 1] = y * a.x + x * a.y;
+                            }
+                        }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float2 a = angles[warp][li * 8 + e];
+                        const float x = v[0][e], y = v[1][e];
+                        v[0][e] = x * a.x - y * a.y;
+                        v[1][e] = y * a.x + x * a.y;
+                    }
+                }
+            }
+            if (norm_mode == 2) normed();
+            if (!live || (!is_q && kv_row < 0)) continue;
+            if (is_q && temp_every > 0) {
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[s][e] *= q_mul;
+            }
+            Pack8* dst = reinterpret_cast<Pack8*>(is_q ? q_out + ((size_t)t * nh + h) * d
+                                                  : is_v ? v_cache + (size_t)(kv_row + (long long)(h - nh - nkv) * page_size) * dv
+                                                         : k_cache + (size_t)(kv_row + (long long)(h - nh) * page_size) * d);
+            dst[li] = xbqk::pack8(v[0]);
+            dst[li + half] = xbqk::pack8(v[1]);
+        }
+    }
+}
+
 XB_EXPORT int xb_qkv_prepare(int dtype, void* q_out, void* k_cache, void* v_cache, const void* qkv, const float* q_w,
                              const float* k_w, const float* inv_freq, const int* positions, const int* req_of_token,
                              const int* block_table, int table_stride, int tokens, int nh, int nkv, int d, int dv, int rot,
@@ -552,6 +693,17 @@ XB_EXPORT int xb_qkv_prepare(int dtype, void* q_out, void* k_cache, void* v_cach
                                                            table_stride, q_start, slots, tokens, nh, nkv, d, dv, page_size,
                                                            num_pages, value_eps, write_kv, err, stream);
         if (done) return xb_launch_status();
+    }
+    // (bfloat16 alone: sums and rotations are contracted in another order there, and a float32 engine's bits must not depend on the step)
+    if (dtype == XB_BF16 && !taps && tokens > 64 && norm_mode != 3 && value_eps < 0.f && d % 16 == 0 && d <= 128 && dv % 16 == 0 && dv <= 128 &&
+        row_len % 8 == 0 && v_off % 8 == 0 && (!inv_freq || interleaved || rot == d) &&
+        !(((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)bias | (uintptr_t)q_w | (uintptr_t)k_w) & 15)) {
+        // a token's heads are shared out among warps until these are some 32 a processor
+        const unsigned bx = (unsigned)((tokens + 7) / 8), by = (unsigned)((heads + 7) / 8), want = (148 * 4 + bx - 1) / bx;
+        return xb_launch_few(qkv_prepare_tokens_kernel, dim3(bx, want < by ? want : by), dim3(256), 0, stream,
+                             (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, (const __nv_bfloat16*)qkv, q_w, k_w, inv_freq,
+                             positions, req_of_token, block_table, table_stride, tokens, nh, nkv, d, dv, rot, interleaved, norm_mode, page_size,
+                             num_pages, eps, write_kv, rot_mag, bias, temp_coef, temp_every, row_len, v_off, err);
     }
 #define XB_PREPARE(T, CONV)                                                                                               \
     xb_launch_few(qkv_prepare_kernel<T, CONV>, dim3(dim3(tokens, spread)), dim3(threads), smem, stream,                                                       \
