@@ -1,0 +1,67 @@
+"""Talking heads of single tokens with keys and values in registers: against 64 bits, over key ranges, windows, sinks, groups of
+heads and pages, and the values that no query sees."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("nh,nkv,contexts,ps,window,sink,parts", [
+    (16, 8, [1, 16, 17, 31, 300], 16, None, False, 1), (16, 2, [5, 129], 8, None, True, 3), (32, 8, [64, 65, 1000], 16, None, True, 8),
+    (32, 4, [40, 700, 3], 32, 50, False, 2), (16, 8, [15, 513], 4, 16, True, 64), (32, 5 - 1, [1], 16, None, True, 2)])
+def test_single_tokens_against_64_bits(nh, nkv, contexts, ps, window, sink, parts):
+    from xinfer_b200 import kernels as k
+    g = torch.Generator().manual_seed(nh + len(contexts))
+    d, T = 128, len(contexts)
+    assert k.attn_talking_decode_takes(nh, nkv, d, d)
+    per = max(contexts) // ps + 1
+    table = torch.randperm(T * per, generator=g).int().view(T, per)
+    kc = torch.full((T * per, nkv, ps, d), float("nan")).bfloat16()      # what is not a request's own is never part of a result
+    vc = torch.full((T * per, nkv, ps, d), float("nan")).bfloat16()
+    ks, vs = [], []
+    for b, n in enumerate(contexts):
+        ks.append(torch.randn(n, nkv, d, generator=g).bfloat16())
+        vs.append(torch.randn(n, nkv, d, generator=g).bfloat16())
+        for i in range(n):
+            kc[table[b, i // ps], :, i % ps], vc[table[b, i // ps], :, i % ps] = ks[b][i], vs[b][i]
+    q = torch.randn(T, nh, d, generator=g).bfloat16()
+    talk = torch.randn(nh, nh, generator=g) / math.sqrt(nh)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out = torch.zeros(T, nh * d, dtype=torch.bfloat16, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    po = torch.zeros(T * parts * nh * d, device=DEV)
+    pml = torch.zeros(T * parts * nh * 2, device=DEV)
+    scale = d ** -0.5
+    starts = i32([n - 1 for n in contexts])
+    args = (kc.to(DEV), vc.to(DEV), talk.to(DEV), i32(list(range(T + 1))), starts, T, table.to(DEV), per, window, scale, sink, 0.5, 1, err, parts, po, pml)
+    k.attn_talking_mma(out, q.to(DEV), *args)
+    assert int(err) == 0
+    for b, n in enumerate(contexts):
+        lo = max(0, n - window) if window else 0
+        s = torch.einsum("hd,khd->hk", q[b].double(), ks[b][lo:].double().repeat_interleave(nh // nkv, 1)) * scale
+        s = talk.double() @ s
+        if sink:
+            s = torch.cat([s, torch.zeros(nh, 1, dtype=torch.float64)], 1)
+        w = torch.softmax(s, 1)[:, : n - lo]
+        ref = 0.5 * torch.einsum("hk,khd->hd", w, vs[b][lo:].double().repeat_interleave(nh // nkv, 1))
+        # weights and results are rounded to bfloat16: 2^-9 of the largest value each, and the float32 sums
+        assert (out[b].double().cpu().view(nh, d) - ref).abs().max() <= 2.0 ** -7 * (1 + ref.abs().max()), (b, n)
+
+
+def test_a_token_of_no_request_and_a_bad_page():
+    from xinfer_b200 import kernels as k
+    nh, nkv, d, ps = 16, 8, 128, 16
+    kc = torch.zeros(4, nkv, ps, d, dtype=torch.bfloat16, device=DEV)
+    q = torch.ones(2, nh, d, dtype=torch.bfloat16, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out = torch.full((2, nh * d), 3.0, dtype=torch.bfloat16, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    table = i32([[0, 9]])
+    run = lambda start: k.attn_talking_mma(out, q, kc, kc, None, i32([0, 1]), i32([start]), 1, table, 2, None, 1.0, False, 1.0, 1, err)
+    run(3)
+    assert int(err) == 0 and torch.count_nonzero(out[0]) == 0 and (out[1] == 3.0).all()
+    run(20)
+    assert int(err) == k.ERR_BAD_PAGE and torch.isfinite(out).all()

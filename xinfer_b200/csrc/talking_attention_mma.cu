@@ -17,6 +17,7 @@
 //   e. per unit: O <- O * correction + P V, O in registers.
 #include "common.cuh"
 #include "mma_sync.cuh"
+#include "talking_decode.h"
 
 using namespace xbmma;
 
@@ -367,6 +368,9 @@ __global__ void __launch_bounds__(TM_THREADS) attn_talking_mma_kernel(__nv_bfloa
 extern "C" int xb_attn_talking_merge_bf16(void* out, const float* part_o, const float* part_ml, int tokens, int H, int dv,
                                           int parts, int ldo, float out_scale, cudaStream_t stream);
 
+// Whether single tokens (a query tile of one) of these sizes run on talk_decode_kernel, two blocks of which share a processor.
+XB_EXPORT int xb_attn_talking_decode_takes(int nh, int nkv, int d, int dv) { return xb_talk_decode_takes(nh, nkv, d, dv) ? 1 : 0; }
+
 // The query tile this kernel takes for these sizes (at most `want`), 0: the sizes are not for it (the FMA
 // kernel takes them).  Needs head sizes in steps of 16 (values up to 128), at most 64 heads, an output row
 // stride and head offsets that keep 4-byte stores aligned.
@@ -411,6 +415,13 @@ XB_EXPORT int xb_attn_talking_mma(void* out, int ldo, const void* q, const void*
     a.page_size = page_size; a.num_pages = num_pages; a.window = window; a.sink = sink; a.bq = bq;
     a.parts = parts < 1 ? 1 : parts; a.ldo = ldo; a.n_mt = (rep * bq + 15) / 16;
     a.scale = scale; a.out_scale = out_scale; a.err = err;
+    if (bq == 1 && xb_talk_decode_takes(nh, nkv, d, dv) && !(((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) {
+        const XbTalkDecode s = {q_start, start_pos, block_table, talk, part_o, part_ml, num_entries, table_stride, nkv, page_size, num_pages, window,
+                                sink, a.parts, ldo, scale, out_scale, err};
+        const int rc = xb_talk_decode(out, q, k_cache, v_cache, s, tokens, nh, stream);
+        if (rc || a.parts == 1) return rc;
+        return xb_attn_talking_merge_bf16(out, part_o, part_ml, tokens, nh, dv, a.parts, ldo, out_scale, stream);
+    }
     const int maxh = nh <= 8 ? 8 : (nh <= 16 ? 16 : (nh <= 32 ? 32 : 64));
     const size_t smem = talk_mma_smem(nh, nkv, d, dv, bq, a.n_mt, maxh).total;
     const dim3 grid((tokens + bq - 1) / bq + num_entries, a.parts);

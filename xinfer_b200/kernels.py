@@ -877,6 +877,11 @@ def attn_talking_mma_tile(nh: int, nkv: int, d: int, dv: int, want: int) -> int:
     return int(kernels_lib().xb_attn_talking_mma_tile(int(nh), int(nkv), int(d), int(dv), int(max(want, 1))))
 
 
+def attn_talking_decode_takes(nh: int, nkv: int, d: int, dv: int) -> bool:
+    """Whether ``attn_talking_mma`` takes single tokens of these sizes a token and range of keys a block, two blocks a processor."""
+    return bool(kernels_lib().xb_attn_talking_decode_takes(int(nh), int(nkv), int(d), int(dv)))
+
+
 def attn_talking_mma(out, q, k_cache, v_cache, talk, q_start, start_pos, num_entries, block_table, table_stride, window, scale,
                      sink, out_scale, bq, err, parts: int = 1, part_o=None, part_ml=None):
     """``attn_talking`` for bfloat16 with both products on tensor cores (mma.sync); the mix across heads, the

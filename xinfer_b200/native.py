@@ -159,6 +159,7 @@ def _declare_kernels(lib):
     _sig(lib, "xb_gemm_batched_plain", I, [I, P, P, P, I, I, I, I, L, L, L, L, L, L, L, P])
     _sig(lib, "xb_attn_talking_tile", I, [I, I, I, I])
     _sig(lib, "xb_attn_talking", I, [I, P, I, P, P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, I, F, I, F, I, I, P, P, P, P])
+    _sig(lib, "xb_attn_talking_decode_takes", I, [I, I, I, I])
     _sig(lib, "xb_attn_talking_mma_tile", I, [I, I, I, I, I])
     _sig(lib, "xb_attn_talking_mma", I, [P, I, P, P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, I, F, I, F, I, I, P, P, P, P])
     _sig(lib, "xb_attn_talking_tc_takes", I, [I, I, I, I, I])

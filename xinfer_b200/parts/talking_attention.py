@@ -41,6 +41,9 @@ _DEFAULT_NORM_NAMES = ("q_norm.weight", "k_norm.weight")
 # blocks and 80.2 us in 256 blocks)
 _DECODE_BLOCKS = 148
 _DECODE_MIN_KEYS = 128
+# the kernel for single tokens that keeps keys and values in registers has two blocks on an SM
+_DECODE_LIGHT_BLOCKS = 296
+_DECODE_LIGHT_MIN_KEYS = 64
 # bfloat16: both products on tensor cores where the sizes allow; tests switch it off to compare the two forms
 USE_TENSOR_CORES = True
 # Scratch memory for the mixed scores of a step of many tokens (in bytes): more queries run one chunk after the other.
@@ -320,7 +323,9 @@ class TalkingAttention(Mixer):
             bound = stride * cache.page_size if ctx.fixed_shapes else ctx.max_context
             if s.window:
                 bound = min(bound, s.window + 32)
-            parts = max(1, min(_DECODE_BLOCKS // max(T, 1), bound // _DECODE_MIN_KEYS, 64))
+            blocks, keys = ((_DECODE_LIGHT_BLOCKS, _DECODE_LIGHT_MIN_KEYS) if mma and kernels.attn_talking_decode_takes(nh, nkv, d, dv)
+                            else (_DECODE_BLOCKS, _DECODE_MIN_KEYS))
+            parts = max(1, min(blocks // max(T, 1), bound // keys, 64))
             if parts > 1:
                 part_o = ws.get("tattn.part_o", (T * parts * nh * dv,), torch.float32)
                 part_ml = ws.get("tattn.part_ml", (T * parts * nh * 2,), torch.float32)
