@@ -1,0 +1,37 @@
+"""Rows in vectors against 64 bits: widths around a thread's vectors, every combination of the row's operands, gathered rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dim", [4, 252, 256, 516, 1024, 4096, 4100, 8192])
+@pytest.mark.parametrize("branch,norm,gain,scale,weight,rows", [
+    (None, False, False, 1.0, True, False), (torch.float32, True, True, 0.5, True, False), (torch.bfloat16, True, False, 1.0, False, False),
+    (torch.bfloat16, False, True, 2.0, True, True), (torch.float32, False, False, 1.0, True, True)])
+def test_rows_in_vectors(dim, branch, norm, gain, scale, weight, rows):
+    from xinfer_b200 import kernels as k
+    g = torch.Generator().manual_seed(dim)
+    n = 5
+    x = torch.randn(n, dim, generator=g)
+    br = torch.randn(n, dim, generator=g).to(branch) if branch else None
+    w, bw, gn = (1 + 0.1 * torch.randn(dim, generator=g) for _ in range(3))
+    idx = [4, 0, 2] if rows else list(range(n))
+    to = lambda t: None if t is None else t.to(DEV)
+    out = torch.empty(len(idx), dim, dtype=torch.bfloat16, device=DEV)
+    total = torch.empty(len(idx), dim, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    k.rms_chain(out, to(x), to(w) if weight else None, 1e-5, err, branch=to(br), branch_weight=to(bw) if norm else None, branch_eps=1e-6,
+                branch_offset=0.25, gain=to(gn) if gain else None, branch_scale=scale, sum_out=total,
+                rows=torch.tensor(idx, dtype=torch.int32, device=DEV) if rows else None, weight_offset=0.5)
+    s = x.double()
+    if br is not None:
+        b = br.double()
+        if norm:
+            b = b * torch.rsqrt((b * b).mean(1, keepdim=True) + 1e-6) * (0.25 + bw.double())
+        s = s + scale * (gn.double() if gain else 1.0) * b
+    y = s * torch.rsqrt((s * s).mean(1, keepdim=True) + 1e-5) * (0.5 + w.double()) if weight else s
+    assert int(err) == 0
+    assert (total.double().cpu() - s[idx]).abs().max() <= 2e-6 * (1 + s.abs().max())      # a few float32 roundings
+    assert (out.double().cpu() - y[idx]).abs().max() <= 2.0 ** -8 * y.abs().max()         # one to bfloat16
