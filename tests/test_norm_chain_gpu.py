@@ -35,3 +35,16 @@ def test_rows_in_vectors(dim, branch, norm, gain, scale, weight, rows):
     assert int(err) == 0
     assert (total.double().cpu() - s[idx]).abs().max() <= 2e-6 * (1 + s.abs().max())      # a few float32 roundings
     assert (out.double().cpu() - y[idx]).abs().max() <= 2.0 ** -8 * y.abs().max()         # one to bfloat16
+
+
+@pytest.mark.parametrize("rows,width", [(65, 4), (66, 1020), (600, 1028), (2000, 3072)])
+@pytest.mark.parametrize("activation", ["silu", "gelu_tanh"])
+def test_gate_with_biases_over_many_rows_gives_the_bits_of_few(rows, width, activation):
+    from xinfer_b200 import kernels as k
+    g = torch.Generator().manual_seed(width)
+    gu, bias = torch.randn(rows, 2 * width, generator=g).to(DEV), torch.randn(2 * width, generator=g).to(DEV)
+    out, few = (torch.zeros(rows, width, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    k.swiglu_bias(out, gu, bias, activation)
+    for a in range(0, rows, 64):
+        k.swiglu_bias(few[a:a + 64], gu[a:a + 64], bias, activation)
+    assert torch.equal(out, few)

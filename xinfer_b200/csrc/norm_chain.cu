@@ -262,9 +262,35 @@ __global__ void swiglu_bias_kernel(TO* __restrict__ out, const TI* gu, const flo
     out[i] = from_f32<TO>(gate_mul_f32<ACT>(g, u));
 }
 
+// The same arithmetic for many float32 rows that leave in bfloat16, in fours: a block walks over rows with its columns' biases in
+// registers.  A value a thread, with a division for its row, took 23 us for 1,802 rows of 3,072 (55 MB), this 9.3.
+template <int ACT>
+__global__ void __launch_bounds__(256) swiglu_bias_rows_kernel(__nv_bfloat16* __restrict__ out, const float* gu, const float* __restrict__ bias, int I, int rows) {
+    pdl_overlap_few();
+    const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (c >= I) return;
+    const float4 bg = *reinterpret_cast<const float4*>(bias + c), bu = *reinterpret_cast<const float4*>(bias + I + c);
+#pragma unroll 4
+    for (int t = blockIdx.y; t < rows; t += gridDim.y) {
+        const float* row = gu + (size_t)t * 2 * I + c;
+        const float4 g = *reinterpret_cast<const float4*>(row), u = *reinterpret_cast<const float4*>(row + I);
+        chain_store4(out + (size_t)t * I + c,
+                     make_float4(gate_mul_f32<ACT>(g.x + bg.x, u.x + bu.x), gate_mul_f32<ACT>(g.y + bg.y, u.y + bu.y),
+                                 gate_mul_f32<ACT>(g.z + bg.z, u.z + bu.z), gate_mul_f32<ACT>(g.w + bg.w, u.w + bu.w)));
+    }
+}
+
 template <typename TI, typename TO>
 static int swiglu_bias_launch(void* out, const void* gu, const float* bias, int rows, int I, int act, cudaStream_t stream) {
     const size_t n = (size_t)rows * I;
+    if (sizeof(TI) == 4 && sizeof(TO) == 2 && rows > 64 && I % 4 == 0 && !(((uintptr_t)gu | (uintptr_t)bias) & 15) && !((uintptr_t)out & 7)) {
+        // about eight blocks a processor, each with at least four rows where there are that many
+        const unsigned bx = (unsigned)((I / 4 + 255) / 256), want = (148 * 8 + bx - 1) / bx, most = (unsigned)((rows + 3) / 4);
+        const dim3 grid(bx, want < most ? want : most);
+        if (act == XB_ACT_GELU_TANH)
+            return xb_launch_few(swiglu_bias_rows_kernel<XB_ACT_GELU_TANH>, grid, dim3(256), 0, stream, (__nv_bfloat16*)out, (const float*)gu, bias, I, rows);
+        return xb_launch_few(swiglu_bias_rows_kernel<XB_ACT_SILU>, grid, dim3(256), 0, stream, (__nv_bfloat16*)out, (const float*)gu, bias, I, rows);
+    }
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (act == XB_ACT_GELU_TANH)
         xb_launch_few(swiglu_bias_kernel<TI, TO, XB_ACT_GELU_TANH>, dim3(blocks), dim3(256), 0, stream, (TO*)out, (const TI*)gu, bias, I, n);
