@@ -48,3 +48,27 @@ def test_gate_with_biases_over_many_rows_gives_the_bits_of_few(rows, width, acti
     for a in range(0, rows, 64):
         k.swiglu_bias(few[a:a + 64], gu[a:a + 64], bias, activation)
     assert torch.equal(out, few)
+
+
+@pytest.mark.parametrize("T,parts,part", [(3, 2, 4), (9, 3, 128), (5, 2, 132), (2, 3, 512), (2, 2, 516), (3, 2, 1024), (2, 1, 1028), (2, 1, 4096), (2, 1, 4100)])
+@pytest.mark.parametrize("after,silu,div", [(False, False, False), (True, False, True), (True, True, False)])
+def test_gated_parts_in_vectors(T, parts, part, after, silu, div):
+    from xinfer_b200 import kernels as k
+    g = torch.Generator().manual_seed(part)
+    W, eps = parts * part, 1e-6
+    y, gate, w = torch.randn(T, W, generator=g), torch.randn(T, W + 8, generator=g), 1 + torch.rand(part, generator=g)
+    d = torch.rand(T, parts, generator=g) + 0.5
+    d[-1, 0] = 0.0
+    out = torch.full((T, W + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    k.gated_head_norm(out[:, 4:4 + W], y.to(DEV), gate.to(DEV), 4, w.to(DEV), part, eps, after, silu, div=d.to(DEV) if div else None, out_scale=-2.0)
+    v, z = y.double().view(T, parts, part), gate.double()[:, 4:4 + W].reshape(T, parts, part)
+    if div:
+        v = v / torch.where(d == 0, 1.0, d.double())[..., None]
+    if not after:
+        v = v * z * torch.sigmoid(z)
+    v = v * (v.square().mean(-1, keepdim=True) + eps).rsqrt() * w.double() * -2.0
+    if after:
+        v = v * torch.sigmoid(z) * (z if silu else 1.0)
+    got = out.double().cpu()
+    assert (got[:, :4] == 7.0).all() and (got[:, 4 + W:] == 7.0).all()
+    assert ((got[:, 4:4 + W] - v.reshape(T, W)).abs() <= 2.0 ** -8 * v.reshape(T, W).abs() + 1e-5).all()     # one rounding to bfloat16, float32 behind it
