@@ -103,3 +103,27 @@ def test_a_padding_token_gives_zeros_and_a_bad_page_is_reported():
     kernels.attention_plain(out, q, kc, vc, torch.tensor([20, 5, 0], dtype=torch.int32, device=dev()),
                             torch.tensor([0, 1, -1], dtype=torch.int32, device=dev()), table, 2, None, 0.2, e)
     assert int(e) == kernels.ERR_BAD_PAGE and torch.isfinite(out).all()
+
+
+def test_tokens_of_a_request_that_are_not_neighbours():
+    """Tokens of two requests in turn: each as it is alone."""
+    from xinfer_b200 import kernels
+    nh, nkv, d, ps = 4, 4, 32, 16
+    kc, vc = rnd(6, nkv, ps, d, seed=1), rnd(6, nkv, ps, d, seed=2)
+    table = torch.tensor([[0, 1, 2], [3, 4, 5]], dtype=torch.int32, device=dev())
+    pos = torch.tensor([5, 3, 40, 41, 17, 0], dtype=torch.int32, device=dev())
+    req = torch.tensor([0, 1, 0, 0, 1, 0], dtype=torch.int32, device=dev())
+    q, e = rnd(6, nh, d, seed=3), err_word()
+
+    def run(rows):
+        out = torch.full((len(rows), nh, d), float("nan"), device=dev())
+        kernels.attention_plain(out, q[rows].contiguous(), kc, vc, pos[rows].contiguous(), req[rows].contiguous(), table, 3, None, 0.2, e)
+        return out
+
+    out = run(list(range(6)))
+    for t in range(6):
+        assert torch.equal(run([t])[0], out[t]), t
+        keys = lambda c: c[table[req[t]].long()].transpose(1, 2).reshape(48, nkv, d)[: int(pos[t]) + 1].double()
+        w = torch.softmax(torch.einsum("hd,khd->hk", q[t].double(), keys(kc)) * 0.2, 1)
+        assert (out[t].double() - torch.einsum("hk,khd->hd", w, keys(vc))).abs().max() <= 2e-5      # (as above)
+    assert int(e) == 0

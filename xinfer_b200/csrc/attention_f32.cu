@@ -85,9 +85,10 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAtten
             }
         }
     }
-    // the tile's tokens by request: their rows walk over that request's keys together
+    // runs of neighbouring tokens of one request: their rows walk over that request's keys together
     for (int s = 0; s < tokens;) {
         const int b = p.req_of_token[t0 + s];
+        const int from = s * heads;              // the run's rows: [from, e * heads), and no others, though a later run may be of the same request
         int e = s, hi = -1, first = 0x7fffffff;
         for (; e < tokens && p.req_of_token[t0 + e] == b; ++e) {
             const int ps = p.positions[t0 + e];
@@ -127,7 +128,8 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAtten
             unsigned vis[R], any = 0u, all = 0xffffffffu;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                const bool sees = req[i] == b && j <= pos[i] && (j >= lo[i] || j < p.keep);
+                const int r = i * WARPS + warp;
+                const bool sees = r >= from && r < s * heads && j <= pos[i] && (j >= lo[i] || j < p.keep);
                 if (sees && rows_now < 0) atomicOr(p.err, XB_ERR_BAD_PAGE);
                 vis[i] = __ballot_sync(0xffffffffu, sees && rows_now >= 0);
                 any |= vis[i];
