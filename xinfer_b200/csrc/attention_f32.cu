@@ -12,7 +12,7 @@ namespace {
 // share a processor and hide each other's waits (with two of each and two blocks: 113 us).  A warp holds up to four rows.  Scores: a lane per key, four sums of every fourth
 // channel each; softmax: the group's maximum and sum over the warp; values: a lane per four channels, keys in order.
 // A row visits the groups that hold a key it sees and no others, each in the same way, so its result depends on its own
-// position and keys alone, not on how many rows run beside it.
+// position and keys alone, not on how many rows run beside it.  A block's rows are of one run: neighbouring tokens of a request.
 // What bounded the kernel with a warp per query were the five shuffles, two exponentials and two dependent loads of every
 // key; here these are shared by 32 keys and by the rows, and the loads of the keys by the rows.  Two prompts of 301 and
 // 145 tokens, 16 heads over 8, head size 128: 292 us a layer before, 58 us now.
@@ -44,37 +44,35 @@ __device__ __forceinline__ void af_copy16(float* dst, const float* src, bool in)
                  "r"(in ? 16 : 0) : "memory");
 }
 
-// R: rows of a warp.  `tile`: tokens of a block, at most ROWS / min(group, ROWS).
+// The tokens [t0, t0 + tokens) of request b, neighbours in the step; R: rows of a warp, tokens * heads <= R * WARPS.
 template <int R>
-__global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAttentionF32 p, int tile) {
-    extern __shared__ __align__(16) float af_smem[];
+__device__ __forceinline__ void attend_run(const XbAttentionF32& p, int t0, int tokens, int b, float* af_smem) {
     const int ldk = p.d + 4, ldv = p.dv;          // a lane per key: rows 16 bytes apart from a multiple of all banks
     float* sk = af_smem;                          // [KEYS][ldk]
     float* sv = sk + KEYS * ldk;                  // [KEYS][ldv]
-    float* sq = sv + KEYS * ldv;                  // [R * WARPS][d], scaled
-    float* sp = sq + R * WARPS * p.d;             // [R * WARPS][KEYS] weights
+    float* sp = sv + KEYS * ldv;                  // [R * WARPS][KEYS] weights
+    float* sq = sp + R * WARPS * KEYS;            // [R * WARPS][d], scaled
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int group = p.nh / p.nkv, g = blockIdx.y, h0 = blockIdx.z * ROWS, heads = min(group - h0, ROWS);
-    const int t0 = blockIdx.x * tile, tokens = min(tile, p.tokens - t0), rows = tokens * heads;
-    for (int i = threadIdx.x; i < rows * p.d; i += WARPS * 32) {
-        const int r = i / p.d, c = i - r * p.d;
-        sq[i] = p.q[(size_t)(t0 + r / heads) * p.q_ts + (size_t)(g * group + h0 + r % heads) * p.q_hs + c] * p.scale;
-    }
-    // row i * WARPS + warp of the block: its token's request and position, the first key beside the kept ones that it sees
-    int req[R], pos[R], lo[R];
+    const int group = p.nh / p.nkv, g = blockIdx.y, h0 = blockIdx.z * ROWS, heads = min(group - h0, ROWS), rows = tokens * heads;
+    if (b >= 0)
+        for (int i = threadIdx.x; i < rows * p.d; i += WARPS * 32) {
+            const int r = i / p.d, c = i - r * p.d;
+            sq[i] = p.q[(size_t)(t0 + r / heads) * p.q_ts + (size_t)(g * group + h0 + r % heads) * p.q_hs + c] * p.scale;
+        }
+    // row i * WARPS + warp of the run: its token's position (-1: no row), the first key beside the kept ones that it sees
+    int pos[R], lo[R];
     float m[R], l[R], slope[R];
     unsigned long long acc[R][2];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         const int r = i * WARPS + warp;
-        req[i] = -1;
-        pos[i] = lo[i] = 0;
+        pos[i] = -1;
+        lo[i] = 0;
         m[i] = -INFINITY;
         l[i] = slope[i] = 0.f;
         acc[i][0] = acc[i][1] = 0ull;
         if (r < rows) {
             const int t = t0 + r / heads, h = g * group + h0 + r % heads;
-            req[i] = p.req_of_token[t];
             pos[i] = p.positions[t];
             lo[i] = p.window > 0 ? max(pos[i] - p.window + 1, 0) : 0;
             if (p.chunk > 0) lo[i] = max(lo[i], pos[i] / p.chunk * p.chunk);
@@ -85,20 +83,15 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAtten
             }
         }
     }
-    // runs of neighbouring tokens of one request: their rows walk over that request's keys together
-    for (int s = 0; s < tokens;) {
-        const int b = p.req_of_token[t0 + s];
-        const int from = s * heads;              // the run's rows: [from, e * heads), and no others, though a later run may be of the same request
-        int e = s, hi = -1, first = 0x7fffffff;
-        for (; e < tokens && p.req_of_token[t0 + e] == b; ++e) {
-            const int ps = p.positions[t0 + e];
+    if (b >= 0) {                                 // (else padding)
+        int hi = -1, first = 0x7fffffff;
+        for (int t = t0; t < t0 + tokens; ++t) {
+            const int ps = p.positions[t];
             int low = p.window > 0 ? max(ps - p.window + 1, 0) : 0;
             if (p.chunk > 0) low = max(low, ps / p.chunk * p.chunk);
             hi = max(hi, ps);
             first = min(first, low);
         }
-        s = e;
-        if (b < 0) continue;      // padding
         const int* table = p.block_table + (size_t)b * p.table_stride;
         const int last = hi / KEYS, begin = first / KEYS;
         const int kept = min(p.keep, first);                     // positions before `first` that some row may see
@@ -128,8 +121,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAtten
             unsigned vis[R], any = 0u, all = 0xffffffffu;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                const int r = i * WARPS + warp;
-                const bool sees = r >= from && r < s * heads && j <= pos[i] && (j >= lo[i] || j < p.keep);
+                const bool sees = j <= pos[i] && (j >= lo[i] || j < p.keep);
                 if (sees && rows_now < 0) atomicOr(p.err, XB_ERR_BAD_PAGE);
                 vis[i] = __ballot_sync(0xffffffffu, sees && rows_now >= 0);
                 any |= vis[i];
@@ -144,7 +136,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAtten
             if (any) {
                 const float* kr = sk + lane * ldk;
                 const float* qb = sq + warp * p.d;
-#pragma unroll 4
+#pragma unroll 8
                 for (int x = 0; x < p.d; x += 4) {
                     const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(kr + x);
 #pragma unroll
@@ -229,7 +221,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAtten
             }
         }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();                           // the buffers are free for the next request's keys
+        __syncthreads();                           // the buffers are free for the next run's keys
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -239,18 +231,65 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const XbAtten
         float* o = p.out + (size_t)(t0 + r / heads) * p.ldo + (size_t)(g * group + h0 + r % heads) * p.dv + lane * 4;
         const float2 a = af_unpack(acc[i][0]), c = af_unpack(acc[i][1]);
         const float v[4] = {a.x, a.y, c.x, c.y};
-        const bool pad = req[i] < 0;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) o[x] = pad ? 0.f : v[x] * inv;
+        for (int x = 0; x < 4; ++x) o[x] = b < 0 ? 0.f : v[x] * inv;
     }
+}
+
+// The first token of the k-th run that does not start a tile, -1 if there are fewer.
+__device__ __forceinline__ int further_run(const XbAttentionF32& p, int tile, int k) {
+    for (int base = 0; base < p.tokens; base += 32) {
+        const int t = base + (int)(threadIdx.x & 31);
+        unsigned starts = __ballot_sync(0xffffffffu, t < p.tokens && t % tile && p.req_of_token[t] != p.req_of_token[t - 1]);
+        const int here = __popc(starts);
+        if (k < here) {
+            for (; k > 0; --k) starts &= starts - 1;
+            return base + __ffs(starts) - 1;
+        }
+        k -= here;
+    }
+    return -1;
+}
+
+// How many tokens the run has in its tile.
+__device__ __forceinline__ int run_length(const XbAttentionF32& p, int tile, int t0) {
+    const int b = p.req_of_token[t0], end = min(t0 / tile * tile + tile, p.tokens);
+    int t = t0 + 1;
+    while (t < end && p.req_of_token[t] == b) ++t;
+    return t - t0;
+}
+
+// The runs from the k-th on, one after the other (a step with more runs than requests).
+template <int R>
+__device__ __noinline__ void attend_rest(const XbAttentionF32& p, int tile, int k, float* af_smem) {
+    for (int t0; (t0 = further_run(p, tile, k)) >= 0; ++k) attend_run<R>(p, t0, run_length(p, tile, t0), p.req_of_token[t0], af_smem);
+}
+
+// The first `tiles` blocks of a grid take the run that starts their tile of `tile` tokens (at most ROWS / min(group, ROWS)), the
+// others the further ones, one each, so that the requests of a decode step are attended side by side; a run of few rows takes
+// the form with one row to a warp.  With the runs of a tile one after the other in its block, 16 tokens at context 1,024 took
+// 1,758 us (8 heads of their own) and 896 (16 over 8), a warp per query 1,221 and 1,225; now 65 each.  (1,500 tokens of one
+// request: 547 and 555; 32 heads of 64 channels 760 and 786.)  A loop over runs around the one call made its steps 8 % longer.
+template <int R>
+__global__ void __launch_bounds__(WARPS * 32, 4) attention_f32_kernel(const __grid_constant__ XbAttentionF32 p, int tile, int tiles) {
+    extern __shared__ __align__(16) float af_smem[];
+    const int heads = min(p.nh / p.nkv - (int)blockIdx.z * ROWS, ROWS);
+    const int k = (int)blockIdx.x - tiles;
+    const int t0 = k < 0 ? blockIdx.x * tile : further_run(p, tile, k);
+    if (t0 < 0) return;
+    const int n = run_length(p, tile, t0);
+    if (R == 1 || n * heads > WARPS) attend_run<R>(p, t0, n, p.req_of_token[t0], af_smem);
+    else attend_run<1>(p, t0, n, p.req_of_token[t0], af_smem);
+    if (k >= 0 && blockIdx.x + 1 == gridDim.x) attend_rest<R>(p, tile, k + 1, af_smem);
 }
 
 template <int R>
 int launch(const XbAttentionF32& p, int tile, cudaStream_t stream) {
-    const int group = p.nh / p.nkv;
+    const int group = p.nh / p.nkv, tiles = (p.tokens + tile - 1) / tile;
+    const int others = min(max(p.requests - 1, 1), p.tokens - tiles);      // (`requests` may be wrong: then a block takes several runs, or none)
     const int smem = (KEYS * (p.d + 4) + KEYS * p.dv + R * WARPS * (p.d + KEYS)) * 4;
     cudaFuncSetAttribute(attention_f32_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attention_f32_kernel<R><<<dim3((p.tokens + tile - 1) / tile, p.nkv, (group + ROWS - 1) / ROWS), WARPS * 32, smem, stream>>>(p, tile);
+    attention_f32_kernel<R><<<dim3(tiles + others, p.nkv, (group + ROWS - 1) / ROWS), WARPS * 32, smem, stream>>>(p, tile, tiles);
     return xb_launch_status();
 }
 
@@ -265,7 +304,12 @@ bool xb_attention_f32_takes(const XbAttentionF32& p) {
 
 int xb_attention_f32(const XbAttentionF32& p, cudaStream_t stream) {
     const int heads = min(p.nh / p.nkv, ROWS);
-    const int tile = max(1, min(ROWS / heads, p.tokens));
+    // Shorter tiles while their blocks are at most two a processor: keys are then read more often, but by more processors.  64
+    // tokens behind 2,048: 228 us in whole tiles, 160 so (16 heads over 8); 32 heads of 64 channels 242 and 170, with a limit of four
+    // blocks a processor 206.
+    const long long columns = (long long)p.nkv * ((p.nh / p.nkv + ROWS - 1) / ROWS);
+    int tile = max(1, min(ROWS / heads, p.tokens));
+    while (tile > 1 && (p.tokens + tile / 2 - 1) / (tile / 2) * columns <= 296) tile /= 2;
     const int rows = tile * heads;
     if (rows <= WARPS) return launch<1>(p, tile, stream);
     if (rows <= 2 * WARPS) return launch<2>(p, tile, stream);

@@ -9,7 +9,7 @@ struct XbAttentionF32 {
     const int *positions, *req_of_token, *block_table;
     int* err;
     long long q_ts, q_hs, ldo;
-    int k_stride, v_stride, table_stride, tokens, nh, nkv, d, dv, page_size, num_pages, window, keep, chunk;
+    int k_stride, v_stride, table_stride, requests, tokens, nh, nkv, d, dv, page_size, num_pages, window, keep, chunk;
     float scale, softcap, slope_exp, out_scale;
 };
 

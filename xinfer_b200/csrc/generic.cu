@@ -491,17 +491,18 @@ static int attention_plain_launch(void* out, const void* q, long long q_ts, long
     return xb_launch_status();
 }
 
+// `requests`: rows of the block table (float32 alone looks at it, to size its grid).
 XB_EXPORT int xb_attention_plain(int dtype, void* out, const void* q, long long q_ts, long long q_hs, const void* k_cache,
                                  const void* v_cache, int k_stride, int v_stride, const float* sink,
                                  const int* positions, const int* req_of_token,
-                                 const int* block_table, int table_stride, int tokens, int nh, int nkv,
+                                 const int* block_table, int table_stride, int requests, int tokens, int nh, int nkv,
                                  int d, int dv, int page_size, int num_pages, int window, int keep, float scale, float softcap,
                                  float slope_exp, int chunk, long long ldo, float out_scale, int* err, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (dtype == XB_F32) {
         const XbAttentionF32 p = {(float*)out, (const float*)q, (const float*)k_cache, (const float*)v_cache, sink, positions,
-                                  req_of_token, block_table, err, q_ts, q_hs, ldo, k_stride, v_stride, table_stride, tokens, nh,
-                                  nkv, d, dv, page_size, num_pages, window, keep, chunk, scale, softcap, slope_exp, out_scale};
+                                  req_of_token, block_table, err, q_ts, q_hs, ldo, k_stride, v_stride, table_stride, requests, tokens,
+                                  nh, nkv, d, dv, page_size, num_pages, window, keep, chunk, scale, softcap, slope_exp, out_scale};
         if (xb_attention_f32_takes(p)) return xb_attention_f32(p, stream);
         return attention_plain_launch<float>(out, q, q_ts, q_hs, k_cache, v_cache, k_stride, v_stride, sink, positions,
                                              req_of_token, block_table,

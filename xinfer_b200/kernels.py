@@ -324,8 +324,8 @@ def qk_norm_rope_write(q_out, k_cache, v_cache, qkv, q_w, k_w, cos_t, sin_t, pos
 def attention_plain(out, q, k_cache, v_cache, positions, req_of_token, block_table, table_stride, window, scale, err, *,
                     sink=None, value_dim=None, softcap=None, slope_exponent=None, chunk=None, keep_first: int = 0,
                     out_scale: float = 1.0):
-    """Attention of every token over its request's cached positions, one warp per (token, head), float32 scores,
-    softmax and value sums.  ``q`` is ``[T, heads, d]``; ``out`` ``[T, heads, dv]``, whose tokens may lie further apart than
+    """Attention of every token over its request's cached positions, in any order of tokens and requests: one warp per
+    (token, head), or in float32 up to 128 channels runs of a request's tokens by block; float32 scores, softmax and value sums.  ``q`` is ``[T, heads, d]``; ``out`` ``[T, heads, dv]``, whose tokens may lie further apart than
     their heads * dv, receives ``out_scale`` times the result.  The caches are
     ``[page, kv_head, slot, d]`` and ``[page, kv_head, slot, dv]``; with ``value_dim`` the values are the first
     ``value_dim`` channels of the key rows themselves (``v_cache`` is then ignored).  ``sink`` (float32 per head):
@@ -358,7 +358,8 @@ def attention_plain(out, q, k_cache, v_cache, positions, req_of_token, block_tab
         raise KernelError(f"head size {max(d, dv)} is larger than the plain attention kernel's limit of 1024")
     _ok(kernels_lib().xb_attention_plain(
         dtype_code(q.dtype), out.data_ptr(), q.data_ptr(), nh * d, d, k_cache.data_ptr(), v_cache.data_ptr(), d, v_stride,
-        _ptr(sink), positions.data_ptr(), req_of_token.data_ptr(), block_table.data_ptr(), int(table_stride), T, nh, nkv, d,
+        _ptr(sink), positions.data_ptr(), req_of_token.data_ptr(), block_table.data_ptr(), int(table_stride),
+        int(block_table.shape[0]) if block_table.dim() == 2 else T, T, nh, nkv, d,
         dv, page_size, num_pages, int(window or 0), int(keep_first), float(scale), float(softcap or 0.0),
         float(slope_exponent or 0.0), int(chunk or 0), ldo, float(out_scale), err.data_ptr(), _stream()), "attention_plain")
 

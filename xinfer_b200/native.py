@@ -103,7 +103,7 @@ def _declare_kernels(lib):
     _sig(lib, "xb_qk_norm_rope_write", I,
          [I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P])
     _sig(lib, "xb_attention_plain", I,
-         [I, P, P, L, L, P, P, I, I, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, F, F, I, L, F, P, P])
+         [I, P, P, L, L, P, P, I, I, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, F, F, I, L, F, P, P])
     _sig(lib, "xb_swiglu", I, [I, P, P, I, I, I, F, F, P])
     _sig(lib, "xb_widen_bf16", I, [P, P, L, P])
     _sig(lib, "xb_sample", I, [P, P, P, P, I, I, I, I, P, P, P])
