@@ -43,3 +43,49 @@ def test_infinities_and_overflow_give_what_float32_gives(M, K):
     fine = torch.isfinite(ref)
     # every row but the two with an infinity and no number, every column but 7 and, in row 2, 9
     assert torch.isfinite(out[fine]).all() and fine.sum() == (M - 2) * (N - 1) - 1
+
+
+@pytest.mark.parametrize("e", [0, -100, -112, -118, -124, -140])
+def test_small_operands_keep_all_their_digits(e):
+    """Single products: 2^-24 of one for its rounding, 2^-24 for the products of parts that are left out and 2^-29 for what tensor
+    memory cuts off the sum of the small ones; of an operand below 2^-126 what is left out may reach its last digit, 2^-149."""
+    from xinfer_b200 import kernels
+    M, N, K = 17, 300, 64
+    for first in (True, False):
+        a, w = torch.zeros(M, K, device=dev()), torch.zeros(N, K, device=dev())
+        a[:, 5], w[:, 5] = rnd(M, seed=8), rnd(N, seed=9)
+        small, large = (a, w) if first else (w, a)
+        small *= 2.0 ** (e // 2)
+        small *= 2.0 ** (e - e // 2)
+        large *= 2.0 ** min(-e, 60)
+        out = torch.empty(M, N, device=dev())
+        kernels.gemm_plain(out, a, w)
+        x, y = a.double().abs()[:, 5, None], w.double().abs()[None, :, 5]
+        ref = a.double() @ w.double().t()
+        assert ((out.double() - ref).abs() <= (2.0 ** -23 + 2.0 ** -29) * ref.abs() + 2.0 ** -149 * (x if large is a else y)).all()
+
+
+@pytest.mark.parametrize("kind,K", [("normal", 64), ("small", 64), ("normal", 1024), ("positive", 1024), ("one term of 30", 1024),
+                                    ("one term of 1000", 1024), ("small", 1024), ("normal", 3072)])
+def test_error_is_no_larger_than_that_of_float32_multiply_adds(kind, K):
+    """In 2-norm over many outputs, against float32's own: 16 terms by fused multiply-adds, these sums added up."""
+    from xinfer_b200 import kernels
+    M, N = 64, 512
+    a, w = rnd(M, K, seed=10), rnd(N, K, seed=11)
+    if kind == "positive":
+        a, w = a.abs(), w.abs()
+    elif kind.startswith("one"):
+        a[:, K // 3] *= float(kind.split()[-1])
+    elif kind == "small":
+        a *= 2.0 ** -118
+    x, y = a.double(), w.double()
+    acc = torch.zeros(M, N, device=dev())
+    for k0 in range(0, K, 16):
+        part = torch.zeros(M, N, device=dev())
+        for k in range(k0, k0 + 16):
+            part = (part.double() + x[:, k, None] * y[None, :, k]).float()
+        acc += part
+    out = torch.empty(M, N, device=dev())
+    kernels.gemm_plain(out, a, w)
+    ref = x @ y.t()
+    assert (out.double() - ref).norm() <= (acc.double() - ref).norm()

@@ -1,20 +1,30 @@
 // Float32 matrix product  out[M, N] = a[M, K] . w[N, K]^T  on the tensor cores, with float32's own precision.
 //
-// Every operand is cut into three bfloat16 numbers that add up to it exactly (8 bits of mantissa each: the leading ones cut off, the
-// middle and last ones rounded), and the six products of parts that are not below 2^-24 of the whole are summed in float32:
-//     w0 a0 + (w0 a1 + w1 a0) + (w1 a1 + w0 a2 + w2 a0).
-// Tensor memory rounds a running sum towards zero, so no sum stays there: the six products of 16 terms go into columns of their
-// own, the small ones first, and are added up in registers, to nearest, in the order of K.
+// Every operand is cut into three bfloat16 numbers that add up to it exactly, each rounded to nearest.  The second and third are kept
+// 2^8 and 2^16 times as large, so that no digit of a small operand falls below the smallest bfloat16.  Of the nine products the
+// six largest are formed; what is left out is below 2^-24 of the whole (of an operand below 2^-126: below its last digit, 2^-149,
+// times the other one):
+//     w0 a0 + 2^-8 ((w0 a1 + w1 a0) + 2^-8 (w1 a1 + w0 a2 + w2 a0)).
+// Tensor memory rounds a running sum towards zero, so little stays there: of 32 terms at a time the products w0 a0, whose digits
+// fit, go to one column, and the small ones, whose cut-off digits do not count, to another; these two are added in registers,
+// to nearest, and so are the sums of 32 terms, in the order of K.  (Splitting a number into parts whose products are exact is
+// Dekker's, 1971.)
 // An output's sum has that one form whatever M, the tile or the operands' alignment is, so a row's result does not depend on
 // what else is in the step.  A sum that is not finite is formed again term by term (an infinity times a part of 0 is no number).
+//
+// Relative error against 64 bits (2-norm), by float32 multiply-adds of 16 terms and so: normal operands, K = 64 8.4e-8 and 5.5e-8,
+// 1,024 1.65e-7 and 1.16e-7, 3,072 2.6e-7 and 1.8e-7; operands near 2^-124 the same; one term 1,000 times the others, K = 1,024
+// 1.85e-7 and 1.30e-7.  Where it is larger: the tensor cores cut every product off near 2^-25 of the largest of its 16, so short
+// sums of one sign, K = 64 5.0e-8 and 5.7e-8, the more the more one term stands out (1,000 times the others, K = 32: 6.6e-8 and
+// 2.1e-7; 10^6 times, K = 1,024: 1.9e-7 and 2.1e-7).
+// With the leading part cut off instead of rounded, parts not scaled and all products in one column (and 446 x 4,096 x 1,024 41
+// instead of 46 us): a single product 5.6e-8, where this has 2.5e-8 as multiply-adds have, operands near 2^-116 3.2e-6.
 //
 // What bounds it is shared memory: with the cut rows of W there too, written once and read by six products, a panel of 64 k took
 // 1,730 cycles at 16 tokens and 1,920 at 32, just those bytes at 128 a cycle.  So the cut rows of W go to tensor memory, from
 // where an operand A costs nothing, and shared memory holds the panels as they come and the cut rows of A: 1,500 and 1,730.
-// Measured, before (float32 FMA) and now: 446 x 4,096 x 1,024 132 -> 40 us, 446 x 1,024 x 3,072 158 -> 44 us, 2,048 x 6,144 x
-// 1,024 781 -> 181 us (142 TFLOP/s), one row of 6,144 x 1,024 19.0 -> 18.0 us; two rows of 151,936 x 1,024 108 -> 113 us, 5,500 GB/s.
-// Relative error against 64 bits at K = 1,024 and 3,072, normal operands: 1.6e-7 and 2.6e-7 -> 1.2e-7 and 1.9e-7 (one term far
-// above all others: 1.3e-7 -> 2.0e-7, of one rounding towards zero instead of to nearest).
+// Measured, before (float32 FMA) and now: 446 x 4,096 x 1,024 145 -> 46 us, 446 x 1,024 x 3,072 209 -> 50 us, 2,048 x 6,144 x
+// 1,024 786 -> 205 us (126 TFLOP/s), one row of 6,144 x 1,024 21.2 -> 23.5 us; two rows of 151,936 x 1,024 123 -> 130 us.
 //
 // Roles of a block (persistent, a tile of 128 rows of W and TOK of A after another): one thread asks for panels by TMA, a ring of
 // them ahead; sixteen warps cut the panels, a thread 16 k of a row of W; two warps issue the products, of 32 k each; four or
@@ -37,8 +47,9 @@ struct Shape {
     static constexpr int RAW = (TILE_W + TOK) * PANEL * 4, RAWS = TOK <= 16 ? 5 : TOK <= 32 ? 4 : 3;
     static constexpr int SMEM = RAWS * RAW + STAGES * STAGE + 1024;
     // columns of tensor memory: the cut rows of W (two numbers a column), then the sums
-    static constexpr int W_COLS = 3 * (PANEL / 2), SUMS = STAGES * W_COLS, BUFS = TOK <= 32 ? 8 : 4;
-    static_assert(SUMS + BUFS * TOK <= 512 && BUFS % ISSUERS == 0, "columns");
+    static constexpr int W_COLS = 3 * (PANEL / 2), SUMS = STAGES * W_COLS, BUF = 2 * TOK, BUFS = TOK <= 16 ? 8 : TOK <= 32 ? 4 : 2;
+    static_assert(SUMS + BUFS * BUF <= 512 && BUFS % ISSUERS == 0, "columns");
+    static constexpr int AT_ONCE = TOK <= 32 ? 16 : 8;                               // columns of either sum that an adding warp reads at once
 };
 
 // one lane of the warp, the same one every time
@@ -59,18 +70,44 @@ __device__ __noinline__ float term_by_term(const float* a, const float* w, int K
     return sum;
 }
 
-// the three parts of two numbers
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// the three parts of two numbers, the second and third 2^8 and 2^16 times their value
 __device__ __forceinline__ void cut2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const uint32_t x0 = __float_as_uint(x), x1 = __float_as_uint(y);
-    hi = __byte_perm(x0, x1, 0x7632);
-    const float r0 = x - __uint_as_float(x0 & 0xffff0000u), r1 = y - __uint_as_float(x1 & 0xffff0000u);
+    const f32x2 minus = pack2(-1.f, -1.f), up = pack2(256.f, 256.f);
+    auto halves = [](uint32_t v) { return pack2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); };
+    float r0, r1;
+    hi = pack_bf16(x, y);
+    const f32x2 r = mul2(fma2(halves(hi), minus, pack2(x, y)), up);      // (no digit of a difference is lost)
+    unpack2(r, r0, r1);
     mid = pack_bf16(r0, r1);
-    // (what is left has no more than eight bits)
-    lo = __byte_perm(__float_as_uint(r0 - __uint_as_float(mid << 16)), __float_as_uint(r1 - __uint_as_float(mid & 0xffff0000u)), 0x7632);
+    unpack2(mul2(fma2(halves(mid), minus, r), up), r0, r1);
+    lo = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);  // (what is left has no more than eight bits)
 }
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
                  "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_nowait(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_nowait(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+}
+// umma_bf16_ta onto 2^-SHIFT times what is there
+template <int SHIFT>
+__device__ __forceinline__ void umma_bf16_ta_scaled(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "n"(SHIFT) : "memory");
 }
 // four numbers of a panel's row as TMA leaves them: halves of 32 numbers, rows of 128 bytes, swizzled
 __device__ __forceinline__ float4 raw4(const unsigned char* rows, int row, int chunk) {
@@ -202,21 +239,22 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                                                  mbar_wait(smem_u32(&s_free[buf]), free_parity, err, true));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d = tm + (uint32_t)(S::SUMS + buf * TOK), sa = mem0 + S::RAWS * S::RAW + stage * S::STAGE + q * (TERMS * 2);
+                const uint32_t d = tm + (uint32_t)(S::SUMS + buf * S::BUF), sa = mem0 + S::RAWS * S::RAW + stage * S::STAGE + q * (TERMS * 2);
                 const uint32_t w0 = tm + (uint32_t)(stage * S::W_COLS + q * (TERMS / 2)), w1 = w0 + PANEL / 2, w2 = w0 + PANEL;
                 const uint64_t a0 = umma_desc(sa), a1 = umma_desc(sa + S::A_BYTES), a2 = umma_desc(sa + 2 * S::A_BYTES);
                 if (elect_one()) {                                // 16 terms are 8 columns and 32 bytes of a row
-                    umma_bf16_ta(d, w2, a0, idesc, 0u);
-                    umma_bf16_ta(d, w0, a2, idesc, 1u);
-                    umma_bf16_ta(d, w1, a1, idesc, 1u);
-                    umma_bf16_ta(d, w1, a0, idesc, 1u);
-                    umma_bf16_ta(d, w0, a1, idesc, 1u);
-                    umma_bf16_ta(d, w2 + 8, a0 + 2, idesc, 1u);
-                    umma_bf16_ta(d, w0 + 8, a2 + 2, idesc, 1u);
-                    umma_bf16_ta(d, w1 + 8, a1 + 2, idesc, 1u);
-                    umma_bf16_ta(d, w1 + 8, a0 + 2, idesc, 1u);
-                    umma_bf16_ta(d, w0 + 8, a1 + 2, idesc, 1u);
-                    umma_bf16_ta(d, w0, a0, idesc, 1u);
+                    const uint32_t small = d + TOK;
+                    umma_bf16_ta(small, w2, a0, idesc, 0u);
+                    umma_bf16_ta(small, w0, a2, idesc, 1u);
+                    umma_bf16_ta(small, w1, a1, idesc, 1u);
+                    umma_bf16_ta(small, w2 + 8, a0 + 2, idesc, 1u);
+                    umma_bf16_ta(small, w0 + 8, a2 + 2, idesc, 1u);
+                    umma_bf16_ta(small, w1 + 8, a1 + 2, idesc, 1u);
+                    umma_bf16_ta_scaled<8>(small, w1, a0, idesc);
+                    umma_bf16_ta(small, w0, a1, idesc, 1u);
+                    umma_bf16_ta(small, w1 + 8, a0 + 2, idesc, 1u);
+                    umma_bf16_ta(small, w0 + 8, a1 + 2, idesc, 1u);
+                    umma_bf16_ta(d, w0, a0, idesc, 0u);
                     umma_bf16_ta(d, w0 + 8, a0 + 2, idesc, 1u);
                     umma_commit(smem_u32(&s_sum[buf]));
                     umma_commit(smem_u32(&s_empty[stage]));
@@ -250,13 +288,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_sum[buf]), parity, err, true));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t from = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(S::SUMS + buf * TOK + c0);
+                const uint32_t from = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(S::SUMS + buf * S::BUF + c0);
 #pragma unroll
-                for (int c = 0; c < S::WIDTH; c += 16) {
-                    float v[16];
-                    tmem_ld16(from + c, v);
+                for (int c = 0; c < S::WIDTH; c += S::AT_ONCE) {
+                    uint32_t large[S::AT_ONCE], small[S::AT_ONCE];
+                    tmem_ld_nowait(from + c, large);
+                    tmem_ld_nowait(from + TOK + c, small);
+                    tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[c + i] += v[i];
+                    for (int i = 0; i < S::AT_ONCE; ++i) acc[c + i] += fmaf(__uint_as_float(small[i]), 0x1p-8f, __uint_as_float(large[i]));
                 }
                 tc_fence_before();
                 __syncwarp();
