@@ -89,3 +89,17 @@ def test_error_is_no_larger_than_that_of_float32_multiply_adds(kind, K):
     kernels.gemm_plain(out, a, w)
     ref = x @ y.t()
     assert (out.double() - ref).norm() <= (acc.double() - ref).norm()
+
+
+@pytest.mark.parametrize("M,N,K", [(449, 4100, 200), (1, 24577, 130), (70, 19000, 65)])
+def test_tiles_of_every_size_form_the_same_bits(M, N, K):
+    """Tiles of 16, 32 and 64 tokens and of any number of rows of W: a row, and some of the columns, as they are alone."""
+    from xinfer_b200 import kernels
+    a, w = rnd(M, K, seed=12), rnd(N, K, seed=13)
+    out = torch.full((M, N), float("nan"), device=dev())
+    kernels.gemm_plain(out, a, w)
+    for rows, cols in (([M // 2], slice(0, N)), (slice(0, min(M, 33)), slice(N - 200, N)), (slice(0, M), slice(88, 130))):
+        x, y = a[rows].contiguous(), w[cols].contiguous()
+        part = torch.full((x.shape[0], y.shape[0]), float("nan"), device=dev())
+        kernels.gemm_plain(part, x, y)
+        assert torch.equal(part, out[rows][:, cols])

@@ -20,14 +20,16 @@
 // With the leading part cut off instead of rounded, parts not scaled and all products in one column (and 446 x 4,096 x 1,024 41
 // instead of 46 us): a single product 5.6e-8, where this has 2.5e-8 as multiply-adds have, operands near 2^-116 3.2e-6.
 //
-// What bounds it is shared memory: with the cut rows of W there too, written once and read by six products, a panel of 64 k took
-// 1,730 cycles at 16 tokens and 1,920 at 32, just those bytes at 128 a cycle.  So the cut rows of W go to tensor memory, from
-// where an operand A costs nothing, and shared memory holds the panels as they come and the cut rows of A: 1,500 and 1,730.
-// Measured, before (float32 FMA) and now: 446 x 4,096 x 1,024 145 -> 46 us, 446 x 1,024 x 3,072 209 -> 50 us, 2,048 x 6,144 x
-// 1,024 786 -> 205 us (126 TFLOP/s), one row of 6,144 x 1,024 21.2 -> 23.5 us; two rows of 151,936 x 1,024 123 -> 130 us.
+// The cut rows of W go to tensor memory, from where an operand A costs no bytes of shared memory; that holds the panels as they come
+// and the cut rows of A (with the cut rows of W there too, a panel of 64 k took 1,730 cycles at 16 tokens instead of 1,500).  What
+// bounds a panel then: at 64 tokens shared memory's bytes, some 1,350 cycles of 2,000; at 16 the time from a panel to its sums, which
+// two teams of cutting warps and two stages overlap: 48 panels of 1,024 rows 46.1 -> 38.9 us with one team -> with two.
+// Measured, float32 multiply-adds and now: 446 x 4,096 x 1,024 145 -> 47 us, 446 x 1,024 x 3,072 209 -> 49 us, 2,048 x 6,144 x
+// 1,024 786 -> 215 us (120 TFLOP/s), one row of 6,144 x 1,024 21.2 -> 20.5 us, two of 151,936 x 1,024 123 -> 121 us, one of 24,576 x
+// 4,096 90 -> 98 us (4,100 GB/s; 117 with one team and all tiles 128 rows high).
 //
 // Roles of a block (persistent, a tile of 128 rows of W and TOK of A after another): one thread asks for panels by TMA, a ring of
-// them ahead; sixteen warps cut the panels, a thread 16 k of a row of W; two warps issue the products, of 32 k each; four or
+// them ahead; sixteen warps cut the panels, a thread 16 k (or 32 of every other panel) of a row of W; two warps issue the products, of 32 k each; four or
 // eight warps add up the sums, through a ring of column buffers, and write the tile.
 #include "common.cuh"
 #include "gemm_f32_tc.h"
@@ -44,7 +46,10 @@ struct Shape {
     static constexpr int ADDERS = TOK > 32 ? 8 : 4, WIDTH = TOK / (ADDERS / 4);      // columns of an adding warp
     static constexpr int THREADS = (CUTTERS + ISSUERS + ADDERS + 1) * 32;
     static constexpr int A_BYTES = TOK * 128, STAGE = 3 * A_BYTES, STAGES = 2;       // the cut rows of A: three parts
-    static constexpr int RAW = (TILE_W + TOK) * PANEL * 4, RAWS = TOK <= 16 ? 5 : TOK <= 32 ? 4 : 3;
+    static constexpr int RAW = (TILE_W + TOK) * PANEL * 4, RAWS = TOK <= 32 ? 4 : 3;
+    // Two teams of cutting warps take every other panel, so that one cuts while the other waits.  A barrier of the ring then has one
+    // team only, which waits for its phases one after the other (a phase that nobody of a team waits for could be taken for the next).
+    static constexpr int TEAMS = RAWS % 2 == 0 ? 2 : 1;
     static constexpr int SMEM = RAWS * RAW + STAGES * STAGE + 1024;
     // columns of tensor memory: the cut rows of W (two numbers a column), then the sums
     static constexpr int W_COLS = 3 * (PANEL / 2), SUMS = STAGES * W_COLS, BUF = 2 * TOK, BUFS = TOK <= 16 ? 8 : TOK <= 32 ? 4 : 2;
@@ -122,7 +127,7 @@ __device__ __forceinline__ float4 any4(const float* p, int left) {
 template <int TOK, bool BY_TMA>
 __global__ void __launch_bounds__(Shape<TOK>::THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* out, const float* a,
-                   const float* w, int M, int N, int K, int* err) {
+                   const float* w, int M, int N, int K, int height, int* err) {
     typedef Shape<TOK> S;
     extern __shared__ unsigned char gf_smem[];
     __shared__ unsigned long long s_full[S::STAGES], s_empty[S::STAGES], s_sum[S::BUFS], s_free[S::BUFS], s_raw[S::RAWS], s_read[S::RAWS];
@@ -132,7 +137,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 32) {
         for (int i = 0; i < S::STAGES; ++i) {
-            mbar_init(smem_u32(&s_full[i]), CUTTERS);
+            mbar_init(smem_u32(&s_full[i]), CUTTERS / S::TEAMS);
             mbar_init(smem_u32(&s_empty[i]), ISSUERS);
         }
         for (int i = 0; i < S::BUFS; ++i) {
@@ -141,7 +146,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         for (int i = 0; i < S::RAWS; ++i) {
             mbar_init(smem_u32(&s_raw[i]), 1);
-            mbar_init(smem_u32(&s_read[i]), CUTTERS);
+            mbar_init(smem_u32(&s_read[i]), CUTTERS / S::TEAMS);
         }
         mbar_init_fence();
     }
@@ -152,78 +157,96 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t tmem = s_tmem;
     pdl_launch_dependents();   // only now: see pdl_launch_dependents on tensor memory
     pdl_wait();
-    const int across = (M + TOK - 1) / TOK, tiles = (N + TILE_W - 1) / TILE_W * across, panels = (K + PANEL - 1) / PANEL;
+    const int across = (M + TOK - 1) / TOK, tiles = (N + height - 1) / height * across, panels = (K + PANEL - 1) / PANEL;
 
     if (warp < CUTTERS) {
-        // 16 k of a row of W, in the quarter of tensor memory's lanes that a warp of this number may write, and eight of a row of A
-        const int part = warp >> 2, row = (warp & 3) * 32 + lane, r = threadIdx.x >> 3, c = threadIdx.x & 7;
-        const bool has_a = r < TOK;
-        int stage = 0, raw = 0;
+        // 16 k of a row of W for every team, in the quarter of tensor memory's lanes that a warp of this number may write, and eight of a
+        // row of A
+        constexpr int TEAMS = S::TEAMS, WARPS = CUTTERS / TEAMS;
+        const int team = warp / WARPS, row = (warp & 3) * 32 + lane, part0 = ((warp % WARPS) >> 2) * TEAMS;
+        const int r = (threadIdx.x % (WARPS * 32)) >> 3, c = threadIdx.x & 7, all_k = panels * PANEL;
+        const bool has_a = r < TOK, has_w = (warp & 3) * 32 < height;      // (rows behind the tile's are not cut: what is there reaches no result)
+        int stage = team % S::STAGES, raw = team, tile = blockIdx.x, k0 = team * PANEL;
         uint32_t parity = 1, raw_parity = 0;                      // (a fresh barrier's phase before its first counts as over)
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-            const int n = tile / across * TILE_W + row, m = tile % across * TOK + r;
-            for (int k0 = 0; k0 < K; k0 += PANEL) {
-                float4 v[4], u[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-                if (BY_TMA) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_raw[raw]), raw_parity, err, true));
-                    if (!ok) break;
-                    const unsigned char* src = mem + raw * S::RAW;
+        for (;; k0 += TEAMS * PANEL) {
+            for (; k0 >= all_k; k0 -= all_k) tile += gridDim.x;
+            if (tile >= tiles) break;
+            float4 v[TEAMS][4], u[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+            if (BY_TMA) {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_raw[raw]), raw_parity, err, true))) break;
+                const unsigned char* src = mem + raw * S::RAW;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) v[i] = raw4(src + (part >> 1) * (TILE_W * 128), row, (part & 1) * 4 + i);
-                    src += TILE_W * PANEL * 4;
-                    if (has_a) {
+                for (int t = 0; t < TEAMS; ++t)
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) u[i] = raw4(src + (c >> 2) * (TOK * 128), r, (c & 3) * 2 + i);
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&s_read[raw]));
-                    if (++raw == S::RAWS) {
-                        raw = 0;
-                        raw_parity ^= 1;
-                    }
-                } else {
-                    const int kw = k0 + part * 16, ka = k0 + c * 8;
+                    for (int i = 0; i < 4; ++i) v[t][i] = raw4(src + ((part0 + t) >> 1) * (TILE_W * 128), row, ((part0 + t) & 1) * 4 + i);
+                src += TILE_W * PANEL * 4;
+                if (has_a) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) v[i] = any4(w + (size_t)n * K + kw + i * 4, n < N ? K - kw - i * 4 : 0);
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) u[i] = any4(a + (size_t)m * K + ka + i * 4, has_a && m < M ? K - ka - i * 4 : 0);
+                    for (int i = 0; i < 2; ++i) u[i] = raw4(src + (c >> 2) * (TOK * 128), r, (c & 3) * 2 + i);
                 }
-                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[stage]), parity, err, true));
-                if (!ok) break;
-                tc_fence_after();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&s_read[raw]));
+                raw += TEAMS;
+                if (raw >= S::RAWS) {
+                    raw -= S::RAWS;
+                    raw_parity ^= 1;
+                }
+            } else {
+                const int n = tile / across * height + row, m = tile % across * TOK + r, ka = k0 + c * 8;
+#pragma unroll
+                for (int t = 0; t < TEAMS; ++t)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int kw = k0 + (part0 + t) * 16 + i * 4;
+                        v[t][i] = any4(w + (size_t)n * K + kw, n < N ? K - kw : 0);
+                    }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) u[i] = any4(a + (size_t)m * K + ka + i * 4, has_a && m < M ? K - ka - i * 4 : 0);
+            }
+#pragma unroll
+            for (int t = 0; t < TEAMS; ++t) {
                 uint32_t hi[8], mid[8], lo[8];
+                if (!has_w) {
+                    if (t == 0 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[stage]), parity, err, true))) goto done;
+                    continue;
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    cut2(v[i].x, v[i].y, hi[2 * i], mid[2 * i], lo[2 * i]);
-                    cut2(v[i].z, v[i].w, hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1]);
+                    cut2(v[t][i].x, v[t][i].y, hi[2 * i], mid[2 * i], lo[2 * i]);
+                    cut2(v[t][i].z, v[t][i].w, hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1]);
                 }
-                const uint32_t to = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(stage * S::W_COLS + part * 8);
+                if (t == 0) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[stage]), parity, err, true))) goto done;
+                    tc_fence_after();
+                }
+                const uint32_t to = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(stage * S::W_COLS + (part0 + t) * 8);
                 tmem_st8(to, hi);
                 tmem_st8(to + PANEL / 2, mid);
                 tmem_st8(to + PANEL, lo);
-                if (has_a) {
-                    unsigned char* dst = mem + S::RAWS * S::RAW + stage * S::STAGE + r * 128 + ((c ^ (r & 7)) << 4);
-                    uint4 h, md, l;
-                    cut2(u[0].x, u[0].y, h.x, md.x, l.x);
-                    cut2(u[0].z, u[0].w, h.y, md.y, l.y);
-                    cut2(u[1].x, u[1].y, h.z, md.z, l.z);
-                    cut2(u[1].z, u[1].w, h.w, md.w, l.w);
-                    *reinterpret_cast<uint4*>(dst) = h;
-                    *reinterpret_cast<uint4*>(dst + S::A_BYTES) = md;
-                    *reinterpret_cast<uint4*>(dst + 2 * S::A_BYTES) = l;
-                }
-                tmem_st_wait();
-                tc_fence_before();
-                fence_async_shared();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&s_full[stage]));
-                if (++stage == S::STAGES) {
-                    stage = 0;
-                    parity ^= 1;
-                }
+            }
+            if (has_a) {
+                unsigned char* dst = mem + S::RAWS * S::RAW + stage * S::STAGE + r * 128 + ((c ^ (r & 7)) << 4);
+                uint4 h, md, l;
+                cut2(u[0].x, u[0].y, h.x, md.x, l.x);
+                cut2(u[0].z, u[0].w, h.y, md.y, l.y);
+                cut2(u[1].x, u[1].y, h.z, md.z, l.z);
+                cut2(u[1].z, u[1].w, h.w, md.w, l.w);
+                *reinterpret_cast<uint4*>(dst) = h;
+                *reinterpret_cast<uint4*>(dst + S::A_BYTES) = md;
+                *reinterpret_cast<uint4*>(dst + 2 * S::A_BYTES) = l;
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            fence_async_shared();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_full[stage]));
+            stage += TEAMS;
+            if (stage >= S::STAGES) {
+                stage -= S::STAGES;
+                parity ^= 1;
             }
         }
+    done:;
     } else if (warp < CUTTERS + ISSUERS) {
         // Issuer q takes the q-th 32 terms of every panel; the whole warp walks along, so that the descriptors are the same in
         // all lanes, and one lane issues.
@@ -306,8 +329,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     parity ^= 1;
                 }
             }
-            const int n = tile / across * TILE_W + quarter * 32 + lane, m0 = tile % across * TOK + c0;
-            if (ok && n < N) {
+            const int n = tile / across * height + quarter * 32 + lane, m0 = tile % across * TOK + c0;
+            if (ok && n < N && quarter * 32 + lane < height) {
 #pragma unroll
                 for (int i = 0; i < S::WIDTH; ++i)
                     if (m0 + i < M) {
@@ -322,12 +345,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t parity = 1;
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-            const int n0 = tile / across * TILE_W, m0 = tile % across * TOK;
+            const int n0 = tile / across * height, m0 = tile % across * TOK;
             for (int k0 = 0; k0 < K; k0 += PANEL) {
                 ok = mbar_wait(smem_u32(&s_read[raw]), parity, err, true);
                 if (!ok) break;
                 const uint32_t dst = base + raw * S::RAW, bar = smem_u32(&s_raw[raw]);
-                mbar_expect_tx(bar, S::RAW);                      // (what lies outside an operand arrives as zeros)
+                mbar_expect_tx(bar, (height + TOK) * PANEL * 4);  // (what lies outside an operand arrives as zeros)
                 for (int h = 0; h < 2; ++h) {
                     tma_load_2d(dst + h * (TILE_W * 128), &map_w, k0 + h * HALF, n0, bar);
                     tma_load_2d(dst + TILE_W * PANEL * 4 + h * (TOK * 128), &map_a, k0 + h * HALF, m0, bar);
@@ -367,15 +390,15 @@ bool rows_map(CUtensorMap* map, const float* p, int rows, int K, int box_rows) {
 }
 
 template <int TOK, bool BY_TMA>
-int launch(float* out, const float* a, const float* w, int M, int N, int K, int* err, int sms, cudaStream_t stream) {
+int launch(float* out, const float* a, const float* w, int M, int N, int K, int height, int* err, int sms, cudaStream_t stream) {
     const cudaError_t rc = cudaFuncSetAttribute(gemm_f32_tc_kernel<TOK, BY_TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<TOK>::SMEM);
     if (rc != cudaSuccess) return (int)rc;
     CUtensorMap map_w = {}, map_a = {};
-    if (BY_TMA && !(rows_map(&map_w, w, N, K, TILE_W) && rows_map(&map_a, a, M, K, TOK))) return (int)cudaErrorInvalidValue;
-    const long long tiles = (long long)((N + TILE_W - 1) / TILE_W) * ((M + TOK - 1) / TOK);
+    if (BY_TMA && !(rows_map(&map_w, w, N, K, height) && rows_map(&map_a, a, M, K, TOK))) return (int)cudaErrorInvalidValue;
+    const long long tiles = (long long)((N + height - 1) / height) * ((M + TOK - 1) / TOK);
     if (tiles > 0x7fffffffLL - sms) return (int)cudaErrorInvalidValue;
     return xb_launch(gemm_f32_tc_kernel<TOK, BY_TMA>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(Shape<TOK>::THREADS), Shape<TOK>::SMEM, stream, map_w,
-                     map_a, out, a, w, M, N, K, err);
+                     map_a, out, a, w, M, N, K, height, err);
 }
 
 }  // namespace
@@ -385,13 +408,20 @@ int xb_gemm_f32_tc(float* out, const float* a, const float* w, int M, int N, int
     if (sms < 1) return (int)cudaErrorInvalidDevice;
     const bool by_tma = K % 4 == 0 && !(((uintptr_t)a | (uintptr_t)w) & 15);
     // tokens of a tile: what takes the fewest rounds of blocks, a round taken to cost 1 at 16 tokens, 1.15 at 32 and
-    // 1.4 at 64 (1,500, 1,730 and 2,000 to 2,300 cycles a panel)
+    // 1.5 at 64 (48 panels: 38.9, 45.1 and 57.4 us; 128 with all processors at work: 98, 111 and 143)
     auto cost = [&](int tok, float round) {
         const long long tiles = (long long)((N + TILE_W - 1) / TILE_W) * ((M + tok - 1) / tok);
         return (float)((tiles + sms - 1) / sms) * round;
     };
-    const float c16 = cost(16, 1.f), c32 = cost(32, 1.15f), c64 = cost(64, 1.4f);
-#define XB_GF(TOK) (by_tma ? launch<TOK, true>(out, a, w, M, N, K, err, sms, stream) : launch<TOK, false>(out, a, w, M, N, K, err, sms, stream))
+    const float c16 = cost(16, 1.f), c32 = cost(32, 1.15f), c64 = cost(64, 1.5f);
+    // rows of W of a tile: as few as the number of rounds allows, so that the last round has work for every processor
+    // (one row of 24,576 x 4,096, 192 tiles of 128 rows or 280 of 88: 111 and 98 us)
+    auto height = [&](int tok) {
+        const long long across = (M + tok - 1) / tok, rounds = ((long long)((N + TILE_W - 1) / TILE_W) * across + sms - 1) / sms, most = rounds * sms / across;
+        const int rows = (int)((N + most - 1) / most);
+        return rows <= 32 ? 32 : (rows + 7) / 8 * 8;
+    };
+#define XB_GF(TOK) (by_tma ? launch<TOK, true>(out, a, w, M, N, K, height(TOK), err, sms, stream) : launch<TOK, false>(out, a, w, M, N, K, height(TOK), err, sms, stream))
     if (c16 <= c32 && c16 <= c64) return XB_GF(16);
     if (c32 <= c64) return XB_GF(32);
     return XB_GF(64);
