@@ -45,3 +45,59 @@ def test_other_stacks_keep_to_the_parts():
     assert ModelRunner.random(cfg, 1, dtype="bf16", **opts).model.dense is None          # heads of more than 128 values
     assert ModelRunner.random(dict(cfg, head_dim=64), 1, dtype="f32", **opts).model.dense is None
     assert ModelRunner.random(dict(cfg, head_dim=64), 1, dtype="bf16", **opts).model.dense is not None
+
+
+CFG = dict(architectures=["Qwen3ForCausalLM"], vocab_size=300, hidden_size=256, intermediate_size=640, num_hidden_layers=3, num_attention_heads=8,
+           num_key_value_heads=2, head_dim=64, rms_norm_eps=1e-6, rope_theta=10000.0, max_position_embeddings=2048, tie_word_embeddings=False)
+
+
+def steps(monkeypatch, native=True):
+    """Logits of a prompt step, a mixed and a decode step."""
+    from xinfer_b200.engine.runner import ModelRunner, StepInput
+    from xinfer_b200.models import dense_layers
+    monkeypatch.setattr(dense_layers, "ENABLED", native)
+    r = ModelRunner.random(CFG, 7, dtype="bf16", block_size=16, num_blocks=64, max_num_seqs=3, max_model_len=512)
+    slots = [r.open_request() for _ in range(3)]
+    rng, out = np.random.default_rng(5), []
+    for step in ([(0, 70), (1, 2)], [(2, 100), (0, 1), (1, 1)], [(0, 1), (1, 1), (2, 1)]):
+        toks = [rng.integers(0, 300, size=n, dtype=np.int32) for _, n in step]
+        out.append(r.step([StepInput(slots[b], t, range(len(t))) for (b, _), t in zip(step, toks)], allow_graph=False).clone())
+    r.check_errors()
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("switch", ["reduced precision", "library", "tunable"])
+def test_torchs_switches_send_products_through_torch(switch, monkeypatch):
+    from xinfer_b200 import kernels
+    called = []
+    whole = kernels.dense_layers
+    monkeypatch.setattr(kernels, "dense_layers", lambda *a: (called.append(1), whole(*a)))
+    steps(monkeypatch)
+    assert len(called) == 3
+    called.clear()
+    blas = torch.backends.cuda.preferred_blas_library()
+    try:
+        if switch == "reduced precision":
+            torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
+        elif switch == "library":
+            torch.backends.cuda.preferred_blas_library("cublaslt")
+        else:
+            monkeypatch.setattr(torch.cuda.tunable, "is_enabled", lambda: True)
+        steps(monkeypatch)
+    finally:
+        torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = True
+        torch.backends.cuda.preferred_blas_library(blas)
+    assert not called
+
+
+def test_without_torchs_library_the_parts_run(monkeypatch):
+    import ctypes
+    from xinfer_b200.engine.runner import ModelRunner
+
+    def none(name, *a, **k):
+        raise OSError(name)
+    opts = dict(block_size=16, num_blocks=8, max_num_seqs=1, max_model_len=64)
+    with monkeypatch.context() as m:
+        m.setattr(ctypes, "CDLL", none)
+        r = ModelRunner.random(CFG, 1, dtype="bf16", **opts)
+        assert r.model.dense is None

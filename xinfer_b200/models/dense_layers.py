@@ -4,6 +4,7 @@ attention, an RMSNorm and a gated feed-forward, all alike, in bfloat16, and the 
 from __future__ import annotations
 
 import ctypes
+import os
 from typing import List, Optional
 
 import torch
@@ -31,20 +32,26 @@ class _Step(ctypes.Structure):
         + [(n, ctypes.c_float) for n in "eps1 offset1 eps2 offset2 qk_eps scale p0 p1".split()])
 
 
-_gemm_ex = None
+def _library_product() -> Optional[int]:
+    """The address of the library product that torch itself calls, in the library that torch has loaded; None if there is none."""
+    try:
+        lib = ctypes.CDLL(f"libcublas.so.{(torch.version.cuda or '').split('.')[0]}", mode=os.RTLD_NOLOAD)
+        return ctypes.cast(lib.cublasGemmEx, ctypes.c_void_p).value
+    except (OSError, AttributeError):
+        return None
 
 
-def _library_product() -> int:
-    """The address of the library product that torch itself calls (the library that torch has loaded)."""
-    global _gemm_ex
-    if _gemm_ex is None:
-        _gemm_ex = ctypes.cast(ctypes.CDLL("libcublas.so.12").cublasGemmEx, ctypes.c_void_p).value
-    return _gemm_ex
+def _torch_calls_the_library() -> bool:
+    """Whether torch's own product would be that call too: its switches choose another library, sums of another kind or an error."""
+    return (torch.backends.cuda.preferred_blas_library().name in ("Default", "Cublas") and not torch.cuda.tunable.is_enabled()
+            and torch._C._get_cublas_allow_bf16_reduced_precision_reduction() in (True, (True, True))
+            and not torch.are_deterministic_algorithms_enabled())
 
 
 class DenseLayers:
-    def __init__(self, layers: List[tuple]):
+    def __init__(self, layers: List[tuple], gemm_ex: int):
         self.layers = layers        # (norm, attention, norm, feed-forward) of every run
+        self.gemm_ex = gemm_ex      # address of the library product
 
     @staticmethod
     def of(plan, blocks, dtype, stream_dtype) -> Optional["DenseLayers"]:
@@ -74,11 +81,13 @@ class DenseLayers:
             return None
         if f.intermediate % 8 or f.intermediate < 64 or a.head_dim % 16 or not 16 <= a.head_dim <= 128 or a.num_heads * a.head_dim < 64:
             return None
-        return DenseLayers(layers)
+        gemm_ex = _library_product()
+        return DenseLayers(layers, gemm_ex) if gemm_ex is not None else None
 
     def takes(self, ctx: StepContext, caches: List[Optional[LayerCache]]) -> bool:
         if not (ENABLED and kernels.vectorized and gemm_backend._enabled and attention_backend._enabled and attention_backend.PREFILL_TC
-                and attention_backend.DECODE_TC) or gemm_backend.FUSE_EPILOGUES or tracing.ENABLED:
+                and attention_backend.DECODE_TC) or gemm_backend.FUSE_EPILOGUES or tracing.ENABLED \
+                or not _torch_calls_the_library():
             return False
         c0, s = caches[0], self.layers[0][1].spec
         if any(c is None or c.group != c0.group or c["k"].shape != c0["k"].shape for c in caches):
@@ -128,7 +137,7 @@ class DenseLayers:
                     skinny=gemm_backend.SKINNY_MAX_TOKENS, many_rows=kernels.many_rows, activation=act)
         reals = dict(eps1=n1.spec.eps, offset1=n1.spec.weight_offset, eps2=n2.spec.eps, offset2=n2.spec.weight_offset, qk_eps=s.qk_norm_eps,
                      scale=s.scale, p0=p0, p1=p1)
-        library = dict(gemm_ex=_library_product(), blas=torch.cuda.current_blas_handle())
+        library = dict(gemm_ex=self.gemm_ex, blas=torch.cuda.current_blas_handle())
         table = [(a.w_qkv, a.w_o, g.w_gate_up, g.w_down, p.weight, q.weight, a.q_norm, a.k_norm, c["k"], c["v"])
                  for (p, a, q, g), c in zip(self.layers, caches)]
         kernels.dense_layers(_Step, bufs, nums, reals, library, table)
