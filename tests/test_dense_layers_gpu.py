@@ -66,6 +66,16 @@ def steps(monkeypatch, native=True):
     return torch.cat(out)
 
 
+class Library:
+    """The native library with another ``xb_dense_layers``."""
+
+    def __init__(self, lib, call):
+        self._lib, self._call = lib, call
+
+    def __getattr__(self, name):
+        return self._call if name == "xb_dense_layers" else getattr(self._lib, name)
+
+
 @pytest.mark.parametrize("switch", ["reduced precision", "library", "tunable"])
 def test_torchs_switches_send_products_through_torch(switch, monkeypatch):
     from xinfer_b200 import kernels
@@ -101,3 +111,53 @@ def test_without_torchs_library_the_parts_run(monkeypatch):
         m.setattr(ctypes, "CDLL", none)
         r = ModelRunner.random(CFG, 1, dtype="bf16", **opts)
         assert r.model.dense is None
+
+
+@pytest.mark.parametrize("layer", [0, 2])
+def test_an_attention_kernel_that_does_not_take_the_step(layer, monkeypatch):
+    """Layer ``layer``'s attention is refused (and what its kernels have written is spoilt): another kernel attends and the call goes on."""
+    import ctypes
+    from xinfer_b200 import kernels, native
+    from xinfer_b200.parts import attention_backend
+    expect = steps(monkeypatch, native=False)
+    real, types = native.kernels_lib(), kernels.dense_types()
+    refused, attend = [], attention_backend.attend
+
+    def refuse(step, layers, begin, end, done, stream):
+        if begin > 2 * layer or end <= 2 * layer:
+            return real.xb_dense_layers(step, layers, begin, end, done, stream)
+        rc = real.xb_dense_layers(step, layers, begin, 2 * layer + 1, done, stream)
+        report = ctypes.cast(done, ctypes.POINTER(types[2])).contents
+        report.half, report.launch = 2 * layer, 4
+        refused.append(report.half)
+        return rc or kernels.ERR_NOT_SUPPORTED
+
+    def attended(out, *a, **k):
+        out.fill_(float("nan"))
+        attend(out, *a, **k)
+    monkeypatch.setattr(kernels, "kernels_lib", lambda: Library(real, refuse))
+    monkeypatch.setattr(attention_backend, "attend", attended)
+    got = steps(monkeypatch)
+    assert refused == [2 * layer] * 3 and torch.equal(got, expect)
+
+
+def test_the_error_names_what_failed(monkeypatch):
+    import ctypes
+    from xinfer_b200 import kernels, native
+    real, types = native.kernels_lib(), kernels.dense_types()
+
+    def fail(step, layers, begin, end, done, stream):
+        report = ctypes.cast(done, ctypes.POINTER(types[2])).contents
+        report.half, report.launch, report.blas_status = 3, 2, 13
+        return 999
+    monkeypatch.setattr(kernels, "kernels_lib", lambda: Library(real, fail))
+    with pytest.raises(kernels.KernelError, match=r"library product of layer 1 \(cuBLAS status 13\): CUDA error 999"):
+        steps(monkeypatch)
+
+
+def test_the_mirrors_members_have_the_librarys_names():
+    from xinfer_b200 import kernels
+    step, layer, done = kernels.dense_types()
+    assert [n for n, _ in step._fields_][:3] == ["x", "h", "qkv"] and [n for n, _ in step._fields_][-2:] == ["p0", "p1"]
+    assert [n for n, _ in layer._fields_] == "w_qkv w_o w_gate_up w_down norm1 norm2 q_norm k_norm k_pages v_pages".split()
+    assert [n for n, _ in done._fields_][3:] == "norms skinny library ropes prefill decode gates".split()

@@ -735,39 +735,59 @@ def attn_prefill_tc(out, q, k_cache, v_cache, q_start, start_pos, block_table, t
     return True
 
 
-def dense_layers(step_type, bufs, nums, reals, library, layers):
-    """The layers of a pre-norm stack, queued by one native call.  ``step_type``: the ctypes mirror of the native step; ``bufs``
-    (tensors), ``nums``, ``reals`` and ``library`` (addresses): its fields by name; ``layers``: for each w_qkv, w_o, w_gate_up,
-    w_down, the weights of the two norms, q and k norm weights (or None), key pages, value pages."""
+_dense_types: list = []
+_DENSE_LAUNCHES = ("rmsnorm_bf16", "gemm_skinny_tc", "library product", "qk_norm_rope_write_bf16", "attn_prefill_tc", "attn_decode_tc", "swiglu_bf16")
+
+
+def dense_types() -> list:
+    """The native step, layer and report of ``dense_layers`` as ctypes structures, laid out as the library describes them."""
+    if not _dense_types:
+        kinds = {"ptr": ctypes.c_void_p, "int": ctypes.c_int, "float": ctypes.c_float}
+        made = []
+        for which, name in enumerate(("DenseStep", "DenseLayer", "DenseDone")):
+            members = [m.split() for m in kernels_lib().xb_dense_fields(which).decode().split(";") if m]
+            made.append(type(name, (ctypes.Structure,), {"_fields_": [(field, kinds[kind]) for kind, field in members]}))
+        _dense_types.extend(made)
+    return _dense_types
+
+
+def dense_layers(bufs, nums, reals, library, layers, attend):
+    """The layers of a pre-norm stack, queued by native calls.  ``bufs`` (tensors), ``nums``, ``reals`` and ``library`` (addresses): the
+    members of the native step by name; ``layers``: the tensors of each layer by name (q and k norm weights may be None).
+    ``attend(i)`` computes layer i's attention from ``q`` into ``o`` by another kernel, where those of the call do not take the step."""
     T, H, nh, nkv, d, I = (nums[k] for k in ("tokens", "hidden", "nh", "nkv", "d", "inter"))
-    bf, width = torch.bfloat16, (nums["nh"] + 2 * nums["nkv"]) * nums["d"]
+    bf, f32, width = torch.bfloat16, torch.float32, (nums["nh"] + 2 * nums["nkv"]) * nums["d"]
     for name, shape in (("x", (T, H)), ("h", (T, H)), ("qkv", (T, width)), ("q", (T, nh, d)), ("o", (T, nh, d)), ("attn_out", (T, H)),
                         ("gate_up", (T, 2 * I)), ("act", (T, I)), ("ffn_out", (T, H))):
         _need(bufs[name], name, bf, shape)
-    pages = layers[0][8].shape
-    table = (ctypes.c_void_p * (10 * len(layers)))()
-    at = 0
-    for ts in layers:
-        for t, name, dtype, shape in zip(ts, ("w_qkv", "w_o", "w_gate_up", "w_down", "norm", "norm", "q norm", "k norm", "k pages", "v pages"),
-                                         (bf, bf, bf, bf, torch.float32, torch.float32, torch.float32, torch.float32, bf, bf),
-                                         ((width, H), (H, nh * d), (2 * I, H), (H, I), (H,), (H,), (d,), (d,), pages, pages)):
+    pages = layers[0]["k_pages"].shape
+    forms = dict(w_qkv=(bf, (width, H)), w_o=(bf, (H, nh * d)), w_gate_up=(bf, (2 * I, H)), w_down=(bf, (H, I)), norm1=(f32, (H,)), norm2=(f32, (H,)),
+                 q_norm=(f32, (d,)), k_norm=(f32, (d,)), k_pages=(bf, pages), v_pages=(bf, pages))
+    step_type, layer_type, done_type = dense_types()
+    table = (layer_type * len(layers))()
+    for row, ts in zip(table, layers):
+        for name, (dtype, shape) in forms.items():
+            t = ts[name]
             if t is not None:
                 _need(t, name, dtype, shape)
-                table[at] = t.data_ptr()
-            at += 1
-    lib, done = kernels_lib(), ctypes.c_int(0)
-    if lib.xb_dense_step_size() != ctypes.sizeof(step_type):
-        raise KernelError("the native step and its mirror differ in size")
-    step = step_type(**{k: t.data_ptr() for k, t in bufs.items()}, **nums, **reals, **library)
-    n = len(layers)
-    rc = lib.xb_dense_layers(ctypes.byref(step), table, n, ctypes.byref(done), _stream())
-    _ok(rc, "rmsnorm_bf16", 2 * n)
-    _ok(0, "qk_norm_rope_write_bf16", n)
-    _ok(0, "swiglu_rows_bf16" if T >= nums["many_rows"] else "swiglu_bf16", n)
-    for name, count in (("gemm_skinny_tc", 4 * n - done.value), ("attn_prefill_tc", n if nums["prefill_ctas"] else 0),
-                        ("attn_decode_tc", n if nums["small"] else 0)):
-        if count:
-            _ok(0, name, count)
+                setattr(row, name, t.data_ptr())
+    step, done = step_type(**{k: t.data_ptr() for k, t in bufs.items()}, **nums, **reals, **library), done_type()
+    half, end = 0, 2 * len(layers)
+    while half < end:
+        rc = kernels_lib().xb_dense_layers(ctypes.byref(step), table, half, end, ctypes.byref(done), _stream())
+        for name, count in (("rmsnorm_bf16", done.norms), ("gemm_skinny_tc", done.skinny), ("qk_norm_rope_write_bf16", done.ropes),
+                            ("attn_prefill_tc", done.prefill), ("attn_decode_tc", done.decode),
+                            ("swiglu_rows_bf16" if T >= nums["many_rows"] else "swiglu_bf16", done.gates)):
+            if count:
+                _ok(0, name, count)
+        if rc == 0:
+            return
+        what = _DENSE_LAUNCHES[done.launch]
+        if rc != ERR_NOT_SUPPORTED or what not in ("attn_prefill_tc", "attn_decode_tc"):
+            status = f" (cuBLAS status {done.blas_status})" if what == "library product" else ""
+            _ok(rc, f"{what} of layer {done.half // 2}{status}")
+        attend(done.half // 2)
+        half = done.half + 1
 
 
 # ---- attention with talking heads and a sink; gated recurrence; polynomial activation; table experts ----

@@ -22,16 +22,6 @@ ENABLED = True
 _PROGRAM = (("norm", "x", "h"), ("mixer", "h", "a"), ("add", "a", "x"), ("norm", "x", "h"), ("feed_forward", "h", "f"), ("add", "f", "x"))
 
 
-class _Step(ctypes.Structure):
-    _fields_ = ([(n, ctypes.c_void_p) for n in (
-        "x h qkv q o attn_out gate_up act ffn_out positions req_of_token table q_start start_pos cos_t sin_t work plan part_o part_ml "
-        "tickets err gemm_ex blas").split()]
-        + [(n, ctypes.c_int) for n in (
-            "tokens hidden nh nkv d inter table_stride page_size num_pages max_pos rot interleaved window prefill_ctas decode_ctas "
-            "splits_max small dec_max overlap skinny many_rows activation").split()]
-        + [(n, ctypes.c_float) for n in "eps1 offset1 eps2 offset2 qk_eps scale p0 p1".split()])
-
-
 def _library_product() -> Optional[int]:
     """The address of the library product that torch itself calls, in the library that torch has loaded; None if there is none."""
     try:
@@ -138,7 +128,8 @@ class DenseLayers:
         reals = dict(eps1=n1.spec.eps, offset1=n1.spec.weight_offset, eps2=n2.spec.eps, offset2=n2.spec.weight_offset, qk_eps=s.qk_norm_eps,
                      scale=s.scale, p0=p0, p1=p1)
         library = dict(gemm_ex=self.gemm_ex, blas=torch.cuda.current_blas_handle())
-        table = [(a.w_qkv, a.w_o, g.w_gate_up, g.w_down, p.weight, q.weight, a.q_norm, a.k_norm, c["k"], c["v"])
-                 for (p, a, q, g), c in zip(self.layers, caches)]
-        kernels.dense_layers(_Step, bufs, nums, reals, library, table)
+        table = [dict(w_qkv=a.w_qkv, w_o=a.w_o, w_gate_up=g.w_gate_up, w_down=g.w_down, norm1=p.weight, norm2=q.weight, q_norm=a.q_norm,
+                      k_norm=a.k_norm, k_pages=c["k"], v_pages=c["v"]) for (p, a, q, g), c in zip(self.layers, caches)]
+        kernels.dense_layers(bufs, nums, reals, library, table, lambda i: attention_backend.attend(
+            bufs["o"], bufs["q"], caches[i], ctx, bufs["table"], nums["table_stride"], s.window, s.scale))
         return bufs["ffn_out"]
