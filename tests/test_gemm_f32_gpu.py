@@ -103,3 +103,26 @@ def test_tiles_of_every_size_form_the_same_bits(M, N, K):
         part = torch.full((x.shape[0], y.shape[0]), float("nan"), device=dev())
         kernels.gemm_plain(part, x, y)
         assert torch.equal(part, out[rows][:, cols])
+
+
+def test_the_word_of_calls_without_one_is_looked_at():
+    """Also where the first such calls are captured: the word is no part of a graph's memory."""
+    from xinfer_b200 import kernels
+    from xinfer_b200.parts import gemm_backend
+    a, w = rnd(3, 64, seed=14), rnd(40, 64, seed=15)
+    out, want = torch.empty(3, 40, device=dev()), torch.empty(3, 40, device=dev())
+    kernels.gemm_plain(want, a, w, torch.zeros(1, dtype=torch.int32, device=dev()))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        kernels.gemm_plain(out, a, w)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    y = torch.empty(3, 40, dtype=torch.bfloat16, device=dev())
+    for call in (lambda: kernels.gemm_plain(out, a, w), lambda: gemm_backend.try_fast(y, a.bfloat16(), w.bfloat16())):
+        kernels.own_err_word().value.value = kernels.ERR_WAIT
+        with pytest.raises(kernels.KernelError, match="bounded wait"):
+            call()
+        call()                  # said once
+        torch.cuda.synchronize()
+        assert kernels.own_err_word().value.value == 0

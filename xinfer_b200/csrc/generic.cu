@@ -9,6 +9,22 @@
 #include "common.cuh"
 #include "gemm_f32_tc.h"
 
+// The error word of calls that bring none: pinned host memory that every device reaches (nullptr if there is none to be had), so
+// that the host can look at it without waiting for a stream.  Also made inside a stream capture, which it is no part of.
+XB_EXPORT int* xb_own_err_word() {
+    static int* const word = []() -> int* {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+        void* p = nullptr;
+        const cudaError_t rc = cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (rc != cudaSuccess) return nullptr;
+        *static_cast<int*>(p) = 0;
+        return static_cast<int*>(p);
+    }();
+    return word;
+}
+
 // ------------------------------------------------------------------------------------------
 // Embedding gather: out[t, :] = table[ids[t], :].  An id -1 - i stands for sampled[i], the id a
 // sampler left on the device (the host has not seen it yet).

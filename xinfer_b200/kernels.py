@@ -257,19 +257,36 @@ def dyt_norm(out, x, alpha, weight, bias, err, *, branch=None, branch_scale: flo
                                   err.data_ptr(), _stream()), "dyt_norm")
 
 
-_err_words: dict = {}
+class _OwnErrWord:
+    """The error word of calls that bring none, in host memory: a wait that expires in such a call is raised by the next one."""
+
+    def __init__(self):
+        self._address = kernels_lib().xb_own_err_word()
+        if not self._address:
+            raise KernelError("no pinned memory for an error word")
+        self.value = ctypes.c_int.from_address(self._address)
+
+    def data_ptr(self) -> int:
+        return self._address
 
 
-def _own_err_word(device) -> torch.Tensor:
-    """The error word of calls that bring none."""
-    if device not in _err_words:
-        _err_words[device] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _err_words[device]
+_own_err = None
+
+
+def own_err_word() -> _OwnErrWord:
+    global _own_err
+    if _own_err is None:
+        _own_err = _OwnErrWord()
+    word = _own_err.value.value
+    if word:
+        _own_err.value.value = 0
+        raise KernelError(f"an earlier product without an error word: {describe_error(word)}")
+    return _own_err
 
 
 def gemm_plain(out, a, w, err=None):
     """out[M, N] = a[M, K] . w[N, K]^T in float32: of float32 operands and result on the tensor cores, in three bfloat16 parts of
-    each number, else by float32 FMA.  ``err``: the step's device error word."""
+    each number, else by float32 FMA.  ``err``: the step's device error word (default: one that the next such call looks at)."""
     M, K = a.shape
     N = w.shape[0]
     _need(a, "a", None, (M, K))
@@ -277,7 +294,7 @@ def gemm_plain(out, a, w, err=None):
     _need(out, "out", None, (M, N))
     _ok(kernels_lib().xb_gemm_plain(dtype_code(a.dtype), dtype_code(w.dtype), dtype_code(out.dtype), out.data_ptr(),
                                     a.data_ptr(), w.data_ptr(), M, N, K,
-                                    (err if err is not None else _own_err_word(out.device)).data_ptr(), _stream()), "gemm_plain")
+                                    (err if err is not None else own_err_word()).data_ptr(), _stream()), "gemm_plain")
 
 
 def rope_table(cos_t, sin_t, inv_freq):

@@ -96,6 +96,7 @@ def _declare_kernels(lib):
     _sig(lib, "xb_logits_post", I, [P, L, F, F, P])
     _sig(lib, "xb_rmsnorm", I, [I, P, P, P, P, P, P, I, I, I, F, F, P, P])
     _sig(lib, "xb_add", I, [I, P, P, P, L, F, P])
+    _sig(lib, "xb_own_err_word", P, [])
     _sig(lib, "xb_gemm_plain", I, [I, I, I, P, P, P, I, I, I, P, P])
     _sig(lib, "xb_dense_fields", ctypes.c_char_p, [I])
     _sig(lib, "xb_dense_layers", I, [P, P, I, I, P, P])
