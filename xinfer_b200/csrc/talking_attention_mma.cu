@@ -417,9 +417,9 @@ XB_EXPORT int xb_attn_talking_mma(void* out, int ldo, const void* q, const void*
     a.scale = scale; a.out_scale = out_scale; a.err = err;
     if (bq == 1 && xb_talk_decode_takes(nh, nkv, d, dv) && !(((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)part_o) & 15) &&
         !((uintptr_t)part_ml & 7)) {
-        const XbTalkDecode s = {q_start, start_pos, block_table, talk, part_o, part_ml, num_entries, table_stride, nkv, page_size, num_pages, window,
+        const XbTalkDecode s = {q_start, start_pos, block_table, talk, part_o, part_ml, num_entries, table_stride, nh, nkv, page_size, num_pages, window,
                                 sink, a.parts, ldo, scale, out_scale, err};
-        const int rc = xb_talk_decode(out, q, k_cache, v_cache, s, tokens, nh, stream);
+        const int rc = xb_talk_decode(out, q, k_cache, v_cache, s, tokens, d, stream);
         if (rc || a.parts == 1) return rc;
         return xb_attn_talking_merge_bf16(out, part_o, part_ml, tokens, nh, dv, a.parts, ldo, out_scale, stream);
     }

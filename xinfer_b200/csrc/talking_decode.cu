@@ -19,7 +19,7 @@
 namespace {
 
 typedef __nv_bfloat16 bf;
-constexpr int D = 128, KEYS = 16, MAX_GROUPS = 8, Q_BYTES = D * 2 + 16;
+constexpr int KEYS = 16, MAX_GROUPS = 8, MAX_HEADS = 64;
 
 __device__ __forceinline__ void mma_keys(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     const uint32_t a[4] = {a0, a1, a2, a3};
@@ -37,23 +37,31 @@ __device__ __forceinline__ unsigned pack2(float a, float b) {
 }
 __device__ __forceinline__ float2 unpack2(unsigned u) { return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
 
-template <int H>
+__device__ __forceinline__ unsigned word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// H: room for heads, ALL: all of it taken (else zeros lie there, which change no sum); D: channels of a head.
+template <int H, bool ALL, int D>
 __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ out, const bf* q, const bf* k_pages, const bf* v_pages,
                                                              const XbTalkDecode a) {
     pdl_overlap_few();
-    constexpr int LDS = H + 4, LDM = KEYS + 1;
+    constexpr int LDS = H + 4, LDM = KEYS + 1, Q_BYTES = D * 2 + 16, KS = D / 32, VS = D / 64, SUMS = D / 16;
     __shared__ __align__(16) float raw[KEYS * LDS];            // [key][head]
     __shared__ float mixed[H * LDM];                           // [head][key]
     __shared__ __align__(16) float talk[H * H];
     __shared__ __align__(16) unsigned char qs[H * Q_BYTES];
     __shared__ int s_entry;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, j = lane & 3;
-    const int G = a.nkv, rep = H / G, t = blockIdx.x;
+    const int heads = ALL ? H : a.nh, G = a.nkv, rep = heads / G, t = blockIdx.x;
     if (tid == 0) s_entry = -1;
     __syncthreads();
     for (int e = tid; e < a.num_entries; e += 256)
         if (a.q_start[e] <= t && t < a.q_start[e + 1]) s_entry = e;
-    for (int i = tid; i < H * H; i += 256) talk[i] = a.talk ? a.talk[i] : (i / H == i % H ? 1.f : 0.f);
+    for (int i = tid; i < H * H; i += 256) {
+        const int to = i / H, from = i % H;
+        talk[i] = to >= heads || from >= heads ? 0.f : a.talk ? a.talk[to * heads + from] : to == from ? 1.f : 0.f;
+    }
+    if (heads < H)
+        for (int i = tid; i < KEYS * LDS; i += 256) raw[i] = 0.f;
     __syncthreads();
     const int b = s_entry;
     if (b < 0) return;
@@ -67,14 +75,14 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
         hi = min(hi, first + per * KEYS);
     }
     const bool first_part = blockIdx.y == 0, works = warp < G;
-    float m[2], l[2], o[8][4];
+    float m[2], l[2], o[SUMS][4];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         m[e] = a.sink && first_part ? 0.f : -INFINITY;
         l[e] = 0.f;                                            // (of this lane's keys; the sink's 1 is added at the end)
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    for (int i = 0; i < SUMS; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     // row of the pages that key `lane & 15` of a chunk has, -1 for none
     auto row_of = [&](int c) -> int {
         const int key = c * KEYS + (lane & 15);
@@ -86,14 +94,14 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
         }
         return (page * G + warp) * a.page_size + key % a.page_size;
     };
-    uint4 k[2][4], v[2][4];
+    uint4 k[2][KS], v[VS][4];
     auto fetch_keys = [&](int rows) {                          // keys g and g + 8 (a key that is not there: any row, its score is not used)
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int row = __shfl_sync(0xffffffffu, rows, u * 8 + g);
             const uint4* src = reinterpret_cast<const uint4*>(k_pages) + (size_t)max(row, 0) * (D / 8) + j;
 #pragma unroll
-            for (int s = 0; s < 4; ++s) k[u][s] = src[s * 4];
+            for (int s = 0; s < KS; ++s) k[u][s] = src[s * 4];
         }
     };
     const int c_lo = lo / KEYS, c_hi = hi > lo ? (hi + KEYS - 1) / KEYS : c_lo;
@@ -103,9 +111,9 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
         fetch_keys(rows);
         if (c_lo + 1 < c_hi) rows_next = row_of(c_lo + 1);
     }
-    for (int i = tid; i < H * (D / 8); i += 256) {
+    for (int i = tid; i < heads * (D / 8); i += 256) {
         const int h = i / (D / 8), c = i % (D / 8);
-        *reinterpret_cast<uint4*>(qs + h * Q_BYTES + c * 16) = *reinterpret_cast<const uint4*>(q + ((size_t)t * H + h) * D + c * 8);
+        *reinterpret_cast<uint4*>(qs + h * Q_BYTES + c * 16) = *reinterpret_cast<const uint4*>(q + ((size_t)t * heads + h) * D + c * 8);
     }
     __syncthreads();
 #pragma unroll 1
@@ -115,7 +123,7 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
             there = __ballot_sync(0xffffffffu, rows >= 0);
             float sc[4] = {0.f, 0.f, 0.f, 0.f};                // (key g, head 2 j), (g, 2 j + 1), (g + 8, 2 j), (g + 8, 2 j + 1)
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
+            for (int s = 0; s < KS; ++s) {
                 uint4 qv = make_uint4(0u, 0u, 0u, 0u);
                 if (g < rep) qv = *reinterpret_cast<const uint4*>(qs + (warp * rep + g) * Q_BYTES + s * 64 + j * 16);
                 mma_keys(sc, k[0][s].x, k[1][s].x, k[0][s].y, k[1][s].y, qv.x, qv.y);
@@ -128,12 +136,14 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
                     raw[(g + 8) * LDS + warp * rep + 2 * j + e] = sc[2 + e] * a.scale;
                 }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {                      // keys 2 j, 2 j + 1, 2 j + 8, 2 j + 9: eight values of either half
+            for (int e = 0; e < 4; ++e) {                      // keys 2 j, 2 j + 1, 2 j + 8, 2 j + 9: eight values of every 64
                 const int row = __shfl_sync(0xffffffffu, rows, 2 * j + (e & 1) + (e >> 1) * 8);
                 const uint4* src = reinterpret_cast<const uint4*>(v_pages) + (size_t)max(row, 0) * (D / 8) + g;
-                v[0][e] = src[0];
-                v[1][e] = src[8];
-                if (row < 0) v[0][e] = v[1][e] = make_uint4(0u, 0u, 0u, 0u);      // (0 times what lies there could be NaN)
+#pragma unroll
+                for (int s = 0; s < VS; ++s) {
+                    v[s][e] = src[s * 8];
+                    if (row < 0) v[s][e] = make_uint4(0u, 0u, 0u, 0u);            // (0 times what lies there could be NaN)
+                }
             }
             if (c + 1 < c_hi) {
                 rows = rows_next;
@@ -146,7 +156,7 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
             const int key = tid & 15;
             const float4* sr = reinterpret_cast<const float4*>(raw + key * LDS);
 #pragma unroll 1
-            for (int h = tid >> 4; h < H; h += 16) {
+            for (int h = tid >> 4; h < heads; h += 16) {
                 const float4* tr = reinterpret_cast<const float4*>(talk + h * H);
                 float m0 = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
 #pragma unroll 4
@@ -188,15 +198,11 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
             }
             const unsigned b0 = transposed(p0), b1 = transposed(p1);
 #pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const unsigned x0 = w == 0 ? v[0][0].x : w == 1 ? v[0][0].y : w == 2 ? v[0][0].z : v[0][0].w;
-                const unsigned x1 = w == 0 ? v[0][1].x : w == 1 ? v[0][1].y : w == 2 ? v[0][1].z : v[0][1].w;
-                const unsigned x2 = w == 0 ? v[0][2].x : w == 1 ? v[0][2].y : w == 2 ? v[0][2].z : v[0][2].w;
-                const unsigned x3 = w == 0 ? v[0][3].x : w == 1 ? v[0][3].y : w == 2 ? v[0][3].z : v[0][3].w;
-                const unsigned y0 = w == 0 ? v[1][0].x : w == 1 ? v[1][0].y : w == 2 ? v[1][0].z : v[1][0].w;
-                const unsigned y1 = w == 0 ? v[1][1].x : w == 1 ? v[1][1].y : w == 2 ? v[1][1].z : v[1][1].w;
-                const unsigned y2 = w == 0 ? v[1][2].x : w == 1 ? v[1][2].y : w == 2 ? v[1][2].z : v[1][2].w;
-                const unsigned y3 = w == 0 ? v[1][3].x : w == 1 ? v[1][3].y : w == 2 ? v[1][3].z : v[1][3].w;
+            for (int w = 0; w < SUMS / 2; ++w) {
+                // rows g of the product: two of the lane's first values; rows g + 8: of the other 64 channels, or of the last four
+                const int wy = VS == 2 ? w : w + 2;
+                const unsigned x0 = word(v[0][0], w), x1 = word(v[0][1], w), x2 = word(v[0][2], w), x3 = word(v[0][3], w);
+                const unsigned y0 = word(v[VS - 1][0], wy), y1 = word(v[VS - 1][1], wy), y2 = word(v[VS - 1][2], wy), y3 = word(v[VS - 1][3], wy);
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     float(&acc)[4] = o[w * 2 + e];
@@ -216,14 +222,15 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
         if (c_lo >= c_hi && a.sink && first_part) l[e] = 1.f;
         if (2 * j + e >= rep) continue;
         const int h = warp * rep + 2 * j + e;
-        // sum i holds values g * 8 + i and 64 + g * 8 + i of the lane's two heads
+        // sum i holds values g * 8 + i and 64 + g * 8 + i of the lane's two heads (of 64 channels: g * 8 + i and g * 8 + 4 + i)
+        constexpr int OTHER = VS == 2 ? 64 : 4;
         if (a.parts > 1) {
-            const size_t at = ((size_t)t * a.parts + blockIdx.y) * H + h;
+            const size_t at = ((size_t)t * a.parts + blockIdx.y) * heads + h;
 #pragma unroll
             for (int hd = 0; hd < 2; ++hd)
 #pragma unroll
-                for (int i = 0; i < 8; i += 4)
-                    *reinterpret_cast<float4*>(a.part_o + at * D + hd * 64 + g * 8 + i) =
+                for (int i = 0; i < SUMS; i += 4)
+                    *reinterpret_cast<float4*>(a.part_o + at * D + hd * OTHER + g * 8 + i) =
                         make_float4(o[i][hd * 2 + e], o[i + 1][hd * 2 + e], o[i + 2][hd * 2 + e], o[i + 3][hd * 2 + e]);
             if (g == 0) *reinterpret_cast<float2*>(a.part_ml + at * 2) = make_float2(m[e], l[e]);
         } else {
@@ -232,21 +239,39 @@ __global__ void __launch_bounds__(256, 2) talk_decode_kernel(bf* __restrict__ ou
 #pragma unroll
             for (int hd = 0; hd < 2; ++hd)
 #pragma unroll
-                for (int i = 0; i < 8; i += 2)
-                    *reinterpret_cast<unsigned*>(dst + hd * 64 + i) = pack2(o[i][hd * 2 + e] * f, o[i + 1][hd * 2 + e] * f);
+                for (int i = 0; i < SUMS; i += 2)
+                    *reinterpret_cast<unsigned*>(dst + hd * OTHER + i) = pack2(o[i][hd * 2 + e] * f, o[i + 1][hd * 2 + e] * f);
         }
     }
 }
 
-}  // namespace
-
-// Heads of 128 channels, 16 or 32 of them over at most eight key/value heads, at most eight to one.
-bool xb_talk_decode_takes(int nh, int nkv, int d, int dv) {
-    return d == D && dv == D && (nh == 16 || nh == 32) && nkv >= 1 && nkv <= MAX_GROUPS && nh % nkv == 0 && nh / nkv <= 8;
+template <int H>
+int launch(bf* out, const bf* q, const bf* k_pages, const bf* v_pages, const XbTalkDecode& a, int tokens, int d, cudaStream_t stream) {
+    const dim3 grid(tokens, a.parts);
+#define XB_GO(ALL, D) return xb_launch_few(talk_decode_kernel<H, ALL, D>, grid, dim3(256), 0, stream, out, q, k_pages, v_pages, a)
+    if (d == 64) {
+        if (a.nh == H) XB_GO(true, 64);
+        XB_GO(false, 64);
+    }
+    if (a.nh == H) XB_GO(true, 128);
+    XB_GO(false, 128);
+#undef XB_GO
 }
 
-int xb_talk_decode(void* out, const void* q, const void* k_pages, const void* v_pages, const XbTalkDecode& a, int tokens, int nh, cudaStream_t stream) {
-    const dim3 grid(tokens, a.parts);
-    if (nh == 16) return xb_launch_few(talk_decode_kernel<16>, grid, dim3(256), 0, stream, (bf*)out, (const bf*)q, (const bf*)k_pages, (const bf*)v_pages, a);
-    return xb_launch_few(talk_decode_kernel<32>, grid, dim3(256), 0, stream, (bf*)out, (const bf*)q, (const bf*)k_pages, (const bf*)v_pages, a);
+}  // namespace
+
+// Heads of 64 or 128 channels (eight values a lane of every 64), keys and values alike; a warp for each of at most eight key/value heads,
+// with at most eight heads each (the eight columns of an mma.sync).  Against the kernel with tiles in shared memory, us, eight tokens at 2,048
+// keys and one at 700: 16 heads over 8 of 128 channels 42.0 -> 33.8 and 44.0 -> 25.7, 64 over 8 66.6 -> 58.4 and 72.7 -> 42.0, 24 over 3 of 64
+// channels 42.0 -> 25.7 and 42.0 -> 23.6, 8 over 1 of 64 27.6 -> 21.5 and 25.6 -> 21.5; nowhere slower.
+bool xb_talk_decode_takes(int nh, int nkv, int d, int dv) {
+    return d == dv && (d == 64 || d == 128) && nkv >= 1 && nkv <= MAX_GROUPS && nh <= MAX_HEADS && nh % nkv == 0 && nh / nkv >= 1 && nh / nkv <= 8;
+}
+
+int xb_talk_decode(void* out, const void* q, const void* k_pages, const void* v_pages, const XbTalkDecode& a, int tokens, int d, cudaStream_t stream) {
+    bf* o = (bf*)out;
+    const bf *qs = (const bf*)q, *ks = (const bf*)k_pages, *vs = (const bf*)v_pages;
+    return a.nh <= 16 ? launch<16>(o, qs, ks, vs, a, tokens, d, stream)
+           : a.nh <= 32 ? launch<32>(o, qs, ks, vs, a, tokens, d, stream)
+                        : launch<64>(o, qs, ks, vs, a, tokens, d, stream);
 }
