@@ -7,16 +7,17 @@
 //     w0 a0 + 2^-8 ((w0 a1 + w1 a0) + 2^-8 (w1 a1 + w0 a2 + w2 a0)).
 // Tensor memory rounds a running sum towards zero, so little stays there: of 32 terms at a time the products w0 a0, whose digits
 // fit, go to one column, and the small ones, whose cut-off digits do not count, to another; these two are added in registers,
-// to nearest, and so are the sums of 32 terms, in the order of K.  (Splitting a number into parts whose products are exact is
-// Dekker's, 1971.)
+// to nearest, and so are the sums of 32 terms.  The four 16 terms of a panel are taken as first and third, second and fourth, so that
+// up to 32 terms nothing is added to a sum in tensor memory.  (Splitting a number into parts whose products are exact is Dekker's,
+// 1971.)
 // An output's sum has that one form whatever M, the tile or the operands' alignment is, so a row's result does not depend on
 // what else is in the step.  A sum that is not finite is formed again term by term (an infinity times a part of 0 is no number).
 //
 // Relative error against 64 bits (2-norm), by float32 multiply-adds of 16 terms and so: normal operands, K = 64 8.4e-8 and 5.5e-8,
 // 1,024 1.65e-7 and 1.16e-7, 3,072 2.6e-7 and 1.8e-7; operands near 2^-124 the same; one term 1,000 times the others, K = 1,024
-// 1.85e-7 and 1.30e-7.  Where it is larger: the tensor cores cut every product off near 2^-25 of the largest of its 16, so short
-// sums of one sign, K = 64 5.0e-8 and 5.7e-8, the more the more one term stands out (1,000 times the others, K = 32: 6.6e-8 and
-// 2.1e-7; 10^6 times, K = 1,024: 1.9e-7 and 2.1e-7).
+// 1.85e-7 and 1.50e-7.  Where it is larger: the tensor cores cut every product off near 2^-25 of the largest of its 16, so short
+// sums of one sign, K = 64 5.0e-8 and 5.6e-8, the more the more one term stands out (1,000 times the others, all of one sign, K =
+// 64 9.3e-8 and 2.2e-7, 1,024 1.55e-7 and 1.75e-7; 10^6 times, 1,024 1.9e-7 and 3.7e-7).
 // With the leading part cut off instead of rounded, parts not scaled and all products in one column (and 446 x 4,096 x 1,024 41
 // instead of 46 us): a single product 5.6e-8, where this has 2.5e-8 as multiply-adds have, operands near 2^-116 3.2e-6.
 //
@@ -248,7 +249,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     done:;
     } else if (warp < CUTTERS + ISSUERS) {
-        // Issuer q takes the q-th 32 terms of every panel; the whole warp walks along, so that the descriptors are the same in
+        // Issuer q takes the q-th and the (q + 2)-th 16 terms of every panel; the whole warp walks along, so that the descriptors are the same in
         // all lanes, and one lane issues.
         const uint32_t idesc = umma_idesc(TOK);
         const int q = __shfl_sync(0xffffffffu, warp, 0) - CUTTERS;
@@ -262,23 +263,23 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                                                  mbar_wait(smem_u32(&s_free[buf]), free_parity, err, true));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d = tm + (uint32_t)(S::SUMS + buf * S::BUF), sa = mem0 + S::RAWS * S::RAW + stage * S::STAGE + q * (TERMS * 2);
-                const uint32_t w0 = tm + (uint32_t)(stage * S::W_COLS + q * (TERMS / 2)), w1 = w0 + PANEL / 2, w2 = w0 + PANEL;
+                const uint32_t d = tm + (uint32_t)(S::SUMS + buf * S::BUF), sa = mem0 + S::RAWS * S::RAW + stage * S::STAGE + q * TERMS;
+                const uint32_t w0 = tm + (uint32_t)(stage * S::W_COLS + q * (TERMS / 4)), w1 = w0 + PANEL / 2, w2 = w0 + PANEL;
                 const uint64_t a0 = umma_desc(sa), a1 = umma_desc(sa + S::A_BYTES), a2 = umma_desc(sa + 2 * S::A_BYTES);
-                if (elect_one()) {                                // 16 terms are 8 columns and 32 bytes of a row
+                if (elect_one()) {                                // 16 terms are 8 columns and 32 bytes of a row, the next 16 of the issuer's twice that further
                     const uint32_t small = d + TOK;
                     umma_bf16_ta(small, w2, a0, idesc, 0u);
                     umma_bf16_ta(small, w0, a2, idesc, 1u);
                     umma_bf16_ta(small, w1, a1, idesc, 1u);
-                    umma_bf16_ta(small, w2 + 8, a0 + 2, idesc, 1u);
-                    umma_bf16_ta(small, w0 + 8, a2 + 2, idesc, 1u);
-                    umma_bf16_ta(small, w1 + 8, a1 + 2, idesc, 1u);
+                    umma_bf16_ta(small, w2 + 16, a0 + 4, idesc, 1u);
+                    umma_bf16_ta(small, w0 + 16, a2 + 4, idesc, 1u);
+                    umma_bf16_ta(small, w1 + 16, a1 + 4, idesc, 1u);
                     umma_bf16_ta_scaled<8>(small, w1, a0, idesc);
                     umma_bf16_ta(small, w0, a1, idesc, 1u);
-                    umma_bf16_ta(small, w1 + 8, a0 + 2, idesc, 1u);
-                    umma_bf16_ta(small, w0 + 8, a1 + 2, idesc, 1u);
+                    umma_bf16_ta(small, w1 + 16, a0 + 4, idesc, 1u);
+                    umma_bf16_ta(small, w0 + 16, a1 + 4, idesc, 1u);
                     umma_bf16_ta(d, w0, a0, idesc, 0u);
-                    umma_bf16_ta(d, w0 + 8, a0 + 2, idesc, 1u);
+                    umma_bf16_ta(d, w0 + 16, a0 + 4, idesc, 1u);
                     umma_commit(smem_u32(&s_sum[buf]));
                     umma_commit(smem_u32(&s_empty[stage]));
                 }
