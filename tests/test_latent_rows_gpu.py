@@ -274,3 +274,35 @@ def test_a_row_that_is_not_finite_reaches_only_the_queries_that_see_it(key, chan
     assert sum(bin(int(b) & 0xFFFFFFFF).count("1") for b in bad) == (1 if key >= first else 0)
     sees = torch.tensor([key <= start + i and (window is None or key > start + i - window) for i in range(n)])
     assert torch.isnan(got[sees]).all() and torch.equal(got[~sees], clean[~sees])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rank,parts,shift", [(8, 2, 0), (72, 64, 0), (512, 18, 0), (512, 65, 0), (512, 130, 0), (136, 3, 2), (512, 70, 2)])
+def test_merge_of_key_ranges_against_64_bits(rank, parts, shift):
+    """Vectors of four columns and single ones (scratch that starts on an 8-byte boundary only), factors for more than 64 ranges, ranges
+    without keys.  Scratch that starts off an 8-byte boundary, where the ranges' sums cannot be stored, is refused by the host."""
+    from xinfer_b200 import kernels as k
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(rank + parts)
+    nh, ps, contexts = 3, 16, [700, 1, 130]
+    dk, T = rank + (-rank % 16) + 16, 3
+    per = 700 // ps + 1
+    rows = torch.randn(T * per, ps, dk, generator=g).bfloat16()
+    q = (torch.randn(T, nh, dk, generator=g) / math.sqrt(dk)).bfloat16()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    table = torch.arange(T * per, dtype=torch.int32, device=dev).view(T, per)
+    out = torch.full((T, nh, rank), float("nan"), dtype=torch.bfloat16, device=dev)
+    po = torch.full((T * nh * parts * rank + 6,), float("nan"), device=dev)[shift:]
+    pml = torch.full((T * nh * parts * 2,), float("nan"), device=dev)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    args = (out, q.to(dev), rows.to(dev), i32([0, 1, 2, 3]), i32([n - 1 for n in contexts]), T, table, per, None, 1.0, None, err)
+    k.attn_latent_mma(*args, parts=parts, part_o=po, part_ml=pml)
+    with pytest.raises(k.KernelError):
+        k.attn_latent_mma(*args, parts=parts, part_o=po[1:], part_ml=pml)
+    assert int(err) == 0
+    for b, n in enumerate(contexts):
+        keys = rows[b * per:(b + 1) * per].reshape(-1, dk)[:n].double()
+        w = torch.softmax(q[b].double() @ keys.t(), 1)
+        ref, terms = w @ keys[:, :rank], w @ keys[:, :rank].abs()
+        # as for any attention with weights in bfloat16: 2^-8 of every term and of their sum, 2^-8 of the result, float32 for the rest
+        assert ((out[b].double().cpu() - ref).abs() <= (2.0 ** -8 + 2.0 ** -16) * terms + 2.0 ** -7 * ref.abs()).all(), (b, n)

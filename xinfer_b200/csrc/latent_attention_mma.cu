@@ -434,7 +434,7 @@ XB_EXPORT int xb_attn_latent_mma_takes(int dk, int rank) {
 
 // q [tokens, heads, dk], cache [pages, page_size, dk], out [tokens, heads, rank], all bfloat16.  `rg`: 16-row
 // groups per block (1 or 2).  `most` > 0: portions of more tokens are left out, `tokens` counts those of the others.
-// `parts` > 1 (with every portion taken) needs part_o (tokens * heads * parts * rank floats) and part_ml
+// `parts` > 1 (with every portion taken) needs part_o (tokens * heads * parts * rank floats, stored two at a time) and part_ml
 // (tokens * heads * parts * 2 floats).
 XB_EXPORT int xb_attn_latent_mma(void* out, const void* q, const void* cache, const int* q_start, const int* start_pos,
                                  int num_entries, const int* block_table, int table_stride, int tokens, int nh, int dk,
@@ -442,7 +442,7 @@ XB_EXPORT int xb_attn_latent_mma(void* out, const void* q, const void* cache, co
                                  int most, int parts, float* part_o, float* part_ml, int* err, cudaStream_t stream) {
     if (tokens <= 0 || num_entries <= 0) return 0;
     if (!xb_attn_latent_mma_takes(dk, rank) || (rg != 1 && rg != 2) || parts < 1 || parts > 65535) return (int)cudaErrorInvalidValue;
-    if (parts > 1 && (part_o == nullptr || part_ml == nullptr || most > 0)) return (int)cudaErrorInvalidValue;
+    if (parts > 1 && (part_o == nullptr || part_ml == nullptr || ((uintptr_t)part_o & 7) || most > 0)) return (int)cudaErrorInvalidValue;
     LatentMmaArgs a;
     a.q_start = q_start; a.start_pos = start_pos; a.block_table = block_table; a.sink = sink;
     a.part_o = part_o; a.part_ml = part_ml;
