@@ -127,3 +127,32 @@ def test_tokens_of_a_request_that_are_not_neighbours():
         w = torch.softmax(torch.einsum("hd,khd->hk", q[t].double(), keys(kc)) * 0.2, 1)
         assert (out[t].double() - torch.einsum("hk,khd->hd", w, keys(vc))).abs().max() <= 2e-5      # (as above)
     assert int(e) == 0
+
+
+def test_a_model_with_head_sizes_on_both_sides_of_the_tiled_kernels():
+    """Layers with heads of 96 and of 160 channels: the float32 logits have the same bits however the tokens are cut into steps."""
+    from xinfer_b200.engine.runner import ModelRunner, StepInput
+    layer = lambda dim, vdim: dict(type="attention", mlp=dict(kind="dense", ff=96), mixer=dict(
+        heads=4, kv_heads=2, dim=dim, vdim=vdim, scale=dim ** -0.5, mask=dict(size=50), rot=dict(dims=16, base=1000.0)))
+    cfg = dict(architecture="Dufitar", vocab=101, width=64, norm=dict(eps=1e-5), residual_mult=0.7, embedding=dict(scale=1.5),
+               layers=[layer(96, 64), layer(160, 144), layer(160, 32), layer(128, 128)])
+    rng = np.random.default_rng(3)
+    a, b = (rng.integers(0, 101, size=n, dtype=np.int32) for n in (90, 41))
+
+    def run(script):
+        r = ModelRunner.random(cfg, 5, dtype="f32", block_size=16, num_blocks=32, max_num_seqs=2, max_model_len=128)
+        slots, at, rows = [r.open_request(), r.open_request()], [0, 0], [[], []]
+        for step in script:
+            parts = [(i, (a, b)[i][at[i]:at[i] + n]) for i, n in step]
+            logits = r.step([StepInput(slots[i], t, range(len(t))) for i, t in parts], allow_graph=False)
+            for i, t in parts:
+                rows[i].append(logits[:len(t)].clone())
+                logits = logits[len(t):]
+                at[i] += len(t)
+        r.check_errors()
+        return [torch.cat(x) for x in rows]
+
+    whole = run([[(0, 90), (1, 41)]])
+    cut = run([[(0, 33)], [(1, 20), (0, 1)], [(0, 55), (1, 20)], [(0, 1), (1, 1)]])
+    for x, y in zip(whole, cut):
+        assert torch.isfinite(x).all() and torch.equal(x, y)

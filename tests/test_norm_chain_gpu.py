@@ -72,3 +72,68 @@ def test_gated_parts_in_vectors(T, parts, part, after, silu, div):
     got = out.double().cpu()
     assert (got[:, :4] == 7.0).all() and (got[:, 4 + W:] == 7.0).all()
     assert ((got[:, 4:4 + W] - v.reshape(T, W)).abs() <= 2.0 ** -8 * v.reshape(T, W).abs() + 1e-5).all()     # one rounding to bfloat16, float32 behind it
+
+
+def same(a, b):
+    """Numbers of the same bits, and no number at the same places."""
+    return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.nan_to_num(a, nan=0.0), torch.nan_to_num(b, nan=0.0))
+
+
+BAD = [float("inf"), float("-inf"), float("nan"), 3e38, 1e20]
+
+
+@pytest.mark.parametrize("where", ["x", "branch"])
+def test_rows_in_vectors_with_infinities_as_the_general_kernel_has_them(where):
+    """Rows that start off a 16-byte boundary run on the general kernel; a row's bad number reaches that row alone."""
+    from xinfer_b200 import kernels as k
+    g = torch.Generator().manual_seed(1)
+    n, dim = len(BAD) + 1, 1024
+    x, br = torch.randn(n, dim, generator=g).to(DEV), torch.randn(n, dim, generator=g).to(DEV)
+    for i, v in enumerate(BAD):
+        (x if where == "x" else br)[i, 77 * (i + 1)] = v
+    w = (1 + 0.1 * torch.randn(dim, generator=g)).to(DEV)
+    off = torch.empty(n * dim + 1, device=DEV)[1:].view(n, dim)
+    off.copy_(x)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for norm in (None, w):
+        a, b = (torch.empty(n, dim, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        k.rms_chain(a, x, w, 1e-5, err, branch=br, branch_weight=norm, branch_eps=1e-6)
+        k.rms_chain(b, off, w, 1e-5, err, branch=br, branch_weight=norm, branch_eps=1e-6)
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.isnan(a[:3]).any(1).all() and torch.isfinite(a[3:]).all()
+        fine = ~torch.isnan(a)
+        assert ((a[fine].float() - b[fine].float()).abs() <= 2.0 ** -7 * b[fine].float().abs()).all()      # one rounding apart
+
+
+@pytest.mark.parametrize("activation", ["silu", "gelu_tanh"])
+def test_gate_over_many_rows_with_infinities(activation):
+    from xinfer_b200 import kernels as k
+    g = torch.Generator().manual_seed(2)
+    rows, width = 70, 64
+    gu, bias = torch.randn(rows, 2 * width, generator=g).to(DEV), torch.zeros(2 * width, device=DEV)
+    for i, v in enumerate(BAD):
+        gu[i, 3], gu[10 + i, width + 5] = v, v
+    out, few = (torch.zeros(rows, width, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    k.swiglu_bias(out, gu, bias, activation)
+    k.swiglu_bias(few[:35], gu[:35], bias, activation)
+    k.swiglu_bias(few[35:], gu[35:], bias, activation)
+    assert same(out, few) and torch.isfinite(out[20:]).all()
+
+
+@pytest.mark.parametrize("part", [64, 512, 1028])
+@pytest.mark.parametrize("after", [False, True])
+def test_gated_parts_with_infinities_as_the_general_kernel_has_them(part, after):
+    """Gates whose columns start off a 16-byte boundary send the call to the general kernel."""
+    from xinfer_b200 import kernels as k
+    g = torch.Generator().manual_seed(3)
+    T, W = len(BAD) + 1, 2 * part
+    y, gate, w = torch.randn(T, W, generator=g).to(DEV), torch.randn(T, W + 8, generator=g).to(DEV), torch.ones(part, device=DEV)
+    for i, v in enumerate(BAD):
+        y[i, 5] = v
+    out, general = (torch.empty(T, W, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    k.gated_head_norm(out, y, gate, 4, w, part, 1e-6, after)
+    other = torch.empty_like(gate)
+    other[:, 5:5 + W] = gate[:, 4:4 + W]
+    k.gated_head_norm(general, y, other, 5, w, part, 1e-6, after)
+    assert torch.equal(torch.isnan(out), torch.isnan(general)) and torch.isfinite(out[:, part:]).all() and torch.isfinite(out[-1]).all()
+    fine = ~torch.isnan(out)
+    assert ((out[fine].float() - general[fine].float()).abs() <= 2.0 ** -7 * general[fine].float().abs()).all()

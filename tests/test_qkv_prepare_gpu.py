@@ -1,4 +1,5 @@
-"""Heads of many tokens, a warp per token: the same as by the block-per-token kernel, which the same tokens take in small steps."""
+"""Heads of many tokens, a warp per token: the same as by the block-per-token kernel, which the same tokens take in small steps, and
+against 64 bits."""
 import pytest
 import torch
 
@@ -38,6 +39,33 @@ def test_many_tokens_as_by_small_steps(nh, nkv, d, dv, rot, interleaved, mode, b
                           interleaved, mode, 1e-5, True, err, rot_magnitude=1.25, bias=b, q_temp=temp)
         return q, kc, vc
 
+    # in 64 bits: bias, norm before or after the rotation, rotation (its angles are formed in float32), temperature
+    x = qkv.double().cpu() + (b.double().cpu() if bias else 0.0)
+    heads = x[:, : (nh + nkv) * d].view(tokens, nh + nkv, d).clone()
+    p = pos.cpu()
+
+    def norm(h):
+        h = h * torch.rsqrt((h * h).mean(-1, keepdim=True) + 1e-5)
+        return h * torch.cat([w.double().cpu().expand(n, d) if w is not None else torch.ones(n, d).double() for w, n in ((qw, nh), (kw, nkv))])
+    if mode == 1:
+        heads = norm(heads)
+    if rot:
+        angle = (p[:, None].float() * freq.cpu()[None]).double()[:, None]
+        cs, sn = torch.cos(angle) * 1.25, torch.sin(angle) * 1.25
+        i, j = (slice(0, rot, 2), slice(1, rot, 2)) if interleaved else (slice(0, rot // 2), slice(rot // 2, rot))
+        u, v = heads[..., i].clone(), heads[..., j].clone()
+        heads[..., i], heads[..., j] = u * cs - v * sn, v * cs + u * sn
+    if mode == 2:
+        heads = norm(heads)
+    if temp:
+        heads[:, :nh] *= 1.0 + temp[0] * torch.log((p[:, None, None] + 1) // temp[1] + 1.0).double()
+    values = x[:, (nh + nkv) * d:].view(tokens, nkv, dv)
+    q, kc, vc = (t.double().cpu() for t in run(tokens))
+    live = req.cpu() >= 0
+    rows = table.cpu()[req.cpu().clamp(min=0).long(), p.long() // ps].long(), p.long() % ps
+    for got, ref in ((q, heads[:, :nh]), (kc[rows[0], :, rows[1]][live], heads[live, nh:]), (vc[rows[0], :, rows[1]][live], values[live])):
+        # the rounding of the result to bfloat16 (eight digits), and 2^-18 of the largest for norm, sine, cosine and rotation in float32
+        assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -18 * ref.abs().max()).all()
     for x, y in zip(run(tokens), run(50)):
         # one rounding to bfloat16 of values that differ by a few float32 roundings
         assert (x.float() - y.float()).abs().max() <= 2.0 ** -7 * float(y.float().abs().max())

@@ -71,3 +71,30 @@ def test_a_token_of_no_request_and_a_bad_page():
     assert int(err) == 0 and torch.count_nonzero(out[0]) == 0 and (out[1] == 3.0).all()
     run(20)
     assert int(err) == k.ERR_BAD_PAGE and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("what", ["key", "value"])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_numbers_that_are_not_finite_reach_what_they_reach_in_the_tiled_kernel(what, bad):
+    """Scratch that is not aligned keeps to the kernel with tiles."""
+    from xinfer_b200 import kernels as k
+    nh, nkv, d, ps, n, parts, T = 16, 4, 64, 16, 200, 2, 2
+    g = torch.Generator().manual_seed(4)
+    kc, vc = (torch.randn(2 * 13, nkv, ps, d, generator=g).bfloat16().to(DEV) for _ in range(2))
+    (kc if what == "key" else vc)[5, 2, 3, 7] = bad            # the first request's key 83
+    q = torch.randn(T, nh, d, generator=g).bfloat16().to(DEV)
+    talk = (torch.randn(nh, nh, generator=g) / 4).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    table = torch.arange(26, dtype=torch.int32, device=DEV).view(2, 13)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = []
+    for shift in (0, 1):
+        po, pml = torch.zeros(T * parts * nh * d + 4, device=DEV), torch.zeros(T * parts * nh * 2 + 4, device=DEV)
+        out = torch.zeros(T, nh * d, dtype=torch.bfloat16, device=DEV)
+        k.attn_talking_mma(out, q, kc, vc, talk, i32([0, 1, 2]), i32([n - 1, n - 1]), 2, table, 13, None, 0.1, True, 1.0, 1, err, parts, po[shift:], pml[shift:])
+        outs.append(out.float())
+    a, b = outs
+    assert int(err) == 0 and torch.isfinite(a[1]).all() and not torch.isfinite(a[0]).all()
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isinf(a), torch.isinf(b))
+    fine = torch.isfinite(a)
+    assert (a[fine] - b[fine]).abs().max() <= 2.0 ** -7 * (1 + b[fine].abs().max())
