@@ -106,6 +106,13 @@ def test_tiles_of_every_size_form_the_same_bits(M, N, K):
         assert torch.equal(part, out[rows][:, cols])
 
 
+def test_no_terms_give_zeros():
+    from xinfer_b200 import kernels
+    out = torch.full((3, 5), float("nan"), device=dev())
+    kernels.gemm_plain(out, torch.empty(3, 0, device=dev()), torch.empty(5, 0, device=dev()))
+    assert torch.count_nonzero(out) == 0 and torch.isfinite(out).all()
+
+
 def test_the_word_of_calls_without_one_is_looked_at():
     """Also where the first such calls are captured: the word is no part of a graph's memory."""
     from xinfer_b200 import kernels

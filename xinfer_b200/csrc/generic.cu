@@ -244,9 +244,11 @@ XB_EXPORT int xb_gemm_plain(int a_dtype, int w_dtype, int out_dtype, void* out, 
     if (M <= 0 || N <= 0) return 0;
     typedef __nv_bfloat16 bf;
     const int code = a_dtype * 4 + w_dtype * 2 + out_dtype;
-    if (code == 0 && K > 0) return xb_gemm_f32_tc((float*)out, (const float*)a, (const float*)w, M, N, K, err, stream);
+    if (code == 0) {
+        if (K <= 0) return (int)cudaMemsetAsync(out, 0, (size_t)M * N * sizeof(float), stream);
+        return xb_gemm_f32_tc((float*)out, (const float*)a, (const float*)w, M, N, K, err, stream);
+    }
     switch (code) {
-        case 0: return gemm_plain_launch<float, float, float>(out, a, w, M, N, K, stream);
         case 1: return gemm_plain_launch<float, float, bf>(out, a, w, M, N, K, stream);
         case 2: return gemm_plain_launch<float, bf, float>(out, a, w, M, N, K, stream);
         case 3: return gemm_plain_launch<float, bf, bf>(out, a, w, M, N, K, stream);

@@ -1392,7 +1392,8 @@ def rms_chain(out, x, weight, eps, err, *, branch=None, branch_weight=None, bran
     """One pass over rows of the float32 stream ``x``: s = x + branch_scale * gain * br, where br is the branch, or with
     ``branch_weight`` its own RMS norm ``branch / rms(branch) * (branch_offset + branch_weight)``; ``sum_out`` receives s
     (it may be x itself when no rows are gathered); ``out`` (either type; None: only the sum) receives
-    ``s / rms(s) * (weight_offset + weight)``, or s itself where ``weight`` is None."""
+    ``s / rms(s) * (weight_offset + weight)``, or s itself where ``weight`` is None.  ``weight``, ``branch_weight`` and ``gain`` are a
+    model's weights: they are read before the engine's kernel ahead in the stream has finished, so none of these may write them."""
     dim = x.shape[-1]
     n = out.shape[0] if out is not None else x.shape[0]
     _need(x, "x", torch.float32, (None, dim))
