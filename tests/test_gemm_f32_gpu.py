@@ -106,6 +106,17 @@ def test_tiles_of_every_size_form_the_same_bits(M, N, K):
         assert torch.equal(part, out[rows][:, cols])
 
 
+def test_the_largest_operands_whose_leading_part_rounds_to_infinity():
+    from xinfer_b200 import kernels
+    a, w = rnd(20, 80, seed=16), rnd(150, 80, seed=17) * 2.0 ** -30
+    a[3, 7], a[5, 64] = 3.4028234663852886e38, -3.4e38
+    out = torch.empty(20, 150, device=dev())
+    kernels.gemm_plain(out, a, w)
+    x, y = a.double(), w.double()
+    # term by term in those rows: 16 multiply-adds, five sums
+    assert ((out.double() - x @ y.t()).abs() <= 21 * 2.0 ** -24 * (x.abs() @ y.abs().t())).all()
+
+
 def test_no_terms_give_zeros():
     from xinfer_b200 import kernels
     out = torch.full((3, 5), float("nan"), device=dev())
