@@ -8,7 +8,7 @@
 // Tensor memory rounds a running sum towards zero, so little stays there: of 32 terms at a time the products w0 a0, whose digits
 // fit, go to one column, and the small ones, whose cut-off digits do not count, to another; these two are added in registers,
 // to nearest, and so are the sums of 32 terms.  The four 16 terms of a panel are taken as first and third, second and fourth, so that
-// up to 32 terms nothing is added to a sum in tensor memory.  (Splitting a number into parts whose products are exact is Dekker's,
+// up to 32 terms nothing is added to a large sum in tensor memory.  (Splitting a number into parts whose products are exact is Dekker's,
 // 1971.)
 // An output's sum has that one form whatever M, the tile or the operands' alignment is, so a row's result does not depend on
 // what else is in the step.  A sum that is not finite is formed again term by term (an infinity times a part of 0 is no number).
@@ -23,15 +23,17 @@
 //
 // The cut rows of W go to tensor memory, from where an operand A costs no bytes of shared memory; that holds the panels as they come
 // and the cut rows of A (with the cut rows of W there too, a panel of 64 k took 1,730 cycles at 16 tokens instead of 1,500).  What
-// bounds a panel then: at 64 tokens shared memory's bytes, some 1,350 cycles of 2,000; at 16 the time from a panel to its sums, which
-// two teams of cutting warps and two stages overlap: 48 panels of 1,024 rows 46.1 -> 38.9 us with one team -> with two.
+// bounds the kernel then at 64 tokens is instructions, 2.9 to 3.1 of four a cycle (the tensor pipe a third of the time): cutting, and
+// the adding warps' reads, of which the small sums are 13 of 215 us at 2,048 x 6,144 x 1,024.  At 16 tokens, 2.7 a cycle while memory
+// is read at half its rate, it is the time from a panel to its sums, which two teams of cutting warps and two stages overlap: 48
+// panels of 1,024 rows 46.1 -> 38.9 us with one team -> with two.
 // Measured, float32 multiply-adds and now: 446 x 4,096 x 1,024 145 -> 47 us, 446 x 1,024 x 3,072 209 -> 49 us, 2,048 x 6,144 x
 // 1,024 786 -> 215 us (120 TFLOP/s), one row of 6,144 x 1,024 21.2 -> 20.5 us, two of 151,936 x 1,024 123 -> 121 us, one of 24,576 x
 // 4,096 90 -> 98 us (4,100 GB/s; 117 with one team and all tiles 128 rows high).
 //
-// Roles of a block (persistent, a tile of 128 rows of W and TOK of A after another): one thread asks for panels by TMA, a ring of
-// them ahead; sixteen warps cut the panels, a thread 16 k (or 32 of every other panel) of a row of W; two warps issue the products, of 32 k each; four or
-// eight warps add up the sums, through a ring of column buffers, and write the tile.
+// Roles of a block (persistent, a tile of up to 128 rows of W and TOK of A after another): one thread asks for panels by TMA, a ring
+// of them ahead; sixteen warps cut the panels, a thread 16 k (or 32 of every other panel) of a row of W; two warps issue the products,
+// of 32 k each; four or eight warps add up the sums, through a ring of column buffers, and write the tile.
 #include "common.cuh"
 #include "gemm_f32_tc.h"
 #include "tc_common.cuh"
